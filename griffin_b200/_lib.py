@@ -97,7 +97,8 @@ def check(code: int, what: str) -> None:
 
 
 _TIMEOUT_NAMES = {1: "a tile load never completed", 2: "the producer never saw a chunk's results",
-                  3: "the wait self-test gave up (as it must)"}
+                  3: "the wait self-test gave up (as it must)",
+                  4: "another block of a time-split cluster never sent its part"}
 
 
 def check_device() -> None:

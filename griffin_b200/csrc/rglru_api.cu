@@ -258,7 +258,9 @@ static int fwd_common(const void* x, const void* u_r, const void* u_i, const flo
 
   FwdMaps maps;
   bool tma = tma_shape_ok(T, D, es) && aligned(x, 16) && aligned(u_r, 16) && aligned(u_i, 16) && aligned(y, 16);
-  const int variant = y ? scan_fwd_variant(B, T, D, bf16) : 0;   // the carry-only pass exists in the 64-channel shape only
+  int variant = y ? scan_fwd_variant(B, T, D, bf16) : 0;   // the carry-only pass exists in the 64-channel shape only
+  if (tma && y) a.split = scan_split(true, bf16, B, T, D);
+  if (a.split > 1) variant = 0;         // so does the time split
   if (tma) {
     const int rows = scan_fwd_box_rows(variant), cols = scan_fwd_box_cols(variant);
     const void* yy = y ? y : x;   // without y the map is never used
@@ -322,6 +324,7 @@ int rglru_bwd(const void* dy, const float* dh_last, const void* x, const void* u
   bool tma = tma_shape_ok(T, D, es) && aligned(dy, 16) && aligned(x, 16) && aligned(u_r, 16) && aligned(u_i, 16) &&
              aligned(dx, 16) && aligned(du_r, 16) && aligned(du_i, 16);
   const int variant = scan_bwd_variant(B, T, D, bf16);
+  if (tma && !carry_only) a.split = scan_split(false, bf16, B, T, D);
   if (tma) {
     const int rows = scan_bwd_box_rows(variant), cols = scan_bwd_box_cols(variant);
     tma = make_map(&maps.dy, dy, bf16, B, T, D, rows, cols) && make_map(&maps.x, x, bf16, B, T, D, rows, cols) &&
@@ -566,6 +569,7 @@ int rglru_grouped_fwd(const void* x, const void* u, const float* gate_bias, cons
   if (ok && merge) ok = make_map(&maps.g, branch, bf16, B, T, D, rows, cols);
   if (!ok) return RGLRU_ERR_UNSUPPORTED;
   maps.ui = maps.ur;
+  a.split = grouped_split(true, bf16, merge, B, T, D);
   const cudaError_t e = launch_grouped_fwd(bf16, merge, maps, a, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
 }
@@ -618,6 +622,7 @@ int rglru_grouped_bwd(const void* dout, const float* dh_last, const void* x, con
   if (!ok) return RGLRU_ERR_UNSUPPORTED;
   maps.ui = maps.ur;
   maps.dui = maps.dur;
+  a.split = grouped_split(false, bf16, merge, B, T, D);
   const cudaError_t e = launch_grouped_bwd(bf16, merge, maps, a, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
 }

@@ -28,6 +28,7 @@ constexpr float POLY_RANGE = -0.25f;
 constexpr int DEV_TIMEOUT_LOAD = 1;   // a tile load never completed
 constexpr int DEV_TIMEOUT_STORE = 2;  // the producer never saw a chunk's results
 constexpr int DEV_TIMEOUT_SELFTEST = 3;  // the wait self-test (a barrier nothing completes) gave up, as it must
+constexpr int DEV_TIMEOUT_SPLIT = 4;     // time split: another CTA of the cluster never sent its chunk's map
 constexpr long long DEV_WAIT_CYCLES = 4000000000LL;   // about two seconds of SM clock
 
 // ---------------------------------------------------------------- PTX wrappers
@@ -180,6 +181,41 @@ __device__ __forceinline__ void prefetch_map(const void* map) {
 // launched with the attribute must come after pdl_wait.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// ---------------------------------------------------------------- thread-block clusters
+// Helpers of the time split: the CTAs of a cluster hold different chunks of one sequence and hand each other
+// eight-byte (product, state) pairs through distributed shared memory.
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+// Address of `p` (shared memory of this CTA) in the CTA of cluster rank `rank`.
+__device__ __forceinline__ uint32_t cluster_map(const void* p, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+  return r;
+}
+// Barrier of all (remaining) threads of the cluster; shared-memory writes before it, remote ones included, are
+// visible after it.
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Store a pair into another CTA's shared memory and report its eight bytes to that CTA's mbarrier.
+__device__ __forceinline__ void st_async_pair(uint32_t dst, float2 v, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(dst),
+               "f"(v.x), "f"(v.y), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void st_cluster_f32(uint32_t dst, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(v) : "memory");
+}
 
 // ---------------------------------------------------------------- fast math
 __device__ __forceinline__ float ex2_approx(float x) {

@@ -35,6 +35,7 @@ struct ScanFwdArgs {
   // gate_bias [2 D] fp32 in the same column layout or nullptr
   const float* gate_bias;
   int gate_bw;
+  int split;    // CTAs of a cluster that share one (batch row, channel tile) along time; 0 or 1: none
   bool paired;  // the four tensor maps are the 5-D paired-row form (32-channel bf16 forward without flags)
   int B, T, D;
   float c;
@@ -69,6 +70,7 @@ struct ScanBwdArgs {
   // the gate-bias gradient, their fold over the batch [2 D]; both in the gate tensor's column layout
   float* dgate_part;
   float* dgate;
+  int split;    // see ScanFwdArgs
   int B, T, D;
   float c;
   int* status;
@@ -190,6 +192,8 @@ cudaError_t launch_grouped_bwd(bool bf16, bool merge, const BwdMaps& maps, const
 int grouped_box_cols();
 int scan_fwd_variant(int B, int T, int D, bool bf16);
 int scan_bwd_variant(int B, int T, int D, bool bf16);
+int scan_split(bool fwd, bool bf16, int B, int T, int D);
+int grouped_split(bool fwd, bool bf16, bool merge, int B, int T, int D);
 int scan_fwd_box_rows(int variant);
 int scan_fwd_box_cols(int variant);
 // True when the call takes the paired-row tile layout, whose tensor maps are 5-D (see rglru_fwd_body).

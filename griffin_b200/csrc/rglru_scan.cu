@@ -38,6 +38,7 @@
 // conv alone, and the self-test of the bounded wait.
 
 #include <atomic>
+#include <cstddef>
 #include <cstdlib>
 
 #include "rglru_device.cuh"
@@ -138,6 +139,59 @@ template <int LANES, int CH>
 struct ChainSmem {
   static constexpr int AGG = LANES * CH * 8;  // float2 per (lane, channel)
   static constexpr int EIN = LANES * CH * 4;  // float per (lane, channel)
+};
+
+// Time split (SPLIT kernels).  A cluster of up to MAX_SPLIT CTAs shares one (batch row, channel tile): in round `it`
+// the CTA of rank r takes chunk it * R + r.  Everything of a chunk but its entering state is worked out locally; then
+// each CTA sends the affine map of its whole chunk, one (product, state) pair per channel, to every CTA of the
+// cluster, and each folds the pairs of the ranks before it onto the carry of the rounds before (all CTAs keep
+// identical copies of that carry, folded in rank order, so the result does not depend on timing).  Two buffers by
+// round parity suffice: nobody can send round it + 2 before it has received everybody's round it + 1, which they
+// send after they are done reading round it.
+// What it buys: with fewer tiles than SMs a sequence is bound by one CTA walking it chunk by chunk.  B = 1, T = 16384,
+// D = 1024 bf16 (16 tiles, six CTAs each): forward 135 -> 67 us, backward 340 -> 80 us; B = 2, T = 2048: 25 -> 13 and
+// 47 -> 21 us; fp32 B = 1, T = 16384: 310 -> 76 and 407 -> 93 us.
+constexpr int MAX_SPLIT = 8;   // the portable cluster size
+template <int CH>
+struct SplitSmem {
+  float2 pair[2][MAX_SPLIT][CH];
+  uint64_t bar[2];
+  float sums[MAX_SPLIT][3 * CH];   // rglru backward only: the per-channel sums of every rank, folded by rank 0
+};
+template <int CH>
+struct SplitChain {
+  SplitSmem<CH>* sm;
+  uint32_t rank, size;
+  __device__ __forceinline__ void init(SplitSmem<CH>* s) { sm = s; rank = cluster_rank(); size = cluster_size(); }
+  __device__ __forceinline__ void arm(int it) { mbar_expect_tx(&sm->bar[it & 1], size * CH * 8); }   // one thread per round
+  // Send this CTA's pair of one channel to the ranks first, first + step, ...
+  __device__ __forceinline__ void send(int it, int ch, float2 v, uint32_t first, uint32_t step) {
+    for (uint32_t r = first; r < size; r += step)
+      st_async_pair(cluster_map(&sm->pair[it & 1][rank][ch], r), v, cluster_map(&sm->bar[it & 1], r));
+  }
+  // State entering this CTA's chunk of round `it`, and the carry behind the whole round.
+  __device__ __forceinline__ float receive(int it, int ch, float& carry, float& prod, volatile int* dead, int* status) {
+    mbar_wait_or_flag(&sm->bar[it & 1], (it >> 1) & 1, dead, status, DEV_TIMEOUT_SPLIT);
+    return fold(it, ch, carry, prod);
+  }
+  __device__ __forceinline__ float receive(int it, int ch, float& carry, float& prod, bool& alive) {
+    if (alive) alive = mbar_wait_bounded(&sm->bar[it & 1], (it >> 1) & 1);
+    return fold(it, ch, carry, prod);
+  }
+  __device__ __forceinline__ float fold(int it, int ch, float& carry, float& prod) {
+    float2 v[MAX_SPLIT];
+#pragma unroll
+    for (int r = 0; r < MAX_SPLIT; ++r) v[r] = r < static_cast<int>(size) ? sm->pair[it & 1][r][ch] : make_float2(1.0f, 0.0f);
+    float e = carry, enter = carry;
+#pragma unroll
+    for (int r = 0; r < MAX_SPLIT; ++r) {
+      if (r == static_cast<int>(rank)) enter = e;
+      e = fmaf(v[r].x, e, v[r].y);
+      prod *= v[r].x;
+    }
+    carry = e;
+    return enter;
+  }
 };
 
 // Grouped gate layout: both gate pre-activations come from ONE tensor [B, T, 2 D] written by a single
@@ -288,7 +342,7 @@ __device__ __forceinline__ void fwd_local(const uint8_t* tx, const uint8_t* tr, 
   }
 }
 
-template <typename IO, int TS, int LANES, int CH, int NSTAGE, bool CONV = false, bool MERGE = false>
+template <typename IO, int TS, int LANES, int CH, int NSTAGE, bool CONV = false, bool MERGE = false, bool SPLIT = false>
 struct FwdSmem {
   static constexpr int TC = LANES * TS;
   static constexpr int TILE = TC * CH * sizeof(IO);
@@ -302,7 +356,8 @@ struct FwdSmem {
   static constexpr int SEGS = (LANES == 32 && CH == 32) ? 4 : 1;
   static constexpr int OFF_SEG = OFF_EIN + ChainSmem<LANES, CH>::EIN;
   static constexpr int OFF_BAR = OFF_SEG + SEGS * CH * 8;   // full[NSTAGE], ready[NSTAGE], dead flag
-  static constexpr int BYTES = OFF_BAR + 2 * NSTAGE * 8 + 16;
+  static constexpr int OFF_SPLIT = OFF_BAR + 2 * NSTAGE * 8 + 16;
+  static constexpr int BYTES = OFF_SPLIT + (SPLIT ? static_cast<int>(sizeof(SplitSmem<CH>)) : 0);
 };
 
 // Threads [0, LANES*NCV) compute; with TMA one extra warp issues every bulk copy so that
@@ -310,9 +365,9 @@ struct FwdSmem {
 // MERGE: the kernel also reads the pre-activation of the block's GeLU branch and writes
 // h_t * gelu(branch_t) (griffin/griffin.py:464, 520 of the reference) instead of h_t.
 template <typename IO, int TS, int LANES, int CH, int NSTAGE, bool USE_TMA, bool CONV, bool MERGE, bool GROUPED, bool PLAIN = false,
-          bool CARRY = false, bool PAIRED = false>
+          bool CARRY = false, bool PAIRED = false, bool SPLIT = false>
 __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFwdArgs& p) {
-  using SM = FwdSmem<IO, TS, LANES, CH, NSTAGE, CONV, MERGE>;
+  using SM = FwdSmem<IO, TS, LANES, CH, NSTAGE, CONV, MERGE, SPLIT>;
   static_assert(!CONV || (SM::HALO % 128 == 0), "the halo must keep the result rows 128-byte aligned for TMA");
   constexpr int NCV = CH / CV;
   constexpr int TC = SM::TC;
@@ -339,12 +394,20 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
   const int d0 = blockIdx.x * CH;
   const int nchunks = (p.T + TC - 1) / TC;
   const int nsave = (p.T + SAVE_EVERY - 1) / SAVE_EVERY;
+  // SPLIT: this CTA's chunks are rank, rank + nranks, ...; every CTA of the cluster goes through `rounds` rounds.
+  static_assert(!SPLIT || (USE_TMA && !CONV && !CARRY), "the time split exists for the TMA-staged scan kernels");
+  SplitChain<CH> split;
+  if constexpr (SPLIT) split.init(reinterpret_cast<SplitSmem<CH>*>(smem + SM::OFF_SPLIT));
+  const int rank = SPLIT ? static_cast<int>(split.rank) : 0, nranks = SPLIT ? static_cast<int>(split.size) : 1;
+  const int rounds = SPLIT ? (nchunks + nranks - 1) / nranks : nchunks;
+  const int mine = SPLIT ? (nchunks - rank + nranks - 1) / nranks : nchunks;   // chunks this CTA loads and stores
   static_assert(!GROUPED || USE_TMA, "the grouped gate layout is staged by TMA only");
   const int rcol = GROUPED ? grouped_col(d0, p.gate_bw) : d0;   // first column of this tile's u_r / u_i
   const int icol = GROUPED ? rcol + p.gate_bw : d0;
 
-  auto issue = [&](int k) {
-    const int sidx = k % NSTAGE;
+  auto issue = [&](int it) {
+    const int sidx = it % NSTAGE;
+    const int k = it * nranks + rank;
     uint8_t* st = smem + sidx * SM::STAGE;
     mbar_expect_tx(&full[sidx], SM::STAGE);
     if constexpr (PAIRED) {
@@ -366,23 +429,25 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
     *dead = 0;
     if (USE_TMA) {
       for (int s = 0; s < NSTAGE; ++s) { mbar_init(&full[s], 1); mbar_init(&ready[s], NCOMP / 32); }
+      if constexpr (SPLIT) { mbar_init(&split.sm->bar[0], 1); mbar_init(&split.sm->bar[1], 1); }
       mbar_fence_init();
       prefetch_map(&maps.x); prefetch_map(&maps.ur); prefetch_map(&maps.ui); prefetch_map(&maps.y);
       if (MERGE) prefetch_map(&maps.g);
       // While the kernel in front of this one on the stream drains, pull the first chunk towards L2.
       if constexpr (PAIRED) {
-        tma_prefetch_5d(&maps.x, d0, 0, 0, 0, b);
-        tma_prefetch_5d(&maps.ur, d0, 0, 0, 0, b);
-        tma_prefetch_5d(&maps.ui, d0, 0, 0, 0, b);
+        tma_prefetch_5d(&maps.x, d0, 0, 0, rank * (TC / 8), b);
+        tma_prefetch_5d(&maps.ur, d0, 0, 0, rank * (TC / 8), b);
+        tma_prefetch_5d(&maps.ui, d0, 0, 0, rank * (TC / 8), b);
       } else {
-        tma_prefetch_3d(&maps.x, d0, -(CONV ? 3 : 0), b);
-        tma_prefetch_3d(&maps.ur, rcol, 0, b);
-        tma_prefetch_3d(&maps.ui, icol, 0, b);
-        if (MERGE) tma_prefetch_3d(&maps.g, d0, 0, b);
+        tma_prefetch_3d(&maps.x, d0, rank * TC - (CONV ? 3 : 0), b);
+        tma_prefetch_3d(&maps.ur, rcol, rank * TC, b);
+        tma_prefetch_3d(&maps.ui, icol, rank * TC, b);
+        if (MERGE) tma_prefetch_3d(&maps.g, d0, rank * TC, b);
       }
     }
   }
-  __syncthreads();
+  if constexpr (SPLIT) cluster_sync_all();   // the barriers of every CTA are there before anybody sends
+  else __syncthreads();
   pdl_wait();   // nothing above touches global memory; everything below may depend on the previous kernel
 
   if (USE_TMA && tid >= NCOMP) {
@@ -393,20 +458,21 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
       // the rest once it has landed, so that no CTA's first chunk queues behind other CTAs' later ones.
       issue(0);
       mbar_wait_or_flag(&full[0], 0, dead, p.status, DEV_TIMEOUT_LOAD);
-      for (int k = 1; k < NSTAGE && k < nchunks; ++k) issue(k);
-      for (int k = 0; k < nchunks; ++k) {
-        const int sidx = k % NSTAGE;
-        mbar_wait_or_flag(&ready[sidx], (k / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
+      for (int it = 1; it < NSTAGE && it < mine; ++it) issue(it);
+      for (int it = 0; it < mine; ++it) {
+        const int sidx = it % NSTAGE, k = it * nranks + rank;
+        mbar_wait_or_flag(&ready[sidx], (it / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
         if constexpr (PAIRED) tma_store_5d(&maps.y, smem + sidx * SM::STAGE, d0, 0, 0, k * (TC / 8), b);
         else if (!CARRY) tma_store_3d(&maps.y, smem + sidx * SM::STAGE + SM::HALO, d0, k * TC, b);
         tma_commit();
-        if (k + NSTAGE < nchunks) {
+        if (it + NSTAGE < mine) {
           tma_wait_read<0>();
-          issue(k + NSTAGE);
+          issue(it + NSTAGE);
         }
       }
       tma_wait_all<0>();
     }
+    if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }
     return;
   }
 
@@ -443,16 +509,21 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
   const int off0 = PAIRED ? ((lane_t >> 1) * TS) * RSTEP + (lane_t & 1) * ROWB + vec * Pack<IO>::BYTES
                           : (lane_t * TS) * ROWB + vec * Pack<IO>::BYTES;
 
-  for (int k = 0; k < nchunks; ++k) {
-    const int stage = USE_TMA ? (k % NSTAGE) : 0;
+  for (int it = 0; it < rounds; ++it) {
+    const int k = it * nranks + rank;
+    const bool idle = SPLIT && it >= mine;     // last round: no chunk left for this CTA, it only takes part in the exchange
+    if constexpr (SPLIT) { if (tid == 0) split.arm(it); }
+    const int stage = USE_TMA ? (it % NSTAGE) : 0;
     uint8_t* tiles = smem + stage * SM::STAGE;
     const int t0 = k * TC;
     uint32_t fl[(TS + 3) / 4];
     const bool masked = !PLAIN && ((p.tok != nullptr) || (t0 + TC > p.T));
     if (masked) load_flags<TS>(p.tok, b, p.T, t0 + lane_t * TS, fl);
 
+    float2 P[TS][2], S[TS][2];
+    if (!idle) {
     if (USE_TMA) {
-      mbar_wait_or_flag(&full[stage], (k / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+      mbar_wait_or_flag(&full[stage], (it / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
     } else {
       tile_load_plain<IO, CH>(tiles, p.x, b, t0 - (CONV ? 3 : 0), d0, TC + (CONV ? 3 : 0), p.T, p.D);
       tile_load_plain<IO, CH>(tiles + SM::TILEX, p.ur, b, t0, d0, TC, p.T, p.D);
@@ -461,7 +532,6 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
       bar_compute(NCOMP);
     }
 
-    float2 P[TS][2], S[TS][2];
     const uint8_t* tx = tiles;
     const uint8_t* tr = tiles + SM::TILEX;
     const uint8_t* ti = tiles + SM::TILEX + SM::TILE;
@@ -483,12 +553,13 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
       dst[0] = make_float4(P[TS - 1][0].x, S[TS - 1][0].x, P[TS - 1][0].y, S[TS - 1][0].y);
       dst[1] = make_float4(P[TS - 1][1].x, S[TS - 1][1].x, P[TS - 1][1].y, S[TS - 1][1].y);
     }
+    }
     bar_compute(NCOMP);
 
     if (chain_thread) {
       float2 ag[SEGL];
 #pragma unroll
-      for (int j = 0; j < SEGL; ++j) ag[j] = agg[(seg * SEGL + j) * CH + cch];
+      for (int j = 0; j < SEGL; ++j) ag[j] = idle ? make_float2(1.0f, 0.0f) : agg[(seg * SEGL + j) * CH + cch];
       auto emit = [&](int lane, float e) {       // state entering a lane; every SAVE_EVERY steps also kept for the backward
         if (((lane * TS) % SAVE_EVERY) == 0) {
           const int t = t0 + lane * TS;
@@ -497,7 +568,7 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
         }
         ein[lane * CH + cch] = e;
       };
-      if (SEGS == 1) {
+      if (SEGS == 1 && !SPLIT) {
         float e = carry;
 #pragma unroll
         for (int j = 0; j < LANES; ++j) {
@@ -522,22 +593,44 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
           sa = fmaf(ag[j].x, sa, ag[j].y);
           pa *= ag[j].x;
         }
-        segtot[seg * CH + cch] = make_float2(pa, sa);
-        bar_chain(SEGS * CH);
-        float e = carry, enter = carry;
+        float enter;
+        if constexpr (!SPLIT) {
+          segtot[seg * CH + cch] = make_float2(pa, sa);
+          bar_chain(SEGS * CH);
+          float e = carry;
+          enter = carry;
 #pragma unroll
-        for (int sgm = 0; sgm < SEGS; ++sgm) {
-          const float2 tot = segtot[sgm * CH + cch];
-          if (sgm == seg) enter = e;
-          e = fmaf(tot.x, e, tot.y);
-          prod_all *= tot.x;
+          for (int sgm = 0; sgm < SEGS; ++sgm) {
+            const float2 tot = segtot[sgm * CH + cch];
+            if (sgm == seg) enter = e;
+            e = fmaf(tot.x, e, tot.y);
+            prod_all *= tot.x;
+          }
+          carry = e;
+        } else {
+          float2 before = make_float2(1.0f, 0.0f), tot = make_float2(pa, sa);   // map of the segments before this one / of the chunk
+          if constexpr (SEGS > 1) {
+            segtot[seg * CH + cch] = tot;
+            bar_chain(SEGS * CH);
+            tot = make_float2(1.0f, 0.0f);
+#pragma unroll
+            for (int sgm = 0; sgm < SEGS; ++sgm) {
+              const float2 t = segtot[sgm * CH + cch];
+              if (sgm == seg) before = tot;
+              tot = make_float2(tot.x * t.x, fmaf(t.x, tot.y, t.y));
+            }
+          }
+          split.send(it, cch, tot, seg, SEGS);
+          enter = fmaf(before.x, split.receive(it, cch, carry, prod_all, dead, p.status), before.y);
         }
-        carry = e;
+        if (!idle) {
 #pragma unroll
-        for (int j = 0; j < SEGL; ++j) emit(seg * SEGL + j, fmaf(pp[j], enter, sp[j]));
+          for (int j = 0; j < SEGL; ++j) emit(seg * SEGL + j, fmaf(pp[j], enter, sp[j]));
+        }
       }
     }
     bar_compute(NCOMP);
+    if (idle) break;
 
     {
       const float4 e4 = *reinterpret_cast<const float4*>(ein + lane_t * CH + vec * CV);
@@ -548,6 +641,15 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
         float2 yv[2];
 #pragma unroll
         for (int cp = 0; cp < 2; ++cp) yv[cp] = fma2(P[st][cp], e[cp], S[st][cp]);
+        if constexpr (SPLIT) {   // the final state is the last step's output to the bit, not the folded carry
+          if (p.h_last && t0 + lane_t * TS + st == p.T - 1) {
+            float* hl = p.h_last + static_cast<size_t>(b) * p.D + d0 + vec * CV;
+            const float v[4] = {yv[0].x, yv[0].y, yv[1].x, yv[1].y};
+#pragma unroll
+            for (int ch = 0; ch < 4; ++ch)
+              if (d0 + vec * CV + ch < p.D) hl[ch] = v[ch];
+          }
+        }
         if (MERGE) {
           float2 gv[2];
           Pack<IO>::unpack2(Pack<IO>::load(tiles + SM::OFF_G + off0 + st * RSTEP), gv);
@@ -567,7 +669,12 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
       bar_compute(NCOMP);
     }
   }
-  if (tid < CH && dch < p.D && p.h_last) p.h_last[static_cast<size_t>(b) * p.D + dch] = carry;   // segment 0's copy
+  if constexpr (SPLIT) {
+    __syncwarp();
+    cluster_sync_all();        // no CTA leaves while another may still send to it
+    if (rank != 0) return;
+  }
+  if (!SPLIT && tid < CH && dch < p.D && p.h_last) p.h_last[static_cast<size_t>(b) * p.D + dch] = carry;   // segment 0's copy
   if (tid < CH && dch < p.D && want_prod) p.decay_prod[static_cast<size_t>(b) * p.D + dch] = prod_all;
 }
 
@@ -575,17 +682,18 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
 // CARRY: the carry-only pass of a time-split sequence: no output tensor, nothing is stored but h_last and decay_prod.
 // PAIRED: 64-byte tile rows staged two to a 128-byte line through 5-D tensor maps (see rglru_fwd_body).
 template <typename IO, int TS, int LANES, int CH, int NSTAGE, bool USE_TMA, bool CONV, bool MERGE, bool GROUPED, bool PLAIN = false,
-          bool CARRY = false, bool PAIRED = false>
+          bool CARRY = false, bool PAIRED = false, bool SPLIT = false>
 __global__ void __launch_bounds__(LANES*(CH / CV) + (USE_TMA ? 32 : 0))
     rglru_fwd_kernel(const __grid_constant__ FwdMaps maps, const ScanFwdArgs p) {
-  rglru_fwd_body<IO, TS, LANES, CH, NSTAGE, USE_TMA, CONV, MERGE, GROUPED, PLAIN, CARRY, PAIRED>(maps, p);
+  rglru_fwd_body<IO, TS, LANES, CH, NSTAGE, USE_TMA, CONV, MERGE, GROUPED, PLAIN, CARRY, PAIRED, SPLIT>(maps, p);
 }
 // The same kernel capped at 96 registers, which lets two 9-warp CTAs share an SM's register files (five warps
 // on one scheduler partition).  Used for the merged / grouped variants, which otherwise take about 112.
-template <typename IO, int TS, int LANES, int CH, int NSTAGE, bool USE_TMA, bool CONV, bool MERGE, bool GROUPED>
+template <typename IO, int TS, int LANES, int CH, int NSTAGE, bool USE_TMA, bool CONV, bool MERGE, bool GROUPED, bool PLAIN = false,
+          bool SPLIT = false>
 __global__ void __maxnreg__(96)
     rglru_fwd_kernel_capped(const __grid_constant__ FwdMaps maps, const ScanFwdArgs p) {
-  rglru_fwd_body<IO, TS, LANES, CH, NSTAGE, USE_TMA, CONV, MERGE, GROUPED>(maps, p);
+  rglru_fwd_body<IO, TS, LANES, CH, NSTAGE, USE_TMA, CONV, MERGE, GROUPED, PLAIN, false, false, SPLIT>(maps, p);
 }
 
 // ======================================================================
@@ -760,7 +868,7 @@ __device__ __forceinline__ void bwd_apply(uint8_t* tiles, int off_dx, int off_dr
   }
 }
 
-template <typename IO, int TS, int LANES, int CH, int NSTAGE, bool CONV = false, bool MERGE = false>
+template <typename IO, int TS, int LANES, int CH, int NSTAGE, bool CONV = false, bool MERGE = false, bool SPLIT = false>
 struct BwdSmem {
   static constexpr int TC = LANES * TS;
   static constexpr int TILE = TC * CH * sizeof(IO);
@@ -777,7 +885,8 @@ struct BwdSmem {
   static constexpr int OFF_EINF = OFF_AGGC + PLANE;
   static constexpr int OFF_EINR = OFF_EINF + PLANE;
   static constexpr int OFF_BAR = OFF_EINR + PLANE;   // full[NSTAGE], ready[NSTAGE], dead flag
-  static constexpr int BYTES = OFF_BAR + 2 * NSTAGE * 8 + 16;
+  static constexpr int OFF_SPLIT = OFF_BAR + 2 * NSTAGE * 8 + 16;
+  static constexpr int BYTES = OFF_SPLIT + (SPLIT ? static_cast<int>(sizeof(SplitSmem<CH>)) : 0);
 };
 
 // SELF_ISSUE: no producer warp.  One thread of the last compute warp (not a chain thread) issues the bulk
@@ -789,11 +898,11 @@ struct BwdSmem {
 // masked; the masked arithmetic is not compiled in (half the code, and registers allotted for this path alone).
 // CARRY: the carry-only pass of a time-split sequence: no gradient tensors, nothing is stored but dh0.
 template <typename IO, int TS, int LANES, int CH, int NSTAGE, bool USE_TMA, bool CONV, bool MERGE, bool GROUPED,
-          bool SELF_ISSUE = false, bool PLAIN = false, bool CARRY = false>
+          bool SELF_ISSUE = false, bool PLAIN = false, bool CARRY = false, bool SPLIT = false>
 __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 32 : 0),
                                   (SELF_ISSUE && CH == 32) ? 2 : 1)
     rglru_bwd_kernel(const __grid_constant__ BwdMaps maps, const ScanBwdArgs p) {
-  using SM = BwdSmem<IO, TS, LANES, CH, NSTAGE, CONV, MERGE>;
+  using SM = BwdSmem<IO, TS, LANES, CH, NSTAGE, CONV, MERGE, SPLIT>;
   static_assert(!CONV || (SM::HALO % 128 == 0), "the halo must keep the result rows 128-byte aligned for TMA");
   constexpr int NCV = CH / CV;
   constexpr int TC = SM::TC;
@@ -818,12 +927,19 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
   const int d0 = blockIdx.x * CH;
   const int nchunks = (p.T + TC - 1) / TC;
   const int nsave = (p.T + SAVE_EVERY - 1) / SAVE_EVERY;
+  // SPLIT: in processing order (from the end of the sequence) this CTA's chunks are rank, rank + nranks, ...
+  static_assert(!SPLIT || (USE_TMA && !CONV && !CARRY), "the time split exists for the TMA-staged scan kernels");
+  SplitChain<CH> split;
+  if constexpr (SPLIT) split.init(reinterpret_cast<SplitSmem<CH>*>(smem + SM::OFF_SPLIT));
+  const int rank = SPLIT ? static_cast<int>(split.rank) : 0, nranks = SPLIT ? static_cast<int>(split.size) : 1;
+  const int rounds = SPLIT ? (nchunks + nranks - 1) / nranks : nchunks;
+  const int mine = SPLIT ? (nchunks - rank + nranks - 1) / nranks : nchunks;   // chunks this CTA loads and stores
   static_assert(!GROUPED || USE_TMA, "the grouped gate layout is staged by TMA only");
   const int rcol = GROUPED ? grouped_col(d0, p.gate_bw) : d0;   // first column of this tile's u_r / u_i (and du_r / du_i)
   const int icol = GROUPED ? rcol + p.gate_bw : d0;
 
-  auto issue = [&](int q) {  // q-th chunk in processing order == chunk nchunks-1-q in time
-    const int k = nchunks - 1 - q;
+  auto issue = [&](int q) {  // this CTA's q-th chunk in processing order, which runs from the end of the sequence
+    const int k = nchunks - 1 - (q * nranks + rank);
     const int sidx = q % NSTAGE;
     uint8_t* st = smem + sidx * SM::STAGE;
     mbar_expect_tx(&full[sidx], SM::STAGE);
@@ -834,7 +950,7 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
     if (MERGE) tma_load_3d(st + SM::OFF_G, &maps.g, d0, k * TC, b, &full[sidx]);
   };
   auto store = [&](int q) {
-    const int k = nchunks - 1 - q;
+    const int k = nchunks - 1 - (q * nranks + rank);
     uint8_t* st = smem + (q % NSTAGE) * SM::STAGE;
     if (!CARRY) {
       tma_store_3d(&maps.dx, st + SM::OFF_X + SM::HALO, d0, k * TC, b);
@@ -855,13 +971,14 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
     *dead = 0;
     if (USE_TMA) {
       for (int s = 0; s < NSTAGE; ++s) { mbar_init(&full[s], 1); mbar_init(&ready[s], NCOMP / 32); }
+      if constexpr (SPLIT) { mbar_init(&split.sm->bar[0], 1); mbar_init(&split.sm->bar[1], 1); }
       mbar_fence_init();
       prefetch_map(&maps.dy); prefetch_map(&maps.x); prefetch_map(&maps.ur); prefetch_map(&maps.ui);
       prefetch_map(&maps.dx); prefetch_map(&maps.dur); prefetch_map(&maps.dui);
       if (MERGE) { prefetch_map(&maps.g); prefetch_map(&maps.dg); }
       // While the kernel in front of this one on the stream drains, pull the first chunk (the last in time)
       // towards L2.
-      const int kl = nchunks - 1;
+      const int kl = nchunks - 1 - rank;
       tma_prefetch_3d(&maps.dy, d0, kl * TC, b);
       tma_prefetch_3d(&maps.x, d0, kl * TC - (CONV ? 3 : 0), b);
       tma_prefetch_3d(&maps.ur, rcol, kl * TC, b);
@@ -869,7 +986,8 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
       if (MERGE) tma_prefetch_3d(&maps.g, d0, kl * TC, b);
     }
   }
-  __syncthreads();
+  if constexpr (SPLIT) cluster_sync_all();   // the barriers of every CTA are there before anybody sends
+  else __syncthreads();
   pdl_wait();   // nothing above touches global memory; everything below may depend on the previous kernel
 
   if (USE_TMA && !SELF_ISSUE && tid >= NCOMP) {
@@ -878,18 +996,19 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
       // the first chunk is asked for alone, the rest once it has landed (see the forward kernel)
       issue(0);
       mbar_wait_or_flag(&full[0], 0, dead, p.status, DEV_TIMEOUT_LOAD);
-      for (int q = 1; q < NSTAGE && q < nchunks; ++q) issue(q);
-      for (int q = 0; q < nchunks; ++q) {
+      for (int q = 1; q < NSTAGE && q < mine; ++q) issue(q);
+      for (int q = 0; q < mine; ++q) {
         const int sidx = q % NSTAGE;
         mbar_wait_or_flag(&ready[sidx], (q / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
         store(q);
-        if (q + NSTAGE < nchunks) {
+        if (q + NSTAGE < mine) {
           tma_wait_read<0>();
           issue(q + NSTAGE);
         }
       }
       tma_wait_all<0>();
     }
+    if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }
     return;
   }
 
@@ -919,26 +1038,31 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
   float2 dsr[2] = {f2(0.0f), f2(0.0f)}, dsi[2] = {f2(0.0f), f2(0.0f)};   // grouped layout: sums over time of du_r, du_i
   const int off0 = (lane_t * TS) * ROWB + vec * Pack<IO>::BYTES;
 
-  for (int q = 0; q < nchunks; ++q) {
-    const int k = nchunks - 1 - q;
+  for (int q = 0; q < rounds; ++q) {
+    const int k = nchunks - 1 - (q * nranks + rank);
+    const bool idle = SPLIT && q >= mine;     // last round: no chunk left for this CTA, it only takes part in the exchange
+    if constexpr (SPLIT) { if (tid == 0) split.arm(q); }
     const int stage = USE_TMA ? (q % NSTAGE) : 0;
     uint8_t* tiles = smem + stage * SM::STAGE;
     const int t0 = k * TC;
     uint32_t fl[(TS + 3) / 4];
     const bool masked = !PLAIN && ((p.tok != nullptr) || (t0 + TC > p.T));
-    if (masked) load_flags<TS>(p.tok, b, p.T, t0 + lane_t * TS, fl);
+    if (masked && !idle) load_flags<TS>(p.tok, b, p.T, t0 + lane_t * TS, fl);
 
     // State entering this chunk (saved by the forward kernel; chunk 0 starts from h0).
     float enter = 0.0f;
-    if (fwd_chain && dch < p.D) {
+    if (fwd_chain && dch < p.D && !idle) {
       if (k == 0) enter = p.h0 ? p.h0[static_cast<size_t>(b) * p.D + dch] : 0.0f;
       else enter = p.states[(static_cast<size_t>(b) * nsave + t0 / SAVE_EVERY) * p.D + dch];
     }
 
+    BwdRegs<IO, TS> R;
+    bool flagged = false;
+    if (!idle) {
     if (USE_TMA) {
       mbar_wait_or_flag(&full[stage], (q / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
       if (self_issuer && q == 0)      // the first chunk was asked for alone; now that it has landed, the rest
-        for (int qq = 1; qq < NSTAGE && qq < nchunks; ++qq) issue(qq);
+        for (int qq = 1; qq < NSTAGE && qq < mine; ++qq) issue(qq);
     } else {
       tile_load_plain<IO, CH>(tiles, p.dy, b, t0, d0, TC, p.T, p.D);
       tile_load_plain<IO, CH>(tiles + SM::OFF_X, p.x, b, t0 - (CONV ? 3 : 0), d0, TC + (CONV ? 3 : 0), p.T, p.D);
@@ -948,9 +1072,8 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
       bar_compute(NCOMP);
     }
 
-    BwdRegs<IO, TS> R;
     float2 prod[2], sfwd[2], crev[2];
-    const bool flagged = masked && any_flag(fl);
+    flagged = masked && any_flag(fl);
     {
       uint8_t* tdy = tiles;
       uint8_t* tg = tiles + SM::OFF_G;
@@ -977,16 +1100,17 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
       *reinterpret_cast<float4*>(aggS + ao) = make_float4(sfwd[0].x, sfwd[0].y, sfwd[1].x, sfwd[1].y);
       *reinterpret_cast<float4*>(aggC + ao) = make_float4(crev[0].x, crev[0].y, crev[1].x, crev[1].y);
     }
+    }
     bar_compute(NCOMP);
     if (self_issuer && q >= 1) {
       store(q - 1);
-      if (q >= 2 && q - 2 + NSTAGE < nchunks) {
+      if (q >= 2 && q - 2 + NSTAGE < mine) {
         tma_wait_read<1>();      // all but the store just committed have been read out: the stage of chunk q-2 is free
         issue(q - 2 + NSTAGE);
       }
     }
 
-    if (fwd_chain || rev_chain) {
+    if ((fwd_chain && !idle) || rev_chain) {
       const float* plane = fwd_chain ? aggS : aggC;
       float* ein = fwd_chain ? einF : einR;
       float ap[LANES], as[LANES];
@@ -999,7 +1123,7 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
           ein[j * CH + cch] = e;
           e = fmaf(ap[j], e, as[j]);
         }
-      } else {
+      } else if constexpr (!SPLIT) {
         float e = carry_rev;
 #pragma unroll
         for (int j = LANES - 1; j >= 0; --j) {
@@ -1007,9 +1131,30 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
           e = fmaf(ap[j], e, as[j]);
         }
         carry_rev = e;
+      } else {
+        // Compose the chunk from the identity, leaving in (ap, as) the map that takes the carry entering the chunk
+        // (at its end) to the carry entering each lane.
+        float pa = 1.0f, sa = 0.0f, unused = 1.0f;
+        if (!idle) {
+#pragma unroll
+          for (int j = LANES - 1; j >= 0; --j) {
+            const float pj = ap[j], sj = as[j];
+            ap[j] = pa;
+            as[j] = sa;
+            sa = fmaf(pj, sa, sj);
+            pa *= pj;
+          }
+        }
+        split.send(q, cch, make_float2(pa, sa), 0, 1);
+        const float e = split.receive(q, cch, carry_rev, unused, dead, p.status);
+        if (!idle) {
+#pragma unroll
+          for (int j = 0; j < LANES; ++j) ein[j * CH + cch] = fmaf(ap[j], e, as[j]);
+        }
       }
     }
     bar_compute(NCOMP);
+    if (idle) break;
 
     {
       const float4 f4 = *reinterpret_cast<const float4*>(einF + lane_t * CH + vec * CV);
@@ -1037,11 +1182,14 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
     }
   }
 
-  if (rev_chain && dch < p.D && p.dh0) p.dh0[static_cast<size_t>(b) * p.D + dch] = carry_rev;
+  if (rev_chain && rank == 0 && dch < p.D && p.dh0) p.dh0[static_cast<size_t>(b) * p.D + dch] = carry_rev;
 
   // Per-row partial of sum_t dl * r: fold the time-lanes in a fixed order.
   bar_compute(NCOMP);
-  if (self_issuer) store(nchunks - 1);     // the last chunk's results; the issuing thread drains its stores on its way out
+  if (self_issuer) {
+    // (in an idle last round the barrier of that round has already sent the last chunk's results off)
+    if (mine == rounds) store(mine - 1);     // the last chunk's results; the issuing thread drains its stores on its way out
+  }
   auto drain = [&]() { if (USE_TMA && SELF_ISSUE && self_issuer) tma_wait_all<0>(); };
   *reinterpret_cast<float4*>(einF + lane_t * CH + vec * CV) = make_float4(dlam[0].x, dlam[0].y, dlam[1].x, dlam[1].y);
   if (GROUPED) {   // the chain planes are free now: the two gate sums go through them the same way
@@ -1056,8 +1204,21 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
     float acc = 0.0f;
 #pragma unroll
     for (int j = 0; j < LANES; ++j) acc += plane[j * CH + cch];
-    if (which == 0) p.dlam_part[static_cast<size_t>(b) * p.D + dch] = acc;
+    if constexpr (SPLIT) { st_cluster_f32(cluster_map(&split.sm->sums[rank][tid], 0), acc); }
+    else if (which == 0) p.dlam_part[static_cast<size_t>(b) * p.D + dch] = acc;
     else if (p.dgate_part) p.dgate_part[static_cast<size_t>(b) * 2 * p.D + (which == 1 ? rcol : icol) + cch] = acc;
+  }
+  if constexpr (SPLIT) {     // rank 0 folds the sums of the cluster in rank order
+    __syncwarp();
+    cluster_sync_all();      // (nothing is sent to any CTA after this)
+    if (rank != 0) { drain(); return; }
+    if (tid < (GROUPED ? 3 * CH : CH) && dch < p.D) {
+      const int which = tid / CH;
+      float acc = 0.0f;
+      for (int r = 0; r < nranks; ++r) acc += split.sm->sums[r][tid];
+      if (which == 0) p.dlam_part[static_cast<size_t>(b) * p.D + dch] = acc;
+      else if (p.dgate_part) p.dgate_part[static_cast<size_t>(b) * 2 * p.D + (which == 1 ? rcol : icol) + cch] = acc;
+    }
   }
   if (!p.ticket) { drain(); return; }   // the caller folds the rows with rglru_dlambda_kernel
 
@@ -1154,64 +1315,122 @@ __global__ void rglru_dlambda_kernel(const float* __restrict__ part, const float
 // for griffin/triton_scan.py:274-276).  Same two-level structure, no gate math.
 // ======================================================================
 
-constexpr int CH = 64;
+// 32-channel tiles (whole 128-byte lines) in four stages, two CTAs per SM: against one CTA per SM on 64-channel tiles,
+// B = 3, T = 1999, D = 1000 takes 16 + 25 us instead of 33 + 45 us with the time split, B = 6, T = 2048, D = 1024
+// 28 + 47 instead of 37 + 51 us without it.
+constexpr int CH = 32;
 constexpr int NCV = CH / CV;
 constexpr int RAW_TS = 4;
 constexpr int RAW_LANES = 16;
 constexpr int RAW_NT = RAW_LANES * NCV;
 constexpr int RAW_TC = RAW_LANES * RAW_TS;
 constexpr int RAW_TILE = RAW_TC * CH * 4;
+constexpr int RAW_STAGES = 4;
 
-template <int NSTAGE>
+// The chain leaves the state entering a lane where the lane's aggregate was (.x of its pair), so that a split backward
+// with two stages stays below half an SM's shared memory.
+template <int NSTAGE, int NTILE, bool SPLIT>
 struct RawSmem {
-  static constexpr int NTILE = 3;
   static constexpr int STAGE = NTILE * RAW_TILE;
   static constexpr int OFF_AGG = NSTAGE * STAGE;
-  static constexpr int OFF_EIN = OFF_AGG + ChainSmem<RAW_LANES, CH>::AGG;
-  static constexpr int OFF_BAR = OFF_EIN + ChainSmem<RAW_LANES, CH>::EIN;
-  static constexpr int BYTES = OFF_BAR + NSTAGE * 8 + 16;
+  static constexpr int OFF_BAR = OFF_AGG + ChainSmem<RAW_LANES, CH>::AGG;
+  static constexpr int OFF_SPLIT = OFF_BAR + NSTAGE * 8 + 16;
+  static constexpr int BYTES = OFF_SPLIT + (SPLIT ? static_cast<int>(offsetof(SplitSmem<CH>, sums)) : 0);
 };
+// The states (carries) of a thread's four channels that enter its lane.
+__device__ __forceinline__ void raw_entering(const float2* agg, int at, float2 (&e)[2]) {
+  const float4 a = *reinterpret_cast<const float4*>(agg + at), b = *reinterpret_cast<const float4*>(agg + at + 2);
+  e[0] = make_float2(a.x, a.z);
+  e[1] = make_float2(b.x, b.z);
+}
+// Level two of a chunk for one channel: chain the lane aggregates onto the carry (lanes in increasing time order, or
+// decreasing with REV) and leave every lane's entering state in place.  `idle`: this CTA has no chunk in the round.
+template <bool REV, bool SPLIT>
+__device__ __forceinline__ void raw_chain(float2* agg, float& carry, SplitChain<CH>& split, int it, bool idle, bool& alive) {
+  constexpr int LANES = RAW_LANES;
+  const int tid = threadIdx.x;
+  float2 ag[LANES];
+#pragma unroll
+  for (int j = 0; j < LANES; ++j) ag[j] = idle ? make_float2(1.0f, 0.0f) : agg[j * CH + tid];
+  if constexpr (!SPLIT) {
+    float e = carry;
+#pragma unroll
+    for (int q = 0; q < LANES; ++q) {
+      const int j = REV ? LANES - 1 - q : q;
+      agg[j * CH + tid].x = e;
+      e = fmaf(ag[j].x, e, ag[j].y);
+    }
+    carry = e;
+  } else {
+    float2 m = make_float2(1.0f, 0.0f);        // map from the state entering the chunk to that entering the lane
+#pragma unroll
+    for (int q = 0; q < LANES; ++q) {
+      const int j = REV ? LANES - 1 - q : q;
+      const float2 a = ag[j];
+      ag[j] = m;
+      m = make_float2(m.x * a.x, fmaf(a.x, m.y, a.y));
+    }
+    split.send(it, tid, m, 0, 1);
+    float unused = 1.0f;
+    const float e = split.receive(it, tid, carry, unused, alive);
+    if (!idle) {
+#pragma unroll
+      for (int j = 0; j < LANES; ++j) agg[j * CH + tid].x = fmaf(ag[j].x, e, ag[j].y);
+    }
+  }
+}
 
-template <int NSTAGE, bool USE_TMA>
+template <int NSTAGE, bool USE_TMA, bool SPLIT>
 __global__ void __launch_bounds__(RAW_NT) rawscan_fwd_kernel(const __grid_constant__ RawFwdMaps maps, const RawScanArgs p) {
-  using SM = RawSmem<NSTAGE>;
-  constexpr int TS = RAW_TS, TC = RAW_TC, ROWB = CH * 4, LANES = RAW_LANES;
+  using SM = RawSmem<NSTAGE, 2, SPLIT>;
+  constexpr int TS = RAW_TS, TC = RAW_TC, ROWB = CH * 4;
   extern __shared__ __align__(128) uint8_t smem[];
   float2* agg = reinterpret_cast<float2*>(smem + SM::OFF_AGG);
-  float* ein = reinterpret_cast<float*>(smem + SM::OFF_EIN);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::OFF_BAR);
   const int tid = threadIdx.x, lane_t = tid / NCV, vec = tid % NCV;
   const int b = blockIdx.y, d0 = blockIdx.x * CH;
   const int nchunks = (p.T + TC - 1) / TC;
+  SplitChain<CH> split;
+  if constexpr (SPLIT) split.init(reinterpret_cast<SplitSmem<CH>*>(smem + SM::OFF_SPLIT));
+  const int rank = SPLIT ? static_cast<int>(split.rank) : 0, nranks = SPLIT ? static_cast<int>(split.size) : 1;
+  const int rounds = SPLIT ? (nchunks + nranks - 1) / nranks : nchunks;
+  const int mine = SPLIT ? (nchunks - rank + nranks - 1) / nranks : nchunks;   // chunks this CTA loads and stores
 
-  auto issue = [&](int k) {
-    const int sidx = k % NSTAGE;
+  auto issue = [&](int it) {
+    const int sidx = it % NSTAGE, k = it * nranks + rank;
     uint8_t* st = smem + sidx * SM::STAGE;
     mbar_expect_tx(&bars[sidx], 2 * RAW_TILE);
     tma_load_3d(st, &maps.drive, d0, k * TC, b, &bars[sidx]);
     tma_load_3d(st + RAW_TILE, &maps.decay, d0, k * TC, b, &bars[sidx]);
   };
+  pdl_launch_dependents();
   if (USE_TMA) {
     if (tid == 0) {
       for (int s = 0; s < NSTAGE; ++s) mbar_init(&bars[s], 1);
+      if constexpr (SPLIT) { mbar_init(&split.sm->bar[0], 1); mbar_init(&split.sm->bar[1], 1); }
       mbar_fence_init();
     }
-    __syncthreads();
-    if (tid == 0)
-      for (int k = 0; k < NSTAGE && k < nchunks; ++k) issue(k);
+    if constexpr (SPLIT) cluster_sync_all();
+    else __syncthreads();
   }
+  pdl_wait();
+  if (USE_TMA && tid == 0)
+    for (int it = 0; it < NSTAGE && it < mine; ++it) issue(it);
   float carry = 0.0f;
   const int dch = d0 + tid;
   if (tid < CH && dch < p.D && p.h0) carry = p.h0[static_cast<size_t>(b) * p.D + dch];
   const int off0 = (lane_t * TS) * ROWB + vec * 16;
   bool alive = true;
 
-  for (int k = 0; k < nchunks; ++k) {
-    const int stage = USE_TMA ? (k % NSTAGE) : 0;
+  for (int it = 0; it < rounds; ++it) {
+    const int k = it * nranks + rank;
+    const bool idle = SPLIT && it >= mine;
+    if constexpr (SPLIT) { if (tid == 0) split.arm(it); }
+    const int stage = USE_TMA ? (it % NSTAGE) : 0;
     uint8_t* tiles = smem + stage * SM::STAGE;
     const int t0 = k * TC;
     if (USE_TMA) {
-      alive = mbar_wait_bounded(&bars[stage], (k / NSTAGE) & 1);
+      if (!idle && alive) alive = mbar_wait_bounded(&bars[stage], (it / NSTAGE) & 1);
     } else {
       tile_load_plain<float, CH>(tiles, p.drive, b, t0, d0, TC, p.T, p.D);
       tile_load_plain<float, CH>(tiles + RAW_TILE, p.decay, b, t0, d0, TC, p.T, p.D);
@@ -1243,23 +1462,13 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_fwd_kernel(const __grid_consta
       dst[1] = make_float4(P[TS - 1][1].x, S[TS - 1][1].x, P[TS - 1][1].y, S[TS - 1][1].y);
     }
     alive = __syncthreads_and(alive);
-    if (!alive) break;
-    if (tid < CH) {
-      float2 ag[LANES];
-#pragma unroll
-      for (int j = 0; j < LANES; ++j) ag[j] = agg[j * CH + tid];
-      float e = carry;
-#pragma unroll
-      for (int j = 0; j < LANES; ++j) {
-        ein[j * CH + tid] = e;
-        e = fmaf(ag[j].x, e, ag[j].y);
-      }
-      carry = e;
-    }
+    if (!SPLIT && !alive) break;
+    if (tid < CH) raw_chain<false, SPLIT>(agg, carry, split, it, idle, alive);
     __syncthreads();
+    if (idle) break;
     {
-      const float4 e4 = *reinterpret_cast<const float4*>(ein + lane_t * CH + vec * CV);
-      const float2 e[2] = {make_float2(e4.x, e4.y), make_float2(e4.z, e4.w)};
+      float2 e[2];
+      raw_entering(agg, lane_t * CH + vec * CV, e);
 #pragma unroll
       for (int st = 0; st < TS; ++st) {
         float2 yv[2];
@@ -1274,10 +1483,10 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_fwd_kernel(const __grid_consta
       if (tid == 0) {
         tma_store_3d(&maps.out, tiles, d0, t0, b);
         tma_commit();
-        const int kp = k - 1;
-        if (kp >= 0 && kp + NSTAGE < nchunks) {
+        const int prev = it - 1;
+        if (prev >= 0 && prev + NSTAGE < mine) {
           tma_wait_read<1>();
-          issue(kp + NSTAGE);
+          issue(prev + NSTAGE);
         }
       }
     } else {
@@ -1286,28 +1495,31 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_fwd_kernel(const __grid_consta
       __syncthreads();
     }
   }
-  if (USE_TMA && tid == 0) {
-    tma_wait_all<0>();
-    if (!alive) atomicExch(p.status, DEV_TIMEOUT_LOAD);
-  }
+  if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }     // no CTA leaves while another may still send to it
+  if (USE_TMA && tid == 0) tma_wait_all<0>();
+  if (USE_TMA && !alive && tid < CH) atomicExch(p.status, DEV_TIMEOUT_LOAD);
 }
 
 // Backward of the raw scan.  Tiles per chunk: d_out, decay, and the forward output
 // shifted one step back in time (row t holds h_{t-1}; the row before t = 0 is h0).
-template <int NSTAGE, bool USE_TMA>
+template <int NSTAGE, bool USE_TMA, bool SPLIT>
 __global__ void __launch_bounds__(RAW_NT) rawscan_bwd_kernel(const __grid_constant__ RawBwdMaps maps, const RawScanArgs p) {
-  using SM = RawSmem<NSTAGE>;
-  constexpr int TS = RAW_TS, TC = RAW_TC, ROWB = CH * 4, LANES = RAW_LANES;
+  using SM = RawSmem<NSTAGE, 3, SPLIT>;
+  constexpr int TS = RAW_TS, TC = RAW_TC, ROWB = CH * 4;
   extern __shared__ __align__(128) uint8_t smem[];
   float2* agg = reinterpret_cast<float2*>(smem + SM::OFF_AGG);
-  float* ein = reinterpret_cast<float*>(smem + SM::OFF_EIN);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::OFF_BAR);
   const int tid = threadIdx.x, lane_t = tid / NCV, vec = tid % NCV;
   const int b = blockIdx.y, d0 = blockIdx.x * CH;
   const int nchunks = (p.T + TC - 1) / TC;
+  SplitChain<CH> split;
+  if constexpr (SPLIT) split.init(reinterpret_cast<SplitSmem<CH>*>(smem + SM::OFF_SPLIT));
+  const int rank = SPLIT ? static_cast<int>(split.rank) : 0, nranks = SPLIT ? static_cast<int>(split.size) : 1;
+  const int rounds = SPLIT ? (nchunks + nranks - 1) / nranks : nchunks;
+  const int mine = SPLIT ? (nchunks - rank + nranks - 1) / nranks : nchunks;   // chunks this CTA loads and stores
 
   auto issue = [&](int q) {
-    const int k = nchunks - 1 - q;
+    const int k = nchunks - 1 - (q * nranks + rank);
     const int sidx = q % NSTAGE;
     uint8_t* st = smem + sidx * SM::STAGE;
     mbar_expect_tx(&bars[sidx], 3 * RAW_TILE);
@@ -1315,27 +1527,33 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_bwd_kernel(const __grid_consta
     tma_load_3d(st + RAW_TILE, &maps.decay, d0, k * TC, b, &bars[sidx]);
     tma_load_3d(st + 2 * RAW_TILE, &maps.out, d0, k * TC - 1, b, &bars[sidx]);
   };
+  pdl_launch_dependents();
   if (USE_TMA) {
     if (tid == 0) {
       for (int s = 0; s < NSTAGE; ++s) mbar_init(&bars[s], 1);
+      if constexpr (SPLIT) { mbar_init(&split.sm->bar[0], 1); mbar_init(&split.sm->bar[1], 1); }
       mbar_fence_init();
     }
-    __syncthreads();
-    if (tid == 0)
-      for (int q = 0; q < NSTAGE && q < nchunks; ++q) issue(q);
+    if constexpr (SPLIT) cluster_sync_all();
+    else __syncthreads();
   }
+  pdl_wait();
+  if (USE_TMA && tid == 0)
+    for (int it = 0; it < NSTAGE && it < mine; ++it) issue(it);
   float carry = 0.0f;  // a_t g_t flowing towards earlier steps
   const int dch = d0 + tid;
   const int off0 = (lane_t * TS) * ROWB + vec * 16;
   bool alive = true;
 
-  for (int q = 0; q < nchunks; ++q) {
-    const int k = nchunks - 1 - q;
+  for (int q = 0; q < rounds; ++q) {
+    const int k = nchunks - 1 - (q * nranks + rank);
+    const bool idle = SPLIT && q >= mine;
+    if constexpr (SPLIT) { if (tid == 0) split.arm(q); }
     const int stage = USE_TMA ? (q % NSTAGE) : 0;
     uint8_t* tiles = smem + stage * SM::STAGE;
     const int t0 = k * TC;
     if (USE_TMA) {
-      alive = mbar_wait_bounded(&bars[stage], (q / NSTAGE) & 1);
+      if (!idle && alive) alive = mbar_wait_bounded(&bars[stage], (q / NSTAGE) & 1);
     } else {
       tile_load_plain<float, CH>(tiles, p.dout, b, t0, d0, TC, p.T, p.D);
       tile_load_plain<float, CH>(tiles + RAW_TILE, p.decay, b, t0, d0, TC, p.T, p.D);
@@ -1373,23 +1591,13 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_bwd_kernel(const __grid_consta
       dst[1] = make_float4(qq[1].x, cc[1].x, qq[1].y, cc[1].y);
     }
     alive = __syncthreads_and(alive);
-    if (!alive) break;
-    if (tid < CH) {
-      float2 ag[LANES];
-#pragma unroll
-      for (int j = 0; j < LANES; ++j) ag[j] = agg[j * CH + tid];
-      float e = carry;
-#pragma unroll
-      for (int j = LANES - 1; j >= 0; --j) {
-        ein[j * CH + tid] = e;
-        e = fmaf(ag[j].x, e, ag[j].y);
-      }
-      carry = e;
-    }
+    if (!SPLIT && !alive) break;
+    if (tid < CH) raw_chain<true, SPLIT>(agg, carry, split, q, idle, alive);
     __syncthreads();
+    if (idle) break;
     {
-      const float4 e4 = *reinterpret_cast<const float4*>(ein + lane_t * CH + vec * CV);
-      float2 c[2] = {make_float2(e4.x, e4.y), make_float2(e4.z, e4.w)};
+      float2 c[2];
+      raw_entering(agg, lane_t * CH + vec * CV, c);
 #pragma unroll
       for (int st = TS - 1; st >= 0; --st) {
         float2 da[2], db[2];
@@ -1412,7 +1620,7 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_bwd_kernel(const __grid_consta
         tma_store_3d(&maps.ddecay, tiles + RAW_TILE, d0, t0, b);
         tma_commit();
         const int qp = q - 1;
-        if (qp >= 0 && qp + NSTAGE < nchunks) {
+        if (qp >= 0 && qp + NSTAGE < mine) {
           tma_wait_read<1>();
           issue(qp + NSTAGE);
         }
@@ -1424,11 +1632,10 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_bwd_kernel(const __grid_consta
       __syncthreads();
     }
   }
-  if (USE_TMA && tid == 0) {
-    tma_wait_all<0>();
-    if (!alive) atomicExch(p.status, DEV_TIMEOUT_LOAD);
-  }
-  if (alive && tid < CH && dch < p.D && p.dh0) p.dh0[static_cast<size_t>(b) * p.D + dch] = carry;
+  if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }     // no CTA leaves while another may still send to it
+  if (USE_TMA && tid == 0) tma_wait_all<0>();
+  if (USE_TMA && !alive && tid < CH) atomicExch(p.status, DEV_TIMEOUT_LOAD);
+  if (alive && rank == 0 && tid < CH && dch < p.D && p.dh0) p.dh0[static_cast<size_t>(b) * p.D + dch] = carry;
 }
 
 // ======================================================================
@@ -1803,15 +2010,16 @@ static int env_override(const char* name) {
   return (v && v[0] >= '0' && v[0] <= '9' && v[1] == 0) ? (v[0] - '0') : -1;
 }
 
-// Measured on B200 (bf16, T = 2048, D = 1024): half-width forward tiles win while 64-channel tiles cannot fill
-// the 148 SMs (B = 8, 128 tiles: 31 us against 50 us) and lose once they can (B = 16: 58 us against 52 us); for
-// fp32 the 64-channel shape is faster throughout.  The backward runs one CTA per SM either way; without the
+// Measured on B200 (T = 2048, D = 1024): half-width forward tiles win while 64-channel tiles cannot fill the 148 SMs
+// (bf16 B = 8, 128 tiles: 28 us against 48 us) and lose once they can (B = 16: 52 us against 50 us); for fp32, whose
+// stages leave one CTA per SM, they win as long as there is an SM for each of them (B = 4, 64 tiles: 25 us against 43;
+// B = 5: 47 against 44).  The backward runs one CTA per SM either way; without the
 // producer warp it is 1 to 2 % faster for bf16 tensors (eight warps leave every thread its registers).
 int scan_fwd_variant(int B, int T, int D, bool bf16) {
   static const int forced = env_override("RGLRU_FWD_VARIANT");
   if (fwd_variant_exists(forced)) return forced;
   const long long tiles = static_cast<long long>(B) * ((D + 63) / 64);
-  return (bf16 && tiles <= 160 && T >= 256) ? 2 : 0;
+  return (tiles <= (bf16 ? 160 : 74) && T >= 256) ? 2 : 0;
 }
 int scan_bwd_variant(int B, int T, int D, bool bf16) {
   static const int forced = env_override("RGLRU_BWD_VARIANT");
@@ -1822,18 +2030,25 @@ int scan_bwd_variant(int B, int T, int D, bool bf16) {
 
 // Launch with programmatic stream serialization, so that this kernel's launch and prologue may overlap
 // the tail of the kernel before it on the stream (the kernels call pdl_wait before touching memory).
+// `split` > 1 makes the grid's z axis the ranks of a cluster.
 template <typename Kern, typename Maps, typename Args>
-static cudaError_t launch_pdl(Kern kern, dim3 grid, int threads, int bytes, cudaStream_t s, const Maps& maps, const Args& a) {
+static cudaError_t launch_pdl(Kern kern, dim3 grid, int threads, int bytes, cudaStream_t s, const Maps& maps, const Args& a,
+                              int split = 1) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = bytes;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = static_cast<unsigned>(split);
+  if (split > 1) cfg.gridDim.z = static_cast<unsigned>(split);
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = split > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, maps, a);
 }
 
@@ -1857,21 +2072,106 @@ static cudaError_t set_smem(Kern kern, int bytes) {
 template <typename... Ts> struct KernelTag {};
 template <int... Vs> struct IntTag {};
 
+// One forward (backward) kernel instantiation with its launch shape.  Kern::get() is the kernel, prepared for its
+// dynamic shared memory.
+template <typename IO, typename V, int STAGES, bool USE_TMA, bool CONV = false, bool MERGE = false, bool GROUPED = false,
+          bool PLAIN = false, bool CARRY = false, bool PAIRED = false, bool SPLIT = false>
+struct FwdKern {
+  static constexpr int ST = USE_TMA ? STAGES : 1;
+  static constexpr bool CAPPED = USE_TMA && !CONV && (MERGE || GROUPED || SPLIT);
+  static constexpr int THREADS = V::LANES * (V::CH / CV) + (USE_TMA ? 32 : 0);
+  static constexpr int BYTES = FwdSmem<IO, V::TS, V::LANES, V::CH, ST, CONV, MERGE, SPLIT>::BYTES;
+  static constexpr int CH = V::CH;
+  static constexpr bool IS_SPLIT = SPLIT;
+  static_assert(BYTES <= 232448, "shared memory of one CTA");
+  using Fn = void (*)(FwdMaps, ScanFwdArgs);
+  static Fn get(cudaError_t& e) {
+    Fn kern;
+    if constexpr (CAPPED) kern = rglru_fwd_kernel_capped<IO, V::TS, V::LANES, V::CH, ST, USE_TMA, CONV, MERGE, GROUPED, PLAIN, SPLIT>;
+    else kern = rglru_fwd_kernel<IO, V::TS, V::LANES, V::CH, ST, USE_TMA, CONV, MERGE, GROUPED, PLAIN, CARRY, PAIRED, SPLIT>;
+    e = set_smem<FwdKern>(kern, BYTES);
+    return kern;
+  }
+};
+template <typename IO, typename V, int STAGES, bool USE_TMA, bool CONV = false, bool MERGE = false, bool GROUPED = false,
+          bool SELF_ISSUE = false, bool PLAIN = false, bool CARRY = false, bool SPLIT = false>
+struct BwdKern {
+  static constexpr int ST = USE_TMA ? STAGES : 1;
+  static constexpr int THREADS = V::LANES * (V::CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 32 : 0);
+  static constexpr int BYTES = BwdSmem<IO, V::TS, V::LANES, V::CH, ST, CONV, MERGE, SPLIT>::BYTES;
+  static constexpr int CH = V::CH;
+  static constexpr bool IS_SPLIT = SPLIT, IS_GROUPED = GROUPED;
+  static_assert(BYTES <= 232448, "shared memory of one CTA");
+  using Fn = void (*)(BwdMaps, ScanBwdArgs);
+  static Fn get(cudaError_t& e) {
+    Fn kern = rglru_bwd_kernel<IO, V::TS, V::LANES, V::CH, ST, USE_TMA, CONV, MERGE, GROUPED, SELF_ISSUE, PLAIN, CARRY, SPLIT>;
+    e = set_smem<BwdKern>(kern, BYTES);
+    return kern;
+  }
+};
+
+// Clusters of `size` CTAs of a kernel that fit on the device at once.  That depends on the chip's GPCs (a cluster
+// lives inside one), so the runtime is asked once per device, kernel (K) and size.
+template <typename K>
+static int resident_clusters(int size) {
+  static std::atomic<int> known[64][MAX_SPLIT + 1];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::atomic<int>& slot = known[dev][size];
+  int n = slot.load(std::memory_order_relaxed);      // 0: not asked yet; else the count + 1
+  if (n == 0) {
+    cudaError_t e;
+    auto kern = K::get(e);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, size);
+    cfg.blockDim = dim3(K::THREADS);
+    cfg.dynamicSmemBytes = K::BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = static_cast<unsigned>(size);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int count = 0;
+    if (e != cudaSuccess || cudaOccupancyMaxActiveClusters(&count, kern, &cfg) != cudaSuccess) count = 0;
+    n = count + 1;
+    slot.store(n, std::memory_order_relaxed);
+  }
+  return n - 1;
+}
+// Cluster size of the time split for `tiles` (batch row, channel tile) pairs: the largest that leaves every CTA a
+// chunk and all clusters resident at once, 1 if not even pairs do.  A round costs about a third more than an unsplit
+// chunk (the exchange through distributed shared memory), so a second wave of clusters gives the gain away again.
+// Measured on B200, T = 2048, D = 1024, bf16, forward / backward us, 64-channel tiles: 16 tiles unsplit 19 / 47, pairs
+// 23 / 32, six CTAs 11 / 16, eight (a second wave in the backward) 17 / 23; 64 tiles unsplit 26 / 48, pairs 24 / 34,
+// three 34 / 47.
+template <typename K>
+static int pick_split(long long tiles, int nchunks) {
+  for (int size = MAX_SPLIT; size > 1; --size)
+    if (size <= nchunks && tiles <= resident_clusters<K>(size)) return size;
+  return 1;
+}
+
+template <typename K>
+static cudaError_t launch_fwd(const FwdMaps& maps, const ScanFwdArgs& a, cudaStream_t s) {
+  cudaError_t e;
+  auto kern = K::get(e);
+  if (e != cudaSuccess) return e;
+  dim3 grid((a.D + K::CH - 1) / K::CH, a.B);
+  return launch_pdl(kern, grid, K::THREADS, K::BYTES, s, maps, a, K::IS_SPLIT ? a.split : 1);
+}
 template <typename IO, typename V, int STAGES, bool USE_TMA, bool CONV = false, bool MERGE = false, bool GROUPED = false,
           bool PLAIN = false, bool CARRY = false, bool PAIRED = false>
 static cudaError_t launch_fwd_t(const FwdMaps& maps, const ScanFwdArgs& a, cudaStream_t s) {
-  constexpr int ST = USE_TMA ? STAGES : 1;
-  constexpr bool CAPPED = USE_TMA && !CONV && (MERGE || GROUPED);
-  void (*kern)(FwdMaps, ScanFwdArgs);
-  if constexpr (CAPPED) kern = rglru_fwd_kernel_capped<IO, V::TS, V::LANES, V::CH, ST, USE_TMA, CONV, MERGE, GROUPED>;
-  else kern = rglru_fwd_kernel<IO, V::TS, V::LANES, V::CH, ST, USE_TMA, CONV, MERGE, GROUPED, PLAIN, CARRY, PAIRED>;
-  constexpr int bytes = FwdSmem<IO, V::TS, V::LANES, V::CH, ST, CONV, MERGE>::BYTES;
-  static_assert(bytes <= 232448, "shared memory of one CTA");
-  cudaError_t e = set_smem<KernelTag<FwdMaps, IO, V, IntTag<ST, USE_TMA, CONV, MERGE, GROUPED, PLAIN, CARRY, PAIRED>>>(kern, bytes);
-  if (e != cudaSuccess) return e;
-  dim3 grid((a.D + V::CH - 1) / V::CH, a.B);
-  return launch_pdl(kern, grid, V::LANES * (V::CH / CV) + (USE_TMA ? 32 : 0), bytes, s, maps, a);
+  return launch_fwd<FwdKern<IO, V, STAGES, USE_TMA, CONV, MERGE, GROUPED, PLAIN, CARRY, PAIRED>>(maps, a, s);
 }
+
+// The time-split kernels.  Three (merged: two) stages leave the bf16 forward small enough for two CTAs per SM.
+template <typename IO, bool PLAIN>
+using SplitFwd = FwdKern<IO, Shape64x16x4, 3, true, false, false, false, PLAIN, false, false, true>;
+template <typename IO, bool MERGE>
+using SplitGroupedFwd = FwdKern<IO, Shape64x16x4, MERGE ? 2 : 3, true, false, MERGE, true, false, false, false, true>;
 
 template <typename IO>
 static cudaError_t launch_fwd_io(bool use_tma, int variant, const FwdMaps& maps, const ScanFwdArgs& a, cudaStream_t s) {
@@ -1881,6 +2181,9 @@ static cudaError_t launch_fwd_io(bool use_tma, int variant, const FwdMaps& maps,
                    : launch_fwd_t<IO, Shape64x16x4, 1, false, false, false, false, false, true>(maps, a, s);
   if (!use_tma) return launch_fwd_t<IO, Shape64x16x4, 1, false>(maps, a, s);
   const bool plain = a.tok == nullptr && a.T % 128 == 0;   // no step of any chunk is masked
+  if (a.split > 1) {
+    return plain ? launch_fwd<SplitFwd<IO, true>>(maps, a, s) : launch_fwd<SplitFwd<IO, false>>(maps, a, s);
+  }
   if (plain && variant == 0) return launch_fwd_t<IO, Shape64x16x4, H ? 4 : 3, true, false, false, false, true>(maps, a, s);
   if (plain && variant == 2) {
     if constexpr (H) {   // 64-byte rows: the paired-row layout when the caller could encode its 5-D maps
@@ -1897,23 +2200,31 @@ cudaError_t launch_scan_fwd(bool bf16, bool use_tma, int variant, const FwdMaps&
   return bf16 ? launch_fwd_io<__nv_bfloat16>(use_tma, variant, maps, a, s) : launch_fwd_io<float>(use_tma, variant, maps, a, s);
 }
 
-template <typename IO, typename V, int STAGES, bool USE_TMA, bool CONV = false, bool MERGE = false, bool GROUPED = false,
-          bool SELF_ISSUE = false, bool PLAIN = false, bool CARRY = false>
-static cudaError_t launch_bwd_t(const BwdMaps& maps, const ScanBwdArgs& a, cudaStream_t s) {
-  constexpr int ST = USE_TMA ? STAGES : 1;
-  auto kern = rglru_bwd_kernel<IO, V::TS, V::LANES, V::CH, ST, USE_TMA, CONV, MERGE, GROUPED, SELF_ISSUE, PLAIN, CARRY>;
-  constexpr int bytes = BwdSmem<IO, V::TS, V::LANES, V::CH, ST, CONV, MERGE>::BYTES;
-  static_assert(bytes <= 232448, "shared memory of one CTA");
-  cudaError_t e = set_smem<KernelTag<BwdMaps, IO, V, IntTag<ST, USE_TMA, CONV, MERGE, GROUPED, SELF_ISSUE, PLAIN, CARRY>>>(kern, bytes);
+template <typename K>
+static cudaError_t launch_bwd(const BwdMaps& maps, const ScanBwdArgs& a, cudaStream_t s) {
+  cudaError_t e;
+  auto kern = K::get(e);
   if (e != cudaSuccess) return e;
-  dim3 grid((a.D + V::CH - 1) / V::CH, a.B);
-  e = launch_pdl(kern, grid, V::LANES * (V::CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 32 : 0), bytes, s, maps, a);
+  dim3 grid((a.D + K::CH - 1) / K::CH, a.B);
+  e = launch_pdl(kern, grid, K::THREADS, K::BYTES, s, maps, a, K::IS_SPLIT ? a.split : 1);
   if (e != cudaSuccess || a.ticket || !a.dlambda) return e;
   rglru_dlambda_kernel<<<(a.D + 255) / 256, 256, 0, s>>>(a.dlam_part, a.lambda, a.dlambda, a.B, a.D, a.c);
-  if (GROUPED && a.dgate && a.dgate_part)
+  if (K::IS_GROUPED && a.dgate && a.dgate_part)
     rglru_colsum_kernel<<<(2 * a.D + 255) / 256, 256, 0, s>>>(a.dgate_part, a.dgate, a.B, 2 * a.D);
   return cudaGetLastError();
 }
+
+template <typename IO, typename V, int STAGES, bool USE_TMA, bool CONV = false, bool MERGE = false, bool GROUPED = false,
+          bool SELF_ISSUE = false, bool PLAIN = false, bool CARRY = false>
+static cudaError_t launch_bwd_t(const BwdMaps& maps, const ScanBwdArgs& a, cudaStream_t s) {
+  return launch_bwd<BwdKern<IO, V, STAGES, USE_TMA, CONV, MERGE, GROUPED, SELF_ISSUE, PLAIN, CARRY>>(maps, a, s);
+}
+
+template <typename IO, bool PLAIN>
+using SplitBwd = BwdKern<IO, Shape64x16x4, sizeof(IO) == 2 ? 5 : 3, true, false, false, false, sizeof(IO) == 2, PLAIN, false, true>;
+template <typename IO, bool MERGE>
+using SplitGroupedBwd = BwdKern<IO, Shape64x16x4, sizeof(IO) == 2 ? (MERGE ? 4 : 5) : (MERGE ? 2 : 3), true, false, MERGE, true,
+                                sizeof(IO) == 2 && !MERGE, false, false, true>;
 
 template <typename IO>
 static cudaError_t launch_bwd_io(bool use_tma, int variant, const BwdMaps& maps, const ScanBwdArgs& a, cudaStream_t s) {
@@ -1923,6 +2234,9 @@ static cudaError_t launch_bwd_io(bool use_tma, int variant, const BwdMaps& maps,
                    : launch_bwd_t<IO, Shape64x16x4, 1, false, false, false, false, false, false, true>(maps, a, s);
   if (!use_tma) return launch_bwd_t<IO, Shape64x16x4, 1, false>(maps, a, s);
   const bool plain = a.tok == nullptr && a.T % 64 == 0;   // no step of any chunk is masked
+  if (a.split > 1) {
+    return plain ? launch_bwd<SplitBwd<IO, true>>(maps, a, s) : launch_bwd<SplitBwd<IO, false>>(maps, a, s);
+  }
   if (variant == 3) {   // bulk copies issued by a compute thread: loads run NSTAGE - 2 chunks ahead, so one more stage
     if (plain) return launch_bwd_t<IO, Shape64x16x4, H ? 5 : 3, true, false, false, false, true, true>(maps, a, s);
     return launch_bwd_t<IO, Shape64x16x4, H ? 5 : 3, true, false, false, false, true>(maps, a, s);
@@ -1985,7 +2299,9 @@ cudaError_t launch_merge_bwd(bool bf16, bool use_tma, bool conv, const BwdMaps& 
 template <typename IO, bool MERGE>
 static cudaError_t launch_grouped_fwd_t(const FwdMaps& maps, const ScanFwdArgs& a, cudaStream_t s) {
   constexpr bool H = sizeof(IO) == 2;
-  return launch_fwd_t<IO, Shape64x16x4, H ? (MERGE ? 3 : 4) : 3, true, false, MERGE, true>(maps, a, s);
+  constexpr int ST = H ? (MERGE ? 3 : 4) : 3;
+  if (a.split > 1) return launch_fwd<SplitGroupedFwd<IO, MERGE>>(maps, a, s);
+  return launch_fwd_t<IO, Shape64x16x4, ST, true, false, MERGE, true>(maps, a, s);
 }
 template <typename IO, bool MERGE>
 static cudaError_t launch_grouped_bwd_t(const BwdMaps& maps, const ScanBwdArgs& a, cudaStream_t s) {
@@ -1993,8 +2309,10 @@ static cudaError_t launch_grouped_bwd_t(const BwdMaps& maps, const ScanBwdArgs& 
   // Measured on B200 at B = 16, T = 2048, D = 1024 bf16: with the branch merge (five loads and four stores per
   // chunk) the producer warp wins although the kernel then spills a little at its 168-register limit (162 us
   // against 169 us with the copies issued by a compute thread); without the merge the compute-thread variant does.
-  if constexpr (H && !MERGE) return launch_bwd_t<IO, Shape64x16x4, 5, true, false, false, true, true>(maps, a, s);
-  else return launch_bwd_t<IO, Shape64x16x4, H ? 4 : (MERGE ? 2 : 3), true, false, MERGE, true>(maps, a, s);
+  constexpr bool SELF = H && !MERGE;
+  constexpr int ST = SELF ? 5 : (H ? 4 : (MERGE ? 2 : 3));
+  if (a.split > 1) return launch_bwd<SplitGroupedBwd<IO, MERGE>>(maps, a, s);
+  return launch_bwd_t<IO, Shape64x16x4, ST, true, false, MERGE, true, SELF>(maps, a, s);
 }
 cudaError_t launch_grouped_fwd(bool bf16, bool merge, const FwdMaps& maps, const ScanFwdArgs& a, cudaStream_t s) {
   if (bf16) return merge ? launch_grouped_fwd_t<__nv_bfloat16, true>(maps, a, s) : launch_grouped_fwd_t<__nv_bfloat16, false>(maps, a, s);
@@ -2006,34 +2324,74 @@ cudaError_t launch_grouped_bwd(bool bf16, bool merge, const BwdMaps& maps, const
 }
 int grouped_box_cols() { return Shape64x16x4::CH; }
 
+// CTAs that share one (batch row, channel tile) along time in a call of this shape, 1 for none (see pick_split).  The
+// plain forward has the 32-channel shape to fall back on, which fills the machine twice as well as 64-channel tiles:
+// pairs of CTAs do not beat it, three or more do (bf16, T = 2048, D = 1024, unsplit 32-channel / split: B = 6 27 / 33 us
+// in pairs, B = 5 27 / 25 us in threes, B = 1 19 / 11 us in eights; fp32 B = 4 25 / 31 in pairs, B = 2 24 / 18 in fours).
+template <bool MERGE, bool GROUPED>
+static int split_of(bool fwd, bool bf16, int B, int T, int D) {
+  const long long tiles = static_cast<long long>(B) * ((D + 63) / 64);
+  const int nchunks = (T + 63) / 64;
+  using H = __nv_bfloat16;
+  if constexpr (GROUPED) {
+    if (fwd) return bf16 ? pick_split<SplitGroupedFwd<H, MERGE>>(tiles, nchunks) : pick_split<SplitGroupedFwd<float, MERGE>>(tiles, nchunks);
+    return bf16 ? pick_split<SplitGroupedBwd<H, MERGE>>(tiles, nchunks) : pick_split<SplitGroupedBwd<float, MERGE>>(tiles, nchunks);
+  } else {
+    if (fwd) return bf16 ? pick_split<SplitFwd<H, false>>(tiles, nchunks) : pick_split<SplitFwd<float, false>>(tiles, nchunks);
+    return bf16 ? pick_split<SplitBwd<H, false>>(tiles, nchunks) : pick_split<SplitBwd<float, false>>(tiles, nchunks);
+  }
+}
+int scan_split(bool fwd, bool bf16, int B, int T, int D) {
+  static const bool forced = fwd_variant_exists(env_override("RGLRU_FWD_VARIANT")) || bwd_variant_exists(env_override("RGLRU_BWD_VARIANT"));
+  if (forced) return 1;
+  const int split = split_of<false, false>(fwd, bf16, B, T, D);
+  return fwd && split < 3 ? 1 : split;      // see scan_fwd_variant
+}
+int grouped_split(bool fwd, bool bf16, bool merge, int B, int T, int D) {
+  return merge ? split_of<true, true>(fwd, bf16, B, T, D) : split_of<false, true>(fwd, bf16, B, T, D);
+}
+
 int raw_box_rows() { return RAW_TC; }
 int raw_box_cols() { return CH; }
 
-template <int NSTAGE, bool USE_TMA>
-static cudaError_t launch_raw_fwd_t(const RawFwdMaps& maps, const RawScanArgs& a, cudaStream_t s) {
-  auto kern = rawscan_fwd_kernel<NSTAGE, USE_TMA>;
-  constexpr int bytes = RawSmem<NSTAGE>::BYTES;
-  cudaError_t e = set_smem<KernelTag<RawFwdMaps, IntTag<NSTAGE, USE_TMA>>>(kern, bytes);
+template <int NSTAGE, bool USE_TMA, bool SPLIT>
+struct RawFwdKern {
+  static constexpr int THREADS = RAW_NT, BYTES = RawSmem<NSTAGE, 2, SPLIT>::BYTES;
+  using Fn = void (*)(RawFwdMaps, RawScanArgs);
+  static Fn get(cudaError_t& e) {
+    Fn kern = rawscan_fwd_kernel<NSTAGE, USE_TMA, SPLIT>;
+    e = set_smem<RawFwdKern>(kern, BYTES);
+    return kern;
+  }
+};
+template <int NSTAGE, bool USE_TMA, bool SPLIT>
+struct RawBwdKern {
+  static constexpr int THREADS = RAW_NT, BYTES = RawSmem<NSTAGE, 3, SPLIT>::BYTES;
+  using Fn = void (*)(RawBwdMaps, RawScanArgs);
+  static Fn get(cudaError_t& e) {
+    Fn kern = rawscan_bwd_kernel<NSTAGE, USE_TMA, SPLIT>;
+    e = set_smem<RawBwdKern>(kern, BYTES);
+    return kern;
+  }
+};
+template <typename K, typename Maps>
+static cudaError_t launch_raw(const Maps& maps, const RawScanArgs& a, int split, cudaStream_t s) {
+  cudaError_t e;
+  auto kern = K::get(e);
   if (e != cudaSuccess) return e;
-  dim3 grid((a.D + CH - 1) / CH, a.B);
-  kern<<<grid, RAW_NT, bytes, s>>>(maps, a);
-  return cudaGetLastError();
+  return launch_pdl(kern, dim3((a.D + CH - 1) / CH, a.B), K::THREADS, K::BYTES, s, maps, a, split);
 }
 cudaError_t launch_raw_fwd(bool use_tma, const RawFwdMaps& maps, const RawScanArgs& a, cudaStream_t s) {
-  return use_tma ? launch_raw_fwd_t<3, true>(maps, a, s) : launch_raw_fwd_t<1, false>(maps, a, s);
-}
-template <int NSTAGE, bool USE_TMA>
-static cudaError_t launch_raw_bwd_t(const RawBwdMaps& maps, const RawScanArgs& a, cudaStream_t s) {
-  auto kern = rawscan_bwd_kernel<NSTAGE, USE_TMA>;
-  constexpr int bytes = RawSmem<NSTAGE>::BYTES;
-  cudaError_t e = set_smem<KernelTag<RawBwdMaps, IntTag<NSTAGE, USE_TMA>>>(kern, bytes);
-  if (e != cudaSuccess) return e;
-  dim3 grid((a.D + CH - 1) / CH, a.B);
-  kern<<<grid, RAW_NT, bytes, s>>>(maps, a);
-  return cudaGetLastError();
+  if (!use_tma) return launch_raw<RawFwdKern<1, false, false>>(maps, a, 1, s);
+  using Split = RawFwdKern<RAW_STAGES, true, true>;
+  const int split = pick_split<Split>(static_cast<long long>(a.B) * ((a.D + CH - 1) / CH), (a.T + RAW_TC - 1) / RAW_TC);
+  return split > 1 ? launch_raw<Split>(maps, a, split, s) : launch_raw<RawFwdKern<RAW_STAGES, true, false>>(maps, a, 1, s);
 }
 cudaError_t launch_raw_bwd(bool use_tma, const RawBwdMaps& maps, const RawScanArgs& a, cudaStream_t s) {
-  return use_tma ? launch_raw_bwd_t<3, true>(maps, a, s) : launch_raw_bwd_t<1, false>(maps, a, s);
+  if (!use_tma) return launch_raw<RawBwdKern<1, false, false>>(maps, a, 1, s);
+  using Split = RawBwdKern<RAW_STAGES, true, true>;
+  const int split = pick_split<Split>(static_cast<long long>(a.B) * ((a.D + CH - 1) / CH), (a.T + RAW_TC - 1) / RAW_TC);
+  return split > 1 ? launch_raw<Split>(maps, a, split, s) : launch_raw<RawBwdKern<RAW_STAGES, true, false>>(maps, a, 1, s);
 }
 
 int conv_tma_box_rows() { return 64 + 3; }
