@@ -52,6 +52,8 @@ SIGNATURES = {
     "rglru_column_sums": (_i, [_vp, _vp, _vp, _sz, ctypes.c_longlong, _i, _i, _vp]),
     "rglru_decode_conv": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]),
     "rglru_decode_step": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _f, _i, _vp]),
+    "rglru_decode_block_workspace_bytes": (_sz, [_i, _i, _i]),
+    "rglru_decode_block": (_i, [_vp] * 19 + [_sz, _i, _i, _i, _f, _i, _i, _vp]),
 }
 
 _lock = threading.Lock()

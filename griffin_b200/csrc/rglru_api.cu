@@ -814,4 +814,46 @@ int rglru_decode_step(const void* x, const void* u_r, const void* u_i, const flo
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
 }
 
+size_t rglru_decode_block_workspace_bytes(int B, int D, int io_dtype) {
+  if (B <= 0 || D <= 0 || (io_dtype != RGLRU_F32 && io_dtype != RGLRU_BF16)) return 0;
+  return static_cast<size_t>(B) * D * (io_dtype == RGLRU_BF16 ? 2 : 4) + B;
+}
+
+int rglru_decode_block(const void* x_in, const void* branch, const void* conv_w, const void* conv_b, const void* conv_in,
+                       void* conv_out, const void* w_r, const void* b_r, const void* w_i, const void* b_i,
+                       const void* lambda, const float* h_in, float* h_out, const int64_t* prev_pos,
+                       const int64_t* seg_pos, const uint8_t* active, int64_t* pos_out, void* y, void* ws,
+                       size_t ws_bytes, int B, int D, int gate_width, float c, int io_dtype, int f32_params,
+                       void* stream) {
+  if (io_dtype != RGLRU_F32 && io_dtype != RGLRU_BF16) return RGLRU_ERR_BAD_DTYPE;
+  if (!x_in || !conv_w || !conv_in || !conv_out || !w_r || !b_r || !w_i || !b_i || !lambda || !h_in || !h_out ||
+      !prev_pos || !pos_out || !y)
+    return RGLRU_ERR_NULL_POINTER;
+  const bool bf16 = io_dtype == RGLRU_BF16;
+  const size_t es = bf16 ? 2 : 4;
+  if (B <= 0 || D <= 0 || gate_width <= 0 || D % gate_width != 0 || (gate_width * es) % 16 != 0 || B > 1000000)
+    return RGLRU_ERR_BAD_SHAPE;
+  if (!aligned(x_in, 16) || !aligned(branch, 16) || !aligned(conv_in, 16) || !aligned(conv_out, 16) || !aligned(w_r, 16) ||
+      !aligned(w_i, 16) || !aligned(h_in, 16) || !aligned(h_out, 16) || !aligned(y, 16) || !aligned(ws, 16) ||
+      !aligned(prev_pos, 8) || !aligned(seg_pos, 8) || !aligned(pos_out, 8) || !aligned(conv_w, 16) || !aligned(conv_b, es) ||
+      !aligned(b_r, es) || !aligned(b_i, es) || !aligned(lambda, es))
+    return RGLRU_ERR_MISALIGNED;
+  if (!ws || ws_bytes < rglru_decode_block_workspace_bytes(B, D, io_dtype)) return RGLRU_ERR_WORKSPACE;
+  int* status = nullptr;
+  const int rc = device_setup(&status);
+  if (rc != RGLRU_OK) return rc;
+  DecodeBlockArgs a = {};
+  a.x_in = x_in; a.branch = branch; a.conv_w = conv_w; a.conv_b = conv_b; a.conv_in = conv_in; a.conv_out = conv_out;
+  a.w_r = w_r; a.b_r = b_r; a.w_i = w_i; a.b_i = b_i; a.lambda = lambda; a.h_in = h_in; a.h_out = h_out;
+  a.prev_pos = reinterpret_cast<const long long*>(prev_pos); a.seg_pos = reinterpret_cast<const long long*>(seg_pos);
+  a.active = active; a.pos_out = reinterpret_cast<long long*>(pos_out); a.y = y;
+  a.x_conv = ws; a.tok = static_cast<uint8_t*>(ws) + static_cast<size_t>(B) * D * es;
+  a.B = B; a.D = D; a.bw = gate_width; a.c = c;
+  a.f32_conv_w = !bf16 || (f32_params & RGLRU_F32_CONV_W);
+  a.f32_conv_b = !bf16 || (f32_params & RGLRU_F32_CONV_B);
+  a.f32_lambda = !bf16 || (f32_params & RGLRU_F32_LAMBDA);
+  const cudaError_t e = launch_decode_block(bf16, a, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
+}
+
 }  // extern "C"

@@ -1,0 +1,406 @@
+// One cached token of the recurrent block between its input projections and its output projection, in two launches:
+//
+//   decode_front_kernel   token flags from the positions, the width-4 conv, the next conv state and position;
+//   decode_gates_kernel   both block-diagonal gate projections, the RG-LRU update, and the product with the GeLU branch.
+//
+// Done operator by operator this is some twenty-five launches (flag arithmetic, state clones, weight casts, two batched
+// GEMMs with a re-layout each, the update, GeLU, the product), which for a token is nearly all launch cost: a block
+// call took 328 us at B = 1, D = 1024 (60 us of device time) and 348 us at B = 512, D = 5632 (217 us), bf16; it now takes
+// 112 (18) and 119 us (109, of which 63 in the three projections).  The conv stays a
+// kernel of its own because every channel slice of a gate head contracts over the whole head: folded in, it would be
+// redone by each of the head's slices (eleven of them at 352 channels).
+//
+// Reference behaviour: griffin/griffin.py:129-154 (gates), :237-258 (update), :309-358 (positions), :459-528 at T = 1.
+
+#include <atomic>
+
+#include "rglru_internal.h"
+#include "rglru_vec.cuh"
+
+namespace rglru {
+
+// A small parameter in the activation type or in fp32.
+template <typename IO>
+__device__ __forceinline__ float load_param(const void* p, size_t i, bool f32) {
+  return f32 ? static_cast<const float*>(p)[i] : Pack<IO>::to_float(static_cast<const IO*>(p)[i]);
+}
+
+// The four taps of VEC channels from d on ([D, 4] row-major), by 16-byte loads: w[k][v] = weight[d + v, k].
+template <typename P, int VEC>
+__device__ __forceinline__ void load_taps_of(const void* weight, int d, float (&w)[CONV_TAPS][VEC]) {
+  constexpr int PV = vec_width<P>(), CHANNELS = PV / CONV_TAPS;     // channels per load
+#pragma unroll
+  for (int v = 0; v < VEC; v += CHANNELS) {
+    float t[PV];
+    Vec<P, PV>::load(static_cast<const P*>(weight) + static_cast<size_t>(d + v) * CONV_TAPS, t);
+#pragma unroll
+    for (int j = 0; j < PV; ++j) w[j % CONV_TAPS][v + j / CONV_TAPS] = t[j];
+  }
+}
+
+// ---------------------------------------------------------------- conv, flags, positions
+// Thread = VEC channels of ROWS consecutive batch rows, so that the taps are fetched once for all of them and the
+// loads of all rows are in flight together (four 16-byte loads a row).
+constexpr int FRONT_THREADS = 128;
+
+template <typename IO, int ROWS>
+__global__ void __launch_bounds__(FRONT_THREADS) decode_front_kernel(const DecodeBlockArgs p) {
+  constexpr int VEC = vec_width<IO>();
+  using V = Vec<IO, VEC>;
+  pdl_launch_dependents();      // the gate kernel may start fetching its weights
+  // Padding anywhere in the batch changes what a new document's first token leaves in the conv state.
+  int padding = 0;
+  if (p.active)
+    for (int b = threadIdx.x; b < p.B; b += FRONT_THREADS) padding |= p.active[b] == 0;
+  const bool padded = p.active && __syncthreads_or(padding);
+
+  const int nvec = p.D / VEC;
+  const int vec = blockIdx.x * FRONT_THREADS + threadIdx.x;
+  if (vec >= nvec) return;
+  const int d = vec * VEC;
+  const int b0 = blockIdx.y * ROWS;
+  const IO* x = static_cast<const IO*>(p.x_in);
+  const IO* cin = static_cast<const IO*>(p.conv_in);
+  IO* cout = static_cast<IO*>(p.conv_out);
+
+  typename V::Raw cur[ROWS], hist[ROWS][3];
+  long long prev[ROWS], seg[ROWS];
+  bool act[ROWS];
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q) {
+    const int b = min(b0 + q, p.B - 1);
+    const IO* st = cin + static_cast<size_t>(b) * 3 * p.D + d;
+    cur[q] = V::load_raw(x + static_cast<size_t>(b) * p.D + d);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) hist[q][k] = V::load_raw(st + static_cast<size_t>(k) * p.D);
+    prev[q] = p.prev_pos[b];
+    seg[q] = p.seg_pos ? p.seg_pos[b] : 0;
+    act[q] = p.active ? p.active[b] != 0 : true;
+  }
+  float w[CONV_TAPS][VEC], bias[VEC];
+  if (p.f32_conv_w) load_taps_of<float, VEC>(p.conv_w, d, w);
+  else load_taps_of<IO, VEC>(p.conv_w, d, w);
+#pragma unroll
+  for (int v = 0; v < VEC; ++v) bias[v] = p.conv_b ? load_param<IO>(p.conv_b, d + v, p.f32_conv_b) : 0.0f;
+
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q) {
+    const int b = b0 + q;
+    if (b >= p.B) break;
+    const long long pos = p.seg_pos ? seg[q] : prev[q] + (act[q] ? 1 : 0);
+    const int reach = pos < 0 ? 0 : (pos > 3 ? 3 : static_cast<int>(pos));    // earlier tokens of this document within the taps
+    const bool wipe = padded && act[q] && pos == 0;
+    if (vec == 0) {
+      p.tok[b] = static_cast<uint8_t>((pos == 0 ? TOK_RESET : 0u) | (act[q] ? 0u : TOK_INACTIVE));
+      p.pos_out[b] = act[q] ? pos : prev[q];
+    }
+    float xv[VEC], s0[VEC], s1[VEC], s2[VEC], out[VEC];
+    V::unpack(cur[q], xv);
+    V::unpack(hist[q][0], s0);
+    V::unpack(hist[q][1], s1);
+    V::unpack(hist[q][2], s2);
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) {
+      float a = fmaf(w[3][v], xv[v], bias[v]);
+      if (reach >= 1) a = fmaf(w[2][v], s2[v], a);
+      if (reach >= 2) a = fmaf(w[1][v], s1[v], a);
+      if (reach >= 3) a = fmaf(w[0][v], s0[v], a);
+      out[v] = act[q] ? a : 0.0f;
+      if (wipe) { s1[v] = 0.0f; s2[v] = 0.0f; }
+    }
+    V::store(static_cast<IO*>(p.x_conv) + static_cast<size_t>(b) * p.D + d, out);
+    IO* st = cout + static_cast<size_t>(b) * 3 * p.D + d;
+    V::store(st, act[q] ? s1 : s0);
+    V::store(st + p.D, act[q] ? s2 : s1);
+    V::store(st + 2 * static_cast<size_t>(p.D), act[q] ? xv : s2);
+  }
+}
+
+// ---------------------------------------------------------------- gate projections and update
+// CTA = (MT batch rows) x (32 channels of one gate head): a [MT, bw] x [bw, 64] product, the 64 columns being the
+// recurrence and the input gate of the same channels, then the update of those channels.  Both operands are staged
+// by cp.async, 128 bytes of the contracted axis per row and stage, rows 144 bytes apart (conflict-free for ldmatrix and
+// for 16-byte loads).  bf16 contracts on mma.sync (a CTA has 64 columns and at most 64 rows, and its time is that of
+// its loads: the tile is too small for a tensor-memory accumulator to pay), fp32 on the FMA pipe in full precision.
+// The first stages' weights, which the kernel in front does not write, are requested before the dependency wait.
+constexpr int GATE_CH = 32;
+constexpr int GATE_COLS = 2 * GATE_CH;
+constexpr int GATE_THREADS = 128;
+constexpr int GATE_ROW = 144;            // bytes between staged rows
+constexpr int GATE_U = GATE_COLS + 4;    // floats between rows of the pre-activations
+
+template <int MT>
+struct GateSmem {
+  static constexpr int STAGES = MT == 64 ? 3 : 4;
+  static constexpr int STAGE = (MT + GATE_COLS) * GATE_ROW;
+  static constexpr int U = MT * GATE_U * 4;
+  static constexpr int BYTES = STAGES * STAGE > U ? STAGES * STAGE : U;
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool ok) {   // zero-filled where not ok
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void ldmatrix4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+template <typename IO, int MT>
+__global__ void __launch_bounds__(GATE_THREADS, sizeof(IO) == 2 ? 4 : 3) decode_gates_kernel(const DecodeBlockArgs p) {
+  using SM = GateSmem<MT>;
+  constexpr bool HALF = sizeof(IO) == 2;
+  constexpr int KC = 128 / sizeof(IO);             // contracted elements per stage
+  extern __shared__ __align__(128) uint8_t smem[];
+  const uint32_t sbase = smem_u32(smem);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int slices = (p.bw + GATE_CH - 1) / GATE_CH;
+  const int head = blockIdx.x / slices, n0 = (blockIdx.x % slices) * GATE_CH;
+  const int b0 = blockIdx.y * MT;
+  const int nk = (p.bw + KC - 1) / KC;
+  const size_t head_w = static_cast<size_t>(head) * p.bw * p.bw;
+  const IO* wr = static_cast<const IO*>(p.w_r) + head_w;
+  const IO* wi = static_cast<const IO*>(p.w_i) + head_w;
+  const IO* xc = static_cast<const IO*>(p.x_conv) + static_cast<size_t>(head) * p.bw;
+
+  auto load_w = [&](int it) {
+    const uint32_t dst = sbase + (it % SM::STAGES) * SM::STAGE + MT * GATE_ROW;
+#pragma unroll
+    for (int i = 0; i < GATE_COLS * 8 / GATE_THREADS; ++i) {
+      const int idx = tid + i * GATE_THREADS, row = idx >> 3, ch = idx & 7;
+      const int n = n0 + (row & (GATE_CH - 1)), k = it * KC + ch * (16 / static_cast<int>(sizeof(IO)));
+      const bool ok = n < p.bw && k < p.bw;
+      const IO* src = (row < GATE_CH ? wr : wi) + (ok ? static_cast<size_t>(n) * p.bw + k : 0);
+      cp_async16(dst + row * GATE_ROW + ch * 16, src, ok);
+    }
+  };
+  auto load_x = [&](int it) {
+    const uint32_t dst = sbase + (it % SM::STAGES) * SM::STAGE;
+#pragma unroll
+    for (int i = 0; i < MT * 8 / GATE_THREADS; ++i) {
+      const int idx = tid + i * GATE_THREADS, row = idx >> 3, ch = idx & 7;
+      const int b = b0 + row, k = it * KC + ch * (16 / static_cast<int>(sizeof(IO)));
+      const bool ok = b < p.B && k < p.bw;
+      cp_async16(dst + row * GATE_ROW + ch * 16, xc + (ok ? static_cast<size_t>(b) * p.D + k : 0), ok);
+    }
+  };
+
+#pragma unroll
+  for (int s = 0; s < SM::STAGES - 1; ++s)
+    if (s < nk) load_w(s);
+
+  // What the update needs beside the projections and the conv output is fetched here, ahead of the contraction: a thread
+  // owns VEC channels of every ROW_STEP-th row.
+  constexpr int VEC = vec_width<IO>();
+  constexpr int CVECS = GATE_CH / VEC, ROW_STEP = GATE_THREADS / CVECS, ROWS = (MT + ROW_STEP - 1) / ROW_STEP;
+  using V = Vec<IO, VEC>;
+  const int cv = (tid % CVECS) * VEC;
+  const bool mine = n0 + cv < p.bw;                // bw is a multiple of VEC
+  const int d = head * p.bw + (mine ? n0 + cv : 0);
+  float rate[VEC];                                 // -c * logsigmoid(Lambda)
+  float kmax = 0.0f;
+#pragma unroll
+  for (int v = 0; v < VEC; ++v) {
+    const float lam = load_param<IO>(p.lambda, d + v, p.f32_lambda);
+    rate[v] = p.c * (lam >= 0.0f ? log1pf(expf(-lam)) : log1pf(expf(lam)) - lam);
+    kmax = fmaxf(kmax, rate[v]);
+  }
+  const bool poly = kmax <= -POLY_RANGE;
+  float hv[ROWS][VEC];
+  typename V::Raw graw[ROWS];
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q) {
+    const size_t at = static_cast<size_t>(min(b0 + tid / CVECS + q * ROW_STEP, p.B - 1)) * p.D + d;
+#pragma unroll
+    for (int v = 0; v < VEC; v += 4) {
+      const float4 t4 = *reinterpret_cast<const float4*>(p.h_in + at + v);
+      hv[q][v] = t4.x; hv[q][v + 1] = t4.y; hv[q][v + 2] = t4.z; hv[q][v + 3] = t4.w;
+    }
+    if (p.branch) graw[q] = V::load_raw(static_cast<const IO*>(p.branch) + at);
+  }
+
+  pdl_wait();
+#pragma unroll
+  for (int s = 0; s < SM::STAGES - 1; ++s) {
+    if (s < nk) load_x(s);
+    cp_async_commit();
+  }
+
+  constexpr int NT = MT == 64 ? 8 : 2;             // bf16: 8-column tiles per warp
+  constexpr int RQ = MT / 8;                       // fp32: rows per thread (of four columns)
+  float acc[HALF ? NT : RQ][4];
+#pragma unroll
+  for (int i = 0; i < (HALF ? NT : RQ); ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+
+  for (int it = 0; it < nk; ++it) {
+    cp_async_wait<SM::STAGES - 2>();
+    __syncthreads();                               // stage `it` is there for all, and all are done with the one refilled next
+    if (it + SM::STAGES - 1 < nk) { load_w(it + SM::STAGES - 1); load_x(it + SM::STAGES - 1); }
+    cp_async_commit();
+    const uint32_t sa = sbase + (it % SM::STAGES) * SM::STAGE;
+    if constexpr (HALF) {
+      const uint32_t arow = sa + ((MT == 64 ? warp * 16 : 0) + (lane & 15)) * GATE_ROW + (lane >> 4) * 16;
+      // weight tiles two at a time: lanes 0-15 address the first tile's rows (both 16-byte halves of 16 k), 16-31 the second's
+      const uint32_t brow = sa + MT * GATE_ROW + (lane & 7) * GATE_ROW + ((lane >> 3) & 1) * 16;
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        uint32_t a[4];
+        ldmatrix4(arow + kk * 32, a);
+#pragma unroll
+        for (int j = 0; j < NT; j += 2) {
+          // tiles j and j + 1; with one row of warps (MT = 16) a warp has 8 channels: tile 0 their r, tile 1 their i columns
+          const int col = MT == 64 ? (j + (lane >> 4)) * 8 : (lane >> 4) * GATE_CH + warp * 8;
+          uint32_t w[4];
+          ldmatrix4(brow + col * GATE_ROW + kk * 32, w);
+          mma_bf16(acc[j], a, w[0], w[1]);
+          mma_bf16(acc[j + 1], a, w[2], w[3]);
+        }
+      }
+    } else {
+      const int cg = tid & 15, rg = tid >> 4;
+      const uint8_t* ta = smem + (it % SM::STAGES) * SM::STAGE + rg * GATE_ROW;
+      const uint8_t* tb = smem + (it % SM::STAGES) * SM::STAGE + (MT + cg) * GATE_ROW;
+#pragma unroll 4
+      for (int k4 = 0; k4 < 8; ++k4) {
+        float4 w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const float4*>(tb + 16 * j * GATE_ROW + k4 * 16);
+#pragma unroll
+        for (int q = 0; q < RQ; ++q) {
+          const float4 a = *reinterpret_cast<const float4*>(ta + 8 * q * GATE_ROW + k4 * 16);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            acc[q][j] = fmaf(a.w, w[j].w, fmaf(a.z, w[j].z, fmaf(a.y, w[j].y, fmaf(a.x, w[j].x, acc[q][j]))));
+        }
+      }
+    }
+  }
+  cp_async_wait<0>();
+  __syncthreads();                                 // the stages are free: the pre-activations take their place
+  float* us = reinterpret_cast<float*>(smem);      // [MT][GATE_U]: r columns 0 .. 31, i columns 32 .. 63
+  if constexpr (HALF) {
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      const int row = (MT == 64 ? warp * 16 : 0) + (lane >> 2);
+      const int col = (MT == 64 ? j * 8 : j * GATE_CH + warp * 8) + (lane & 3) * 2;
+      *reinterpret_cast<float2*>(us + row * GATE_U + col) = make_float2(acc[j][0], acc[j][1]);
+      *reinterpret_cast<float2*>(us + (row + 8) * GATE_U + col) = make_float2(acc[j][2], acc[j][3]);
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < RQ; ++q)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) us[((tid >> 4) + 8 * q) * GATE_U + (tid & 15) + 16 * j] = acc[q][j];
+  }
+  __syncthreads();
+
+  // The update.
+  if (!mine) return;
+  float br[VEC], bi[VEC];
+#pragma unroll
+  for (int v = 0; v < VEC; ++v) {
+    br[v] = Pack<IO>::to_float(static_cast<const IO*>(p.b_r)[d + v]);
+    bi[v] = Pack<IO>::to_float(static_cast<const IO*>(p.b_i)[d + v]);
+  }
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q) {
+    const int row = tid / CVECS + q * ROW_STEP;
+    if (row >= MT || b0 + row >= p.B) break;
+    const size_t at = static_cast<size_t>(b0 + row) * p.D + d;
+    float xv[VEC], gv[VEC], yv[VEC];
+    V::load(static_cast<const IO*>(p.x_conv) + at, xv);
+    if (p.branch) V::unpack(graw[q], gv);
+    const uint32_t f = p.tok[b0 + row];
+    const float keep = (f & TOK_RESET) ? 0.0f : 1.0f;
+    const float live = (f & TOK_INACTIVE) ? 0.0f : 1.0f;
+    const float* ur = us + row * GATE_U + cv;
+    const float* ui = ur + GATE_CH;
+#pragma unroll
+    for (int v = 0; v < VEC; v += 2) {             // the arithmetic of the scan kernels' forward
+      float2 r, i;
+      sigmoid_pair2<HALF>(make_float2(ur[v] + br[v], ur[v + 1] + br[v + 1]),
+                          make_float2(ui[v] + bi[v], ui[v + 1] + bi[v + 1]), r, i);
+      const float2 y2 = mul2(r, make_float2(rate[v], rate[v + 1]));
+      const float2 e = poly ? one_minus_exp_neg2<true, HALF>(y2) : one_minus_exp_neg2<false, HALF>(y2);
+      float2 a = fma2(e, f2(-1.0f), f2(1.0f));
+      const float2 gq = add2(mul2(e, fma2(e, f2(-1.0f), f2(2.0f))), f2(1e-30f));
+      float2 gam = mul2(gq, make_float2(rsqrt_approx(gq.x), rsqrt_approx(gq.y)));
+      if (f) {
+        a = fma2(mul2(a, f2(keep)), f2(live), f2(1.0f - live));
+        gam = mul2(fma2(gam, f2(keep), f2(1.0f - keep)), f2(live));
+      }
+      const float2 h2 = fma2(a, make_float2(hv[q][v], hv[q][v + 1]), mul2(mul2(gam, i), make_float2(xv[v], xv[v + 1])));
+      hv[q][v] = h2.x; hv[q][v + 1] = h2.y;
+      float2 out = h2;
+      if (p.branch) {
+        const float2 g = make_float2(gv[v], gv[v + 1]);
+        out = mul2(h2, mul2(g, gelu_sigmoid2<false>(g)));
+      }
+      yv[v] = out.x; yv[v + 1] = out.y;
+    }
+    V::store(static_cast<IO*>(p.y) + at, yv);
+#pragma unroll
+    for (int v = 0; v < VEC; v += 4)
+      *reinterpret_cast<float4*>(p.h_out + at + v) = make_float4(hv[q][v], hv[q][v + 1], hv[q][v + 2], hv[q][v + 3]);
+  }
+}
+
+// ---------------------------------------------------------------- launchers
+template <typename IO, int MT>
+static cudaError_t launch_gates(const DecodeBlockArgs& a, cudaStream_t s) {
+  auto kern = decode_gates_kernel<IO, MT>;
+  static std::atomic<unsigned long long> done{0ull};   // the attribute is per device and set once
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = (dev >= 0 && dev < 64) ? (1ull << dev) : 0ull;
+  if (!bit || !(done.load(std::memory_order_acquire) & bit)) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GateSmem<MT>::BYTES);
+    if (e != cudaSuccess) return e;
+    if (bit) done.fetch_or(bit, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>((a.D / a.bw) * ((a.bw + GATE_CH - 1) / GATE_CH)), static_cast<unsigned>((a.B + MT - 1) / MT));
+  cfg.blockDim = dim3(GATE_THREADS);
+  cfg.dynamicSmemBytes = GateSmem<MT>::BYTES;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, a);
+}
+
+template <typename IO, int ROWS>
+static cudaError_t launch_front(const DecodeBlockArgs& a, cudaStream_t s) {
+  const dim3 grid(static_cast<unsigned>((a.D / vec_width<IO>() + FRONT_THREADS - 1) / FRONT_THREADS),
+                  static_cast<unsigned>((a.B + ROWS - 1) / ROWS));
+  decode_front_kernel<IO, ROWS><<<grid, FRONT_THREADS, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
+// Up to 32 rows the 64-row tile would be at least half empty and half as many CTAs as the 16-row one; the conv gives a
+// thread several rows once there are enough of them to fill the machine anyway.
+template <typename IO>
+static cudaError_t decode_block_t(const DecodeBlockArgs& a, cudaStream_t s) {
+  const cudaError_t e = a.B > 32 ? launch_front<IO, 4>(a, s) : launch_front<IO, 1>(a, s);
+  if (e != cudaSuccess) return e;
+  return a.B > 32 ? launch_gates<IO, 64>(a, s) : launch_gates<IO, 16>(a, s);
+}
+cudaError_t launch_decode_block(bool bf16, const DecodeBlockArgs& a, cudaStream_t s) {
+  return bf16 ? decode_block_t<__nv_bfloat16>(a, s) : decode_block_t<float>(a, s);
+}
+
+}  // namespace rglru

@@ -161,6 +161,33 @@ struct DecodeArgs {
   bool vector_ok;
 };
 
+// One cached token of the recurrent block (see rglru_decode_block in the public header).
+struct DecodeBlockArgs {
+  const void* x_in;
+  const void* branch;       // pre-activation of the GeLU branch, or nullptr
+  const void* conv_w;
+  const void* conv_b;       // or nullptr
+  const void* conv_in;
+  void* conv_out;
+  const void* w_r;
+  const void* b_r;
+  const void* w_i;
+  const void* b_i;
+  const void* lambda;
+  const float* h_in;
+  float* h_out;
+  const long long* prev_pos;
+  const long long* seg_pos;   // or nullptr
+  const uint8_t* active;      // or nullptr
+  long long* pos_out;
+  void* x_conv;               // workspace: conv output [B, D] and flag bytes [B]
+  uint8_t* tok;
+  void* y;
+  int B, D, bw;
+  float c;
+  bool f32_conv_w, f32_conv_b, f32_lambda;
+};
+
 cudaError_t launch_raw_fwd(bool use_tma, const RawFwdMaps& maps, const RawScanArgs& args, cudaStream_t s);
 cudaError_t launch_raw_bwd(bool use_tma, const RawBwdMaps& maps, const RawScanArgs& args, cudaStream_t s);
 int raw_box_rows();
@@ -173,6 +200,7 @@ int conv_tma_box_rows();
 int conv_tma_box_cols();
 cudaError_t launch_decode_conv(bool bf16, const ConvArgs& a, cudaStream_t s);
 cudaError_t launch_decode_step(bool bf16, const DecodeArgs& a, cudaStream_t s);
+cudaError_t launch_decode_block(bool bf16, const DecodeBlockArgs& a, cudaStream_t s);
 int colsum_row_blocks(long long rows, int cols);   // partial rows a column-sum call leaves in its workspace
 cudaError_t launch_column_sums(bool bf16, const void* src, float* out, float* part, long long rows, int cols,
                                bool vector_ok, cudaStream_t s);

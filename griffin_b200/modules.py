@@ -349,12 +349,17 @@ def _shared_between_blocks(owners: tuple, device, build):
     return value
 
 
+def _is_stock(layer: nn.Module, kind: type) -> bool:
+    """Whether a submodule is the one this package put there: not replaced, not parametrised, without hooks."""
+    return type(layer) is kind and not (layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks
+                                        or layer._backward_pre_hooks)
+
+
 def _project(layer: nn.Module, x: Tensor) -> Tensor:
     """One of the block's three projections.  A stock ``nn.Linear`` without hooks goes through ``ops.linear`` (same
     GEMMs; the bias gradient comes from the library's column-sum kernel); anything else — a replaced layer, a layer
     with hooks — is called as the module it is."""
-    if type(layer) is nn.Linear and not (layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks
-                                         or layer._backward_pre_hooks):
+    if _is_stock(layer, nn.Linear):
         return ops.linear(x, layer.weight, layer.bias)
     return layer(x)
 
@@ -403,6 +408,49 @@ class RecurrentBlock(nn.Module):
         for bias in (self.linear_x.bias, self.linear_y.bias, self.linear_out.bias, self.temporal_conv.bias):
             nn.init.zeros_(bias)
 
+    def _decodes_fused(self, x: Tensor, cache: RecurrentBlockCache, segment_pos: Optional[Tensor]) -> bool:
+        """Whether ``ops.decode_block`` does this cached token: this package's own layers in the dtype of ``x`` (the conv
+        and Lambda may be fp32), a cache of the right shapes, no autograd, no autocast, no tracing.  Whatever it does not
+        do -- and whatever has to be refused -- goes operator by operator."""
+        if (torch.is_grad_enabled() or not x.is_cuda or ops._library_ops_active() or torch.is_autocast_enabled("cuda")
+                or not ops.decode_block_supported(x, self.rg_lru.recurrence_gate.block_width)):
+            return False
+        lru, conv = self.rg_lru, self.temporal_conv
+        if not (_is_stock(self.linear_x, nn.Linear) and _is_stock(self.linear_y, nn.Linear)
+                and _is_stock(lru.recurrence_gate, BlockDiagonalLinear) and _is_stock(lru.input_gate, BlockDiagonalLinear)
+                and type(lru) is RG_LRU):
+            return False
+        batch, width = x.shape[0], self.rnn_width
+        for gate in (lru.recurrence_gate, lru.input_gate):
+            if gate.bias is None or gate.weight.shape != (gate.num_blocks, gate.block_width, gate.block_width):
+                return False
+        same = (self.linear_x.weight, self.linear_y.weight, lru.recurrence_gate.weight, lru.recurrence_gate.bias,
+                lru.input_gate.weight, lru.input_gate.bias)
+        either = (conv.weight, lru.Lambda) if conv.bias is None else (conv.weight, conv.bias, lru.Lambda)
+        device = x.device
+        if not (all(t.dtype == x.dtype and t.device == device and t.is_contiguous() for t in same)
+                and all(t.dtype in (x.dtype, torch.float32) and t.device == device and t.is_contiguous() for t in either)):
+            return False
+        return (cache.rnn_state.shape == (batch, width) and cache.conv_state.shape == (batch, 3, width)
+                and cache.segment_position.shape == (batch,) and (segment_pos is None or segment_pos.shape == (batch, 1)))
+
+    def _decode_fused(self, x: Tensor, cache: RecurrentBlockCache, segment_pos: Optional[Tensor],
+                      active_mask: Optional[Tensor], return_cache: bool):
+        lru, conv, device = self.rg_lru, self.temporal_conv, x.device
+        branch = _project(self.linear_y, x)[:, 0]
+        x_in = _project(self.linear_x, x)[:, 0]
+        y, new_rnn, new_conv, position = ops.decode_block(
+            x_in, branch, conv.weight[:, 0, :], conv.bias, cache.conv_state.to(device=device, dtype=x.dtype),
+            lru.recurrence_gate.weight, lru.recurrence_gate.bias, lru.input_gate.weight, lru.input_gate.bias, lru.Lambda,
+            cache.rnn_state.to(device=device, dtype=torch.float32),
+            cache.segment_position.to(device=device, dtype=torch.long).contiguous(),
+            None if segment_pos is None else segment_pos.to(device=device, dtype=torch.long)[:, 0].contiguous(),
+            None if active_mask is None else active_mask[:, 0].contiguous(), lru.c)
+        out = _project(self.linear_out, y[:, None, :])
+        if active_mask is not None:
+            out = torch.where(active_mask[..., None], out, 0.0)
+        return (out, RecurrentBlockCache(new_rnn, new_conv, position)) if return_cache else out
+
     def forward(self, x: Tensor, cache: Optional[RecurrentBlockCache] = None, segment_pos: Optional[Tensor] = None, *,
                 active_mask: Optional[Tensor] = None, return_cache: bool = False):
         if x.dim() != 3:
@@ -413,6 +461,8 @@ class RecurrentBlock(nn.Module):
             if active_mask.shape != (batch, steps):
                 raise ValueError("active_mask must match the input [batch, sequence] dimensions")
             active_mask = active_mask.to(device=x.device, dtype=torch.bool)
+        if steps == 1 and cache is not None and self._decodes_fused(x, cache, segment_pos):
+            return self._decode_fused(x, cache, segment_pos, active_mask, return_cache)
         previous = None if cache is None else cache.segment_position
         plain = segment_pos is None and cache is None and active_mask is None
         if plain and steps == 0:
@@ -459,8 +509,8 @@ class RecurrentBlock(nn.Module):
         conv_w = self.temporal_conv.weight[:, 0, :]
         rnn_state = None if cache is None else cache.rnn_state
         if steps == 1 and cache is not None and not torch.is_grad_enabled() and x_in.is_cuda:
-            # Cached single-token decode (inference): the two in-place decode kernels on copies of the cached
-            # states (the cache stays a value: the caller's old cache is not modified).
+            # Cached single-token decode (inference) that the fused form does not take: the two in-place decode kernels
+            # on copies of the cached states (the cache stays a value: the caller's old cache is not modified).
             if rnn_state.shape != (batch, self.rnn_width):
                 raise ValueError(f"ht_minus_1 must have shape ({batch}, {self.rnn_width}), got {tuple(rnn_state.shape)}")
             lru = self.rg_lru

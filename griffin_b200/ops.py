@@ -954,3 +954,42 @@ def decode_step(x: Tensor, u_r: Tensor, u_i: Tensor, lam: Tensor, h: Tensor, tok
                                    _ptr(h), _ptr(tok), _ptr(y), B, D, float(c), dt, _stream(x))
     _lib.check(rc, "rglru_decode_step")
     return y
+
+
+def _aligned_dense(t: Optional[Tensor]) -> Optional[Tensor]:
+    """``t`` as a contiguous tensor on a 16-byte boundary (a copy where it is not one)."""
+    return None if t is None else _aligned16(t.contiguous())
+
+
+def decode_block_supported(x: Tensor, gate_width: int) -> bool:
+    """Whether :func:`decode_block` takes these activations: gate heads whose rows are whole 16-byte groups."""
+    return x.is_cuda and x.dtype in _DTYPES and gate_width * x.element_size() % 16 == 0
+
+
+def decode_block(x_in: Tensor, branch: Optional[Tensor], conv_w: Tensor, conv_b: Optional[Tensor], conv_state: Tensor,
+                 w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor, h: Tensor, position: Tensor,
+                 segment_pos: Optional[Tensor] = None, active: Optional[Tensor] = None, c: float = 8.0
+                 ) -> tuple[Tensor, Tensor, Tensor, Tensor]:
+    """(y, next h, next conv state, next position) of one cached token between the block's input projections and its
+    output projection (``rglru_decode_block``): conv, both gate projections, the update and, with ``branch`` given, the
+    product with its GeLU.  ``x_in`` / ``branch`` [B, D]; conv weights, biases and Lambda in the activation dtype or
+    (conv and Lambda) fp32; ``position`` / ``segment_pos`` [B] int64; ``active`` [B] bool.  The states are not modified."""
+    lib = _lib.load()
+    _require_cuda(x_in, branch, conv_w, conv_b, conv_state, w_r, b_r, w_i, b_i, lam, h, position, segment_pos, active)
+    dt = _io_dtype(x_in, "decode block")
+    B, D = x_in.shape
+    f32 = ((1 if conv_w.dtype == torch.float32 else 0) | (2 if conv_b is not None and conv_b.dtype == torch.float32 else 0)
+           | (4 if lam.dtype == torch.float32 else 0))
+    x_in, branch, conv_state, h = (_aligned_dense(t) for t in (x_in, branch, conv_state, h))
+    w_r, w_i, conv_w = _aligned_dense(w_r), _aligned_dense(w_i), _aligned_dense(conv_w)
+    y, h_new, conv_new = torch.empty_like(x_in), torch.empty_like(h), torch.empty_like(conv_state)
+    pos_new = torch.empty_like(position)
+    nbytes = B * D * x_in.element_size() + B
+    ws = torch.empty(nbytes, device=x_in.device, dtype=torch.uint8)
+    with _on(x_in, "rglru_decode_block"):
+        rc = lib.rglru_decode_block(_ptr(x_in), _ptr(branch), _ptr(conv_w), _ptr(conv_b), _ptr(conv_state), _ptr(conv_new),
+                                    _ptr(w_r), _ptr(b_r), _ptr(w_i), _ptr(b_i), _ptr(lam), _ptr(h), _ptr(h_new),
+                                    _ptr(position), _ptr(segment_pos), _ptr(active), _ptr(pos_new), _ptr(y), _ptr(ws),
+                                    nbytes, B, D, w_r.shape[1], float(c), dt, f32, _stream(x_in))
+    _lib.check(rc, "rglru_decode_block")
+    return y, h_new, conv_new, pos_new

@@ -276,6 +276,32 @@ int rglru_decode_conv(const void* x_in, const float* conv_w, const float* conv_b
 int rglru_decode_step(const void* x, const void* u_r, const void* u_i, const float* lambda, float* h,
                       const uint8_t* tok, void* y, int B, int D, float c, int io_dtype, void* stream);
 
+/* One cached token of the recurrent block between its input projections and its output projection, in two launches:
+ * positions and flags, conv, both gate projections, the update and the product with the GeLU branch
+ * (griffin/griffin.py:309-358, :459-528 at T = 1; :129-154, :237-258).  Same results as rglru_decode_conv, two gate GEMMs,
+ * rglru_decode_step and the branch product, with the states written to outputs of their own (h_out may be h_in and
+ * conv_out may be conv_in; pos_out may not be prev_pos).
+ *   x_in, branch : [B,D] io_dtype; branch is the PRE-activation of the GeLU branch, or NULL for no product
+ *   conv_w [D,4], conv_b [D] or NULL, lambda [D] : io_dtype, or fp32 where f32_params says so
+ *   conv_in, conv_out : [B,3,D] io_dtype       h_in, h_out : [B,D] fp32
+ *   w_r, w_i : [D/gate_width, gate_width, gate_width] (out, in) io_dtype      b_r, b_i : [D] io_dtype
+ *   prev_pos : [B] position of each row's last real token      seg_pos : [B] position of this token, or NULL (prev + 1)
+ *   active : [B] bytes, 0 = padding (state and position stay), or NULL       pos_out : [B]
+ *   y : [B,D] io_dtype out     ws : rglru_decode_block_workspace_bytes(B,D,io_dtype) bytes
+ * gate_width * element size must be a multiple of 16 bytes, activations, states, weights (conv_w too) and ws
+ * 16-byte aligned.
+ */
+#define RGLRU_F32_CONV_W 1
+#define RGLRU_F32_CONV_B 2
+#define RGLRU_F32_LAMBDA 4
+size_t rglru_decode_block_workspace_bytes(int B, int D, int io_dtype);
+int rglru_decode_block(const void* x_in, const void* branch, const void* conv_w, const void* conv_b, const void* conv_in,
+                       void* conv_out, const void* w_r, const void* b_r, const void* w_i, const void* b_i,
+                       const void* lambda, const float* h_in, float* h_out, const int64_t* prev_pos,
+                       const int64_t* seg_pos, const uint8_t* active, int64_t* pos_out, void* y, void* ws,
+                       size_t ws_bytes, int B, int D, int gate_width, float c, int io_dtype, int f32_params,
+                       void* stream);
+
 #ifdef __cplusplus
 }
 #endif
