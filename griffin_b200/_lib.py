@@ -41,6 +41,12 @@ SIGNATURES = {
     "rglru_merge_bwd": (_i, [_vp] * 12 + [_vp, _sz] + [_vp] * 6 + [_i, _i, _i, _f, _i, _vp]),
     "rglru_grouped_fwd": (_i, [_vp] * 9 + [_vp, _sz, _i, _i, _i, _i, _f, _i, _vp]),
     "rglru_grouped_bwd": (_i, [_vp] * 9 + [_vp, _sz] + [_vp] * 6 + [_i, _i, _i, _i, _f, _i, _vp]),
+    "rglru_gated_fwd": (_i, [_vp] * 9 + [_vp, _sz, _i, _i, _i, _i, _f, _i, _vp]),
+    "rglru_gated_bwd": (_i, [_vp] * 9 + [_vp, _sz] + [_vp] * 6 + [_i, _i, _i, _i, _f, _i, _vp]),
+    "rglru_gate_pack": (_i, [_vp] * 7 + [_i] * 7 + [_vp]),
+    "rglru_gate_unpack": (_i, [_vp, _i] + [_vp] * 7 + [_i] * 7 + [_vp]),
+    "rglru_gate_dw_splits": (_i, [ctypes.c_longlong, _i, _i]),
+    "rglru_gate_dw": (_i, [_vp, _vp, _vp, _i, ctypes.c_longlong, _i, _i, _vp]),
     "rglru_linear_scan_fwd": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _vp]),
     "rglru_linear_scan_bwd": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]),
     "rglru_conv_fwd": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),

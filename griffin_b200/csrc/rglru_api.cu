@@ -101,15 +101,38 @@ static bool encode_map_paired(CUtensorMap* map, const void* base, bool bf16, int
   return r == CUDA_SUCCESS;
 }
 
+// 5-D map over a gate tensor [B, T, 2 D] whose columns alternate between the two gates in groups of `unit` channels:
+// dimensions (channel in the group, gate, group, time, batch).  A box of [unit, 1, cols / unit, rows, 1] is the tile of
+// `cols` adjacent channels of one gate, dense in shared memory; groups past D read as zero and are dropped on store.
+static bool encode_map_gates(CUtensorMap* map, const void* base, bool bf16, int B, int T, int D, int rows, int cols, int unit) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  const size_t es = bf16 ? 2 : 4;
+  const cuuint64_t group = static_cast<cuuint64_t>(unit) * es, pitch = 2 * static_cast<cuuint64_t>(D) * es;
+  const cuuint64_t dims[5] = {static_cast<cuuint64_t>(unit), 2u, static_cast<cuuint64_t>(D / unit), static_cast<cuuint64_t>(T),
+                              static_cast<cuuint64_t>(B)};
+  const cuuint64_t strides[4] = {group, 2 * group, pitch, pitch * T};
+  const cuuint32_t box[5] = {static_cast<cuuint32_t>(unit), 1u, static_cast<cuuint32_t>(cols / unit), static_cast<cuuint32_t>(rows), 1u};
+  const cuuint32_t estr[5] = {1u, 1u, 1u, 1u, 1u};
+  const CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5,
+                        const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS;
+}
+
 // A tensor map is a pure function of (base address, element type, shape, box), and a training loop calls with
 // the same handful of buffers step after step (the caching allocator hands the same blocks back), so encoded
 // maps are kept in a small per-thread table: a hit costs a compare and a 128-byte copy instead of a driver call
 // per map (seven to nine of them per backward call).
+// `form` is 0 for the plain 3-D map, MAP_PAIRED, or the group width of an interleaved gate tensor.
+constexpr int MAP_PAIRED = -1;
 struct MapKey {
   const void* base;
-  int B, T, D, rows, cols, bf16;
+  int B, T, D, rows, cols, bf16, form;
   bool operator==(const MapKey& o) const {
-    return base == o.base && B == o.B && T == o.T && D == o.D && rows == o.rows && cols == o.cols && bf16 == o.bf16;
+    return base == o.base && B == o.B && T == o.T && D == o.D && rows == o.rows && cols == o.cols && bf16 == o.bf16 &&
+           form == o.form;
   }
 };
 struct MapSlot {
@@ -120,9 +143,9 @@ struct MapSlot {
 constexpr int MAP_CACHE_SLOTS = 256;   // direct-mapped
 
 static bool make_map(CUtensorMap* map, const void* base, bool bf16, int B, int T, int D, int rows, int cols,
-                     bool paired = false) {
+                     int form = 0) {
   static thread_local MapSlot table[MAP_CACHE_SLOTS] = {};
-  const MapKey key{base, B, T, D, paired ? -rows : rows, cols, bf16 ? 1 : 0};   // negative rows: the paired 5-D form
+  const MapKey key{base, B, T, D, rows, cols, bf16 ? 1 : 0, form};
   uint64_t h = reinterpret_cast<uintptr_t>(base) >> 8;
   h ^= (static_cast<uint64_t>(rows) << 3) ^ (static_cast<uint64_t>(cols) << 11) ^ (static_cast<uint64_t>(D) << 17) ^
        (static_cast<uint64_t>(T) << 29) ^ (static_cast<uint64_t>(B) << 41);
@@ -132,12 +155,26 @@ static bool make_map(CUtensorMap* map, const void* base, bool bf16, int B, int T
     *map = slot.map;
     return true;
   }
-  if (!(paired ? encode_map_paired(map, base, bf16, B, T, D, rows, cols) : encode_map(map, base, bf16, B, T, D, rows, cols)))
-    return false;
+  auto encode = [&]() {
+    if (form == 0) return encode_map(map, base, bf16, B, T, D, rows, cols);
+    if (form == MAP_PAIRED) return encode_map_paired(map, base, bf16, B, T, D, rows, cols);
+    return encode_map_gates(map, base, bf16, B, T, D, rows, cols, form);
+  };
+  // The driver encodes only on a thread that has the device's context, which a thread whose first CUDA call this is (an
+  // autograd worker, say) does not have yet: choosing its device gives it one.
+  if (!encode()) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess || !encode()) return false;
+  }
   slot.key = key;
   slot.map = *map;
   slot.used = true;
   return true;
+}
+
+static bool make_gate_map(CUtensorMap* map, const void* base, bool bf16, int B, int T, int D, int rows, int cols, int gate_width) {
+  return gate_width < cols ? make_map(map, base, bf16, B, T, D, rows, cols, gate_width)
+                           : make_map(map, base, bf16, B, T, 2 * D, rows, cols);
 }
 
 static bool aligned(const void* p, size_t n) { return (reinterpret_cast<uintptr_t>(p) % n) == 0; }
@@ -264,9 +301,9 @@ static int fwd_common(const void* x, const void* u_r, const void* u_i, const flo
   if (tma) {
     const int rows = scan_fwd_box_rows(variant), cols = scan_fwd_box_cols(variant);
     const void* yy = y ? y : x;   // without y the map is never used
-    a.paired = scan_fwd_paired(variant, bf16, tok, T) && make_map(&maps.x, x, bf16, B, T, D, rows, cols, true) &&
-               make_map(&maps.ur, u_r, bf16, B, T, D, rows, cols, true) &&
-               make_map(&maps.ui, u_i, bf16, B, T, D, rows, cols, true) && make_map(&maps.y, yy, bf16, B, T, D, rows, cols, true);
+    a.paired = scan_fwd_paired(variant, bf16, tok, T) && make_map(&maps.x, x, bf16, B, T, D, rows, cols, MAP_PAIRED) &&
+               make_map(&maps.ur, u_r, bf16, B, T, D, rows, cols, MAP_PAIRED) &&
+               make_map(&maps.ui, u_i, bf16, B, T, D, rows, cols, MAP_PAIRED) && make_map(&maps.y, yy, bf16, B, T, D, rows, cols, MAP_PAIRED);
     if (!a.paired)
       tma = make_map(&maps.x, x, bf16, B, T, D, rows, cols) && make_map(&maps.ur, u_r, bf16, B, T, D, rows, cols) &&
             make_map(&maps.ui, u_i, bf16, B, T, D, rows, cols) && make_map(&maps.y, yy, bf16, B, T, D, rows, cols);
@@ -522,17 +559,20 @@ int rglru_merge_bwd(const void* dout, const float* dh_last, const void* x, const
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
 }
 
-// Grouped gate layout: TMA staging only, so everything the copy engine touches must be 16-byte aligned and a
-// channel tile must not straddle a gate head.
-static int check_grouped(int D, int gate_width, size_t es) {
-  if (gate_width <= 0 || D % gate_width != 0 || gate_width % grouped_box_cols() != 0) return RGLRU_ERR_BAD_SHAPE;
+// Grouped gate layout: TMA staging only, so everything the copy engine touches must be 16-byte aligned.  Column groups
+// are a multiple of the channel tile or, for the rglru_gated_* entry points, a power of two of at least 16 bytes below it.
+static int check_grouped(int D, int gate_width, size_t es, bool narrow) {
+  if (gate_width <= 0 || D % gate_width != 0) return RGLRU_ERR_BAD_SHAPE;
+  const bool wide_ok = gate_width % grouped_box_cols() == 0;
+  const bool narrow_ok = gate_width < grouped_box_cols() && (gate_width & (gate_width - 1)) == 0 && gate_width * es >= 16;
+  if (!wide_ok && !(narrow && narrow_ok)) return RGLRU_ERR_BAD_SHAPE;
   if ((static_cast<size_t>(D) * es) % 16 != 0) return RGLRU_ERR_BAD_SHAPE;
   return RGLRU_OK;
 }
 
-int rglru_grouped_fwd(const void* x, const void* u, const float* gate_bias, const void* branch, const float* lambda,
+static int grouped_fwd_common(const void* x, const void* u, const float* gate_bias, const void* branch, const float* lambda,
                       const float* h0, const uint8_t* tok, void* out, float* h_last, void* ws, size_t ws_bytes, int B,
-                      int T, int D, int gate_width, float c, int io_dtype, void* stream) {
+                      int T, int D, int gate_width, float c, int io_dtype, void* stream, bool narrow) {
   if (io_dtype != RGLRU_F32 && io_dtype != RGLRU_BF16) return RGLRU_ERR_BAD_DTYPE;
   if (!x || !u || !lambda || !out) return RGLRU_ERR_NULL_POINTER;
   int rc = check_dims(B, T, D);
@@ -540,7 +580,7 @@ int rglru_grouped_fwd(const void* x, const void* u, const float* gate_bias, cons
   const bool bf16 = io_dtype == RGLRU_BF16;
   const bool merge = branch != nullptr;
   const size_t es = bf16 ? 2 : 4;
-  rc = check_grouped(D, gate_width, es);
+  rc = check_grouped(D, gate_width, es, narrow);
   if (rc != RGLRU_OK) return rc;
   if (!aligned(x, 16) || !aligned(u, 16) || !aligned(branch, 16) || !aligned(out, 16) || !aligned(gate_bias, 16) ||
       !aligned(lambda, 4) || !aligned(h0, 4) || !aligned(h_last, 4) || !aligned(ws, 4))
@@ -564,7 +604,7 @@ int rglru_grouped_fwd(const void* x, const void* u, const float* gate_bias, cons
 
   FwdMaps maps;
   const int rows = scan_fwd_box_rows(0), cols = grouped_box_cols();
-  bool ok = make_map(&maps.x, x, bf16, B, T, D, rows, cols) && make_map(&maps.ur, u, bf16, B, T, 2 * D, rows, cols) &&
+  bool ok = make_map(&maps.x, x, bf16, B, T, D, rows, cols) && make_gate_map(&maps.ur, u, bf16, B, T, D, rows, cols, gate_width) &&
             make_map(&maps.y, out, bf16, B, T, D, rows, cols);
   if (ok && merge) ok = make_map(&maps.g, branch, bf16, B, T, D, rows, cols);
   if (!ok) return RGLRU_ERR_UNSUPPORTED;
@@ -574,10 +614,10 @@ int rglru_grouped_fwd(const void* x, const void* u, const float* gate_bias, cons
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
 }
 
-int rglru_grouped_bwd(const void* dout, const float* dh_last, const void* x, const void* u, const float* gate_bias,
+static int grouped_bwd_common(const void* dout, const float* dh_last, const void* x, const void* u, const float* gate_bias,
                       const void* branch, const float* lambda, const float* h0, const uint8_t* tok, void* ws,
                       size_t ws_bytes, void* dx, void* du, void* dbranch, float* dlambda, float* dh0, float* d_gate_bias,
-                      int B, int T, int D, int gate_width, float c, int io_dtype, void* stream) {
+                      int B, int T, int D, int gate_width, float c, int io_dtype, void* stream, bool narrow) {
   if (io_dtype != RGLRU_F32 && io_dtype != RGLRU_BF16) return RGLRU_ERR_BAD_DTYPE;
   if (!dout || !x || !u || !lambda || !dx || !du || !dlambda || (branch && !dbranch)) return RGLRU_ERR_NULL_POINTER;
   int rc = check_dims(B, T, D);
@@ -585,7 +625,7 @@ int rglru_grouped_bwd(const void* dout, const float* dh_last, const void* x, con
   const bool bf16 = io_dtype == RGLRU_BF16;
   const bool merge = branch != nullptr;
   const size_t es = bf16 ? 2 : 4;
-  rc = check_grouped(D, gate_width, es);
+  rc = check_grouped(D, gate_width, es, narrow);
   if (rc != RGLRU_OK) return rc;
   if (!aligned(dout, 16) || !aligned(x, 16) || !aligned(u, 16) || !aligned(branch, 16) || !aligned(dx, 16) ||
       !aligned(du, 16) || !aligned(dbranch, 16) || !aligned(gate_bias, 16) || !aligned(d_gate_bias, 16) ||
@@ -615,8 +655,8 @@ int rglru_grouped_bwd(const void* dout, const float* dh_last, const void* x, con
   BwdMaps maps;
   const int rows = scan_bwd_box_rows(0), cols = grouped_box_cols();
   bool ok = make_map(&maps.dy, dout, bf16, B, T, D, rows, cols) && make_map(&maps.x, x, bf16, B, T, D, rows, cols) &&
-            make_map(&maps.ur, u, bf16, B, T, 2 * D, rows, cols) && make_map(&maps.dx, dx, bf16, B, T, D, rows, cols) &&
-            make_map(&maps.dur, du, bf16, B, T, 2 * D, rows, cols);
+            make_gate_map(&maps.ur, u, bf16, B, T, D, rows, cols, gate_width) && make_map(&maps.dx, dx, bf16, B, T, D, rows, cols) &&
+            make_gate_map(&maps.dur, du, bf16, B, T, D, rows, cols, gate_width);
   if (ok && merge)
     ok = make_map(&maps.g, branch, bf16, B, T, D, rows, cols) && make_map(&maps.dg, dbranch, bf16, B, T, D, rows, cols);
   if (!ok) return RGLRU_ERR_UNSUPPORTED;
@@ -625,6 +665,34 @@ int rglru_grouped_bwd(const void* dout, const float* dh_last, const void* x, con
   a.split = grouped_split(false, bf16, merge, B, T, D);
   const cudaError_t e = launch_grouped_bwd(bf16, merge, maps, a, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
+}
+
+int rglru_grouped_fwd(const void* x, const void* u, const float* gate_bias, const void* branch, const float* lambda,
+                      const float* h0, const uint8_t* tok, void* out, float* h_last, void* ws, size_t ws_bytes,
+                      int B, int T, int D, int gate_width, float c, int io_dtype, void* stream) {
+  return grouped_fwd_common(x, u, gate_bias, branch, lambda, h0, tok, out, h_last, ws, ws_bytes, B, T, D, gate_width,
+                            c, io_dtype, stream, false);
+}
+int rglru_gated_fwd(const void* x, const void* u, const float* gate_bias, const void* branch, const float* lambda,
+                    const float* h0, const uint8_t* tok, void* out, float* h_last, void* ws, size_t ws_bytes, int B,
+                    int T, int D, int gate_width, float c, int io_dtype, void* stream) {
+  return grouped_fwd_common(x, u, gate_bias, branch, lambda, h0, tok, out, h_last, ws, ws_bytes, B, T, D, gate_width,
+                            c, io_dtype, stream, true);
+}
+
+int rglru_grouped_bwd(const void* dout, const float* dh_last, const void* x, const void* u, const float* gate_bias,
+                      const void* branch, const float* lambda, const float* h0, const uint8_t* tok, void* ws,
+                      size_t ws_bytes, void* dx, void* du, void* dbranch, float* dlambda, float* dh0,
+                      float* d_gate_bias, int B, int T, int D, int gate_width, float c, int io_dtype, void* stream) {
+  return grouped_bwd_common(dout, dh_last, x, u, gate_bias, branch, lambda, h0, tok, ws, ws_bytes, dx, du, dbranch,
+                            dlambda, dh0, d_gate_bias, B, T, D, gate_width, c, io_dtype, stream, false);
+}
+int rglru_gated_bwd(const void* dout, const float* dh_last, const void* x, const void* u, const float* gate_bias,
+                    const void* branch, const float* lambda, const float* h0, const uint8_t* tok, void* ws,
+                    size_t ws_bytes, void* dx, void* du, void* dbranch, float* dlambda, float* dh0,
+                    float* d_gate_bias, int B, int T, int D, int gate_width, float c, int io_dtype, void* stream) {
+  return grouped_bwd_common(dout, dh_last, x, u, gate_bias, branch, lambda, h0, tok, ws, ws_bytes, dx, du, dbranch,
+                            dlambda, dh0, d_gate_bias, B, T, D, gate_width, c, io_dtype, stream, true);
 }
 
 int rglru_linear_scan_fwd(const float* decay, const float* drive, const float* h0, float* out, int B, int T, int D,
@@ -811,6 +879,72 @@ int rglru_decode_step(const void* x, const void* u_r, const void* u_i, const flo
   a.vector_ok = (static_cast<size_t>(D) * es) % 16 == 0 && aligned(x, 16) && aligned(u_r, 16) && aligned(u_i, 16) &&
                 aligned(y, 16) && aligned(h, 16);
   const cudaError_t e = launch_decode_step(bf16, a, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
+}
+
+static bool gate_groups_ok(int D, int head_width, int gate_width) {
+  return D > 0 && head_width > 0 && D % head_width == 0 && gate_width >= 4 && gate_width % 4 == 0 && head_width % gate_width == 0;
+}
+static bool io_dtype_ok(int t) { return t == RGLRU_F32 || t == RGLRU_BF16; }
+
+int rglru_gate_pack(const void* w_r, const void* b_r, const void* w_i, const void* b_i, const void* lambda, void* wcat,
+                    float* params, int D, int head_width, int gate_width, int weight_dtype, int bias_dtype,
+                    int lambda_dtype, int io_dtype, void* stream) {
+  if (!io_dtype_ok(weight_dtype) || !io_dtype_ok(bias_dtype) || !io_dtype_ok(lambda_dtype) || !io_dtype_ok(io_dtype))
+    return RGLRU_ERR_BAD_DTYPE;
+  if (!w_r || !b_r || !w_i || !b_i || !lambda || !wcat || !params) return RGLRU_ERR_NULL_POINTER;
+  if (!gate_groups_ok(D, head_width, gate_width)) return RGLRU_ERR_BAD_SHAPE;
+  if (!aligned(w_r, 16) || !aligned(w_i, 16) || !aligned(wcat, 16) || !aligned(params, 4) || !aligned(b_r, 2) ||
+      !aligned(b_i, 2) || !aligned(lambda, 2))
+    return RGLRU_ERR_MISALIGNED;
+  int* status = nullptr;
+  const int rc = device_setup(&status);
+  if (rc != RGLRU_OK) return rc;
+  GatePackArgs a = {};
+  a.w_r = w_r; a.b_r = b_r; a.w_i = w_i; a.b_i = b_i; a.lambda = lambda; a.wcat = wcat; a.params = params;
+  a.D = D; a.bw = head_width; a.unit = gate_width; a.f32_bias = bias_dtype == RGLRU_F32; a.f32_lambda = lambda_dtype == RGLRU_F32;
+  const cudaError_t e = launch_gate_pack(weight_dtype == RGLRU_F32, io_dtype == RGLRU_BF16, a, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
+}
+
+int rglru_gate_unpack(const void* dw, int splits, const float* dbias, const float* dlam, void* dw_r, void* db_r, void* dw_i,
+                      void* db_i, void* dlambda, int D, int head_width, int gate_width, int io_dtype, int weight_dtype,
+                      int bias_dtype, int lambda_dtype, void* stream) {
+  if (!io_dtype_ok(weight_dtype) || !io_dtype_ok(bias_dtype) || !io_dtype_ok(lambda_dtype) || !io_dtype_ok(io_dtype))
+    return RGLRU_ERR_BAD_DTYPE;
+  if (!dw || !dbias || !dlam || !dw_r || !db_r || !dw_i || !db_i || !dlambda) return RGLRU_ERR_NULL_POINTER;
+  if (!gate_groups_ok(D, head_width, gate_width) || splits < 1) return RGLRU_ERR_BAD_SHAPE;
+  if (!aligned(dw, 16) || !aligned(dw_r, 16) || !aligned(dw_i, 16) || !aligned(dbias, 4) || !aligned(dlam, 4) ||
+      !aligned(db_r, 2) || !aligned(db_i, 2) || !aligned(dlambda, 2))
+    return RGLRU_ERR_MISALIGNED;
+  int* status = nullptr;
+  const int rc = device_setup(&status);
+  if (rc != RGLRU_OK) return rc;
+  GateUnpackArgs a = {};
+  a.dw = dw; a.splits = splits; a.dbias = dbias; a.dlam = dlam; a.dw_r = dw_r; a.db_r = db_r; a.dw_i = dw_i; a.db_i = db_i;
+  a.dlambda = dlambda; a.D = D; a.bw = head_width; a.unit = gate_width;
+  a.f32_bias = bias_dtype == RGLRU_F32; a.f32_lambda = lambda_dtype == RGLRU_F32;
+  const cudaError_t e = launch_gate_unpack(io_dtype == RGLRU_BF16, weight_dtype == RGLRU_F32, a, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
+}
+
+int rglru_gate_dw_splits(long long rows, int D, int head_width) {
+  if (rows <= 0 || D <= 0 || head_width <= 0 || D % head_width != 0) return 0;
+  return gate_dw_splits(rows, D, head_width);
+}
+
+int rglru_gate_dw(const float* du, const float* x, float* dw, int splits, long long rows, int D, int head_width, void* stream) {
+  if (!du || !x || !dw) return RGLRU_ERR_NULL_POINTER;
+  if (rows <= 0 || rows > (1ll << 40) || D <= 0 || head_width <= 0 || D % head_width != 0 || head_width % 4 != 0 ||
+      D / head_width > 65535 || splits < 1 || splits > 65535)
+    return RGLRU_ERR_BAD_SHAPE;
+  if (!aligned(du, 16) || !aligned(x, 16) || !aligned(dw, 16)) return RGLRU_ERR_MISALIGNED;
+  int* status = nullptr;
+  const int rc = device_setup(&status);
+  if (rc != RGLRU_OK) return rc;
+  GateDwArgs a = {};
+  a.du = du; a.x = x; a.part = dw; a.rows = rows; a.D = D; a.bw = head_width;
+  const cudaError_t e = launch_gate_dw(a, splits, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
 }
 

@@ -31,8 +31,8 @@ struct ScanFwdArgs {
   const float* conv_b;
   const void* conv_state;
   const void* g;     // merged variant only: pre-activation of the GeLU branch [B, T, D]; y receives h * gelu(g)
-  // grouped gate layout only: ur == ui == one [B, T, 2 D] tensor, gate_bw channels per gate head,
-  // gate_bias [2 D] fp32 in the same column layout or nullptr
+  // grouped gate layout only: ur == ui == one [B, T, 2 D] tensor, gate_bw channels per group of its columns (below 64
+  // the two tensor maps are the 5-D interleaved form), gate_bias [2 D] fp32 in the same column layout or nullptr
   const float* gate_bias;
   int gate_bw;
   int split;    // CTAs of a cluster that share one (batch row, channel tile) along time; 0 or 1: none
@@ -161,6 +161,38 @@ struct DecodeArgs {
   bool vector_ok;
 };
 
+// Gate parameters into and out of the interleaved gate layout (see rglru_gates.cu).
+struct GatePackArgs {
+  const void* w_r;
+  const void* b_r;
+  const void* w_i;
+  const void* b_i;
+  const void* lambda;
+  void* wcat;
+  float* params;     // [3 D]: the biases in the gate tensor's column order [2 D], then Lambda [D]
+  int D, bw, unit;
+  bool f32_bias, f32_lambda;
+};
+struct GateUnpackArgs {
+  const void* dw;
+  const float* dbias;
+  const float* dlam;
+  void* dw_r;
+  void* db_r;
+  void* dw_i;
+  void* db_i;
+  void* dlambda;
+  int splits, D, bw, unit;
+  bool f32_bias, f32_lambda;
+};
+struct GateDwArgs {
+  const float* du;   // [rows, 2 D]
+  const float* x;    // [rows, D]
+  float* part;       // [splits, G, 2 bw, bw]
+  long long rows, per_split;
+  int D, bw;
+};
+
 // One cached token of the recurrent block (see rglru_decode_block in the public header).
 struct DecodeBlockArgs {
   const void* x_in;
@@ -200,6 +232,10 @@ int conv_tma_box_rows();
 int conv_tma_box_cols();
 cudaError_t launch_decode_conv(bool bf16, const ConvArgs& a, cudaStream_t s);
 cudaError_t launch_decode_step(bool bf16, const DecodeArgs& a, cudaStream_t s);
+cudaError_t launch_gate_pack(bool f32_weights, bool bf16, const GatePackArgs& a, cudaStream_t s);
+cudaError_t launch_gate_unpack(bool bf16, bool f32_weights, const GateUnpackArgs& a, cudaStream_t s);
+cudaError_t launch_gate_dw(const GateDwArgs& a, int splits, cudaStream_t s);
+int gate_dw_splits(long long rows, int D, int bw);
 cudaError_t launch_decode_block(bool bf16, const DecodeBlockArgs& a, cudaStream_t s);
 int colsum_row_blocks(long long rows, int cols);   // partial rows a column-sum call leaves in its workspace
 cudaError_t launch_column_sums(bool bf16, const void* src, float* out, float* part, long long rows, int cols,

@@ -31,7 +31,8 @@
 //           an x tile with a three-row halo;
 //   MERGE   the block's GeLU-branch product (:464, :520) is formed in the store stage and differentiated in
 //           the backward's load stage;
-//   GROUPED both gate pre-activations come from one [B, T, 2 D] tensor written by a single grouped GEMM, the
+//   GROUPED both gate pre-activations come from one [B, T, 2 D] tensor written by a single grouped GEMM (its columns
+//           alternate between the gates in groups that divide the head width, so any head width will do), the
 //           gate biases are added here, and the backward also returns their gradient (column sums of du);
 //   PLAIN   no token flags and a whole number of chunks: the masked arithmetic is not compiled in.
 // The file also holds the raw affine scan operator (triton_scan.py:274-276), the TMA-staged kernels of the
@@ -195,25 +196,47 @@ struct SplitChain {
 };
 
 // Grouped gate layout: both gate pre-activations come from ONE tensor [B, T, 2 D] written by a single
-// grouped GEMM with the two weight blocks of a gate head stacked, i.e. per head of width bw the columns are
-// [u_r (bw) | u_i (bw)].  The channel tile at d0 (which never straddles a head: bw is a multiple of the tile
-// width) finds its u_r columns at (d0 / bw) * 2 bw + d0 % bw and its u_i columns bw further.  The gate biases
-// (same column layout, fp32) are added in the kernel, pre-scaled for the sigmoid.
+// grouped GEMM with the two weight blocks of a gate head stacked.  Its columns alternate between the gates in groups of
+// `bw` channels, [u_r (bw) | u_i (bw)] and so on: channel d's recurrence gate is column (d / bw) * 2 bw + d % bw, its
+// input gate bw columns further.  A group is a multiple of the tile width -- a tile's columns of one gate are then
+// adjacent -- or a power of two below it: a tile then takes every other group of 2 * 64 columns, which the copy engine
+// gathers through a 5-D tensor map (channel in the group, gate, group, time, batch) into the same dense tile.  The
+// gate biases (same column layout, fp32) are added in the kernel, pre-scaled for the sigmoid.
 struct GateBias {
   float2 r[2], i[2];
 };
-__device__ __forceinline__ int grouped_col(int d0, int bw) { return (d0 / bw) * 2 * bw + d0 % bw; }
+__device__ __forceinline__ int grouped_col(int d, int bw) { return (d / bw) * 2 * bw + d % bw; }
 template <bool HALF_IO>
-__device__ __forceinline__ void load_gate_bias(const float* bias, int rcol, int icol, GateBias& gb) {
+__device__ __forceinline__ void load_gate_bias(const float* bias, int d, int D, int bw, GateBias& gb) {
   const float sc = gate_bias_scale<HALF_IO>();
   float4 br = make_float4(0.f, 0.f, 0.f, 0.f), bi = br;
-  if (bias) {
-    br = *reinterpret_cast<const float4*>(bias + rcol);
-    bi = *reinterpret_cast<const float4*>(bias + icol);
+  if (bias && d < D) {
+    const int col = grouped_col(d, bw);
+    br = *reinterpret_cast<const float4*>(bias + col);
+    bi = *reinterpret_cast<const float4*>(bias + col + bw);
   }
   gb.r[0] = make_float2(br.x * sc, br.y * sc); gb.r[1] = make_float2(br.z * sc, br.w * sc);
   gb.i[0] = make_float2(bi.x * sc, bi.y * sc); gb.i[1] = make_float2(bi.z * sc, bi.w * sc);
 }
+// The tile of one gate (which: 0 recurrence, 1 input) of the channels from d0 on, at time t of batch row b.
+template <bool GROUPED, int CH>
+struct GateTile {
+  int col, group, step;      // first column of a wide group, or first group of a narrow one (step 0)
+  __device__ __forceinline__ GateTile(int d0, int bw)
+      : col(GROUPED ? grouped_col(d0, bw) : d0), group(GROUPED ? d0 / bw : 0), step(GROUPED && bw >= CH ? bw : 0) {}
+  __device__ __forceinline__ void load(void* dst, const void* map, int which, int t, int b, uint64_t* bar) const {
+    if (!GROUPED || step) tma_load_3d(dst, map, col + which * step, t, b, bar);
+    else tma_load_5d(dst, map, 0, which, group, t, b, bar);
+  }
+  __device__ __forceinline__ void prefetch(const void* map, int which, int t, int b) const {
+    if (!GROUPED || step) tma_prefetch_3d(map, col + which * step, t, b);
+    else tma_prefetch_5d(map, 0, which, group, t, b);
+  }
+  __device__ __forceinline__ void store(const void* map, const void* src, int which, int t, int b) const {
+    if (!GROUPED || step) tma_store_3d(map, src, col + which * step, t, b);
+    else tma_store_5d(map, src, 0, which, group, t, b);
+  }
+};
 
 // Taps of the width-4 causal depthwise conv for the four channels a thread owns (column 3 of the
 // [D, 4] weight multiplies the current token; griffin/griffin.py:474-486 of the reference).
@@ -402,8 +425,7 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
   const int rounds = SPLIT ? (nchunks + nranks - 1) / nranks : nchunks;
   const int mine = SPLIT ? (nchunks - rank + nranks - 1) / nranks : nchunks;   // chunks this CTA loads and stores
   static_assert(!GROUPED || USE_TMA, "the grouped gate layout is staged by TMA only");
-  const int rcol = GROUPED ? grouped_col(d0, p.gate_bw) : d0;   // first column of this tile's u_r / u_i
-  const int icol = GROUPED ? rcol + p.gate_bw : d0;
+  const GateTile<GROUPED, CH> gate(d0, p.gate_bw);
 
   auto issue = [&](int it) {
     const int sidx = it % NSTAGE;
@@ -416,8 +438,8 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
       tma_load_5d(st + SM::TILEX + SM::TILE, &maps.ui, d0, 0, 0, k * (TC / 8), b, &full[sidx]);
     } else {
       tma_load_3d(st, &maps.x, d0, k * TC - (CONV ? 3 : 0), b, &full[sidx]);   // rows before t = 0 read as zero
-      tma_load_3d(st + SM::TILEX, &maps.ur, rcol, k * TC, b, &full[sidx]);
-      tma_load_3d(st + SM::TILEX + SM::TILE, &maps.ui, icol, k * TC, b, &full[sidx]);
+      gate.load(st + SM::TILEX, &maps.ur, 0, k * TC, b, &full[sidx]);
+      gate.load(st + SM::TILEX + SM::TILE, &maps.ui, 1, k * TC, b, &full[sidx]);
       if (MERGE) tma_load_3d(st + SM::OFF_G, &maps.g, d0, k * TC, b, &full[sidx]);
     }
   };
@@ -440,8 +462,8 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
         tma_prefetch_5d(&maps.ui, d0, 0, 0, rank * (TC / 8), b);
       } else {
         tma_prefetch_3d(&maps.x, d0, rank * TC - (CONV ? 3 : 0), b);
-        tma_prefetch_3d(&maps.ur, rcol, rank * TC, b);
-        tma_prefetch_3d(&maps.ui, icol, rank * TC, b);
+        gate.prefetch(&maps.ur, 0, rank * TC, b);
+        gate.prefetch(&maps.ui, 1, rank * TC, b);
         if (MERGE) tma_prefetch_3d(&maps.g, d0, rank * TC, b);
       }
     }
@@ -489,7 +511,7 @@ __device__ __forceinline__ void rglru_fwd_body(const FwdMaps& maps, const ScanFw
   ConvTaps ct;
   if (CONV) load_taps(p.conv_w, p.conv_b, d0 + vec * CV, p.D, ct);
   GateBias gb;
-  if (GROUPED) load_gate_bias<sizeof(IO) == 2>(p.gate_bias, rcol + vec * CV, icol + vec * CV, gb);
+  if (GROUPED) load_gate_bias<sizeof(IO) == 2>(p.gate_bias, d0 + vec * CV, p.D, p.gate_bw, gb);
 
   // Level-two chain: SEGS threads per channel (thread tid: channel d0 + tid % CH, lane segment tid / CH), each
   // of which carries the channel's state across chunks (identical copies).
@@ -935,8 +957,7 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
   const int rounds = SPLIT ? (nchunks + nranks - 1) / nranks : nchunks;
   const int mine = SPLIT ? (nchunks - rank + nranks - 1) / nranks : nchunks;   // chunks this CTA loads and stores
   static_assert(!GROUPED || USE_TMA, "the grouped gate layout is staged by TMA only");
-  const int rcol = GROUPED ? grouped_col(d0, p.gate_bw) : d0;   // first column of this tile's u_r / u_i (and du_r / du_i)
-  const int icol = GROUPED ? rcol + p.gate_bw : d0;
+  const GateTile<GROUPED, CH> gate(d0, p.gate_bw);
 
   auto issue = [&](int q) {  // this CTA's q-th chunk in processing order, which runs from the end of the sequence
     const int k = nchunks - 1 - (q * nranks + rank);
@@ -945,8 +966,8 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
     mbar_expect_tx(&full[sidx], SM::STAGE);
     tma_load_3d(st, &maps.dy, d0, k * TC, b, &full[sidx]);
     tma_load_3d(st + SM::OFF_X, &maps.x, d0, k * TC - (CONV ? 3 : 0), b, &full[sidx]);
-    tma_load_3d(st + SM::OFF_UR, &maps.ur, rcol, k * TC, b, &full[sidx]);
-    tma_load_3d(st + SM::OFF_UI, &maps.ui, icol, k * TC, b, &full[sidx]);
+    gate.load(st + SM::OFF_UR, &maps.ur, 0, k * TC, b, &full[sidx]);
+    gate.load(st + SM::OFF_UI, &maps.ui, 1, k * TC, b, &full[sidx]);
     if (MERGE) tma_load_3d(st + SM::OFF_G, &maps.g, d0, k * TC, b, &full[sidx]);
   };
   auto store = [&](int q) {
@@ -954,8 +975,8 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
     uint8_t* st = smem + (q % NSTAGE) * SM::STAGE;
     if (!CARRY) {
       tma_store_3d(&maps.dx, st + SM::OFF_X + SM::HALO, d0, k * TC, b);
-      tma_store_3d(&maps.dur, st + SM::OFF_UR, rcol, k * TC, b);
-      tma_store_3d(&maps.dui, st + SM::OFF_UI, icol, k * TC, b);
+      gate.store(&maps.dur, st + SM::OFF_UR, 0, k * TC, b);
+      gate.store(&maps.dui, st + SM::OFF_UI, 1, k * TC, b);
       if (MERGE) tma_store_3d(&maps.dg, st + SM::OFF_G, d0, k * TC, b);
     }
     tma_commit();
@@ -981,8 +1002,8 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
       const int kl = nchunks - 1 - rank;
       tma_prefetch_3d(&maps.dy, d0, kl * TC, b);
       tma_prefetch_3d(&maps.x, d0, kl * TC - (CONV ? 3 : 0), b);
-      tma_prefetch_3d(&maps.ur, rcol, kl * TC, b);
-      tma_prefetch_3d(&maps.ui, icol, kl * TC, b);
+      gate.prefetch(&maps.ur, 0, kl * TC, b);
+      gate.prefetch(&maps.ui, 1, kl * TC, b);
       if (MERGE) tma_prefetch_3d(&maps.g, d0, kl * TC, b);
     }
   }
@@ -1032,7 +1053,7 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
   ConvTaps ct;
   if (CONV) load_taps(p.conv_w, p.conv_b, d0 + vec * CV, p.D, ct);
   GateBias gb;
-  if (GROUPED) load_gate_bias<sizeof(IO) == 2>(p.gate_bias, rcol + vec * CV, icol + vec * CV, gb);
+  if (GROUPED) load_gate_bias<sizeof(IO) == 2>(p.gate_bias, d0 + vec * CV, p.D, p.gate_bw, gb);
 
   float2 dlam[2] = {f2(0.0f), f2(0.0f)};
   float2 dsr[2] = {f2(0.0f), f2(0.0f)}, dsi[2] = {f2(0.0f), f2(0.0f)};   // grouped layout: sums over time of du_r, du_i
@@ -1206,7 +1227,7 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
     for (int j = 0; j < LANES; ++j) acc += plane[j * CH + cch];
     if constexpr (SPLIT) { st_cluster_f32(cluster_map(&split.sm->sums[rank][tid], 0), acc); }
     else if (which == 0) p.dlam_part[static_cast<size_t>(b) * p.D + dch] = acc;
-    else if (p.dgate_part) p.dgate_part[static_cast<size_t>(b) * 2 * p.D + (which == 1 ? rcol : icol) + cch] = acc;
+    else if (p.dgate_part) p.dgate_part[static_cast<size_t>(b) * 2 * p.D + grouped_col(dch, p.gate_bw) + (which - 1) * p.gate_bw] = acc;
   }
   if constexpr (SPLIT) {     // rank 0 folds the sums of the cluster in rank order
     __syncwarp();
@@ -1217,7 +1238,7 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
       float acc = 0.0f;
       for (int r = 0; r < nranks; ++r) acc += split.sm->sums[r][tid];
       if (which == 0) p.dlam_part[static_cast<size_t>(b) * p.D + dch] = acc;
-      else if (p.dgate_part) p.dgate_part[static_cast<size_t>(b) * 2 * p.D + (which == 1 ? rcol : icol) + cch] = acc;
+      else if (p.dgate_part) p.dgate_part[static_cast<size_t>(b) * 2 * p.D + grouped_col(dch, p.gate_bw) + (which - 1) * p.gate_bw] = acc;
     }
   }
   if (!p.ticket) { drain(); return; }   // the caller folds the rows with rglru_dlambda_kernel
@@ -1268,7 +1289,7 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
     }
   }
   if (GROUPED && p.dgate && p.dgate_part) {     // gate-bias gradient: column sums of du over the batch rows
-    const int N2 = 2 * p.D;                     // a multiple of 4: the grouped layout needs 64-channel gate heads
+    const int N2 = 2 * p.D;                     // a multiple of 4: groups of four channels or more
     for (int d = tid * 4; d < N2; d += NCOMP * 4) {
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
       for (int r0 = 0; r0 < p.B; r0 += 8) {

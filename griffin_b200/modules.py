@@ -55,6 +55,12 @@ def _largest_block_count(width: int, requested: int) -> int:
     return count
 
 
+def _is_stock(layer: nn.Module, kind: type) -> bool:
+    """Whether a submodule is the one this package put there: not replaced, not parametrised, without hooks."""
+    return type(layer) is kind and not (layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks
+                                        or layer._backward_pre_hooks)
+
+
 class BlockDiagonalLinear(nn.Module):
     """Gate projection with independent diagonal blocks (griffin/griffin.py:129-154).
 
@@ -168,6 +174,24 @@ class RG_LRU(nn.Module):
             target = torch.empty_like(self.Lambda).uniform_(0.9, 0.999)
             self.Lambda.copy_(torch.logit(target.pow(1.0 / self.c)))
 
+    def _gates_in_node(self, xt: Tensor) -> bool:
+        """Whether both gate projections run inside the scan's autograd node (``ops.rglru_gated``).  Heads of a multiple of 64
+        channels always do; of other widths, wherever the projections called as modules would compute the same thing:
+        this package's own layers, in the dtype of ``xt`` or cast to it by autocast."""
+        r, i = self.recurrence_gate, self.input_gate
+        if not self.group_gates:
+            return False
+        if ops.grouped_gates_supported(xt, r.block_width):
+            return True
+        if not (ops.gated_supported(xt, r.block_width) and _is_stock(r, BlockDiagonalLinear) and _is_stock(i, BlockDiagonalLinear)):
+            return False
+        params = (r.weight, r.bias, i.weight, i.bias)
+        if torch.is_autocast_enabled("cuda"):
+            alike = xt.dtype == torch.get_autocast_dtype("cuda") and all(t.dtype in (torch.float32, xt.dtype) for t in params)
+        else:
+            alike = all(t.dtype == xt.dtype for t in params)
+        return alike and all(t.device == xt.device for t in params)
+
     def forward(self, xt: Tensor, ht_minus_1: Optional[Tensor] = None, *, reset_mask: Optional[Tensor] = None,
                 active_mask: Optional[Tensor] = None, return_state: bool = False, _flags: Optional[Tensor] = None,
                 _branch: Optional[Tensor] = None):
@@ -194,10 +218,10 @@ class RG_LRU(nn.Module):
             raise TypeError(f"scan_mode='cuda' supports float32 and bfloat16 activations, got {xt.dtype}")
 
         flags = _flags if _flags is not None else token_flags(batch, steps, xt.device, reset=reset_mask, active=active_mask)
-        if self.group_gates and ops.grouped_gates_supported(xt, self.recurrence_gate.block_width):
-            yt, h_last = ops.rglru_grouped(xt, self.recurrence_gate.weight, self.recurrence_gate.bias,
-                                           self.input_gate.weight, self.input_gate.bias, self.Lambda, ht_minus_1, flags,
-                                           self.c, _branch)
+        if self._gates_in_node(xt):
+            yt, h_last = ops.rglru_gated(xt, self.recurrence_gate.weight, self.recurrence_gate.bias,
+                                         self.input_gate.weight, self.input_gate.bias, self.Lambda, ht_minus_1, flags,
+                                         self.c, _branch)
             return (yt, h_last) if return_state else yt
         u_r = self.recurrence_gate(xt).to(xt.dtype)
         u_i = self.input_gate(xt).to(xt.dtype)
@@ -347,12 +371,6 @@ def _shared_between_blocks(owners: tuple, device, build):
             _MASK_PLANS.clear()
         _MASK_PLANS[key] = (stamps, value)
     return value
-
-
-def _is_stock(layer: nn.Module, kind: type) -> bool:
-    """Whether a submodule is the one this package put there: not replaced, not parametrised, without hooks."""
-    return type(layer) is kind and not (layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks
-                                        or layer._backward_pre_hooks)
 
 
 def _project(layer: nn.Module, x: Tensor) -> Tensor:

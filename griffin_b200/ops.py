@@ -565,12 +565,63 @@ def _aligned16(t: Optional[Tensor]) -> Optional[Tensor]:
     return t if t is None or t.data_ptr() % 16 == 0 else t.clone()
 
 
-def _stacked_gates(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor) -> tuple[Tensor, Tensor]:
-    """The two [G, bw, bw] gate weights stacked per head in the activation dtype, and the biases [2 D] fp32 in the
-    same column layout."""
-    wcat = torch.cat([w_r, w_i], dim=1).to(x.dtype)                                   # [G, 2 bw, bw]
-    bias = torch.cat([b_r, b_i], dim=1).to(torch.float32).reshape(-1).contiguous()    # [2 D]
-    return wcat, bias
+def _aligned_dense(t: Optional[Tensor]) -> Optional[Tensor]:
+    """``t`` as a contiguous tensor on a 16-byte boundary (a copy where it is not one)."""
+    return None if t is None else _aligned16(t.contiguous())
+
+
+def _gate_group(head_width: int, element_size: int) -> int:
+    """Channels per column group of the gate tensor (see ``rglru_gated_fwd``): the largest power of two up to 64 that divides
+    the head width; 0 where such a group would be less than 16 bytes."""
+    group = min(head_width & -head_width, 64)
+    return group if group * element_size >= 16 else 0
+
+
+def gated_supported(x: Tensor, head_width: int) -> bool:
+    """Whether :func:`rglru_gated` applies: CUDA tensors and gate heads of whole 16-byte groups (four fp32 or eight bf16
+    channels)."""
+    return x.is_cuda and _gate_group(head_width, x.element_size()) > 0
+
+
+def _packed_gates(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor) -> tuple[Tensor, Tensor]:
+    """The two [G, bw, bw] gate weights as one [G, 2 bw, bw] operand in the activation dtype whose rows alternate between
+    the gates in column groups, and [3 D] fp32: the biases in that order, then Lambda (``rglru_gate_pack``)."""
+    G, bw, _ = w_r.shape
+    if w_r.dtype != w_i.dtype or w_r.dtype not in _DTYPES:
+        w_r, w_i = w_r.float(), w_i.float()
+    if b_r.dtype != b_i.dtype or b_r.dtype not in _DTYPES:
+        b_r, b_i = b_r.float(), b_i.float()
+    if lam.dtype not in _DTYPES:
+        lam = lam.float()
+    w_r, w_i, b_r, b_i, lam = _aligned_dense(w_r), _aligned_dense(w_i), b_r.contiguous(), b_i.contiguous(), lam.contiguous()
+    _require_cuda(w_r, b_r, w_i, b_i, lam)
+    D = G * bw
+    wcat = torch.empty(G, 2 * bw, bw, device=x.device, dtype=x.dtype)
+    params = torch.empty(3 * D, device=x.device, dtype=torch.float32)
+    rc = _lib.load().rglru_gate_pack(_ptr(w_r), _ptr(b_r), _ptr(w_i), _ptr(b_i), _ptr(lam), _ptr(wcat), _ptr(params), D, bw,
+                                     _gate_group(bw, x.element_size()), _DTYPES[w_r.dtype], _DTYPES[b_r.dtype],
+                                     _DTYPES[lam.dtype], _DTYPES[x.dtype], _stream(x))
+    _lib.check(rc, "rglru_gate_pack")
+    return wcat, params
+
+
+def _unpacked_gate_grads(dw: Tensor, dbias: Tensor, dlam: Tensor, dtypes: tuple) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor]:
+    """Gradients of (w_r, b_r, w_i, b_i, Lambda) in their dtypes from ``dw`` [splits, G, 2 bw, bw], ``dbias`` [G, 2 bw] and
+    ``dlam`` [D] (``rglru_gate_unpack``)."""
+    splits, G, bw2, bw = dw.shape
+    device = dw.device
+    kernel = [t if t in _DTYPES else torch.float32 for t in dtypes]
+    wt = kernel[0] if kernel[0] == kernel[2] else torch.float32
+    bt = kernel[1] if kernel[1] == kernel[3] else torch.float32
+    dw_r, dw_i = (torch.empty(G, bw, bw, device=device, dtype=wt) for _ in range(2))
+    db_r, db_i = (torch.empty(G, bw, device=device, dtype=bt) for _ in range(2))
+    dl = torch.empty(G * bw, device=device, dtype=kernel[4])
+    with _on(dw, "rglru_gate_unpack"):
+        rc = _lib.load().rglru_gate_unpack(_ptr(dw), splits, _ptr(dbias), _ptr(dlam), _ptr(dw_r), _ptr(db_r), _ptr(dw_i),
+                                           _ptr(db_i), _ptr(dl), G * bw, bw, _gate_group(bw, dw.element_size()),
+                                           _DTYPES[dw.dtype], _DTYPES[wt], _DTYPES[bt], _DTYPES[dl.dtype], _stream(dw))
+    _lib.check(rc, "rglru_gate_unpack")
+    return tuple(g if g.dtype == t else g.to(t) for g, t in zip((dw_r, db_r, dw_i, db_i, dl), dtypes))
 
 
 def _grouped_fwd_impl(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor, h0: Optional[Tensor],
@@ -578,20 +629,22 @@ def _grouped_fwd_impl(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Ten
                  ) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor, Tensor]:
     """Gate projections + RG-LRU (+ optional GeLU-branch product) around ONE grouped GEMM.
 
-    The two [G, bw, bw] gate weights are stacked per head and a single batched GEMM writes both gate
-    pre-activations straight into a [B, T, G, 2 bw] tensor (cuBLAS takes the strided output, so there is no
-    re-layout pass); the kernels read that layout, add the biases themselves and return the gradient in the
+    The two [G, bw, bw] gate weights are stacked per head, their output rows alternating in groups, and a single batched
+    GEMM writes both gate pre-activations straight into a [B, T, G, 2 bw] tensor (cuBLAS takes the strided output, so
+    there is no re-layout pass); the kernels read that layout, add the biases themselves and return the gradient in the
     same layout, from which two more batched GEMMs give the input and weight gradients.
     Reference: BlockDiagonalLinear griffin/griffin.py:129-154 called twice at :237-238.
-    Returns (out, h_last, the gate tensor u, the workspace, the stacked weights, the stacked biases); the last four
-    are what the backward needs beside the inputs."""
+    Returns (out, h_last, the gate tensor u, the workspace, the stacked weights, the stacked biases and Lambda in fp32);
+    the last four are what the backward needs beside the inputs."""
     lib = _lib.load()
     with torch.autocast("cuda", enabled=False):
         x = _aligned16(x)
         B, T, D = x.shape
         G, bw, _ = w_r.shape
         dt = _io_dtype(x, "grouped forward")
-        wcat, bias = _stacked_gates(x, w_r, b_r, w_i, b_i)
+        group = _gate_group(bw, x.element_size())
+        with _on(x, "rglru_gate_pack"):
+            wcat, params = _packed_gates(x, w_r, b_r, w_i, b_i, lam)
         rows = x.view(B * T, G, bw).transpose(0, 1)                                       # [G, N, bw] view
         u = torch.empty(B, T, 2 * D, device=x.device, dtype=x.dtype)
         torch.bmm(rows, wcat.transpose(1, 2), out=u.view(B * T, G, 2 * bw).transpose(0, 1))
@@ -600,12 +653,12 @@ def _grouped_fwd_impl(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Ten
         h_last = torch.empty(B, D, device=x.device, dtype=torch.float32)
         nbytes = lib.rglru_workspace_bytes(B, T, D, dt) if save else 0
         ws = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
-        with _on(x, "rglru_grouped_fwd"):
-            rc = lib.rglru_grouped_fwd(_ptr(x), _ptr(u), _ptr(bias), _ptr(branch), _ptr(lam), _ptr(h0), _ptr(tok),
-                                       _ptr(out), _ptr(h_last), _ptr(ws) if save else None, nbytes, B, T, D, bw,
-                                       c, dt, _stream(x))
-        _lib.check(rc, "rglru_grouped_fwd")
-    return out, h_last, u, ws, wcat, bias
+        with _on(x, "rglru_gated_fwd"):
+            rc = lib.rglru_gated_fwd(_ptr(x), _ptr(u), _ptr(params), _ptr(branch), _ptr(params) + 8 * D, _ptr(h0), _ptr(tok),
+                                     _ptr(out), _ptr(h_last), _ptr(ws) if save else None, nbytes, B, T, D, group, c, dt,
+                                     _stream(x))
+        _lib.check(rc, "rglru_gated_fwd")
+    return out, h_last, u, ws, wcat, params
 
 
 _grouped_fwd = torch.library.custom_op("griffin_b200::grouped_fwd", _grouped_fwd_impl, mutates_args=())
@@ -617,16 +670,32 @@ def _(x, w_r, b_r, w_i, b_i, lam, h0, tok, c, branch, save):
     G, bw, _ = w_r.shape
     return (torch.empty_like(x), x.new_empty((B, D), dtype=torch.float32), x.new_empty((B, T, 2 * D)),
             x.new_empty((workspace_bytes(B, T, D) if save else 0,), dtype=torch.uint8),
-            x.new_empty((G, 2 * bw, bw)), x.new_empty((2 * D,), dtype=torch.float32))
+            x.new_empty((G, 2 * bw, bw)), x.new_empty((3 * D,), dtype=torch.float32))
 
 
-def _grouped_bwd_impl(dout: Tensor, dh_last: Optional[Tensor], x: Tensor, u: Tensor, wcat: Tensor, bias: Tensor,
-                 branch: Optional[Tensor], lam: Tensor, h0: Optional[Tensor], tok: Optional[Tensor],
-                 ws: Tensor, c: float, want_dh0: bool
-                 ) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor, Tensor]:
-    """(dx, d stacked weights [G, 2 bw, bw], d stacked biases [G, 2 bw] fp32, dLambda, dh0, dbranch) from the stacked
-    weights and biases the forward built; absent results are empty tensors.  The caller slices the two stacked
-    gradients into the gates' own."""
+def _gate_weight_grad(du: Tensor, x: Tensor, G: int, bw: int) -> Tensor:
+    """d stacked weights [splits, G, 2 bw, bw] from the gate tensor's gradient: one batched GEMM for bf16; for fp32, where
+    the library's GEMM walks all tokens with the few CTAs so small an output gives, ``rglru_gate_dw``, whose partial
+    sums over stretches of the tokens are left for the caller to add."""
+    rows, D = du.shape[0] * du.shape[1], G * bw
+    if du.dtype != torch.float32:
+        return torch.bmm(du.view(rows, G, 2 * bw).transpose(0, 1).transpose(1, 2), x.view(rows, G, bw).transpose(0, 1))[None]
+    lib = _lib.load()
+    splits = lib.rglru_gate_dw_splits(rows, D, bw)
+    dw = torch.empty(splits, G, 2 * bw, bw, device=du.device, dtype=torch.float32)
+    with _on(x, "rglru_gate_dw"):
+        rc = lib.rglru_gate_dw(_ptr(du), _ptr(x), _ptr(dw), splits, rows, D, bw, _stream(x))
+    _lib.check(rc, "rglru_gate_dw")
+    return dw
+
+
+def _grouped_bwd_parts(dout: Tensor, dh_last: Optional[Tensor], x: Tensor, u: Tensor, wcat: Tensor, bias: Tensor,
+                       branch: Optional[Tensor], lam: Tensor, h0: Optional[Tensor], tok: Optional[Tensor],
+                       ws: Tensor, c: float, want_dh0: bool
+                       ) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor, Tensor]:
+    """(dx, d stacked weights [splits, G, 2 bw, bw], d stacked biases [G, 2 bw] fp32, dLambda, dh0, dbranch) from the stacked
+    weights and biases the forward built; absent results are empty tensors.  The caller takes the two stacked
+    gradients apart into the gates' own."""
     lib = _lib.load()
     with torch.autocast("cuda", enabled=False):
         x = _aligned16(x)
@@ -641,17 +710,26 @@ def _grouped_bwd_impl(dout: Tensor, dh_last: Optional[Tensor], x: Tensor, u: Ten
         dlam = torch.empty(D, device=x.device, dtype=torch.float32)
         dh0 = torch.empty((B, D) if want_dh0 else (0,), device=x.device, dtype=torch.float32)
         dbias = torch.empty(G, bw2, device=x.device, dtype=torch.float32)    # [2 D] in the gate tensor's column layout
-        with _on(x, "rglru_grouped_bwd"):
-            rc = lib.rglru_grouped_bwd(_ptr(dout), _ptr(dh_last), _ptr(x), _ptr(u), _ptr(bias), _ptr(branch),
-                                       _ptr(lam), _ptr(h0), _ptr(tok), _ptr(ws), ws.numel(), _ptr(dx), _ptr(du),
-                                       _ptr(dbranch) if branch is not None else None, _ptr(dlam),
-                                       _ptr(dh0) if want_dh0 else None, _ptr(dbias), B, T, D, bw, c, dt, _stream(x))
-        _lib.check(rc, "rglru_grouped_bwd")
+        with _on(x, "rglru_gated_bwd"):
+            rc = lib.rglru_gated_bwd(_ptr(dout), _ptr(dh_last), _ptr(x), _ptr(u), _ptr(bias), _ptr(branch),
+                                     _ptr(lam), _ptr(h0), _ptr(tok), _ptr(ws), ws.numel(), _ptr(dx), _ptr(du),
+                                     _ptr(dbranch) if branch is not None else None, _ptr(dlam),
+                                     _ptr(dh0) if want_dh0 else None, _ptr(dbias), B, T, D,
+                                     _gate_group(bw, x.element_size()), c, dt, _stream(x))
+        _lib.check(rc, "rglru_gated_bwd")
         dg = du.view(B * T, G, bw2).transpose(0, 1)                    # [G, N, 2 bw] view
-        rows = x.view(B * T, G, bw).transpose(0, 1)                    # [G, N, bw] view
         dx.view(B * T, G, bw).transpose(0, 1).baddbmm_(dg, wcat)       # gate path added onto the direct path
-        dwcat = torch.bmm(dg.transpose(1, 2), rows)                    # [G, 2 bw, bw]
-    return dx, dwcat, dbias, dlam, dh0, dbranch
+        dw = _gate_weight_grad(du, x, G, bw)
+    return dx, dw, dbias, dlam, dh0, dbranch
+
+
+def _grouped_bwd_impl(dout: Tensor, dh_last: Optional[Tensor], x: Tensor, u: Tensor, wcat: Tensor, bias: Tensor,
+                 branch: Optional[Tensor], lam: Tensor, h0: Optional[Tensor], tok: Optional[Tensor],
+                 ws: Tensor, c: float, want_dh0: bool
+                 ) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor, Tensor]:
+    """:func:`_grouped_bwd_parts` with the weight gradient's stretches added up: [G, 2 bw, bw]."""
+    dx, dw, dbias, dlam, dh0, dbranch = _grouped_bwd_parts(dout, dh_last, x, u, wcat, bias, branch, lam, h0, tok, ws, c, want_dh0)
+    return dx, dw.sum(0) if dw.shape[0] > 1 else dw[0].clone(), dbias, dlam, dh0, dbranch
 
 
 _grouped_bwd = torch.library.custom_op("griffin_b200::grouped_bwd", _grouped_bwd_impl, mutates_args=())
@@ -669,9 +747,9 @@ def _(dout, dh_last, x, u, wcat, bias, branch, lam, h0, tok, ws, c, want_dh0):
 def _grouped_setup(ctx, inputs, output):
     x, w_r, b_r, w_i, b_i, lam, h0, tok, c, branch, save = inputs
     _, _, u, ws, wcat, bias = output
-    ctx.save_for_backward(x, u, wcat, bias, branch, lam, h0, tok, ws)
+    ctx.save_for_backward(x, u, wcat, bias, branch, lam if lam.dtype == torch.float32 else None, h0, tok, ws)
     ctx.c, ctx.saved = c, save
-    ctx.param_dtypes = (w_r.dtype, b_r.dtype, w_i.dtype, b_i.dtype)
+    ctx.param_dtypes = (w_r.dtype, b_r.dtype, w_i.dtype, b_i.dtype, lam.dtype)
     ctx.want_dh0 = h0 is not None and ctx.needs_input_grad[6]
 
 
@@ -681,21 +759,30 @@ def _grouped_backward(ctx, dout, dh_last, _du, _dws, _dwcat, _dbias, _bwd=None):
     x, u, wcat, bias, branch, lam, h0, tok, ws = ctx.saved_tensors
     dout = torch.zeros_like(x) if dout is None else dout.to(x.dtype).contiguous()
     dh_last = None if dh_last is None else dh_last.to(torch.float32).contiguous()
-    dx, dwcat, dbias, dlam, dh0, dbranch = (_bwd or _grouped_bwd)(
+    if lam is None:                       # the fp32 copy the forward left behind the biases
+        lam = bias[2 * x.shape[2]:]
+    dx, dw, dbias, dlam, dh0, dbranch = (_bwd or _grouped_bwd)(
         dout, dh_last, x, u, wcat, bias, branch, lam, h0, tok, ws, ctx.c, ctx.want_dh0)
-    bw = wcat.shape[2]
-    dt_wr, dt_br, dt_wi, dt_bi = ctx.param_dtypes
-    return (dx, dwcat[:, :bw].to(dt_wr), dbias[:, :bw].to(dt_br), dwcat[:, bw:].to(dt_wi), dbias[:, bw:].to(dt_bi),
-            dlam, (dh0 if ctx.want_dh0 else None), None, None, (dbranch if branch is not None else None), None)
+    if _bwd is None:                      # traced: the same by views and casts
+        G, bw2, bw = wcat.shape
+        shape = (G, -1, 2, _gate_group(bw, x.element_size()))
+        w, b = dw.view(*shape, bw), dbias.view(shape)
+        dt_wr, dt_br, dt_wi, dt_bi, _ = ctx.param_dtypes
+        dw_r, dw_i = w[:, :, 0].reshape(G, bw, bw).to(dt_wr), w[:, :, 1].reshape(G, bw, bw).to(dt_wi)
+        db_r, db_i = b[:, :, 0].reshape(G, bw).to(dt_br), b[:, :, 1].reshape(G, bw).to(dt_bi)
+    else:
+        dw_r, db_r, dw_i, db_i, dlam = _unpacked_gate_grads(dw, dbias, dlam, ctx.param_dtypes)
+    return (dx, dw_r, db_r, dw_i, db_i, dlam, (dh0 if ctx.want_dh0 else None), None, None,
+            (dbranch if branch is not None else None), None)
 
 
 _grouped_fwd.register_autograd(_grouped_backward, setup_context=_grouped_setup)
-_GroupedNode = _eager_node("GroupedRGLRU", _grouped_fwd_impl, _grouped_setup, _grouped_backward, _grouped_bwd_impl)
+_GroupedNode = _eager_node("GroupedRGLRU", _grouped_fwd_impl, _grouped_setup, _grouped_backward, _grouped_bwd_parts)
 
 
-def rglru_grouped(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor,
-                  h0: Optional[Tensor] = None, tok: Optional[Tensor] = None, c: float = 8.0,
-                  branch: Optional[Tensor] = None) -> tuple[Tensor, Tensor]:
+def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor,
+                h0: Optional[Tensor] = None, tok: Optional[Tensor] = None, c: float = 8.0,
+                branch: Optional[Tensor] = None) -> tuple[Tensor, Tensor]:
     """y, h_last = RG-LRU(x) with both block-diagonal gate projections (weights [G, out, in], biases [G, out])
     computed inside the node by one grouped GEMM; with ``branch`` the first result is y * gelu_tanh(branch)."""
     if x.dim() != 3:
@@ -707,16 +794,28 @@ def rglru_grouped(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor,
         raise ValueError("Lambda must have shape [width]")
     if branch is not None and branch.shape != x.shape:
         raise ValueError("branch must have the shape of x")
-    if not grouped_gates_supported(x, bw):
-        raise ValueError("the grouped gate layout needs CUDA tensors, gate heads of a multiple of 64 channels and "
-                         "rows that are a multiple of 16 bytes")
+    if not gated_supported(x, bw):
+        raise ValueError("the gate layout needs CUDA tensors and gate heads of whole 16-byte groups of channels")
     save = torch.is_grad_enabled() and any(
         t is not None and t.requires_grad for t in (x, w_r, b_r, w_i, b_i, lam, h0, branch))
-    out, h_last, _, _, _, _ = (_grouped_fwd if _library_ops_active() else _GroupedNode.apply)(
-        x.contiguous(), w_r, b_r, w_i, b_i, lam.to(torch.float32).contiguous(),
+    traced = _library_ops_active()
+    if traced or lam.dtype not in _DTYPES:
+        lam = lam.to(torch.float32)
+    out, h_last, _, _, _, _ = (_grouped_fwd if traced else _GroupedNode.apply)(
+        x.contiguous(), w_r, b_r, w_i, b_i, lam.contiguous(),
         None if h0 is None else h0.to(torch.float32).contiguous(), None if tok is None else tok.contiguous(), float(c),
         None if branch is None else branch.to(x.dtype).contiguous(), save)
     return out, h_last
+
+
+def rglru_grouped(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor,
+                  h0: Optional[Tensor] = None, tok: Optional[Tensor] = None, c: float = 8.0,
+                  branch: Optional[Tensor] = None) -> tuple[Tensor, Tensor]:
+    """:func:`rglru_gated` for gate heads of a multiple of 64 channels."""
+    if x.dim() == 3 and w_r.dim() == 3 and not grouped_gates_supported(x, w_r.shape[1]):
+        raise ValueError("the grouped gate layout needs CUDA tensors, gate heads of a multiple of 64 channels and "
+                         "rows that are a multiple of 16 bytes")
+    return rglru_gated(x, w_r, b_r, w_i, b_i, lam, h0, tok, c, branch)
 
 
 def _gate(x: Tensor, weight: Tensor, bias: Tensor) -> Tensor:
@@ -954,11 +1053,6 @@ def decode_step(x: Tensor, u_r: Tensor, u_i: Tensor, lam: Tensor, h: Tensor, tok
                                    _ptr(h), _ptr(tok), _ptr(y), B, D, float(c), dt, _stream(x))
     _lib.check(rc, "rglru_decode_step")
     return y
-
-
-def _aligned_dense(t: Optional[Tensor]) -> Optional[Tensor]:
-    """``t`` as a contiguous tensor on a 16-byte boundary (a copy where it is not one)."""
-    return None if t is None else _aligned16(t.contiguous())
 
 
 def decode_block_supported(x: Tensor, gate_width: int) -> bool:

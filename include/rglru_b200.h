@@ -180,6 +180,36 @@ int rglru_grouped_bwd(const void* dout, const float* dh_last, const void* x, con
                       size_t ws_bytes, void* dx, void* du, void* dbranch, float* dlambda, float* dh0, float* d_gate_bias,
                       int B, int T, int D, int gate_width, float c, int io_dtype, void* stream);
 
+/* The same for gate heads of any width: the columns of u / du alternate between the two gates in groups of gate_width
+ * channels that divide the head width, [u_r | u_i] per group whatever head it is in.  gate_width is a multiple of 64 as
+ * above, or 4, 8, 16 or 32 with gate_width * sizeof(element) >= 16. */
+int rglru_gated_fwd(const void* x, const void* u, const float* gate_bias, const void* branch, const float* lambda,
+                    const float* h0, const uint8_t* tok, void* out, float* h_last, void* ws, size_t ws_bytes, int B,
+                    int T, int D, int gate_width, float c, int io_dtype, void* stream);
+int rglru_gated_bwd(const void* dout, const float* dh_last, const void* x, const void* u, const float* gate_bias,
+                    const void* branch, const float* lambda, const float* h0, const uint8_t* tok, void* ws,
+                    size_t ws_bytes, void* dx, void* du, void* dbranch, float* dlambda, float* dh0, float* d_gate_bias,
+                    int B, int T, int D, int gate_width, float c, int io_dtype, void* stream);
+
+/* The gate parameters into that layout and their gradients out of it (BlockDiagonalLinear, griffin/griffin.py:129-154).
+ * G = D / head_width heads; gate_width (a multiple of 4) divides head_width; every *_dtype is RGLRU_F32 or RGLRU_BF16.
+ *   rglru_gate_pack   : w_r, w_i [G, head_width, head_width], b_r, b_i [D], lambda [D] in their own types ->
+ *                       wcat [G, 2 head_width, head_width] io_dtype with the output rows in the column order of u, and
+ *                       params [3 D] fp32: the biases in that order, then lambda.
+ *   rglru_gate_unpack : dw [splits, G, 2 head_width, head_width] (io_dtype; splits > 1 are added in index order), dbias
+ *                       [2 D] and dlam [D] fp32 -> the five gradients in the parameters' types and shapes.
+ *   rglru_gate_dw     : fp32 dw[s] = the share of du^T x (per head) of the s-th of `splits` stretches of the rows; du
+ *                       [rows, 2 D], x [rows, D].  rglru_gate_dw_splits says how many stretches fill the machine.
+ * Weights, wcat, dw, du and x must be 16-byte aligned. */
+int rglru_gate_pack(const void* w_r, const void* b_r, const void* w_i, const void* b_i, const void* lambda, void* wcat,
+                    float* params, int D, int head_width, int gate_width, int weight_dtype, int bias_dtype,
+                    int lambda_dtype, int io_dtype, void* stream);
+int rglru_gate_unpack(const void* dw, int splits, const float* dbias, const float* dlam, void* dw_r, void* db_r, void* dw_i,
+                      void* db_i, void* dlambda, int D, int head_width, int gate_width, int io_dtype, int weight_dtype,
+                      int bias_dtype, int lambda_dtype, void* stream);
+int rglru_gate_dw_splits(long long rows, int D, int head_width);
+int rglru_gate_dw(const float* du, const float* x, float* dw, int splits, long long rows, int D, int head_width, void* stream);
+
 /* Raw affine scan h_t = a_t h_{t-1} + b_t on fp32 tensors: the operator
  * fused_rglru_scan(decay, current_input, initial_state) of griffin/triton_scan.py:274-276
  * (forward kernel :31-60).  decay, drive, out: [B,T,D] fp32; h0: [B,D] fp32 or NULL. */

@@ -1,0 +1,110 @@
+"""Gate heads of any width through ``ops.rglru_gated`` against the projections called as modules: column groups of 4 to 64
+channels, tiles that straddle heads, a last tile that is cut off, padding, resets, the time split, the branch product; and
+the parameters' way into and out of the layout."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _rel(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30)).item()
+
+
+def _run(layer, x, dy, h0, resets, active, branch, dh):
+    x = x.clone().requires_grad_(True)
+    h0 = h0.clone().requires_grad_(True)
+    branch = None if branch is None else branch.clone().requires_grad_(True)
+    layer.zero_grad(set_to_none=True)
+    y, h = layer(x, h0, reset_mask=resets, active_mask=active, return_state=True, _branch=branch)
+    torch.autograd.backward([y, h], [dy, dh])
+    out = [y.detach(), h.detach(), x.grad, h0.grad] + [p.grad.clone() for p in layer.parameters()]
+    return out + ([branch.grad] if branch is not None else [])
+
+
+# (batch, steps, heads, head width): fp32 groups of 4 (4, 12), 8 (8, 24, 40), 16 (16, 48), 32 (32, 96, 352), 64 (64)
+SHAPES = [(1, 1, 3, 4), (2, 70, 5, 12), (3, 64, 1, 8), (2, 129, 3, 24), (1, 1000, 2, 40), (4, 65, 7, 16), (5, 200, 3, 48),
+          (2, 64, 2, 32), (1, 300, 3, 96), (2, 130, 2, 352), (2, 80, 3, 64)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("merge", [False, True])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_any_head_width_matches_the_modules(shape, dtype, merge, monkeypatch):
+    from griffin_b200 import RG_LRU, ops
+    batch, steps, heads, bw = shape
+    if dtype == torch.bfloat16 and bw % 8:
+        pytest.skip("a group of four bf16 channels is below 16 bytes")
+    torch.manual_seed(0)
+    width = heads * bw
+    layer = RG_LRU(width, gate_blocks=heads).to(DEV)
+    with torch.no_grad():
+        layer.recurrence_gate.bias.normal_(std=0.3)
+        layer.input_gate.bias.normal_(std=0.3)
+        for p in layer.parameters():          # values that bf16 holds: both dtypes run on the same numbers
+            p.copy_(p.to(torch.bfloat16).float())
+    draw = lambda *s: torch.randn(*s, device=DEV).to(torch.bfloat16)
+    x, dy, branch = draw(batch, steps, width), draw(batch, steps, width), (draw(batch, steps, width) if merge else None)
+    h0, dh = torch.randn(batch, width, device=DEV), torch.randn(batch, width, device=DEV)
+    masked = steps > 64
+    resets = (torch.rand(batch, steps, device=DEV) < 0.05) if masked else None
+    active = (torch.arange(steps, device=DEV)[None] < torch.randint(1, steps + 1, (batch, 1), device=DEV)) if masked else None
+    used = []
+    gated = ops.rglru_gated
+    monkeypatch.setattr(ops, "rglru_gated", lambda *a, **k: used.append(1) or gated(*a, **k))
+    cast = lambda t: None if t is None else t.to(dtype)
+    got = _run(layer.to(dtype), cast(x), cast(dy), h0, resets, active, cast(branch), dh)
+    assert used == [1]
+    plain = layer.float()
+    plain.group_gates = False
+    want = _run(plain, x.float(), dy.float(), h0, resets, active, None if branch is None else branch.float(), dh)
+    assert used == [1]
+    # fp32: sums in another order.  bf16: the bound of the layer's other bf16 tests.
+    bound = 1e-5 if dtype == torch.float32 else 2e-2
+    for k, (a, b) in enumerate(zip(got, want)):
+        assert a.shape == b.shape and torch.isfinite(a).all()
+        assert _rel(a, b) <= bound, (k, _rel(a, b))
+    assert all(g.dtype == dtype for g in got[4:])
+
+
+@pytest.mark.parametrize("weights,biases,lam", [(torch.float32, torch.bfloat16, torch.float32), (torch.bfloat16, torch.float32, torch.bfloat16),
+                                                (torch.float64, torch.float16, torch.float64)])
+@pytest.mark.parametrize("io", [torch.float32, torch.bfloat16])
+def test_parameters_into_and_out_of_the_layout(weights, biases, lam, io):
+    from griffin_b200 import ops
+    torch.manual_seed(1)
+    G, bw = 3, 24
+    D, group = G * bw, 8
+    w_r, w_i = (torch.randn(G, bw, bw, device=DEV, dtype=weights) for _ in range(2))
+    b_r, b_i = (torch.randn(G, bw, device=DEV).to(biases) for _ in range(2))
+    lv = torch.randn(D, device=DEV).to(lam)
+    x = torch.empty(1, 1, D, device=DEV, dtype=io)
+    wcat, params = ops._packed_gates(x, w_r, b_r, w_i, b_i, lv)
+    stack = lambda a, c, *tail: torch.stack([a.reshape(G, -1, group, *tail), c.reshape(G, -1, group, *tail)], 2)
+    assert torch.equal(wcat, stack(w_r.float().to(io), w_i.float().to(io), bw).reshape(G, 2 * bw, bw))
+    assert torch.equal(params, torch.cat([stack(b_r.float(), b_i.float()).reshape(-1), lv.float()]))
+    dw = wcat[None] if io == torch.bfloat16 else torch.stack([wcat * (k + 1) for k in range(11)])
+    scale = 1.0 if io == torch.bfloat16 else 66.0
+    back = ops._unpacked_gate_grads(dw, params[:2 * D].view(G, 2 * bw), params[2 * D:], (weights, biases, weights, biases, lam))
+    for g, t in zip(back, (w_r, b_r, w_i, b_i, lv)):
+        assert g.dtype == t.dtype and g.shape == t.shape
+    for g, t in ((back[0], w_r), (back[2], w_i)):
+        torch.testing.assert_close(g.double(), scale * t.float().to(io).double(), rtol=1e-2 if weights == torch.bfloat16 else 1e-6, atol=0)
+    assert torch.equal(back[1], b_r) and torch.equal(back[3], b_i)
+    torch.testing.assert_close(back[4].double(), lv.double(), rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("rows,heads,bw", [(1, 1, 4), (127, 2, 12), (129, 3, 48), (1000, 2, 72), (4099, 1, 100), (513, 2, 352)])
+def test_fp32_gate_weight_gradient(rows, heads, bw):
+    """Against float64.  Each of the two levels adds fewer than 4,200 fp32 products in order: a relative error of a few
+    roundings of 6e-8 norm-wise, 1e-6 at most."""
+    from griffin_b200 import ops
+    torch.manual_seed(2)
+    du, x = torch.randn(1, rows, 2 * heads * bw, device=DEV), torch.randn(1, rows, heads * bw, device=DEV)
+    got = ops._gate_weight_grad(du, x, heads, bw).double().sum(0)
+    want = torch.einsum("ngo,ngi->goi", du[0].double().view(rows, heads, 2 * bw), x[0].double().view(rows, heads, bw))
+    assert _rel(got, want) <= 1e-6
