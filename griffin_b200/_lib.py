@@ -55,7 +55,11 @@ SIGNATURES = {
     "rglru_conv_bwd_noalloc_max_bytes": (_sz, []),
     "rglru_conv_bwd_noalloc": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),
     "rglru_column_sums_workspace_bytes": (_sz, [ctypes.c_longlong, _i]),
+    "rglru_column_sums_as": (_i, [_vp, _vp, _vp, _sz, ctypes.c_longlong, _i, _i, _i, _vp]),
     "rglru_column_sums": (_i, [_vp, _vp, _vp, _sz, ctypes.c_longlong, _i, _i, _vp]),
+    "rglru_token_plan": (_i, [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _vp]),
+    "rglru_gelu_mul_fwd": (_i, [_vp, _vp, _vp, ctypes.c_longlong, _i, _vp]),
+    "rglru_gelu_mul_bwd": (_i, [_vp, _vp, _vp, _vp, _vp, ctypes.c_longlong, _i, _vp]),
     "rglru_decode_conv": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]),
     "rglru_decode_step": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _f, _i, _vp]),
     "rglru_decode_block_workspace_bytes": (_sz, [_i, _i, _i]),

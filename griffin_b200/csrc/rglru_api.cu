@@ -822,18 +822,24 @@ size_t rglru_column_sums_workspace_bytes(long long rows, int cols) {
 
 int rglru_column_sums(const void* src, float* out, void* ws, size_t ws_bytes, long long rows, int cols, int io_dtype,
                       void* stream) {
+  return rglru_column_sums_as(src, out, ws, ws_bytes, rows, cols, io_dtype, RGLRU_F32, stream);
+}
+
+int rglru_column_sums_as(const void* src, void* out, void* ws, size_t ws_bytes, long long rows, int cols, int io_dtype,
+                         int out_dtype, void* stream) {
   if (io_dtype != RGLRU_F32 && io_dtype != RGLRU_BF16) return RGLRU_ERR_BAD_DTYPE;
+  if (out_dtype != RGLRU_F32 && out_dtype != RGLRU_BF16) return RGLRU_ERR_BAD_DTYPE;
   if (!src || !out) return RGLRU_ERR_NULL_POINTER;
   if (rows <= 0 || cols <= 0 || rows > (1ll << 40)) return RGLRU_ERR_BAD_SHAPE;
-  const bool bf16 = io_dtype == RGLRU_BF16;
+  const bool bf16 = io_dtype == RGLRU_BF16, out_bf16 = out_dtype == RGLRU_BF16;
   const size_t es = bf16 ? 2 : 4;
-  if (!aligned(src, es) || !aligned(out, 4) || !aligned(ws, 4)) return RGLRU_ERR_MISALIGNED;
+  if (!aligned(src, es) || !aligned(out, out_bf16 ? 2 : 4) || !aligned(ws, 4)) return RGLRU_ERR_MISALIGNED;
   if (!ws || ws_bytes < rglru_column_sums_workspace_bytes(rows, cols)) return RGLRU_ERR_WORKSPACE;
   int* status = nullptr;
   const int rc = device_setup(&status);
   if (rc != RGLRU_OK) return rc;
   const bool vector_ok = (static_cast<size_t>(cols) * es) % 16 == 0 && aligned(src, 16);
-  const cudaError_t e = launch_column_sums(bf16, src, out, static_cast<float*>(ws), rows, cols, vector_ok,
+  const cudaError_t e = launch_column_sums(bf16, src, out, out_bf16, static_cast<float*>(ws), rows, cols, vector_ok,
                                            static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
 }
@@ -946,6 +952,46 @@ int rglru_gate_dw(const float* du, const float* x, float* dw, int splits, long l
   a.du = du; a.x = x; a.part = dw; a.rows = rows; a.D = D; a.bw = head_width;
   const cudaError_t e = launch_gate_dw(a, splits, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
+}
+
+int rglru_token_plan(const int64_t* seg_pos, const int64_t* prev_pos, const uint8_t* active, const uint8_t* reset,
+                     int positions, uint8_t* flags, int64_t* last_pos, int B, int T, void* stream) {
+  if (!flags) return RGLRU_ERR_NULL_POINTER;
+  if (B <= 0 || T <= 0 || T > (1 << 30)) return RGLRU_ERR_BAD_SHAPE;
+  if (!aligned(seg_pos, 8) || !aligned(prev_pos, 8) || !aligned(last_pos, 8)) return RGLRU_ERR_MISALIGNED;
+  int* status = nullptr;
+  const int rc = device_setup(&status);
+  if (rc != RGLRU_OK) return rc;
+  TokenPlanArgs a = {};
+  a.seg = reinterpret_cast<const long long*>(seg_pos); a.prev = reinterpret_cast<const long long*>(prev_pos);
+  a.active = active; a.reset = reset; a.flags = flags; a.last = reinterpret_cast<long long*>(last_pos);
+  a.positions = positions != 0; a.B = B; a.T = T;
+  const cudaError_t e = launch_token_plan(a, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
+}
+
+static int gelu_mul(const GeluMulArgs& a, int io_dtype, void* stream) {
+  if (io_dtype != RGLRU_F32 && io_dtype != RGLRU_BF16) return RGLRU_ERR_BAD_DTYPE;
+  if (!a.y || !a.g || !a.out) return RGLRU_ERR_NULL_POINTER;
+  if (a.n <= 0 || a.n > (1ll << 38)) return RGLRU_ERR_BAD_SHAPE;
+  const size_t es = io_dtype == RGLRU_BF16 ? 2 : 4;
+  if (!aligned(a.y, es) || !aligned(a.g, es) || !aligned(a.dout, es) || !aligned(a.out, es) || !aligned(a.dg, es))
+    return RGLRU_ERR_MISALIGNED;
+  int* status = nullptr;
+  const int rc = device_setup(&status);
+  if (rc != RGLRU_OK) return rc;
+  const bool vector_ok = (static_cast<size_t>(a.n) * es) % 16 == 0 && aligned(a.y, 16) && aligned(a.g, 16) && aligned(a.dout, 16) &&
+                         aligned(a.out, 16) && aligned(a.dg, 16);
+  const cudaError_t e = launch_gelu_mul(io_dtype == RGLRU_BF16, a, vector_ok, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
+}
+int rglru_gelu_mul_fwd(const void* y, const void* branch, void* out, long long n, int io_dtype, void* stream) {
+  return gelu_mul(GeluMulArgs{y, branch, nullptr, out, nullptr, n}, io_dtype, stream);
+}
+int rglru_gelu_mul_bwd(const void* dout, const void* y, const void* branch, void* dy, void* dbranch, long long n, int io_dtype,
+                       void* stream) {
+  if (!dout || !dbranch) return RGLRU_ERR_NULL_POINTER;
+  return gelu_mul(GeluMulArgs{y, branch, dout, dy, dbranch, n}, io_dtype, stream);
 }
 
 size_t rglru_decode_block_workspace_bytes(int B, int D, int io_dtype) {

@@ -448,8 +448,9 @@ __global__ void __launch_bounds__(32 * COLSUM_LANES) colsum_partial_kernel(const
   }
 }
 
+template <typename OUT>
 __global__ void __launch_bounds__(32 * COLSUM_LANES) colsum_fold_kernel(const float* __restrict__ part,
-                                                                       float* __restrict__ out, int nrow, int cols) {
+                                                                       OUT* __restrict__ out, int nrow, int cols) {
   __shared__ float red[COLSUM_LANES][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + tx;
@@ -462,7 +463,7 @@ __global__ void __launch_bounds__(32 * COLSUM_LANES) colsum_fold_kernel(const fl
     float t = red[0][tx];
 #pragma unroll
     for (int l = 1; l < COLSUM_LANES; ++l) t += red[l][tx];
-    out[col] = t;
+    out[col] = Pack<OUT>::from_float(t);
   }
 }
 
@@ -478,8 +479,8 @@ int colsum_row_blocks(long long rows, int cols) {
 }
 
 template <typename IO>
-static cudaError_t column_sums_t(const void* src, float* out, float* part, long long rows, int cols, bool vector_ok,
-                                 cudaStream_t s) {
+static cudaError_t column_sums_t(const void* src, void* out, bool out_bf16, float* part, long long rows, int cols,
+                                 bool vector_ok, cudaStream_t s) {
   constexpr int V = vec_width<IO>();
   const int nblk = colsum_row_blocks(rows, cols);
   const long long per = (rows + nblk - 1) / nblk;
@@ -493,14 +494,16 @@ static cudaError_t column_sums_t(const void* src, float* out, float* part, long 
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  colsum_fold_kernel<<<(cols + 31) / 32, 32 * COLSUM_LANES, 0, s>>>(part, out, nblk, cols);
+  const int folds = (cols + 31) / 32;
+  if (out_bf16) colsum_fold_kernel<<<folds, 32 * COLSUM_LANES, 0, s>>>(part, static_cast<__nv_bfloat16*>(out), nblk, cols);
+  else colsum_fold_kernel<<<folds, 32 * COLSUM_LANES, 0, s>>>(part, static_cast<float*>(out), nblk, cols);
   return cudaGetLastError();
 }
 
-cudaError_t launch_column_sums(bool bf16, const void* src, float* out, float* part, long long rows, int cols,
+cudaError_t launch_column_sums(bool bf16, const void* src, void* out, bool out_bf16, float* part, long long rows, int cols,
                                bool vector_ok, cudaStream_t s) {
-  return bf16 ? column_sums_t<__nv_bfloat16>(src, out, part, rows, cols, vector_ok, s)
-              : column_sums_t<float>(src, out, part, rows, cols, vector_ok, s);
+  return bf16 ? column_sums_t<__nv_bfloat16>(src, out, out_bf16, part, rows, cols, vector_ok, s)
+              : column_sums_t<float>(src, out, out_bf16, part, rows, cols, vector_ok, s);
 }
 
 // ---------------------------------------------------------------- decode

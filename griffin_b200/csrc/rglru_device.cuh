@@ -314,7 +314,7 @@ __device__ __forceinline__ float2 gelu_sigmoid2(float2 v) {
   const float2 z = mul2(mul2(v, f2(GELU_K0)), fma2(mul2(v, v), f2(GELU_K1), f2(1.0f)));
   if (HALF_IO) return fma2(make_float2(tanh_approx(z.x), tanh_approx(z.y)), f2(0.5f), f2(0.5f));
   const float2 t = mul2(z, f2(-2.0f * LOG2E));
-  const float2 d = add2(make_float2(ex2_approx(fminf(t.x, 60.0f)), ex2_approx(fminf(t.y, 60.0f))), f2(1.0f));
+  const float2 d = add2(make_float2(ex2_approx(t.x), ex2_approx(t.y)), f2(1.0f));   // infinite far out: s = 0
   return make_float2(rcp_approx(d.x), rcp_approx(d.y));
 }
 // d gelu / d v = s + v s (1 - s) * 2 z',  2 z' = 2 k0 (1 + 3 k1 v^2)

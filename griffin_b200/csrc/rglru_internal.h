@@ -161,6 +161,27 @@ struct DecodeArgs {
   bool vector_ok;
 };
 
+// Masks of a call as flag bytes (see rglru_token_plan in the public header).
+struct TokenPlanArgs {
+  const long long* seg;
+  const long long* prev;
+  const uint8_t* active;
+  const uint8_t* reset;
+  uint8_t* flags;
+  long long* last;
+  bool positions;      // flags of a block call from positions, not of a bare layer from its reset mask
+  int B, T;
+};
+// out = y * gelu(g), or with dout given out = dy and dg.
+struct GeluMulArgs {
+  const void* y;
+  const void* g;
+  const void* dout;
+  void* out;
+  void* dg;
+  long long n;
+};
+
 // Gate parameters into and out of the interleaved gate layout (see rglru_gates.cu).
 struct GatePackArgs {
   const void* w_r;
@@ -232,13 +253,15 @@ int conv_tma_box_rows();
 int conv_tma_box_cols();
 cudaError_t launch_decode_conv(bool bf16, const ConvArgs& a, cudaStream_t s);
 cudaError_t launch_decode_step(bool bf16, const DecodeArgs& a, cudaStream_t s);
+cudaError_t launch_token_plan(const TokenPlanArgs& a, cudaStream_t s);
+cudaError_t launch_gelu_mul(bool bf16, const GeluMulArgs& a, bool vector_ok, cudaStream_t s);
 cudaError_t launch_gate_pack(bool f32_weights, bool bf16, const GatePackArgs& a, cudaStream_t s);
 cudaError_t launch_gate_unpack(bool bf16, bool f32_weights, const GateUnpackArgs& a, cudaStream_t s);
 cudaError_t launch_gate_dw(const GateDwArgs& a, int splits, cudaStream_t s);
 int gate_dw_splits(long long rows, int D, int bw);
 cudaError_t launch_decode_block(bool bf16, const DecodeBlockArgs& a, cudaStream_t s);
 int colsum_row_blocks(long long rows, int cols);   // partial rows a column-sum call leaves in its workspace
-cudaError_t launch_column_sums(bool bf16, const void* src, float* out, float* part, long long rows, int cols,
+cudaError_t launch_column_sums(bool bf16, const void* src, void* out, bool out_bf16, float* part, long long rows, int cols,
                                bool vector_ok, cudaStream_t s);
 
 // use_tma == false selects the bounds-checked plain-load staging path that accepts any D.

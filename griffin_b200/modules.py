@@ -93,6 +93,11 @@ def token_flags(batch: int, steps: int, device, *, reset: Optional[Tensor] = Non
     """Pack the per-token masks into the flag byte the kernels read ([B, T] uint8), or None if all are absent."""
     if reset is None and active is None and segment_pos is None:
         return None
+    if segment_pos is None and not ops._library_ops_active() and all(
+            m is None or (m.is_cuda and m.dtype == torch.bool and m.shape == (batch, steps) and m.device == torch.device(device))
+            for m in (reset, active)) and batch > 0 and steps > 0:
+        return ops.token_plan(batch, steps, device, reset=None if reset is None else reset.contiguous(),
+                              active=None if active is None else active.contiguous(), positions=False)[0]
     flags = torch.zeros(batch, steps, device=device, dtype=torch.uint8)
     if segment_pos is not None:
         cut = (3 - segment_pos.clamp(min=0, max=3)).to(torch.uint8)
@@ -234,20 +239,26 @@ class RG_LRU(nn.Module):
         return yt
 
 
-def _positions(x: Tensor, segment_pos: Optional[Tensor], previous: Optional[Tensor], active: Optional[Tensor]) -> Tensor:
-    """Per-token position inside its document (behaviour of griffin/griffin.py:309-338)."""
+def _check_positions(x: Tensor, segment_pos: Optional[Tensor], previous: Optional[Tensor]) -> None:
     batch, steps = x.shape[:2]
     if steps == 0:
         raise ValueError("Empty token sequences are not supported")
     if segment_pos is not None:
         if segment_pos.shape != (batch, steps):
             raise ValueError(f"segment_pos must have shape ({batch}, {steps}), got {tuple(segment_pos.shape)}")
+    elif previous is not None and previous.shape != (batch,):
+        raise ValueError("Cached segment positions have an incompatible shape")
+
+
+def _positions(x: Tensor, segment_pos: Optional[Tensor], previous: Optional[Tensor], active: Optional[Tensor]) -> Tensor:
+    """Per-token position inside its document (behaviour of griffin/griffin.py:309-338)."""
+    _check_positions(x, segment_pos, previous)
+    batch, steps = x.shape[:2]
+    if segment_pos is not None:
         return segment_pos.to(device=x.device, dtype=torch.long)
     if previous is None:
         start = torch.full((batch, 1), -1, device=x.device, dtype=torch.long)
     else:
-        if previous.shape != (batch,):
-            raise ValueError("Cached segment positions have an incompatible shape")
         start = previous.to(device=x.device, dtype=torch.long)[:, None]
     if active is None:
         return start + torch.arange(1, steps + 1, device=x.device, dtype=torch.long)[None, :]
@@ -458,7 +469,7 @@ class RecurrentBlock(nn.Module):
         branch = _project(self.linear_y, x)[:, 0]
         x_in = _project(self.linear_x, x)[:, 0]
         y, new_rnn, new_conv, position = ops.decode_block(
-            x_in, branch, conv.weight[:, 0, :], conv.bias, cache.conv_state.to(device=device, dtype=x.dtype),
+            x_in, branch, conv.weight.squeeze(1), conv.bias, cache.conv_state.to(device=device, dtype=x.dtype),
             lru.recurrence_gate.weight, lru.recurrence_gate.bias, lru.input_gate.weight, lru.input_gate.bias, lru.Lambda,
             cache.rnn_state.to(device=device, dtype=torch.float32),
             cache.segment_position.to(device=device, dtype=torch.long).contiguous(),
@@ -489,15 +500,25 @@ class RecurrentBlock(nn.Module):
         device = x.device
 
         def mask_plan():
-            """(positions, flag bytes, flat indices of the row partition or None) for this call's masks."""
-            # rows that are one fresh document each need no position tensor unless a cache is asked for
-            pos = None if plain and not return_cache else _positions(x, segment_pos, previous, active_mask)
+            """(flag bytes, flat indices of the row partition or None, position of every row's last real token, positions) for
+            this call's masks; of the last two whichever the cache can be made from."""
             if plain:
                 # contiguous positions 0..T-1: only the first three tokens lose taps, token 0 is a reset
-                return pos, _plain_flags(batch, steps, device), None
+                last = torch.full((batch,), steps - 1, device=device, dtype=torch.long) if return_cache else None
+                return _plain_flags(batch, steps, device), None, last, None
+            _check_positions(x, segment_pos, previous)
+            split = active_mask is not None and steps > 1 and _needs_partition(active_mask, caller_mask)
+            if (not split and x.is_cuda and not ops._library_ops_active() and batch > 0
+                    and (previous is None or previous.shape == (batch,))):
+                as_long = lambda t: None if t is None else t.to(device=device, dtype=torch.long).contiguous()
+                # (with positions of its own a call needs the cached ones only for rows that are all padding)
+                flags, last = ops.token_plan(batch, steps, device, segment_pos=as_long(segment_pos), previous=as_long(previous),
+                                             active=None if active_mask is None else active_mask.contiguous())
+                return flags, None, last, None
+            pos = _positions(x, segment_pos, previous, active_mask)
             moves = None
             kernel_pos, kernel_active = pos, active_mask
-            if active_mask is not None and steps > 1 and _needs_partition(active_mask, caller_mask):
+            if split:
                 # a real token follows padding somewhere: stable partition of every row, real tokens first
                 order, restore = _stable_partition(active_mask)
                 moves = (_flat_rows(order), _flat_rows(restore))
@@ -505,16 +526,16 @@ class RecurrentBlock(nn.Module):
             padded = None if kernel_active is None else ~kernel_active.all()
             flags = token_flags(batch, steps, device, reset=kernel_pos == 0, active=kernel_active,
                                 segment_pos=kernel_pos, padded=padded)
-            return pos, flags, moves
+            return flags, moves, None, pos
 
         if plain or cache is not None:      # (the plain flags have a memo of their own; a cache differs per block)
-            pos, flags, moves = mask_plan()
+            flags, moves, last, pos = mask_plan()
         else:
-            pos, flags, moves = _shared_between_blocks((caller_pos, caller_mask), device, mask_plan)
+            flags, moves, last, pos = _shared_between_blocks((caller_pos, caller_mask), device, mask_plan)
+            if return_cache and last is not None:
+                last = last.clone()         # the plan is shared between blocks, a cache belongs to one
 
-        y_branch = _project(self.linear_y, x)
-        if not self.fold_merge:
-            y_branch = F.gelu(y_branch, approximate="tanh")
+        y_branch = _project(self.linear_y, x)       # before its GeLU
         x_in = _project(self.linear_x, x)
         if moves is not None:
             x_in = _PermuteRows.apply(x_in, moves[0], moves[1])
@@ -524,7 +545,8 @@ class RecurrentBlock(nn.Module):
         if conv_state is not None and conv_state.shape != (batch, self.conv_kernel_size - 1, self.rnn_width):
             raise ValueError("Recurrent convolution cache has an incompatible shape")
 
-        conv_w = self.temporal_conv.weight[:, 0, :]
+        conv_w = self.temporal_conv.weight.squeeze(1)      # (a view whose gradient is a view)
+        merged = self.fold_merge                           # whether the kernels form the branch product
         rnn_state = None if cache is None else cache.rnn_state
         if steps == 1 and cache is not None and not torch.is_grad_enabled() and x_in.is_cuda:
             # Cached single-token decode (inference) that the fused form does not take: the two in-place decode kernels
@@ -541,8 +563,7 @@ class RecurrentBlock(nn.Module):
             u_i = lru.input_gate(x_conv).to(x_conv.dtype)
             new_rnn = rnn_state.to(device=x_in.device, dtype=torch.float32).clone()
             y = ops.decode_step(x_conv, u_r, u_i, lru.Lambda.float().contiguous(), new_rnn, tok, lru.c)[:, None, :]
-            if self.fold_merge:
-                y = y * F.gelu(y_branch, approximate="tanh")
+            merged = False
         elif self.fold_conv:
             if not x_in.is_cuda:
                 raise RuntimeError("scan_mode='cuda' requires CUDA tensors; there is no CPU fallback")
@@ -560,9 +581,11 @@ class RecurrentBlock(nn.Module):
                                      _branch=y_branch if self.fold_merge else None)
         if moves is not None:
             y = _PermuteRows.apply(y, moves[1], moves[0])
-        out = _project(self.linear_out, y if self.fold_merge else y * y_branch)
+        out = _project(self.linear_out, y if merged else ops.gelu_mul(y, y_branch))
         if active_mask is not None:
             out = torch.where(active_mask[..., None], out, 0.0)     # (a scalar: no tensor of zeros to write and read)
         if return_cache:
-            return out, RecurrentBlockCache(new_rnn, new_conv, _last_real_position(pos, active_mask, previous))
+            if last is None:
+                last = _last_real_position(pos, active_mask, previous)
+            return out, RecurrentBlockCache(new_rnn, new_conv, last)
         return out

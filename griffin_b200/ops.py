@@ -964,9 +964,9 @@ def recurrent_core(x_in: Tensor, conv_w: Tensor, conv_b: Optional[Tensor], conv_
 
 
 # ----------------------------------------------------------------------------- linear layers around the recurrence
-def column_sums(m: Tensor) -> Tensor:
-    """fp32 column sums of a dense [rows, cols] CUDA matrix (``rglru_column_sums``): fixed summation order, one
-    streaming pass.  The bias gradient of a linear layer from the gradient of its output."""
+def column_sums(m: Tensor, dtype: torch.dtype = torch.float32) -> Tensor:
+    """Column sums (added in fp32, returned in ``dtype``: float32 or bfloat16) of a dense [rows, cols] CUDA matrix (``rglru_column_sums_as``): fixed summation
+    order, one streaming pass.  The bias gradient of a linear layer from the gradient of its output."""
     if m.dim() != 2:
         raise ValueError("column_sums takes a [rows, cols] matrix")
     _require_cuda(m)
@@ -974,13 +974,13 @@ def column_sums(m: Tensor) -> Tensor:
     dt = _io_dtype(m, "column sums")
     m = m.contiguous()
     rows, cols = m.shape
-    out = torch.empty(cols, device=m.device, dtype=torch.float32)
+    out = torch.empty(cols, device=m.device, dtype=dtype)
     if rows == 0:
         return out.zero_()
     nbytes = lib.rglru_column_sums_workspace_bytes(rows, cols)
     ws = torch.empty(nbytes, device=m.device, dtype=torch.uint8)
     with _on(m, "rglru_column_sums"):
-        rc = lib.rglru_column_sums(_ptr(m), _ptr(out), _ptr(ws), nbytes, rows, cols, dt, _stream(m))
+        rc = lib.rglru_column_sums_as(_ptr(m), _ptr(out), _ptr(ws), nbytes, rows, cols, dt, _DTYPES[dtype], _stream(m))
     _lib.check(rc, "rglru_column_sums")
     return out
 
@@ -1001,7 +1001,8 @@ class _BiasGradTap(torch.autograd.Function):
     def backward(ctx, dy):
         db = None
         if ctx.needs_input_grad[1]:
-            db = column_sums(dy.reshape(-1, dy.shape[-1])).to(ctx.bias_dtype)
+            dt = ctx.bias_dtype
+            db = column_sums(dy.reshape(-1, dy.shape[-1]), dt if dt in _DTYPES else torch.float32).to(dt)
         return dy, db
 
 
@@ -1018,6 +1019,56 @@ def linear(x: Tensor, weight: Tensor, bias: Optional[Tensor]) -> Tensor:
         return torch.nn.functional.linear(x, weight, bias)
     y = torch.nn.functional.linear(x, weight, bias.detach())
     return _BiasGradTap.apply(y, bias)
+
+
+# ----------------------------------------------------------------------------- masks and branch of the block
+def token_plan(batch: int, steps: int, device, *, segment_pos: Optional[Tensor] = None, previous: Optional[Tensor] = None,
+               active: Optional[Tensor] = None, reset: Optional[Tensor] = None, positions: bool = True
+               ) -> tuple[Tensor, Optional[Tensor]]:
+    """(flag bytes [B, T], position of every row's last real token [B]) of a block call's masks, or with
+    ``positions=False`` (flag bytes, None) of a bare layer's reset and padding masks, in one launch (``rglru_token_plan``).
+    Contiguous CUDA tensors: int64 positions, bool masks."""
+    flags = torch.empty(batch, steps, device=device, dtype=torch.uint8)
+    last = torch.empty(batch, device=device, dtype=torch.long) if positions else None
+    with _on(flags, "rglru_token_plan"):
+        rc = _lib.load().rglru_token_plan(_ptr(segment_pos), _ptr(previous), _ptr(active), _ptr(reset), int(positions),
+                                          _ptr(flags), _ptr(last), batch, steps, _stream(flags))
+    _lib.check(rc, "rglru_token_plan")
+    return flags, last
+
+
+class _GeluMul(torch.autograd.Function):
+    """y * gelu_tanh(branch), keeping only the two factors."""
+
+    @staticmethod
+    def forward(ctx, y, branch):
+        ctx.save_for_backward(y, branch)
+        out = torch.empty_like(y)
+        with _on(y, "rglru_gelu_mul_fwd"):
+            rc = _lib.load().rglru_gelu_mul_fwd(_ptr(y), _ptr(branch), _ptr(out), y.numel(), _DTYPES[y.dtype], _stream(y))
+        _lib.check(rc, "rglru_gelu_mul_fwd")
+        return out
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, dout):
+        y, branch = ctx.saved_tensors
+        dout = dout.to(y.dtype).contiguous()
+        dy, dbranch = torch.empty_like(y), torch.empty_like(branch)
+        with _on(y, "rglru_gelu_mul_bwd"):
+            rc = _lib.load().rglru_gelu_mul_bwd(_ptr(dout), _ptr(y), _ptr(branch), _ptr(dy), _ptr(dbranch), y.numel(),
+                                                _DTYPES[y.dtype], _stream(y))
+        _lib.check(rc, "rglru_gelu_mul_bwd")
+        return dy, dbranch
+
+
+def gelu_mul(y: Tensor, branch: Tensor) -> Tensor:
+    """``y * gelu(branch, approximate="tanh")``: one pass each way for CUDA tensors of one kernel dtype and shape outside
+    tracing, the two torch operators otherwise."""
+    if (y.is_cuda and branch.is_cuda and y.device == branch.device and y.dtype == branch.dtype and y.dtype in _DTYPES
+            and y.shape == branch.shape and y.numel() > 0 and not _library_ops_active()):
+        return _GeluMul.apply(y.contiguous(), branch.contiguous())
+    return y * torch.nn.functional.gelu(branch, approximate="tanh")
 
 
 # ----------------------------------------------------------------------------- decode (in-place state, no autograd)

@@ -286,6 +286,9 @@ int rglru_conv_bwd_noalloc(const void* d_conv, const void* x_in, const float* co
 size_t rglru_column_sums_workspace_bytes(long long rows, int cols);
 int rglru_column_sums(const void* src, float* out, void* ws, size_t ws_bytes, long long rows, int cols, int io_dtype,
                       void* stream);
+/* The same with the sums rounded to out_dtype (RGLRU_F32 or RGLRU_BF16) as they are stored. */
+int rglru_column_sums_as(const void* src, void* out, void* ws, size_t ws_bytes, long long rows, int cols, int io_dtype,
+                         int out_dtype, void* stream);
 
 /* Single-token decode update: the T = 1 case of RecurrentBlock.forward with a cache,
  * griffin/griffin.py:459-528, split at the gate projections (which stay ordinary GEMMs):
@@ -305,6 +308,22 @@ int rglru_decode_conv(const void* x_in, const float* conv_w, const float* conv_b
  */
 int rglru_decode_step(const void* x, const void* u_r, const void* u_i, const float* lambda, float* h,
                       const uint8_t* tok, void* y, int B, int D, float c, int io_dtype, void* stream);
+
+/* What the masks of a call mean for every token, as the flag byte the kernels read, in one launch
+ * (griffin/griffin.py:309-358).
+ *   positions != 0 : a block call.  A token's position in its document is seg_pos, else prev_pos + the number of active
+ *                    tokens of its row up to it (prev_pos NULL: -1); it gives the tap cuts, the resets and, where any
+ *                    token of the batch is padding, RGLRU_TOK_ZERO_HISTORY.
+ *   positions == 0 : a bare layer call: resets from `reset`.
+ *   seg_pos [B,T], prev_pos [B], active [B,T] bytes (0 = padding), reset [B,T] bytes: each may be NULL
+ *   flags : [B,T] out     last_pos : [B] out or NULL: position of the row's last active token, prev_pos if it has none */
+int rglru_token_plan(const int64_t* seg_pos, const int64_t* prev_pos, const uint8_t* active, const uint8_t* reset,
+                     int positions, uint8_t* flags, int64_t* last_pos, int B, int T, void* stream);
+
+/* out = y * gelu_tanh(branch) of n elements, and its gradient (griffin/griffin.py:464, 520). */
+int rglru_gelu_mul_fwd(const void* y, const void* branch, void* out, long long n, int io_dtype, void* stream);
+int rglru_gelu_mul_bwd(const void* dout, const void* y, const void* branch, void* dy, void* dbranch, long long n, int io_dtype,
+                       void* stream);
 
 /* One cached token of the recurrent block between its input projections and its output projection, in two launches:
  * positions and flags, conv, both gate projections, the update and the product with the GeLU branch
