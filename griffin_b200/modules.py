@@ -535,8 +535,11 @@ class RecurrentBlock(nn.Module):
             if return_cache and last is not None:
                 last = last.clone()         # the plan is shared between blocks, a cache belongs to one
 
-        y_branch = _project(self.linear_y, x)       # before its GeLU
-        x_in = _project(self.linear_x, x)
+        lx, ly = self.linear_x, self.linear_y
+        if _is_stock(lx, nn.Linear) and _is_stock(ly, nn.Linear):
+            x_in, y_branch = ops.linear_pair(x, lx.weight, lx.bias, ly.weight, ly.bias)
+        else:
+            x_in, y_branch = _project(lx, x), _project(ly, x)       # the branch before its GeLU
         if moves is not None:
             x_in = _PermuteRows.apply(x_in, moves[0], moves[1])
             if self.fold_merge:   # the kernels multiply by the branch, so it travels with its tokens

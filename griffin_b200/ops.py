@@ -1021,6 +1021,68 @@ def linear(x: Tensor, weight: Tensor, bias: Optional[Tensor]) -> Tensor:
     return _BiasGradTap.apply(y, bias)
 
 
+def _mm(a: Tensor, b: Tensor, dtype: torch.dtype) -> Tensor:
+    return torch.mm(a, b) if a.dtype == dtype else torch.mm(a, b, out_dtype=dtype)
+
+
+class _LinearPair(torch.autograd.Function):
+    """Two linear layers of one input.  Their two shares of the input gradient meet in the second GEMM's accumulator, not in
+    a pass of its own over three tensors (21 us at [32768, 768] bf16), in the input's type: under autocast an fp32 input
+    is cast once, and neither share is rounded on its way.  Weight gradients leave their GEMMs in the weights' types, the
+    bias gradients come from :func:`column_sums`."""
+
+    @staticmethod
+    def forward(ctx, x, w1, b1, w2, b2, dtype):
+        ctx.set_materialize_grads(False)
+        with torch.autocast("cuda", enabled=False):
+            xc, m1, m2 = x.to(dtype), w1.to(dtype), w2.to(dtype)
+            y1 = torch.nn.functional.linear(xc, m1, b1.to(dtype))
+            y2 = torch.nn.functional.linear(xc, m2, b2.to(dtype))
+        ctx.save_for_backward(xc, m1, m2)
+        ctx.dtypes = (x.dtype, w1.dtype, b1.dtype, w2.dtype, b2.dtype)
+        return y1, y2
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, d1, d2):
+        x, m1, m2 = ctx.saved_tensors
+        need, dtypes = ctx.needs_input_grad, ctx.dtypes
+        rows = x.reshape(-1, x.shape[-1])
+        dx = None
+        grads = [None] * 4
+        with torch.autocast("cuda", enabled=False):
+            for k, (d, m) in enumerate(((d1, m1), (d2, m2))):
+                if d is None:
+                    continue
+                d = d.reshape(-1, d.shape[-1])
+                if need[0]:
+                    if dx is None:
+                        dx = _mm(d, m, dtypes[0])
+                    elif d.dtype == dx.dtype:
+                        dx.addmm_(d, m)
+                    else:
+                        torch.addmm(dx, d, m, out_dtype=dx.dtype, out=dx)
+                if need[1 + 2 * k]:
+                    grads[2 * k] = _mm(d.t(), rows, dtypes[1 + 2 * k])
+                if need[2 + 2 * k]:
+                    grads[2 * k + 1] = column_sums(d, dtypes[2 + 2 * k])
+        return (None if dx is None else dx.view(x.shape), *grads, None)
+
+
+def linear_pair(x: Tensor, w1: Tensor, b1: Optional[Tensor], w2: Tensor, b2: Optional[Tensor]) -> tuple[Tensor, Tensor]:
+    """``(F.linear(x, w1, b1), F.linear(x, w2, b2))``, in one autograd node where gradients are wanted on CUDA tensors of the
+    kernel dtypes outside tracing; anything else is two calls of :func:`linear`."""
+    tensors = (x, w1, b1, w2, b2)
+    if (b1 is not None and b2 is not None and x.is_cuda and x.numel() > 0 and torch.is_grad_enabled()
+            and any(t.requires_grad for t in tensors) and not _library_ops_active()):
+        autocast = torch.is_autocast_enabled("cuda")
+        dtype = torch.get_autocast_dtype("cuda") if autocast else x.dtype
+        if dtype in _DTYPES and all(t.device == x.device and (t.dtype == dtype or autocast and t.dtype == torch.float32)
+                                    for t in tensors):
+            return _LinearPair.apply(x, w1, b1, w2, b2, dtype)
+    return linear(x, w1, b1), linear(x, w2, b2)
+
+
 # ----------------------------------------------------------------------------- masks and branch of the block
 def token_plan(batch: int, steps: int, device, *, segment_pos: Optional[Tensor] = None, previous: Optional[Tensor] = None,
                active: Optional[Tensor] = None, reset: Optional[Tensor] = None, positions: bool = True
