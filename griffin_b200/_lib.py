@@ -73,6 +73,8 @@ _lib = None
 def load() -> ctypes.CDLL:
     """Load the library once; raise RuntimeError if it has not been built."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None:
             if not os.path.exists(LIB_PATH):

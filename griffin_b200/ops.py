@@ -16,6 +16,7 @@ CUDA stream; nothing here computes on the CPU.
 from __future__ import annotations
 
 import contextlib
+import functools
 import os
 from typing import Optional
 
@@ -66,6 +67,16 @@ def _on(t: Tensor, name: str):
     return torch.cuda.device(t.device)
 
 
+def _no_autocast():
+    """Context without autocast (nothing to do where it is off already)."""
+    return torch.autocast("cuda", enabled=False) if torch.is_autocast_enabled("cuda") else _SAME_DEVICE
+
+
+def _or_empty(t: Optional[Tensor], like: Tensor, dtype: Optional[torch.dtype] = None) -> Tensor:
+    """A custom op returns tensors only: an empty one stands for an absent result."""
+    return like.new_empty((0,), dtype=dtype) if t is None else t
+
+
 def _ptr(t: Optional[Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
@@ -103,7 +114,9 @@ def _library_ops_active() -> bool:
 
 
 def _eager_node(name: str, fwd_impl, setup, backward_rule, bwd_impl):
-    """The autograd.Function twin of a custom op: same forward implementation, same set-up and backward rule."""
+    """The autograd.Function twin of a custom op: same forward implementation, same set-up and backward rule.
+    ``Node.run(differentiated, *args)`` calls the implementation by itself where nothing is to be differentiated (except
+    under forward-mode differentiation, which the Function refuses)."""
 
     class Node(torch.autograd.Function):
         @staticmethod
@@ -119,6 +132,11 @@ def _eager_node(name: str, fwd_impl, setup, backward_rule, bwd_impl):
             return backward_rule(ctx, *grads, _bwd=bwd_impl)
 
     Node.__name__ = Node.__qualname__ = name
+
+    def run(differentiated, *args):
+        return Node.apply(*args) if differentiated or torch.autograd.forward_ad._current_level >= 0 else fwd_impl(*args)
+
+    Node.run = staticmethod(run)
     return Node
 
 
@@ -131,7 +149,7 @@ def _rglru_fwd_impl(x: Tensor, u_r: Tensor, u_i: Tensor, lam: Tensor, h0: Option
     B, T, D = x.shape
     y = torch.empty_like(x)
     h_last = torch.empty(B, D, device=x.device, dtype=torch.float32)
-    nbytes = lib.rglru_workspace_bytes(B, T, D, dt) if save else 0
+    nbytes = workspace_bytes(B, T, D) if save else 0
     ws = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
     with _on(x, "rglru_fwd"):
         rc = lib.rglru_fwd(_ptr(x), _ptr(u_r), _ptr(u_i), _ptr(lam), _ptr(h0), _ptr(tok), _ptr(y), _ptr(h_last),
@@ -157,9 +175,9 @@ def _(x, u_r, u_i, lam, h0, tok, c, save):
             x.new_empty((workspace_bytes(B, T, D) if save else 0,), dtype=torch.uint8))
 
 
-def _rglru_bwd_impl(dy: Tensor, dh_last: Optional[Tensor], x: Tensor, u_r: Tensor, u_i: Tensor, lam: Tensor,
-               h0: Optional[Tensor], tok: Optional[Tensor], ws: Tensor, c: float, want_dh0: bool
-               ) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor]:
+def _rglru_bwd_parts(dy: Tensor, dh_last: Optional[Tensor], x: Tensor, u_r: Tensor, u_i: Tensor, lam: Tensor,
+                     h0: Optional[Tensor], tok: Optional[Tensor], ws: Tensor, c: float, want_dh0: bool
+                     ) -> tuple[Tensor, Tensor, Tensor, Tensor, Optional[Tensor]]:
     lib = _lib.load()
     dt = _io_dtype(x, "backward")
     B, T, D = x.shape
@@ -167,13 +185,20 @@ def _rglru_bwd_impl(dy: Tensor, dh_last: Optional[Tensor], x: Tensor, u_r: Tenso
     du_r = torch.empty_like(x)
     du_i = torch.empty_like(x)
     dlam = torch.empty(D, device=x.device, dtype=torch.float32)
-    dh0 = torch.empty((B, D) if want_dh0 else (0,), device=x.device, dtype=torch.float32)
+    dh0 = torch.empty(B, D, device=x.device, dtype=torch.float32) if want_dh0 else None
     with _on(x, "rglru_bwd"):
         rc = lib.rglru_bwd(_ptr(dy), _ptr(dh_last), _ptr(x), _ptr(u_r), _ptr(u_i), _ptr(lam), _ptr(h0), _ptr(tok),
-                           _ptr(ws), ws.numel(), _ptr(dx), _ptr(du_r), _ptr(du_i), _ptr(dlam),
-                           _ptr(dh0) if want_dh0 else None, B, T, D, c, dt, _stream(x))
+                           _ptr(ws), ws.numel(), _ptr(dx), _ptr(du_r), _ptr(du_i), _ptr(dlam), _ptr(dh0), B, T, D, c, dt,
+                           _stream(x))
     _lib.check(rc, "rglru_bwd")
     return dx, du_r, du_i, dlam, dh0
+
+
+def _rglru_bwd_impl(dy: Tensor, dh_last: Optional[Tensor], x: Tensor, u_r: Tensor, u_i: Tensor, lam: Tensor,
+               h0: Optional[Tensor], tok: Optional[Tensor], ws: Tensor, c: float, want_dh0: bool
+               ) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor]:
+    *grads, dh0 = _rglru_bwd_parts(dy, dh_last, x, u_r, u_i, lam, h0, tok, ws, c, want_dh0)
+    return *grads, _or_empty(dh0, x, torch.float32)
 
 
 _rglru_bwd = torch.library.custom_op("griffin_b200::rglru_bwd", _rglru_bwd_impl, mutates_args=())
@@ -209,7 +234,7 @@ def _rglru_backward(ctx, dy, dh_last, _dws, _bwd=None):
 
 
 _rglru_fwd.register_autograd(_rglru_backward, setup_context=_rglru_setup)
-_RglruNode = _eager_node("RglruScan", _rglru_fwd_impl, _rglru_setup, _rglru_backward, _rglru_bwd_impl)
+_RglruNode = _eager_node("RglruScan", _rglru_fwd_impl, _rglru_setup, _rglru_backward, _rglru_bwd_parts)
 
 
 def rglru(x: Tensor, u_r: Tensor, u_i: Tensor, lam: Tensor, h0: Optional[Tensor] = None,
@@ -223,7 +248,7 @@ def rglru(x: Tensor, u_r: Tensor, u_i: Tensor, lam: Tensor, h0: Optional[Tensor]
         raise ValueError("Lambda must have shape [width]")
     save = torch.is_grad_enabled() and any(
         t is not None and t.requires_grad for t in (x, u_r, u_i, lam, h0))
-    y, h_last, _ = (_rglru_fwd if _library_ops_active() else _RglruNode.apply)(
+    y, h_last, _ = (_rglru_fwd if _library_ops_active() else functools.partial(_RglruNode.run, save))(
         x.contiguous(), u_r.contiguous(), u_i.contiguous(),
                               lam.to(torch.float32).contiguous(),
                               None if h0 is None else h0.to(torch.float32).contiguous(),
@@ -393,7 +418,8 @@ def causal_conv(x_in: Tensor, weight: Tensor, bias: Optional[Tensor], conv_state
     w = weight.to(torch.float32).contiguous()
     b = None if bias is None else bias.to(torch.float32).contiguous()
     st = None if conv_state is None else conv_state.to(x_in.dtype).contiguous()
-    return (_conv_fwd if _library_ops_active() else _ConvNode.apply)(
+    differentiated = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x_in, w, b, st))
+    return (_conv_fwd if _library_ops_active() else functools.partial(_ConvNode.run, differentiated))(
         x_in.contiguous(), w, b, st, None if tok is None else tok.contiguous(), want_state)
 
 
@@ -547,7 +573,7 @@ def rglru_merged(x: Tensor, u_r: Tensor, u_i: Tensor, branch: Tensor, lam: Tenso
     if lam.shape != (x.shape[2],):
         raise ValueError("Lambda must have shape [width]")
     save = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, u_r, u_i, branch, lam, h0))
-    out, h_last, _ = (_merged_fwd if _library_ops_active() else _MergedNode.apply)(
+    out, h_last, _ = (_merged_fwd if _library_ops_active() else functools.partial(_MergedNode.run, save))(
         x.contiguous(), u_r.contiguous(), u_i.contiguous(), branch.to(x.dtype).contiguous(),
         lam.to(torch.float32).contiguous(), None if h0 is None else h0.to(torch.float32).contiguous(),
         None if tok is None else tok.contiguous(), float(c), save)
@@ -637,7 +663,7 @@ def _grouped_fwd_impl(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Ten
     Returns (out, h_last, the gate tensor u, the workspace, the stacked weights, the stacked biases and Lambda in fp32);
     the last four are what the backward needs beside the inputs."""
     lib = _lib.load()
-    with torch.autocast("cuda", enabled=False):
+    with _no_autocast():
         x = _aligned16(x)
         B, T, D = x.shape
         G, bw, _ = w_r.shape
@@ -645,13 +671,12 @@ def _grouped_fwd_impl(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Ten
         group = _gate_group(bw, x.element_size())
         with _on(x, "rglru_gate_pack"):
             wcat, params = _packed_gates(x, w_r, b_r, w_i, b_i, lam)
-        rows = x.view(B * T, G, bw).transpose(0, 1)                                       # [G, N, bw] view
         u = torch.empty(B, T, 2 * D, device=x.device, dtype=x.dtype)
-        torch.bmm(rows, wcat.transpose(1, 2), out=u.view(B * T, G, 2 * bw).transpose(0, 1))
+        torch.bmm(_heads_first(x, B * T, G), wcat.transpose(1, 2), out=_heads_first(u, B * T, G))
         branch = _aligned16(branch)
         out = torch.empty_like(x)
         h_last = torch.empty(B, D, device=x.device, dtype=torch.float32)
-        nbytes = lib.rglru_workspace_bytes(B, T, D, dt) if save else 0
+        nbytes = workspace_bytes(B, T, D) if save else 0
         ws = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
         with _on(x, "rglru_gated_fwd"):
             rc = lib.rglru_gated_fwd(_ptr(x), _ptr(u), _ptr(params), _ptr(branch), _ptr(params) + 8 * D, _ptr(h0), _ptr(tok),
@@ -673,13 +698,19 @@ def _(x, w_r, b_r, w_i, b_i, lam, h0, tok, c, branch, save):
             x.new_empty((G, 2 * bw, bw)), x.new_empty((3 * D,), dtype=torch.float32))
 
 
+def _heads_first(t: Tensor, rows: int, G: int) -> Tensor:
+    """[B, T, C] (dense) as its [G, rows, C / G] view."""
+    C = t.shape[-1]
+    return t.as_strided((G, rows, C // G), (C // G, C, 1))
+
+
 def _gate_weight_grad(du: Tensor, x: Tensor, G: int, bw: int) -> Tensor:
     """d stacked weights [splits, G, 2 bw, bw] from the gate tensor's gradient: one batched GEMM for bf16; for fp32, where
     the library's GEMM walks all tokens with the few CTAs so small an output gives, ``rglru_gate_dw``, whose partial
     sums over stretches of the tokens are left for the caller to add."""
     rows, D = du.shape[0] * du.shape[1], G * bw
     if du.dtype != torch.float32:
-        return torch.bmm(du.view(rows, G, 2 * bw).transpose(0, 1).transpose(1, 2), x.view(rows, G, bw).transpose(0, 1))[None]
+        return torch.bmm(_heads_first(du, rows, G).transpose(1, 2), _heads_first(x, rows, G))[None]
     lib = _lib.load()
     splits = lib.rglru_gate_dw_splits(rows, D, bw)
     dw = torch.empty(splits, G, 2 * bw, bw, device=du.device, dtype=torch.float32)
@@ -692,12 +723,11 @@ def _gate_weight_grad(du: Tensor, x: Tensor, G: int, bw: int) -> Tensor:
 def _grouped_bwd_parts(dout: Tensor, dh_last: Optional[Tensor], x: Tensor, u: Tensor, wcat: Tensor, bias: Tensor,
                        branch: Optional[Tensor], lam: Tensor, h0: Optional[Tensor], tok: Optional[Tensor],
                        ws: Tensor, c: float, want_dh0: bool
-                       ) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor, Tensor]:
+                       ) -> tuple[Tensor, Tensor, Tensor, Tensor, Optional[Tensor], Optional[Tensor]]:
     """(dx, d stacked weights [splits, G, 2 bw, bw], d stacked biases [G, 2 bw] fp32, dLambda, dh0, dbranch) from the stacked
-    weights and biases the forward built; absent results are empty tensors.  The caller takes the two stacked
-    gradients apart into the gates' own."""
+    weights and biases the forward built.  The caller takes the two stacked gradients apart into the gates' own."""
     lib = _lib.load()
-    with torch.autocast("cuda", enabled=False):
+    with _no_autocast():
         x = _aligned16(x)
         B, T, D = x.shape
         G, bw2, bw = wcat.shape
@@ -706,19 +736,17 @@ def _grouped_bwd_parts(dout: Tensor, dh_last: Optional[Tensor], x: Tensor, u: Te
         branch = _aligned16(branch)
         dx = torch.empty_like(x)
         du = torch.empty_like(u)
-        dbranch = torch.empty_like(x) if branch is not None else x.new_empty((0,))
+        dbranch = None if branch is None else torch.empty_like(x)
         dlam = torch.empty(D, device=x.device, dtype=torch.float32)
-        dh0 = torch.empty((B, D) if want_dh0 else (0,), device=x.device, dtype=torch.float32)
+        dh0 = torch.empty(B, D, device=x.device, dtype=torch.float32) if want_dh0 else None
         dbias = torch.empty(G, bw2, device=x.device, dtype=torch.float32)    # [2 D] in the gate tensor's column layout
         with _on(x, "rglru_gated_bwd"):
             rc = lib.rglru_gated_bwd(_ptr(dout), _ptr(dh_last), _ptr(x), _ptr(u), _ptr(bias), _ptr(branch),
                                      _ptr(lam), _ptr(h0), _ptr(tok), _ptr(ws), ws.numel(), _ptr(dx), _ptr(du),
-                                     _ptr(dbranch) if branch is not None else None, _ptr(dlam),
-                                     _ptr(dh0) if want_dh0 else None, _ptr(dbias), B, T, D,
+                                     _ptr(dbranch), _ptr(dlam), _ptr(dh0), _ptr(dbias), B, T, D,
                                      _gate_group(bw, x.element_size()), c, dt, _stream(x))
         _lib.check(rc, "rglru_gated_bwd")
-        dg = du.view(B * T, G, bw2).transpose(0, 1)                    # [G, N, 2 bw] view
-        dx.view(B * T, G, bw).transpose(0, 1).baddbmm_(dg, wcat)       # gate path added onto the direct path
+        _heads_first(dx, B * T, G).baddbmm_(_heads_first(du, B * T, G), wcat)       # gate path added onto the direct path
         dw = _gate_weight_grad(du, x, G, bw)
     return dx, dw, dbias, dlam, dh0, dbranch
 
@@ -727,9 +755,10 @@ def _grouped_bwd_impl(dout: Tensor, dh_last: Optional[Tensor], x: Tensor, u: Ten
                  branch: Optional[Tensor], lam: Tensor, h0: Optional[Tensor], tok: Optional[Tensor],
                  ws: Tensor, c: float, want_dh0: bool
                  ) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor, Tensor]:
-    """:func:`_grouped_bwd_parts` with the weight gradient's stretches added up: [G, 2 bw, bw]."""
+    """:func:`_grouped_bwd_parts` with the weight gradient's stretches added up, [G, 2 bw, bw]; absent results are empty."""
     dx, dw, dbias, dlam, dh0, dbranch = _grouped_bwd_parts(dout, dh_last, x, u, wcat, bias, branch, lam, h0, tok, ws, c, want_dh0)
-    return dx, dw.sum(0) if dw.shape[0] > 1 else dw[0].clone(), dbias, dlam, dh0, dbranch
+    return (dx, dw.sum(0) if dw.shape[0] > 1 else dw[0].clone(), dbias, dlam, _or_empty(dh0, x, torch.float32),
+            _or_empty(dbranch, x))
 
 
 _grouped_bwd = torch.library.custom_op("griffin_b200::grouped_bwd", _grouped_bwd_impl, mutates_args=())
@@ -801,7 +830,7 @@ def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, l
     traced = _library_ops_active()
     if traced or lam.dtype not in _DTYPES:
         lam = lam.to(torch.float32)
-    out, h_last, _, _, _, _ = (_grouped_fwd if traced else _GroupedNode.apply)(
+    out, h_last, _, _, _, _ = (_grouped_fwd if traced else functools.partial(_GroupedNode.run, save))(
         x.contiguous(), w_r, b_r, w_i, b_i, lam.contiguous(),
         None if h0 is None else h0.to(torch.float32).contiguous(), None if tok is None else tok.contiguous(), float(c),
         None if branch is None else branch.to(x.dtype).contiguous(), save)
@@ -845,7 +874,7 @@ def _core_fwd_impl(x_in: Tensor, conv_w: Tensor, conv_b: Optional[Tensor], conv_
     The conv output is materialised once for the two gate GEMMs and dropped; the scan kernels read the conv
     input and redo the four taps in their load stage.  ``conv_w`` [D,4], ``conv_b``, ``lam``, ``h0`` fp32.
     Returns (y, h_last, next conv state, u_r, u_i, workspace)."""
-    with torch.autocast("cuda", enabled=False):
+    with _no_autocast():
         x_conv, new_state = _conv_fwd_impl(x_in, conv_w, conv_b, conv_state, tok)
         u_r = _gate(x_conv, w_r, b_r)
         u_i = _gate(x_conv, w_i, b_i)
@@ -876,7 +905,7 @@ def _core_bwd_impl(dy: Tensor, dh_last: Optional[Tensor], x_in: Tensor, conv_w: 
     """Backward of ``core_fwd``: recomputes the conv output (one streaming pass) for the gate-weight gradients,
     sums the direct and gate paths and runs a single conv backward.  Returns (dx_in, d conv_w, d conv_b,
     d conv_state, dw_r, db_r, dw_i, db_i, dLambda, dh0, dbranch); absent results are empty tensors."""
-    with torch.autocast("cuda", enabled=False):
+    with _no_autocast():
         empty = x_in.new_empty((0,))
         dbranch = empty
         if branch is None:
@@ -953,7 +982,7 @@ def recurrent_core(x_in: Tensor, conv_w: Tensor, conv_b: Optional[Tensor], conv_
         raise ValueError("x_in must be [batch, sequence, width] and conv_w [width, 4]")
     save = torch.is_grad_enabled() and any(
         t is not None and t.requires_grad for t in (x_in, conv_w, conv_b, conv_state, w_r, b_r, w_i, b_i, lam, h0, branch))
-    y, h_last, new_state, _, _, _ = (_core_fwd if _library_ops_active() else _CoreNode.apply)(
+    y, h_last, new_state, _, _, _ = (_core_fwd if _library_ops_active() else functools.partial(_CoreNode.run, save))(
         x_in.contiguous(), conv_w.to(torch.float32).contiguous(),
         None if conv_b is None else conv_b.to(torch.float32).contiguous(),
         None if conv_state is None else conv_state.to(x_in.dtype).contiguous(), w_r, b_r, w_i, b_i,
@@ -1034,7 +1063,7 @@ class _LinearPair(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w1, b1, w2, b2, dtype):
         ctx.set_materialize_grads(False)
-        with torch.autocast("cuda", enabled=False):
+        with _no_autocast():
             xc, m1, m2 = x.to(dtype), w1.to(dtype), w2.to(dtype)
             y1 = torch.nn.functional.linear(xc, m1, b1.to(dtype))
             y2 = torch.nn.functional.linear(xc, m2, b2.to(dtype))
@@ -1050,7 +1079,7 @@ class _LinearPair(torch.autograd.Function):
         rows = x.reshape(-1, x.shape[-1])
         dx = None
         grads = [None] * 4
-        with torch.autocast("cuda", enabled=False):
+        with _no_autocast():
             for k, (d, m) in enumerate(((d1, m1), (d2, m2))):
                 if d is None:
                     continue
