@@ -45,8 +45,13 @@ SIGNATURES = {
     "rglru_gated_bwd": (_i, [_vp] * 9 + [_vp, _sz] + [_vp] * 6 + [_i, _i, _i, _i, _f, _i, _vp]),
     "rglru_gate_pack": (_i, [_vp] * 7 + [_i] * 7 + [_vp]),
     "rglru_gate_unpack": (_i, [_vp, _i] + [_vp] * 7 + [_i] * 7 + [_vp]),
-    "rglru_gate_dw_splits": (_i, [ctypes.c_longlong, _i, _i]),
-    "rglru_gate_dw": (_i, [_vp, _vp, _vp, _i, ctypes.c_longlong, _i, _i, _vp]),
+    "rglru_gate_project": (_i, [_vp, _vp, _vp, _i, ctypes.c_longlong, _i, _i, _i, _vp]),
+    "rglru_gate_dw_splits": (_i, [ctypes.c_longlong, _i, _i, _i]),
+    "rglru_gate_dw": (_i, [_vp, _vp, _vp, _i, ctypes.c_longlong, _i, _i, _i, _vp]),
+    "rglru_layer_workspace_bytes": (_sz, [_i] * 6),
+    "rglru_layer_scratch_bytes": (_sz, [_i] * 5),
+    "rglru_layer_fwd": (_i, [_vp] * 13 + [_sz] + [_i] * 6 + [_f] + [_i] * 4 + [_vp]),
+    "rglru_layer_bwd": (_i, [_vp] * 8 + [_sz] + [_vp] * 10 + [_sz] + [_i] * 5 + [_f] + [_i] * 4 + [_vp]),
     "rglru_linear_scan_fwd": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _vp]),
     "rglru_linear_scan_bwd": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]),
     "rglru_conv_fwd": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),

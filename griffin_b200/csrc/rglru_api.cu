@@ -934,24 +934,106 @@ int rglru_gate_unpack(const void* dw, int splits, const float* dbias, const floa
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
 }
 
-int rglru_gate_dw_splits(long long rows, int D, int head_width) {
-  if (rows <= 0 || D <= 0 || head_width <= 0 || D % head_width != 0) return 0;
-  return gate_dw_splits(rows, D, head_width);
+static int check_gate_gemm(long long rows, int D, int head_width, int io_dtype) {
+  if (!io_dtype_ok(io_dtype)) return RGLRU_ERR_BAD_DTYPE;
+  if (rows <= 0 || rows > (1ll << 32) || D <= 0 || head_width <= 0 || D % head_width != 0 ||
+      head_width % (io_dtype == RGLRU_BF16 ? 8 : 4) != 0 || D / head_width > 65535)
+    return RGLRU_ERR_BAD_SHAPE;
+  return RGLRU_OK;
 }
 
-int rglru_gate_dw(const float* du, const float* x, float* dw, int splits, long long rows, int D, int head_width, void* stream) {
+int rglru_gate_project(const void* a, const void* wcat, void* out, int backward, long long rows, int D, int head_width,
+                       int io_dtype, void* stream) {
+  if (!a || !wcat || !out) return RGLRU_ERR_NULL_POINTER;
+  int rc = check_gate_gemm(rows, D, head_width, io_dtype);
+  if (rc != RGLRU_OK) return rc;
+  if (!aligned(a, 16) || !aligned(wcat, 16) || !aligned(out, 16)) return RGLRU_ERR_MISALIGNED;
+  int* status = nullptr;
+  rc = device_setup(&status);
+  if (rc != RGLRU_OK) return rc;
+  const GateProjectArgs p = {a, wcat, out, rows, D, head_width};
+  const cudaError_t e = launch_gate_project(io_dtype == RGLRU_BF16, backward != 0, p, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
+}
+
+int rglru_gate_dw_splits(long long rows, int D, int head_width, int io_dtype) {
+  return check_gate_gemm(rows, D, head_width, io_dtype) == RGLRU_OK ? gate_dw_splits(io_dtype == RGLRU_BF16, rows, D, head_width) : 0;
+}
+
+int rglru_gate_dw(const void* du, const void* x, float* dw, int splits, long long rows, int D, int head_width, int io_dtype,
+                  void* stream) {
   if (!du || !x || !dw) return RGLRU_ERR_NULL_POINTER;
-  if (rows <= 0 || rows > (1ll << 40) || D <= 0 || head_width <= 0 || D % head_width != 0 || head_width % 4 != 0 ||
-      D / head_width > 65535 || splits < 1 || splits > 65535)
-    return RGLRU_ERR_BAD_SHAPE;
+  int rc = check_gate_gemm(rows, D, head_width, io_dtype);
+  if (rc != RGLRU_OK) return rc;
+  if (splits < 1 || splits > 65535) return RGLRU_ERR_BAD_SHAPE;
   if (!aligned(du, 16) || !aligned(x, 16) || !aligned(dw, 16)) return RGLRU_ERR_MISALIGNED;
   int* status = nullptr;
-  const int rc = device_setup(&status);
+  rc = device_setup(&status);
   if (rc != RGLRU_OK) return rc;
   GateDwArgs a = {};
   a.du = du; a.x = x; a.part = dw; a.rows = rows; a.D = D; a.bw = head_width;
-  const cudaError_t e = launch_gate_dw(a, splits, static_cast<cudaStream_t>(stream));
+  const cudaError_t e = launch_gate_dw(io_dtype == RGLRU_BF16, a, splits, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
+}
+
+// The layer's workspace: packed weights, packed biases and Lambda, then (where a backward follows) the scan's own.
+static size_t up256(size_t n) { return (n + 255) / 256 * 256; }
+static size_t packed_bytes(int D, int head_width, size_t es) {
+  return up256(static_cast<size_t>(2) * D * head_width * es) + up256(static_cast<size_t>(3) * D * sizeof(float));
+}
+size_t rglru_layer_workspace_bytes(int B, int T, int D, int head_width, int io_dtype, int save) {
+  if (B <= 0 || T <= 0 || D <= 0 || head_width <= 0 || !io_dtype_ok(io_dtype)) return 0;
+  return packed_bytes(D, head_width, io_dtype == RGLRU_BF16 ? 2 : 4) + (save ? rglru_workspace_bytes(B, T, D, io_dtype) : 0);
+}
+size_t rglru_layer_scratch_bytes(int B, int T, int D, int head_width, int io_dtype) {
+  const int splits = rglru_gate_dw_splits(static_cast<long long>(B) * T, D, head_width, io_dtype);
+  return up256(static_cast<size_t>(splits) * 2 * D * head_width * sizeof(float)) + static_cast<size_t>(3) * D * sizeof(float);
+}
+
+int rglru_layer_fwd(const void* x, const void* w_r, const void* b_r, const void* w_i, const void* b_i, const void* lambda,
+                    const void* branch, const float* h0, const uint8_t* tok, void* out, float* h_last, void* u, void* ws,
+                    size_t ws_bytes, int save, int B, int T, int D, int head_width, int gate_width, float c,
+                    int weight_dtype, int bias_dtype, int lambda_dtype, int io_dtype, void* stream) {
+  const size_t need = rglru_layer_workspace_bytes(B, T, D, head_width, io_dtype, save);
+  if (!ws || need == 0 || ws_bytes < need) return RGLRU_ERR_WORKSPACE;
+  const size_t es = io_dtype == RGLRU_BF16 ? 2 : 4, packed = packed_bytes(D, head_width, es);
+  uint8_t* w = static_cast<uint8_t*>(ws);
+  float* params = reinterpret_cast<float*>(w + up256(static_cast<size_t>(2) * D * head_width * es));
+  int rc = rglru_gate_pack(w_r, b_r, w_i, b_i, lambda, w, params, D, head_width, gate_width, weight_dtype, bias_dtype,
+                           lambda_dtype, io_dtype, stream);
+  if (rc != RGLRU_OK) return rc;
+  rc = rglru_gate_project(x, w, u, 0, static_cast<long long>(B) * T, D, head_width, io_dtype, stream);
+  if (rc != RGLRU_OK) return rc;
+  return rglru_gated_fwd(x, u, params, branch, params + 2 * static_cast<size_t>(D), h0, tok, out, h_last,
+                         save ? w + packed : nullptr, save ? ws_bytes - packed : 0, B, T, D, gate_width, c, io_dtype, stream);
+}
+
+int rglru_layer_bwd(const void* dout, const float* dh_last, const void* x, const void* u, const void* branch, const float* h0,
+                    const uint8_t* tok, void* ws, size_t ws_bytes, void* dx, void* du, void* dbranch, void* dw_r, void* db_r,
+                    void* dw_i, void* db_i, void* dlambda, float* dh0, void* scratch, size_t scratch_bytes, int B, int T,
+                    int D, int head_width, int gate_width, float c, int weight_dtype, int bias_dtype, int lambda_dtype,
+                    int io_dtype, void* stream) {
+  const size_t need = rglru_layer_workspace_bytes(B, T, D, head_width, io_dtype, 1);
+  if (!ws || need == 0 || ws_bytes < need) return RGLRU_ERR_WORKSPACE;
+  if (!scratch || scratch_bytes < rglru_layer_scratch_bytes(B, T, D, head_width, io_dtype)) return RGLRU_ERR_WORKSPACE;
+  const long long rows = static_cast<long long>(B) * T;
+  const int splits = rglru_gate_dw_splits(rows, D, head_width, io_dtype);
+  if (splits < 1) return RGLRU_ERR_BAD_SHAPE;
+  const size_t es = io_dtype == RGLRU_BF16 ? 2 : 4, packed = packed_bytes(D, head_width, es);
+  uint8_t* w = static_cast<uint8_t*>(ws);
+  const float* params = reinterpret_cast<const float*>(w + up256(static_cast<size_t>(2) * D * head_width * es));
+  float* part = static_cast<float*>(scratch);
+  float* dbias = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + up256(static_cast<size_t>(splits) * 2 * D * head_width * sizeof(float)));
+  float* dlam = dbias + 2 * static_cast<size_t>(D);
+  int rc = rglru_gated_bwd(dout, dh_last, x, u, params, branch, params + 2 * static_cast<size_t>(D), h0, tok, w + packed,
+                           ws_bytes - packed, dx, du, dbranch, dlam, dh0, dbias, B, T, D, gate_width, c, io_dtype, stream);
+  if (rc != RGLRU_OK) return rc;
+  rc = rglru_gate_dw(du, x, part, splits, rows, D, head_width, io_dtype, stream);
+  if (rc != RGLRU_OK) return rc;
+  rc = rglru_gate_unpack(part, splits, dbias, dlam, dw_r, db_r, dw_i, db_i, dlambda, D, head_width, gate_width, RGLRU_F32,
+                         weight_dtype, bias_dtype, lambda_dtype, stream);
+  if (rc != RGLRU_OK) return rc;
+  return rglru_gate_project(du, w, dx, 1, rows, D, head_width, io_dtype, stream);
 }
 
 int rglru_token_plan(const int64_t* seg_pos, const int64_t* prev_pos, const uint8_t* active, const uint8_t* reset,

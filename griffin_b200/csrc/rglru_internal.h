@@ -206,9 +206,16 @@ struct GateUnpackArgs {
   int splits, D, bw, unit;
   bool f32_bias, f32_lambda;
 };
+struct GateProjectArgs {
+  const void* a;     // x [rows, D], or backward du [rows, 2 D]
+  const void* w;     // [G, 2 bw, bw]
+  void* out;         // u [rows, 2 D], or backward dx [rows, D], added to
+  long long rows;
+  int D, bw;
+};
 struct GateDwArgs {
-  const float* du;   // [rows, 2 D]
-  const float* x;    // [rows, D]
+  const void* du;    // [rows, 2 D]
+  const void* x;     // [rows, D]
   float* part;       // [splits, G, 2 bw, bw]
   long long rows, per_split;
   int D, bw;
@@ -257,8 +264,9 @@ cudaError_t launch_token_plan(const TokenPlanArgs& a, cudaStream_t s);
 cudaError_t launch_gelu_mul(bool bf16, const GeluMulArgs& a, bool vector_ok, cudaStream_t s);
 cudaError_t launch_gate_pack(bool f32_weights, bool bf16, const GatePackArgs& a, cudaStream_t s);
 cudaError_t launch_gate_unpack(bool bf16, bool f32_weights, const GateUnpackArgs& a, cudaStream_t s);
-cudaError_t launch_gate_dw(const GateDwArgs& a, int splits, cudaStream_t s);
-int gate_dw_splits(long long rows, int D, int bw);
+cudaError_t launch_gate_dw(bool bf16, const GateDwArgs& a, int splits, cudaStream_t s);
+cudaError_t launch_gate_project(bool bf16, bool backward, const GateProjectArgs& a, cudaStream_t s);
+int gate_dw_splits(bool bf16, long long rows, int D, int bw);
 cudaError_t launch_decode_block(bool bf16, const DecodeBlockArgs& a, cudaStream_t s);
 int colsum_row_blocks(long long rows, int cols);   // partial rows a column-sum call leaves in its workspace
 cudaError_t launch_column_sums(bool bf16, const void* src, void* out, bool out_bf16, float* part, long long rows, int cols,

@@ -57,8 +57,8 @@ def _largest_block_count(width: int, requested: int) -> int:
 
 def _is_stock(layer: nn.Module, kind: type) -> bool:
     """Whether a submodule is the one this package put there: not replaced, not parametrised, without hooks."""
-    return type(layer) is kind and not (layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks
-                                        or layer._backward_pre_hooks)
+    return type(layer) is kind and "forward" not in layer.__dict__ and not (
+        layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks)
 
 
 class BlockDiagonalLinear(nn.Module):

@@ -609,18 +609,33 @@ def gated_supported(x: Tensor, head_width: int) -> bool:
     return x.is_cuda and _gate_group(head_width, x.element_size()) > 0
 
 
-def _packed_gates(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor) -> tuple[Tensor, Tensor]:
-    """The two [G, bw, bw] gate weights as one [G, 2 bw, bw] operand in the activation dtype whose rows alternate between
-    the gates in column groups, and [3 D] fp32: the biases in that order, then Lambda (``rglru_gate_pack``)."""
-    G, bw, _ = w_r.shape
+def _kernel_params(w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor) -> tuple:
+    """The gate parameters as ``rglru_gate_pack`` takes them: dense CUDA tensors, weights and biases each of one kernel dtype."""
     if w_r.dtype != w_i.dtype or w_r.dtype not in _DTYPES:
         w_r, w_i = w_r.float(), w_i.float()
     if b_r.dtype != b_i.dtype or b_r.dtype not in _DTYPES:
         b_r, b_i = b_r.float(), b_i.float()
     if lam.dtype not in _DTYPES:
         lam = lam.float()
-    w_r, w_i, b_r, b_i, lam = _aligned_dense(w_r), _aligned_dense(w_i), b_r.contiguous(), b_i.contiguous(), lam.contiguous()
     _require_cuda(w_r, b_r, w_i, b_i, lam)
+    return _aligned_dense(w_r), b_r.contiguous(), _aligned_dense(w_i), b_i.contiguous(), lam.contiguous()
+
+
+def _gate_grad_buffers(dtypes: tuple, G: int, bw: int, device) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor]:
+    """Buffers for the gradients of (w_r, b_r, w_i, b_i, Lambda) in the dtypes ``_kernel_params`` gives parameters of ``dtypes``."""
+    kernel = [t if t in _DTYPES else torch.float32 for t in dtypes]
+    wt = kernel[0] if kernel[0] == kernel[2] else torch.float32
+    bt = kernel[1] if kernel[1] == kernel[3] else torch.float32
+    return (torch.empty(G, bw, bw, device=device, dtype=wt), torch.empty(G, bw, device=device, dtype=bt),
+            torch.empty(G, bw, bw, device=device, dtype=wt), torch.empty(G, bw, device=device, dtype=bt),
+            torch.empty(G * bw, device=device, dtype=kernel[4]))
+
+
+def _packed_gates(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor) -> tuple[Tensor, Tensor]:
+    """The two [G, bw, bw] gate weights as one [G, 2 bw, bw] operand in the activation dtype whose rows alternate between
+    the gates in column groups, and [3 D] fp32: the biases in that order, then Lambda (``rglru_gate_pack``)."""
+    w_r, b_r, w_i, b_i, lam = _kernel_params(w_r, b_r, w_i, b_i, lam)
+    G, bw, _ = w_r.shape
     D = G * bw
     wcat = torch.empty(G, 2 * bw, bw, device=x.device, dtype=x.dtype)
     params = torch.empty(3 * D, device=x.device, dtype=torch.float32)
@@ -635,19 +650,14 @@ def _unpacked_gate_grads(dw: Tensor, dbias: Tensor, dlam: Tensor, dtypes: tuple)
     """Gradients of (w_r, b_r, w_i, b_i, Lambda) in their dtypes from ``dw`` [splits, G, 2 bw, bw], ``dbias`` [G, 2 bw] and
     ``dlam`` [D] (``rglru_gate_unpack``)."""
     splits, G, bw2, bw = dw.shape
-    device = dw.device
-    kernel = [t if t in _DTYPES else torch.float32 for t in dtypes]
-    wt = kernel[0] if kernel[0] == kernel[2] else torch.float32
-    bt = kernel[1] if kernel[1] == kernel[3] else torch.float32
-    dw_r, dw_i = (torch.empty(G, bw, bw, device=device, dtype=wt) for _ in range(2))
-    db_r, db_i = (torch.empty(G, bw, device=device, dtype=bt) for _ in range(2))
-    dl = torch.empty(G * bw, device=device, dtype=kernel[4])
+    dw_r, db_r, dw_i, db_i, dl = grads = _gate_grad_buffers(dtypes, G, bw, dw.device)
     with _on(dw, "rglru_gate_unpack"):
         rc = _lib.load().rglru_gate_unpack(_ptr(dw), splits, _ptr(dbias), _ptr(dlam), _ptr(dw_r), _ptr(db_r), _ptr(dw_i),
                                            _ptr(db_i), _ptr(dl), G * bw, bw, _gate_group(bw, dw.element_size()),
-                                           _DTYPES[dw.dtype], _DTYPES[wt], _DTYPES[bt], _DTYPES[dl.dtype], _stream(dw))
+                                           _DTYPES[dw.dtype], _DTYPES[dw_r.dtype], _DTYPES[db_r.dtype], _DTYPES[dl.dtype],
+                                           _stream(dw))
     _lib.check(rc, "rglru_gate_unpack")
-    return tuple(g if g.dtype == t else g.to(t) for g, t in zip((dw_r, db_r, dw_i, db_i, dl), dtypes))
+    return tuple(g if g.dtype == t else g.to(t) for g, t in zip(grads, dtypes))
 
 
 def _grouped_fwd_impl(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor, h0: Optional[Tensor],
@@ -705,17 +715,18 @@ def _heads_first(t: Tensor, rows: int, G: int) -> Tensor:
 
 
 def _gate_weight_grad(du: Tensor, x: Tensor, G: int, bw: int) -> Tensor:
-    """d stacked weights [splits, G, 2 bw, bw] from the gate tensor's gradient: one batched GEMM for bf16; for fp32, where
-    the library's GEMM walks all tokens with the few CTAs so small an output gives, ``rglru_gate_dw``, whose partial
-    sums over stretches of the tokens are left for the caller to add."""
+    """d stacked weights [splits, G, 2 bw, bw] from the gate tensor's gradient: one batched GEMM; for fp32 with fewer 64 x 64
+    output tiles than SMs, where that GEMM walks all tokens with the few CTAs so small an output gives (8 heads of 128,
+    16384 tokens: 384 against 254 us; 16 of 176, 8192 tokens, the other way round: 321 against 529), ``rglru_gate_dw``,
+    whose partial sums over stretches of the tokens are left for the caller to add."""
     rows, D = du.shape[0] * du.shape[1], G * bw
-    if du.dtype != torch.float32:
+    if du.dtype != torch.float32 or G * -(-2 * bw // 64) * -(-bw // 64) >= 148:
         return torch.bmm(_heads_first(du, rows, G).transpose(1, 2), _heads_first(x, rows, G))[None]
     lib = _lib.load()
-    splits = lib.rglru_gate_dw_splits(rows, D, bw)
+    splits = lib.rglru_gate_dw_splits(rows, D, bw, _lib.F32)
     dw = torch.empty(splits, G, 2 * bw, bw, device=du.device, dtype=torch.float32)
     with _on(x, "rglru_gate_dw"):
-        rc = lib.rglru_gate_dw(_ptr(du), _ptr(x), _ptr(dw), splits, rows, D, bw, _stream(x))
+        rc = lib.rglru_gate_dw(_ptr(du), _ptr(x), _ptr(dw), splits, rows, D, bw, _lib.F32, _stream(x))
     _lib.check(rc, "rglru_gate_dw")
     return dw
 
@@ -809,6 +820,78 @@ _grouped_fwd.register_autograd(_grouped_backward, setup_context=_grouped_setup)
 _GroupedNode = _eager_node("GroupedRGLRU", _grouped_fwd_impl, _grouped_setup, _grouped_backward, _grouped_bwd_parts)
 
 
+def _layer_in_library(x: Tensor, head_width: int) -> bool:
+    """Whether the layer's projections too are the library's kernels, each direction being one library call, or batched GEMMs
+    between its calls.  One call a direction saves some 105 us of host time in a training step; the batched GEMMs are
+    faster from a few hundred CTAs' worth of work on, by a time that grows with elements x head width.  The line is where
+    that reaches about half of what the host saves (see rglru_gates.cu for both sides' times)."""
+    work = x.numel() * head_width
+    return x.numel() <= 1 << 24 and work <= (1 << 30 if x.dtype == torch.bfloat16 else 1 << 29)
+
+
+def _layer_fwd(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor, h0: Optional[Tensor],
+               tok: Optional[Tensor], c: float, branch: Optional[Tensor], save: bool) -> tuple[Tensor, Tensor, Tensor, Tensor]:
+    """(out, h_last, gate tensor u, workspace) of the whole layer (``rglru_layer_fwd``); ``x`` and ``branch`` dense and aligned."""
+    lib = _lib.load()
+    dt = _io_dtype(x, "layer forward")
+    B, T, D = x.shape
+    w_r, b_r, w_i, b_i, lam = _kernel_params(w_r, b_r, w_i, b_i, lam)
+    bw = w_r.shape[1]
+    u = torch.empty(B, T, 2 * D, device=x.device, dtype=x.dtype)
+    out = torch.empty_like(x)
+    h_last = torch.empty(B, D, device=x.device, dtype=torch.float32)
+    nbytes = lib.rglru_layer_workspace_bytes(B, T, D, bw, dt, int(save))
+    ws = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
+    with _on(x, "rglru_layer_fwd"):
+        rc = lib.rglru_layer_fwd(_ptr(x), _ptr(w_r), _ptr(b_r), _ptr(w_i), _ptr(b_i), _ptr(lam), _ptr(branch), _ptr(h0),
+                                 _ptr(tok), _ptr(out), _ptr(h_last), _ptr(u), _ptr(ws), nbytes, int(save), B, T, D, bw,
+                                 _gate_group(bw, x.element_size()), c, _DTYPES[w_r.dtype], _DTYPES[b_r.dtype],
+                                 _DTYPES[lam.dtype], dt, _stream(x))
+    _lib.check(rc, "rglru_layer_fwd")
+    return out, h_last, u, ws
+
+
+class _LayerNode(torch.autograd.Function):
+    """The layer with both directions as one library call each."""
+
+    @staticmethod
+    def forward(ctx, x, w_r, b_r, w_i, b_i, lam, h0, tok, c, branch):
+        ctx.set_materialize_grads(False)
+        x, branch = _aligned16(x), _aligned16(branch)
+        out, h_last, u, ws = _layer_fwd(x, w_r, b_r, w_i, b_i, lam, h0, tok, c, branch, True)
+        ctx.save_for_backward(x, u, ws, branch, h0, tok)
+        ctx.c, ctx.heads = c, w_r.shape[:2]
+        ctx.param_dtypes = (w_r.dtype, b_r.dtype, w_i.dtype, b_i.dtype, lam.dtype)
+        ctx.want_dh0 = h0 is not None and ctx.needs_input_grad[6]
+        return out, h_last
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, dout, dh_last):
+        x, u, ws, branch, h0, tok = ctx.saved_tensors
+        lib = _lib.load()
+        dt = _DTYPES[x.dtype]
+        B, T, D = x.shape
+        G, bw = ctx.heads
+        dout = torch.zeros_like(x) if dout is None else _aligned16(dout.to(x.dtype).contiguous())
+        dh_last = None if dh_last is None else dh_last.to(torch.float32).contiguous()
+        dx, du = torch.empty_like(x), torch.empty_like(u)
+        dbranch = None if branch is None else torch.empty_like(x)
+        dh0 = torch.empty(B, D, device=x.device, dtype=torch.float32) if ctx.want_dh0 else None
+        dw_r, db_r, dw_i, db_i, dlam = grads = _gate_grad_buffers(ctx.param_dtypes, G, bw, x.device)
+        nbytes = lib.rglru_layer_scratch_bytes(B, T, D, bw, dt)
+        scratch = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
+        with _on(x, "rglru_layer_bwd"):
+            rc = lib.rglru_layer_bwd(_ptr(dout), _ptr(dh_last), _ptr(x), _ptr(u), _ptr(branch), _ptr(h0), _ptr(tok), _ptr(ws),
+                                     ws.numel(), _ptr(dx), _ptr(du), _ptr(dbranch), _ptr(dw_r), _ptr(db_r), _ptr(dw_i),
+                                     _ptr(db_i), _ptr(dlam), _ptr(dh0), _ptr(scratch), nbytes, B, T, D, bw,
+                                     _gate_group(bw, x.element_size()), ctx.c, _DTYPES[dw_r.dtype], _DTYPES[db_r.dtype],
+                                     _DTYPES[dlam.dtype], dt, _stream(x))
+        _lib.check(rc, "rglru_layer_bwd")
+        dw_r, db_r, dw_i, db_i, dlam = (g if g.dtype == t else g.to(t) for g, t in zip(grads, ctx.param_dtypes))
+        return dx, dw_r, db_r, dw_i, db_i, dlam, dh0, None, None, dbranch
+
+
 def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor,
                 h0: Optional[Tensor] = None, tok: Optional[Tensor] = None, c: float = 8.0,
                 branch: Optional[Tensor] = None) -> tuple[Tensor, Tensor]:
@@ -830,6 +913,12 @@ def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, l
     traced = _library_ops_active()
     if traced or lam.dtype not in _DTYPES:
         lam = lam.to(torch.float32)
+    if not traced and _layer_in_library(x, bw):
+        args = (x.contiguous(), w_r, b_r, w_i, b_i, lam, None if h0 is None else h0.to(torch.float32).contiguous(),
+                None if tok is None else tok.contiguous(), float(c), None if branch is None else branch.to(x.dtype).contiguous())
+        if save or torch.autograd.forward_ad._current_level >= 0:
+            return _LayerNode.apply(*args)
+        return _layer_fwd(_aligned16(args[0]), *args[1:9], _aligned16(args[9]), False)[:2]
     out, h_last, _, _, _, _ = (_grouped_fwd if traced else functools.partial(_GroupedNode.run, save))(
         x.contiguous(), w_r, b_r, w_i, b_i, lam.contiguous(),
         None if h0 is None else h0.to(torch.float32).contiguous(), None if tok is None else tok.contiguous(), float(c),

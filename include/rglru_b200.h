@@ -198,17 +198,40 @@ int rglru_gated_bwd(const void* dout, const float* dh_last, const void* x, const
  *                       params [3 D] fp32: the biases in that order, then lambda.
  *   rglru_gate_unpack : dw [splits, G, 2 head_width, head_width] (io_dtype; splits > 1 are added in index order), dbias
  *                       [2 D] and dlam [D] fp32 -> the five gradients in the parameters' types and shapes.
- *   rglru_gate_dw     : fp32 dw[s] = the share of du^T x (per head) of the s-th of `splits` stretches of the rows; du
+ *   rglru_gate_dw     : dw[s] (fp32) = the share of du^T x (per head) of the s-th of `splits` stretches of the rows; du
  *                       [rows, 2 D], x [rows, D].  rglru_gate_dw_splits says how many stretches fill the machine.
- * Weights, wcat, dw, du and x must be 16-byte aligned. */
+ *   rglru_gate_project: u [rows, 2 D] from a = x [rows, D], or with backward != 0 dx [rows, D] += from a = du [rows, 2 D],
+ *                       fp32 accumulation.  (Both: head_width a multiple of 16 bytes.)
+ * Weights, wcat, dw, du, dx, u and x must be 16-byte aligned. */
 int rglru_gate_pack(const void* w_r, const void* b_r, const void* w_i, const void* b_i, const void* lambda, void* wcat,
                     float* params, int D, int head_width, int gate_width, int weight_dtype, int bias_dtype,
                     int lambda_dtype, int io_dtype, void* stream);
 int rglru_gate_unpack(const void* dw, int splits, const float* dbias, const float* dlam, void* dw_r, void* db_r, void* dw_i,
                       void* db_i, void* dlambda, int D, int head_width, int gate_width, int io_dtype, int weight_dtype,
                       int bias_dtype, int lambda_dtype, void* stream);
-int rglru_gate_dw_splits(long long rows, int D, int head_width);
-int rglru_gate_dw(const float* du, const float* x, float* dw, int splits, long long rows, int D, int head_width, void* stream);
+int rglru_gate_project(const void* a, const void* wcat, void* out, int backward, long long rows, int D, int head_width,
+                       int io_dtype, void* stream);
+int rglru_gate_dw_splits(long long rows, int D, int head_width, int io_dtype);
+int rglru_gate_dw(const void* du, const void* x, float* dw, int splits, long long rows, int D, int head_width, int io_dtype,
+                  void* stream);
+
+/* The whole layer from x and its parameters (griffin/griffin.py:190-286), each direction in one call: pack, projections and
+ * scan; scan backward, weight gradient, unpacking and the gates' share of the input gradient.
+ *   x, branch, out, u ([B,T,2D]), dout, dx, du, dbranch : io_dtype, 16-byte aligned     h0, h_last, dh_last, dh0 : [B,D] fp32
+ *   parameters and their gradients as in rglru_gate_pack / rglru_gate_unpack, gate_width as in rglru_gated_fwd
+ *   ws      : rglru_layer_workspace_bytes(..., save) bytes, 16-byte aligned; with save != 0 it is what the backward needs
+ *   scratch : rglru_layer_scratch_bytes(...) bytes, 16-byte aligned, of the backward alone */
+size_t rglru_layer_workspace_bytes(int B, int T, int D, int head_width, int io_dtype, int save);
+size_t rglru_layer_scratch_bytes(int B, int T, int D, int head_width, int io_dtype);
+int rglru_layer_fwd(const void* x, const void* w_r, const void* b_r, const void* w_i, const void* b_i, const void* lambda,
+                    const void* branch, const float* h0, const uint8_t* tok, void* out, float* h_last, void* u, void* ws,
+                    size_t ws_bytes, int save, int B, int T, int D, int head_width, int gate_width, float c,
+                    int weight_dtype, int bias_dtype, int lambda_dtype, int io_dtype, void* stream);
+int rglru_layer_bwd(const void* dout, const float* dh_last, const void* x, const void* u, const void* branch, const float* h0,
+                    const uint8_t* tok, void* ws, size_t ws_bytes, void* dx, void* du, void* dbranch, void* dw_r, void* db_r,
+                    void* dw_i, void* db_i, void* dlambda, float* dh0, void* scratch, size_t scratch_bytes, int B, int T,
+                    int D, int head_width, int gate_width, float c, int weight_dtype, int bias_dtype, int lambda_dtype,
+                    int io_dtype, void* stream);
 
 /* Raw affine scan h_t = a_t h_{t-1} + b_t on fp32 tensors: the operator
  * fused_rglru_scan(decay, current_input, initial_state) of griffin/triton_scan.py:274-276

@@ -28,14 +28,16 @@ def _run(layer, x, dy, h0, resets, active, branch, dh):
 
 # (batch, steps, heads, head width): fp32 groups of 4 (4, 12), 8 (8, 24, 40), 16 (16, 48), 32 (32, 96, 352), 64 (64)
 SHAPES = [(1, 1, 3, 4), (2, 70, 5, 12), (3, 64, 1, 8), (2, 129, 3, 24), (1, 1000, 2, 40), (4, 65, 7, 16), (5, 200, 3, 48),
-          (2, 64, 2, 32), (1, 300, 3, 96), (2, 130, 2, 352), (2, 80, 3, 64)]
+          (2, 64, 2, 32), (1, 300, 3, 96), (2, 130, 2, 352), (2, 80, 3, 64), (1, 70, 150, 8)]   # (the last: more output tiles than SMs)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("merge", [False, True])
+@pytest.mark.parametrize("own_projections", [False, True])
 @pytest.mark.parametrize("shape", SHAPES)
-def test_any_head_width_matches_the_modules(shape, dtype, merge, monkeypatch):
+def test_any_head_width_matches_the_modules(shape, dtype, merge, own_projections, monkeypatch):
     from griffin_b200 import RG_LRU, ops
+    monkeypatch.setattr(ops, "_layer_in_library", lambda *a: own_projections)
     batch, steps, heads, bw = shape
     if dtype == torch.bfloat16 and bw % 8:
         pytest.skip("a group of four bf16 channels is below 16 bytes")
@@ -98,13 +100,29 @@ def test_parameters_into_and_out_of_the_layout(weights, biases, lam, io):
     torch.testing.assert_close(back[4].double(), lv.double(), rtol=1e-6, atol=0)
 
 
-@pytest.mark.parametrize("rows,heads,bw", [(1, 1, 4), (127, 2, 12), (129, 3, 48), (1000, 2, 72), (4099, 1, 100), (513, 2, 352)])
-def test_fp32_gate_weight_gradient(rows, heads, bw):
-    """Against float64.  Each of the two levels adds fewer than 4,200 fp32 products in order: a relative error of a few
-    roundings of 6e-8 norm-wise, 1e-6 at most."""
-    from griffin_b200 import ops
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,heads,bw", [(1, 1, 4), (1, 2, 8), (127, 2, 12), (128, 3, 48), (129, 3, 48), (1000, 2, 72), (4099, 1, 104), (60000, 2, 16),
+                                           (513, 2, 352)])
+def test_gate_projections_and_weight_gradient(rows, heads, bw, dtype):
+    """The three contractions against float64, fp32 accumulators throughout: fewer than 4,200 products added in order, a
+    relative error of a few roundings of 6e-8 norm-wise (1e-6 at most), and the results of the two projections rounded once
+    to the type."""
+    from griffin_b200 import _lib, ops
+    if dtype == torch.bfloat16 and bw % 8:
+        pytest.skip("rows of whole 16-byte groups")
     torch.manual_seed(2)
-    du, x = torch.randn(1, rows, 2 * heads * bw, device=DEV), torch.randn(1, rows, heads * bw, device=DEV)
-    got = ops._gate_weight_grad(du, x, heads, bw).double().sum(0)
-    want = torch.einsum("ngo,ngi->goi", du[0].double().view(rows, heads, 2 * bw), x[0].double().view(rows, heads, bw))
-    assert _rel(got, want) <= 1e-6
+    lib, io, st = _lib.load(), ops._DTYPES[dtype], torch.cuda.current_stream().cuda_stream
+    D = heads * bw
+    du, x, dx = (torch.randn(rows, n, device=DEV).to(dtype) for n in (2 * D, D, D))
+    w = (torch.randn(heads, 2 * bw, bw, device=DEV) / bw ** 0.5).to(dtype)
+    u, dx0 = torch.empty(rows, 2 * D, device=DEV, dtype=dtype), dx.clone()
+    _lib.check(lib.rglru_gate_project(x.data_ptr(), w.data_ptr(), u.data_ptr(), 0, rows, D, bw, io, st), "project")
+    _lib.check(lib.rglru_gate_project(du.data_ptr(), w.data_ptr(), dx.data_ptr(), 1, rows, D, bw, io, st), "project back")
+    splits = lib.rglru_gate_dw_splits(rows, D, bw, io)
+    dw = torch.full((splits, heads, 2 * bw, bw), float("nan"), device=DEV)
+    _lib.check(lib.rglru_gate_dw(du.data_ptr(), x.data_ptr(), dw.data_ptr(), splits, rows, D, bw, io, st), "dw")
+    d64, x64, w64 = du.double().view(rows, heads, 2 * bw), x.double().view(rows, heads, bw), w.double()
+    once = 1e-6 if dtype == torch.float32 else 2.0 ** -9
+    assert _rel(u, torch.einsum("ngi,goi->ngo", x64, w64).reshape(rows, -1)) <= once
+    assert _rel(dx, dx0.double() + torch.einsum("ngo,goi->ngi", d64, w64).reshape(rows, -1)) <= once
+    assert _rel(dw.double().sum(0), torch.einsum("ngo,ngi->goi", d64, x64)) <= 1e-6
