@@ -609,15 +609,23 @@ def gated_supported(x: Tensor, head_width: int) -> bool:
     return x.is_cuda and _gate_group(head_width, x.element_size()) > 0
 
 
-def _kernel_params(w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor) -> tuple:
-    """The gate parameters as ``rglru_gate_pack`` takes them: dense CUDA tensors, weights and biases each of one kernel dtype."""
+def _same_device(x: Tensor, *tensors: Optional[Tensor]) -> None:
+    """The kernels read raw pointers on the device of ``x``: everything else has to be there too."""
+    for t in tensors:
+        if t is not None and t.device != x.device:
+            raise RuntimeError(f"CUDA RG-LRU kernels require all tensors on one device, got {x.device} and {t.device}")
+
+
+def _kernel_params(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor) -> tuple:
+    """The gate parameters as ``rglru_gate_pack`` takes them: dense tensors on the device of ``x``, weights and biases each of
+    one kernel dtype."""
+    _same_device(x, w_r, b_r, w_i, b_i, lam)
     if w_r.dtype != w_i.dtype or w_r.dtype not in _DTYPES:
         w_r, w_i = w_r.float(), w_i.float()
     if b_r.dtype != b_i.dtype or b_r.dtype not in _DTYPES:
         b_r, b_i = b_r.float(), b_i.float()
     if lam.dtype not in _DTYPES:
         lam = lam.float()
-    _require_cuda(w_r, b_r, w_i, b_i, lam)
     return _aligned_dense(w_r), b_r.contiguous(), _aligned_dense(w_i), b_i.contiguous(), lam.contiguous()
 
 
@@ -634,7 +642,7 @@ def _gate_grad_buffers(dtypes: tuple, G: int, bw: int, device) -> tuple[Tensor, 
 def _packed_gates(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor) -> tuple[Tensor, Tensor]:
     """The two [G, bw, bw] gate weights as one [G, 2 bw, bw] operand in the activation dtype whose rows alternate between
     the gates in column groups, and [3 D] fp32: the biases in that order, then Lambda (``rglru_gate_pack``)."""
-    w_r, b_r, w_i, b_i, lam = _kernel_params(w_r, b_r, w_i, b_i, lam)
+    w_r, b_r, w_i, b_i, lam = _kernel_params(x, w_r, b_r, w_i, b_i, lam)
     G, bw, _ = w_r.shape
     D = G * bw
     wcat = torch.empty(G, 2 * bw, bw, device=x.device, dtype=x.dtype)
@@ -835,7 +843,7 @@ def _layer_fwd(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, la
     lib = _lib.load()
     dt = _io_dtype(x, "layer forward")
     B, T, D = x.shape
-    w_r, b_r, w_i, b_i, lam = _kernel_params(w_r, b_r, w_i, b_i, lam)
+    w_r, b_r, w_i, b_i, lam = _kernel_params(x, w_r, b_r, w_i, b_i, lam)
     bw = w_r.shape[1]
     u = torch.empty(B, T, 2 * D, device=x.device, dtype=x.dtype)
     out = torch.empty_like(x)
@@ -869,6 +877,7 @@ class _LayerNode(torch.autograd.Function):
     @torch.autograd.function.once_differentiable
     def backward(ctx, dout, dh_last):
         x, u, ws, branch, h0, tok = ctx.saved_tensors
+        x, branch = _aligned16(x), _aligned16(branch)
         lib = _lib.load()
         dt = _DTYPES[x.dtype]
         B, T, D = x.shape
@@ -1300,7 +1309,8 @@ def decode_block(x_in: Tensor, branch: Optional[Tensor], conv_w: Tensor, conv_b:
     product with its GeLU.  ``x_in`` / ``branch`` [B, D]; conv weights, biases and Lambda in the activation dtype or
     (conv and Lambda) fp32; ``position`` / ``segment_pos`` [B] int64; ``active`` [B] bool.  The states are not modified."""
     lib = _lib.load()
-    _require_cuda(x_in, branch, conv_w, conv_b, conv_state, w_r, b_r, w_i, b_i, lam, h, position, segment_pos, active)
+    _require_cuda(x_in)
+    _same_device(x_in, branch, conv_w, conv_b, conv_state, w_r, b_r, w_i, b_i, lam, h, position, segment_pos, active)
     dt = _io_dtype(x_in, "decode block")
     B, D = x_in.shape
     f32 = ((1 if conv_w.dtype == torch.float32 else 0) | (2 if conv_b is not None and conv_b.dtype == torch.float32 else 0)

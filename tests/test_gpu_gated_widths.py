@@ -28,7 +28,7 @@ def _run(layer, x, dy, h0, resets, active, branch, dh):
 
 # (batch, steps, heads, head width): fp32 groups of 4 (4, 12), 8 (8, 24, 40), 16 (16, 48), 32 (32, 96, 352), 64 (64)
 SHAPES = [(1, 1, 3, 4), (2, 70, 5, 12), (3, 64, 1, 8), (2, 129, 3, 24), (1, 1000, 2, 40), (4, 65, 7, 16), (5, 200, 3, 48),
-          (2, 64, 2, 32), (1, 300, 3, 96), (2, 130, 2, 352), (2, 80, 3, 64), (1, 70, 150, 8)]   # (the last: more output tiles than SMs)
+          (2, 64, 2, 32), (1, 300, 3, 96), (2, 130, 2, 352), (2, 80, 3, 64), (1, 70, 150, 8), (70, 65, 2, 24)]   # (more output tiles than SMs; a batch whose sums a second kernel folds)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
@@ -126,3 +126,11 @@ def test_gate_projections_and_weight_gradient(rows, heads, bw, dtype):
     assert _rel(u, torch.einsum("ngi,goi->ngo", x64, w64).reshape(rows, -1)) <= once
     assert _rel(dx, dx0.double() + torch.einsum("ngo,goi->ngi", d64, w64).reshape(rows, -1)) <= once
     assert _rel(dw.double().sum(0), torch.einsum("ngo,ngi->goi", d64, x64)) <= 1e-6
+
+
+def test_parameters_elsewhere_are_refused():
+    from griffin_b200 import RG_LRU
+    layer = RG_LRU(128, gate_blocks=2).to(DEV)
+    layer.input_gate.weight.data = layer.input_gate.weight.data.cpu()
+    with pytest.raises(RuntimeError):
+        layer(torch.randn(1, 4, 128, device=DEV))
