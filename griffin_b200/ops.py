@@ -616,6 +616,12 @@ def _same_device(x: Tensor, *tensors: Optional[Tensor]) -> None:
             raise RuntimeError(f"CUDA RG-LRU kernels require all tensors on one device, got {x.device} and {t.device}")
 
 
+def _expect(name: str, t: Optional[Tensor], shape: tuple, *dtypes: torch.dtype) -> None:
+    """The kernels take raw pointers: an argument of another shape or dtype would be read (or written) out of range."""
+    if t is not None and (t.shape != shape or t.dtype not in dtypes):
+        raise ValueError(f"{name} must be {list(shape)} of {' or '.join(str(d) for d in dtypes)}, got {list(t.shape)} of {t.dtype}")
+
+
 def _kernel_params(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor) -> tuple:
     """The gate parameters as ``rglru_gate_pack`` takes them: dense tensors on the device of ``x``, weights and biases each of
     one kernel dtype."""
@@ -1308,11 +1314,31 @@ def decode_block(x_in: Tensor, branch: Optional[Tensor], conv_w: Tensor, conv_b:
     output projection (``rglru_decode_block``): conv, both gate projections, the update and, with ``branch`` given, the
     product with its GeLU.  ``x_in`` / ``branch`` [B, D]; conv weights, biases and Lambda in the activation dtype or
     (conv and Lambda) fp32; ``position`` / ``segment_pos`` [B] int64; ``active`` [B] bool.  The states are not modified."""
-    lib = _lib.load()
     _require_cuda(x_in)
     _same_device(x_in, branch, conv_w, conv_b, conv_state, w_r, b_r, w_i, b_i, lam, h, position, segment_pos, active)
     dt = _io_dtype(x_in, "decode block")
+    if x_in.dim() != 2 or w_r.dim() != 3:
+        raise ValueError("x_in must be [batch, width] and the gate weights [heads, width/heads, width/heads]")
     B, D = x_in.shape
+    io, (G, bw) = x_in.dtype, w_r.shape[:2]
+    if G * bw != D:
+        raise ValueError(f"gate weights of {G} heads of {bw} channels do not make up a width of {D}")
+    _expect("branch", branch, (B, D), io)
+    _expect("conv_w", conv_w, (D, 4), io, torch.float32)
+    _expect("conv_b", conv_b, (D,), io, torch.float32)
+    _expect("conv_state", conv_state, (B, 3, D), io)
+    _expect("w_r", w_r, (G, bw, bw), io)
+    _expect("b_r", b_r, (G, bw), io)
+    _expect("w_i", w_i, (G, bw, bw), io)
+    _expect("b_i", b_i, (G, bw), io)
+    _expect("Lambda", lam, (D,), io, torch.float32)
+    _expect("h", h, (B, D), torch.float32)
+    _expect("position", position, (B,), torch.long)
+    _expect("segment_pos", segment_pos, (B,), torch.long)
+    _expect("active", active, (B,), torch.bool)
+    conv_b, b_r, b_i, lam, position, segment_pos, active = (
+        t if t is None else t.contiguous() for t in (conv_b, b_r, b_i, lam, position, segment_pos, active))
+    lib = _lib.load()
     f32 = ((1 if conv_w.dtype == torch.float32 else 0) | (2 if conv_b is not None and conv_b.dtype == torch.float32 else 0)
            | (4 if lam.dtype == torch.float32 else 0))
     x_in, branch, conv_state, h = (_aligned_dense(t) for t in (x_in, branch, conv_state, h))

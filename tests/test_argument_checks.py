@@ -1,0 +1,53 @@
+"""Arguments that the library would read or write out of range are refused on the host, before the library is reached: the
+operators run here on CPU tensors with the CUDA requirement lifted and a library that fails the test when it is asked for."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+
+class _Reached(Exception):
+    pass
+
+
+@pytest.fixture
+def ops(monkeypatch):
+    from griffin_b200 import _lib, ops
+
+    def reached():
+        raise _Reached
+    monkeypatch.setattr(_lib, "load", reached)
+    monkeypatch.setattr(ops, "_require_cuda", lambda *tensors: None)
+    return ops
+
+
+def _decode_args(dtype=torch.bfloat16, B=3, D=48, G=2):
+    bw = D // G
+    r = lambda *s: torch.randn(*s).to(dtype)
+    return dict(x_in=r(B, D), branch=r(B, D), conv_w=torch.randn(D, 4), conv_b=r(D), conv_state=r(B, 3, D), w_r=r(G, bw, bw),
+                b_r=r(G, bw), w_i=r(G, bw, bw), b_i=r(G, bw), lam=torch.randn(D), h=torch.randn(B, D),
+                position=torch.zeros(B, dtype=torch.long), segment_pos=torch.zeros(B, dtype=torch.long),
+                active=torch.ones(B, dtype=torch.bool))
+
+
+def test_decode_block_takes_what_it_is_meant_for(ops):
+    with pytest.raises(_Reached):
+        ops.decode_block(**_decode_args())
+    with pytest.raises(_Reached):
+        ops.decode_block(**{**_decode_args(torch.float32), "branch": None, "conv_b": None, "segment_pos": None, "active": None})
+
+
+@pytest.mark.parametrize("name,change", [
+    ("h", lambda t: t.bfloat16()), ("h", lambda t: t[:2]), ("conv_state", lambda t: t[:, :2]), ("conv_state", lambda t: t.float()),
+    ("position", lambda t: t.int()), ("position", lambda t: t[:2]), ("segment_pos", lambda t: t.int()),
+    ("segment_pos", lambda t: t[:, None]), ("active", lambda t: t.long()), ("active", lambda t: t[:1]), ("branch", lambda t: t[:, :8]),
+    ("branch", lambda t: t.float()), ("w_r", lambda t: t.float()), ("w_i", lambda t: t[:1]), ("w_r", lambda t: t[..., :8]),
+    ("w_r", lambda t: t[:1]), ("b_r", lambda t: t.float()), ("b_i", lambda t: t[:1]), ("conv_w", lambda t: t[:, :3]),
+    ("conv_w", lambda t: t.half()), ("conv_b", lambda t: t[:8]), ("lam", lambda t: t[:8]), ("lam", lambda t: t.double()),
+    ("x_in", lambda t: t[0])])
+def test_decode_block_refuses_other_shapes_and_dtypes(ops, name, change):
+    args = _decode_args()
+    args[name] = change(args[name])
+    with pytest.raises((ValueError, TypeError)):
+        ops.decode_block(**args)
