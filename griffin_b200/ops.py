@@ -1222,8 +1222,15 @@ def token_plan(batch: int, steps: int, device, *, segment_pos: Optional[Tensor] 
                ) -> tuple[Tensor, Optional[Tensor]]:
     """(flag bytes [B, T], position of every row's last real token [B]) of a block call's masks, or with
     ``positions=False`` (flag bytes, None) of a bare layer's reset and padding masks, in one launch (``rglru_token_plan``).
-    Contiguous CUDA tensors: int64 positions, bool masks."""
+    CUDA tensors on ``device``: int64 positions [B, T] and [B], bool masks [B, T]."""
     flags = torch.empty(batch, steps, device=device, dtype=torch.uint8)
+    _require_cuda(flags)
+    _same_device(flags, segment_pos, previous, active, reset)
+    _expect("segment_pos", segment_pos, (batch, steps), torch.long)
+    _expect("previous", previous, (batch,), torch.long)
+    _expect("active", active, (batch, steps), torch.bool)
+    _expect("reset", reset, (batch, steps), torch.bool)
+    segment_pos, previous, active, reset = (t if t is None else t.contiguous() for t in (segment_pos, previous, active, reset))
     last = torch.empty(batch, device=device, dtype=torch.long) if positions else None
     with _on(flags, "rglru_token_plan"):
         rc = _lib.load().rglru_token_plan(_ptr(segment_pos), _ptr(previous), _ptr(active), _ptr(reset), int(positions),

@@ -19,6 +19,7 @@ def ops(monkeypatch):
         raise _Reached
     monkeypatch.setattr(_lib, "load", reached)
     monkeypatch.setattr(ops, "_require_cuda", lambda *tensors: None)
+    monkeypatch.setattr(ops, "_on", lambda t, name: ops._SAME_DEVICE)
     return ops
 
 
@@ -51,3 +52,40 @@ def test_decode_block_refuses_other_shapes_and_dtypes(ops, name, change):
     args[name] = change(args[name])
     with pytest.raises((ValueError, TypeError)):
         ops.decode_block(**args)
+
+
+def _plan_args(B=3, T=5):
+    return dict(segment_pos=torch.zeros(B, T, dtype=torch.long), previous=torch.zeros(B, dtype=torch.long),
+                active=torch.ones(B, T, dtype=torch.bool), reset=torch.zeros(B, T, dtype=torch.bool))
+
+
+@pytest.mark.parametrize("name,change", [
+    ("segment_pos", lambda t: t.int()), ("segment_pos", lambda t: t[:, :4]), ("previous", lambda t: t.int()),
+    ("previous", lambda t: t[:1]), ("active", lambda t: t.long()), ("active", lambda t: t[:2]), ("reset", lambda t: t.float()),
+    ("reset", lambda t: t[0]), ("active", lambda t: t.to("meta")), ("segment_pos", lambda t: t.to("meta"))])
+def test_token_plan_refuses_other_shapes_dtypes_and_devices(ops, name, change):
+    args = _plan_args()
+    with pytest.raises(_Reached):
+        ops.token_plan(3, 5, torch.device("cpu"), **args)
+    args[name] = change(args[name])
+    with pytest.raises((ValueError, RuntimeError)):
+        ops.token_plan(3, 5, torch.device("cpu"), **args)
+
+
+def test_token_plan_refuses_tensors_that_are_not_on_a_gpu():
+    from griffin_b200 import ops
+    with pytest.raises(RuntimeError):
+        ops.token_plan(3, 5, torch.device("cpu"), **_plan_args())
+
+
+def test_token_plan_makes_strided_masks_dense(ops, monkeypatch):
+    seen = []
+    ptr = ops._ptr
+    monkeypatch.setattr(ops, "_ptr", lambda t: seen.append(t) or ptr(t))
+    monkeypatch.setattr(ops, "_stream", lambda t: 0)
+    monkeypatch.setattr(ops._lib, "load", lambda: type("L", (), {"rglru_token_plan": staticmethod(lambda *a: 0)}))
+    args = _plan_args()
+    args["active"] = torch.ones(5, 3, dtype=torch.bool).T
+    args["segment_pos"] = torch.zeros(5, 3, dtype=torch.long).T
+    ops.token_plan(3, 5, torch.device("cpu"), **args)
+    assert len(seen) >= 6 and all(t is None or t.is_contiguous() for t in seen)
