@@ -622,10 +622,8 @@ def _expect(name: str, t: Optional[Tensor], shape: tuple, *dtypes: torch.dtype) 
         raise ValueError(f"{name} must be {list(shape)} of {' or '.join(str(d) for d in dtypes)}, got {list(t.shape)} of {t.dtype}")
 
 
-def _kernel_params(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor) -> tuple:
-    """The gate parameters as ``rglru_gate_pack`` takes them: dense tensors on the device of ``x``, weights and biases each of
-    one kernel dtype."""
-    _same_device(x, w_r, b_r, w_i, b_i, lam)
+def _kernel_params(w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor) -> tuple:
+    """The gate parameters as ``rglru_gate_pack`` takes them: dense tensors, weights and biases each of one kernel dtype."""
     if w_r.dtype != w_i.dtype or w_r.dtype not in _DTYPES:
         w_r, w_i = w_r.float(), w_i.float()
     if b_r.dtype != b_i.dtype or b_r.dtype not in _DTYPES:
@@ -648,7 +646,8 @@ def _gate_grad_buffers(dtypes: tuple, G: int, bw: int, device) -> tuple[Tensor, 
 def _packed_gates(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor) -> tuple[Tensor, Tensor]:
     """The two [G, bw, bw] gate weights as one [G, 2 bw, bw] operand in the activation dtype whose rows alternate between
     the gates in column groups, and [3 D] fp32: the biases in that order, then Lambda (``rglru_gate_pack``)."""
-    w_r, b_r, w_i, b_i, lam = _kernel_params(x, w_r, b_r, w_i, b_i, lam)
+    _same_device(x, w_r, b_r, w_i, b_i, lam)
+    w_r, b_r, w_i, b_i, lam = _kernel_params(w_r, b_r, w_i, b_i, lam)
     G, bw, _ = w_r.shape
     D = G * bw
     wcat = torch.empty(G, 2 * bw, bw, device=x.device, dtype=x.dtype)
@@ -849,7 +848,7 @@ def _layer_fwd(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, la
     lib = _lib.load()
     dt = _io_dtype(x, "layer forward")
     B, T, D = x.shape
-    w_r, b_r, w_i, b_i, lam = _kernel_params(x, w_r, b_r, w_i, b_i, lam)
+    w_r, b_r, w_i, b_i, lam = _kernel_params(w_r, b_r, w_i, b_i, lam)
     bw = w_r.shape[1]
     u = torch.empty(B, T, 2 * D, device=x.device, dtype=x.dtype)
     out = torch.empty_like(x)
@@ -923,6 +922,10 @@ def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, l
         raise ValueError("branch must have the shape of x")
     if not gated_supported(x, bw):
         raise ValueError("the gate layout needs CUDA tensors and gate heads of whole 16-byte groups of channels")
+    _same_device(x, w_r, b_r, w_i, b_i, lam, h0, tok, branch)
+    if h0 is not None and h0.shape != (x.shape[0], x.shape[2]):
+        raise ValueError(f"h0 must be [batch, width], got {list(h0.shape)}")
+    _expect("tok", tok, (x.shape[0], x.shape[1]), torch.uint8)
     save = torch.is_grad_enabled() and any(
         t is not None and t.requires_grad for t in (x, w_r, b_r, w_i, b_i, lam, h0, branch))
     traced = _library_ops_active()

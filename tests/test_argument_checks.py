@@ -89,3 +89,22 @@ def test_token_plan_makes_strided_masks_dense(ops, monkeypatch):
     args["segment_pos"] = torch.zeros(5, 3, dtype=torch.long).T
     ops.token_plan(3, 5, torch.device("cpu"), **args)
     assert len(seen) >= 6 and all(t is None or t.is_contiguous() for t in seen)
+
+
+@pytest.mark.parametrize("one_call", [False, True])
+@pytest.mark.parametrize("name,change", [
+    ("h0", lambda t: t[:1]), ("h0", lambda t: t[:, :8]), ("h0", lambda t: t.to("meta")), ("tok", lambda t: t[:, :4]),
+    ("tok", lambda t: t.int()), ("tok", lambda t: t.to("meta")), ("branch", lambda t: t.to("meta")),
+    ("w_i", lambda t: t.to("meta")), ("lam", lambda t: t.to("meta"))])
+def test_gated_layer_refuses_states_flags_and_branches_it_cannot_read(ops, monkeypatch, one_call, name, change):
+    monkeypatch.setattr(ops, "_layer_in_library", lambda *a: one_call)
+    monkeypatch.setattr(ops, "gated_supported", lambda *a: True)
+    B, T, D, G = 2, 5, 128, 2
+    w, b = torch.randn(G, D // G, D // G), torch.randn(G, D // G)
+    args = dict(x=torch.randn(B, T, D), w_r=w, b_r=b, w_i=w, b_i=b, lam=torch.randn(D), h0=torch.randn(B, D),
+                tok=torch.zeros(B, T, dtype=torch.uint8), branch=torch.randn(B, T, D))
+    with torch.no_grad(), pytest.raises(_Reached):
+        ops.rglru_gated(**args)
+    args[name] = change(args[name])
+    with torch.no_grad(), pytest.raises((ValueError, RuntimeError)):
+        ops.rglru_gated(**args)
