@@ -1093,7 +1093,9 @@ int rglru_decode_block(const void* x_in, const void* branch, const void* conv_w,
     return RGLRU_ERR_NULL_POINTER;
   const bool bf16 = io_dtype == RGLRU_BF16;
   const size_t es = bf16 ? 2 : 4;
-  if (B <= 0 || D <= 0 || gate_width <= 0 || D % gate_width != 0 || (gate_width * es) % 16 != 0 || B > 1000000)
+  // (the grids' y axes hold rows / 64 and channels / 512 or more, so these keep them below 65536)
+  if (B <= 0 || D <= 0 || gate_width <= 0 || D % gate_width != 0 || (gate_width * es) % 16 != 0 ||
+      B > RGLRU_DECODE_BLOCK_MAX_BATCH || D > RGLRU_DECODE_BLOCK_MAX_WIDTH)
     return RGLRU_ERR_BAD_SHAPE;
   if (!aligned(x_in, 16) || !aligned(branch, 16) || !aligned(conv_in, 16) || !aligned(conv_out, 16) || !aligned(w_r, 16) ||
       !aligned(w_i, 16) || !aligned(h_in, 16) || !aligned(h_out, 16) || !aligned(y, 16) || !aligned(ws, 16) ||

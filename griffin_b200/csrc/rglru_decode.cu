@@ -56,10 +56,10 @@ __global__ void __launch_bounds__(FRONT_THREADS) decode_front_kernel(const Decod
   const bool padded = p.active && __syncthreads_or(padding);
 
   const int nvec = p.D / VEC;
-  const int vec = blockIdx.x * FRONT_THREADS + threadIdx.x;
+  const int vec = blockIdx.y * FRONT_THREADS + threadIdx.x;
   if (vec >= nvec) return;
   const int d = vec * VEC;
-  const int b0 = blockIdx.y * ROWS;
+  const int b0 = blockIdx.x * ROWS;
   const IO* x = static_cast<const IO*>(p.x_in);
   const IO* cin = static_cast<const IO*>(p.conv_in);
   IO* cout = static_cast<IO*>(p.conv_out);
@@ -368,8 +368,9 @@ static cudaError_t launch_gates(const DecodeBlockArgs& a, cudaStream_t s) {
 
 template <typename IO, int ROWS>
 static cudaError_t launch_front(const DecodeBlockArgs& a, cudaStream_t s) {
-  const dim3 grid(static_cast<unsigned>((a.D / vec_width<IO>() + FRONT_THREADS - 1) / FRONT_THREADS),
-                  static_cast<unsigned>((a.B + ROWS - 1) / ROWS));
+  // batch rows on the x axis: the only one that goes past 65535 blocks
+  const dim3 grid(static_cast<unsigned>((a.B + ROWS - 1) / ROWS),
+                  static_cast<unsigned>((a.D / vec_width<IO>() + FRONT_THREADS - 1) / FRONT_THREADS));
   decode_front_kernel<IO, ROWS><<<grid, FRONT_THREADS, 0, s>>>(a);
   return cudaGetLastError();
 }

@@ -1312,8 +1312,10 @@ def decode_step(x: Tensor, u_r: Tensor, u_i: Tensor, lam: Tensor, h: Tensor, tok
 
 
 def decode_block_supported(x: Tensor, gate_width: int) -> bool:
-    """Whether :func:`decode_block` takes these activations: gate heads whose rows are whole 16-byte groups."""
-    return x.is_cuda and x.dtype in _DTYPES and gate_width * x.element_size() % 16 == 0
+    """Whether the recurrent block hands these activations to :func:`decode_block`: gate heads whose rows are whole 16-byte
+    groups, and at most 65536 rows (every block of its first kernel looks through the whole padding mask, which is nothing
+    at serving batches and a pass of its own beyond; the library itself takes a million rows)."""
+    return x.is_cuda and x.dtype in _DTYPES and gate_width * x.element_size() % 16 == 0 and x.shape[0] <= 65536
 
 
 def decode_block(x_in: Tensor, branch: Optional[Tensor], conv_w: Tensor, conv_b: Optional[Tensor], conv_state: Tensor,

@@ -361,8 +361,10 @@ int rglru_gelu_mul_bwd(const void* dout, const void* y, const void* branch, void
  *   active : [B] bytes, 0 = padding (state and position stay), or NULL       pos_out : [B]
  *   y : [B,D] io_dtype out     ws : rglru_decode_block_workspace_bytes(B,D,io_dtype) bytes
  * gate_width * element size must be a multiple of 16 bytes, activations, states, weights (conv_w too) and ws
- * 16-byte aligned.
+ * 16-byte aligned; B and D at most the two limits below.
  */
+#define RGLRU_DECODE_BLOCK_MAX_BATCH 1000000
+#define RGLRU_DECODE_BLOCK_MAX_WIDTH (1 << 24)
 #define RGLRU_F32_CONV_W 1
 #define RGLRU_F32_CONV_B 2
 #define RGLRU_F32_LAMBDA 4

@@ -68,3 +68,33 @@ def test_fused_token_matches_the_operators(dtype, batch, heads, head_width, mask
         assert torch.equal(new.rnn_state[rows], cache.rnn_state[rows])
         assert torch.equal(new.conv_state[rows], cache.conv_state[rows])
         assert torch.equal(new.segment_position[rows], cache.segment_position[rows])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_batches_past_one_grid_axis(dtype):
+    """262145 rows: one more than 65535 blocks of four rows hold.  Rows do not depend on each other, so the first and the
+    last ones are what a call on them alone gives, to the bit."""
+    from griffin_b200 import _lib, ops
+    torch.manual_seed(0)
+    batch, heads, bw = 262145, 1, 8
+    D = heads * bw
+    r = lambda *s: torch.randn(*s, device=DEV).to(dtype)
+    shared = dict(conv_w=r(D, 4), conv_b=r(D), w_r=r(heads, bw, bw), b_r=r(heads, bw), w_i=r(heads, bw, bw), b_i=r(heads, bw),
+                  lam=torch.randn(D, device=DEV))
+    rows = dict(x_in=r(batch, D), branch=r(batch, D), conv_state=r(batch, 3, D), h=torch.randn(batch, D, device=DEV),
+                position=torch.randint(0, 5, (batch,), device=DEV))
+    whole = ops.decode_block(**rows, **shared)
+    for part in (slice(0, 100), slice(batch - 97, batch)):
+        alone = ops.decode_block(**{k: v[part] for k, v in rows.items()}, **shared)
+        for a, b in zip(whole, alone):
+            assert torch.equal(a[part], b)
+    assert _lib.device_status() == 0
+
+
+def test_very_large_batches_go_by_operators(monkeypatch):
+    from griffin_b200 import ops
+    block, x, cache, _, _ = _setup(65537, 1, 8, torch.bfloat16, False, False)
+    monkeypatch.setattr(ops, "decode_block", None)
+    with torch.no_grad():
+        out, _ = block.bfloat16()(x, cache, return_cache=True)
+    assert torch.isfinite(out).all()
