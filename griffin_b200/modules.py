@@ -441,13 +441,13 @@ class RecurrentBlock(nn.Module):
         """Whether ``ops.decode_block`` does this cached token: this package's own layers in the dtype of ``x`` (the conv
         and Lambda may be fp32), a cache of the right shapes, no autograd, no autocast, no tracing.  Whatever it does not
         do -- and whatever has to be refused -- goes operator by operator."""
-        if (torch.is_grad_enabled() or not x.is_cuda or ops._library_ops_active() or torch.is_autocast_enabled("cuda")
-                or not ops.decode_block_supported(x, self.rg_lru.recurrence_gate.block_width)):
+        if torch.is_grad_enabled() or not x.is_cuda or ops._library_ops_active() or torch.is_autocast_enabled("cuda"):
             return False
         lru, conv = self.rg_lru, self.temporal_conv
-        if not (_is_stock(self.linear_x, nn.Linear) and _is_stock(self.linear_y, nn.Linear)
+        # (replaced layers need not have any of the attributes read below)
+        if not (type(lru) is RG_LRU and _is_stock(self.linear_x, nn.Linear) and _is_stock(self.linear_y, nn.Linear)
                 and _is_stock(lru.recurrence_gate, BlockDiagonalLinear) and _is_stock(lru.input_gate, BlockDiagonalLinear)
-                and type(lru) is RG_LRU):
+                and ops.decode_block_supported(x, lru.recurrence_gate.block_width)):
             return False
         batch, width = x.shape[0], self.rnn_width
         for gate in (lru.recurrence_gate, lru.input_gate):

@@ -108,3 +108,22 @@ def test_gated_layer_refuses_states_flags_and_branches_it_cannot_read(ops, monke
     args[name] = change(args[name])
     with torch.no_grad(), pytest.raises((ValueError, RuntimeError)):
         ops.rglru_gated(**args)
+
+
+def test_a_cached_token_through_a_replaced_gate_is_not_taken_by_the_fused_form():
+    """The decision reads nothing that a replaced layer need not have."""
+    from griffin_b200 import RecurrentBlock
+
+    class OnGpu:
+        is_cuda, shape, dtype = True, (1, 1, 32), torch.float32
+        element_size = staticmethod(lambda: 4)
+
+    for replace in ("recurrence_gate", "input_gate"):
+        block = RecurrentBlock(32, 64, gate_blocks=2)
+        setattr(block.rg_lru, replace, torch.nn.Identity())
+        with torch.no_grad():
+            assert block._decodes_fused(OnGpu(), None, None) is False
+    block = RecurrentBlock(32, 64, gate_blocks=2)
+    block.rg_lru = torch.nn.Identity()
+    with torch.no_grad():
+        assert block._decodes_fused(OnGpu(), None, None) is False

@@ -98,3 +98,23 @@ def test_very_large_batches_go_by_operators(monkeypatch):
     with torch.no_grad():
         out, _ = block.bfloat16()(x, cache, return_cache=True)
     assert torch.isfinite(out).all()
+
+
+class _Scale(torch.nn.Module):
+    """A gate without any attribute of the layer it replaces."""
+
+    def forward(self, x):
+        return x * 0.5
+
+
+def test_a_replaced_gate_goes_by_operators():
+    block, x, cache, _, _ = _setup(3, 2, 16, torch.float32, False, False)
+    block.rg_lru.group_gates = False
+    block.rg_lru.recurrence_gate = _Scale()
+    with torch.no_grad():
+        out, new = block(x, cache, return_cache=True)
+        # with gradients the token takes the scan kernels
+        with torch.enable_grad():
+            want, ref = block(x, cache, return_cache=True)
+    torch.testing.assert_close(out, want, rtol=1e-5, atol=1e-5)
+    torch.testing.assert_close(new.rnn_state, ref.rnn_state, rtol=1e-5, atol=1e-5)
