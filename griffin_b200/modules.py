@@ -56,9 +56,11 @@ def _largest_block_count(width: int, requested: int) -> int:
 
 
 def _is_stock(layer: nn.Module, kind: type) -> bool:
-    """Whether a submodule is the one this package put there: not replaced, not parametrised, without hooks."""
+    """Whether a submodule is the one this package put there: not replaced, not parametrised, without hooks of its own or
+    for all modules (``torch.nn.modules.module.register_module_forward_hook`` and its like)."""
     return type(layer) is kind and "forward" not in layer.__dict__ and not (
-        layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks)
+        layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks
+        or torch.nn.modules.module._has_any_global_hook())
 
 
 class BlockDiagonalLinear(nn.Module):

@@ -127,3 +127,18 @@ def test_a_cached_token_through_a_replaced_gate_is_not_taken_by_the_fused_form()
     block.rg_lru = torch.nn.Identity()
     with torch.no_grad():
         assert block._decodes_fused(OnGpu(), None, None) is False
+
+
+@pytest.mark.parametrize("register", ["register_module_forward_hook", "register_module_forward_pre_hook",
+                                      "register_module_full_backward_hook"])
+def test_hooks_for_all_modules_keep_the_gates_modules(register):
+    """A hook registered for every module has to see the gate projections, so they are called as the modules they are."""
+    from griffin_b200 import RG_LRU, modules
+    gate = RG_LRU(96, gate_blocks=2).recurrence_gate
+    assert modules._is_stock(gate, modules.BlockDiagonalLinear)
+    handle = getattr(torch.nn.modules.module, register)(lambda *args: None)
+    try:
+        assert not modules._is_stock(gate, modules.BlockDiagonalLinear)
+    finally:
+        handle.remove()
+    assert modules._is_stock(gate, modules.BlockDiagonalLinear)

@@ -134,3 +134,15 @@ def test_parameters_elsewhere_are_refused():
     layer.input_gate.weight.data = layer.input_gate.weight.data.cpu()
     with pytest.raises(RuntimeError):
         layer(torch.randn(1, 4, 128, device=DEV))
+
+
+def test_hooks_for_all_modules_see_the_gates():
+    from griffin_b200 import RG_LRU, BlockDiagonalLinear
+    layer = RG_LRU(96, gate_blocks=2).to(DEV)
+    seen = []
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda module, args, out: seen.append(type(module)))
+    try:
+        layer(torch.randn(1, 4, 96, device=DEV))
+    finally:
+        handle.remove()
+    assert seen.count(BlockDiagonalLinear) == 2
