@@ -213,6 +213,10 @@ __device__ __forceinline__ void st_async_pair(uint32_t dst, float2 v, uint32_t b
                "f"(v.x), "f"(v.y), "r"(bar)
                : "memory");
 }
+__device__ __forceinline__ void st_async_f32(uint32_t dst, float v, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(dst), "f"(v), "r"(bar)
+               : "memory");
+}
 __device__ __forceinline__ void st_cluster_f32(uint32_t dst, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(v) : "memory");
 }

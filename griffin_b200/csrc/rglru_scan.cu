@@ -39,6 +39,7 @@
 // conv alone, and the self-test of the bounded wait.
 
 #include <atomic>
+#include <cfloat>
 #include <cstddef>
 #include <cstdlib>
 
@@ -1348,6 +1349,19 @@ constexpr int RAW_TC = RAW_LANES * RAW_TS;
 constexpr int RAW_TILE = RAW_TC * CH * 4;
 constexpr int RAW_STAGES = 4;
 
+// The decays of this operator are the caller's and may be of any size, so the map of a whole chunk is not always what
+// the steps it is made of are: a product of 64 decays above one overflows, or takes the digits of a state that the steps
+// would have left small (h = 4 h - 3 stays at 1 for ever, 4^64 1 - (4^64 - 1) does not), and one that underflows turns an
+// infinite state into NaN.  Maps of decays up to one do neither.  So a channel whose round has a lane's product above one,
+// or a state that is not finite, is chained lane by lane instead, the ranks of the cluster one after another, each
+// handing the state behind its chunk to all: the same arithmetic as the unsplit kernel's.  CH is one warp, so which
+// channels these are is a ballot, and every CTA of the cluster, having the same pairs, comes to the same answer.
+struct RawSerial {
+  float exact[MAX_SPLIT][CH];    // state behind rank r's chunk of this round
+  uint64_t bar[MAX_SPLIT];
+};
+static_assert(CH == 32, "the channels of a tile are one warp");
+
 // The chain leaves the state entering a lane where the lane's aggregate was (.x of its pair), so that a split backward
 // with two stages stays below half an SM's shared memory.
 template <int NSTAGE, int NTILE, bool SPLIT>
@@ -1356,7 +1370,8 @@ struct RawSmem {
   static constexpr int OFF_AGG = NSTAGE * STAGE;
   static constexpr int OFF_BAR = OFF_AGG + ChainSmem<RAW_LANES, CH>::AGG;
   static constexpr int OFF_SPLIT = OFF_BAR + NSTAGE * 8 + 16;
-  static constexpr int BYTES = OFF_SPLIT + (SPLIT ? static_cast<int>(offsetof(SplitSmem<CH>, sums)) : 0);
+  static constexpr int OFF_SERIAL = OFF_SPLIT + static_cast<int>(offsetof(SplitSmem<CH>, sums));
+  static constexpr int BYTES = SPLIT ? OFF_SERIAL + static_cast<int>(sizeof(RawSerial)) : OFF_SPLIT;
 };
 // The states (carries) of a thread's four channels that enter its lane.
 __device__ __forceinline__ void raw_entering(const float2* agg, int at, float2 (&e)[2]) {
@@ -1364,10 +1379,11 @@ __device__ __forceinline__ void raw_entering(const float2* agg, int at, float2 (
   e[0] = make_float2(a.x, a.z);
   e[1] = make_float2(b.x, b.z);
 }
-// Level two of a chunk for one channel: chain the lane aggregates onto the carry (lanes in increasing time order, or
-// decreasing with REV) and leave every lane's entering state in place.  `idle`: this CTA has no chunk in the round.
+// Level two of a chunk for one channel (thread): chain the lane aggregates onto the carry (lanes in increasing time order,
+// or decreasing with REV) and leave every lane's entering state in place.  `idle`: this CTA has no chunk in the round.
 template <bool REV, bool SPLIT>
-__device__ __forceinline__ void raw_chain(float2* agg, float& carry, SplitChain<CH>& split, int it, bool idle, bool& alive) {
+__device__ __forceinline__ void raw_chain(float2* agg, float& carry, SplitChain<CH>& split, RawSerial* serial, int& serial_rounds,
+                                          int it, bool idle, bool& alive) {
   constexpr int LANES = RAW_LANES;
   const int tid = threadIdx.x;
   float2 ag[LANES];
@@ -1384,19 +1400,51 @@ __device__ __forceinline__ void raw_chain(float2* agg, float& carry, SplitChain<
     carry = e;
   } else {
     float2 m = make_float2(1.0f, 0.0f);        // map from the state entering the chunk to that entering the lane
+    bool composable = true;
 #pragma unroll
     for (int q = 0; q < LANES; ++q) {
       const int j = REV ? LANES - 1 - q : q;
       const float2 a = ag[j];
+      composable = composable && fabsf(a.x) <= 1.0f;
       ag[j] = m;
       m = make_float2(m.x * a.x, fmaf(a.x, m.y, a.y));
     }
+    if (!composable) m.x = __int_as_float(0x7f800000);      // tells every rank
     split.send(it, tid, m, 0, 1);
     float unused = 1.0f;
+    const float before = carry;
     const float e = split.receive(it, tid, carry, unused, alive);
-    if (!idle) {
+    bool steady = fabsf(carry) <= FLT_MAX;     // (a state that is not finite stays so to the end of the round)
+    for (uint32_t r = 0; r < split.size; ++r) steady = steady && fabsf(split.sm->pair[it & 1][r][tid].x) <= 1.0f;
+    const unsigned wild = __ballot_sync(0xffffffffu, !steady);
+    if (steady && !idle) {
 #pragma unroll
       for (int j = 0; j < LANES; ++j) agg[j * CH + tid].x = fmaf(ag[j].x, e, ag[j].y);
+    }
+    if (wild) {
+      if (tid == 0)
+        for (uint32_t r = 0; r < split.size; ++r) mbar_expect_tx(&serial->bar[r], 4 * __popc(wild));
+      __syncwarp();
+      float state = before;
+      for (uint32_t r = 0; r < split.size; ++r) {
+        if (r == split.rank && !steady) {
+          if (!idle) {
+            for (int q = 0; q < LANES; ++q) {
+              float2* lane = agg + (REV ? LANES - 1 - q : q) * CH + tid;
+              const float2 a = *lane;
+              lane->x = state;
+              state = fmaf(a.x, state, a.y);
+            }
+          }
+          for (uint32_t to = 0; to < split.size; ++to)
+            st_async_f32(cluster_map(&serial->exact[r][tid], to), state, cluster_map(&serial->bar[r], to));
+        }
+        __syncwarp();
+        if (alive) alive = mbar_wait_bounded(&serial->bar[r], serial_rounds & 1);
+        if (!steady) state = serial->exact[r][tid];
+      }
+      if (!steady) carry = state;
+      ++serial_rounds;
     }
   }
 }
@@ -1413,6 +1461,8 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_fwd_kernel(const __grid_consta
   const int nchunks = (p.T + TC - 1) / TC;
   SplitChain<CH> split;
   if constexpr (SPLIT) split.init(reinterpret_cast<SplitSmem<CH>*>(smem + SM::OFF_SPLIT));
+  [[maybe_unused]] RawSerial* serial = reinterpret_cast<RawSerial*>(smem + SM::OFF_SERIAL);      // SPLIT only
+  [[maybe_unused]] int serial_rounds = 0;
   const int rank = SPLIT ? static_cast<int>(split.rank) : 0, nranks = SPLIT ? static_cast<int>(split.size) : 1;
   const int rounds = SPLIT ? (nchunks + nranks - 1) / nranks : nchunks;
   const int mine = SPLIT ? (nchunks - rank + nranks - 1) / nranks : nchunks;   // chunks this CTA loads and stores
@@ -1428,7 +1478,11 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_fwd_kernel(const __grid_consta
   if (USE_TMA) {
     if (tid == 0) {
       for (int s = 0; s < NSTAGE; ++s) mbar_init(&bars[s], 1);
-      if constexpr (SPLIT) { mbar_init(&split.sm->bar[0], 1); mbar_init(&split.sm->bar[1], 1); }
+      if constexpr (SPLIT) {
+        mbar_init(&split.sm->bar[0], 1);
+        mbar_init(&split.sm->bar[1], 1);
+        for (int r = 0; r < MAX_SPLIT; ++r) mbar_init(&serial->bar[r], 1);
+      }
       mbar_fence_init();
     }
     if constexpr (SPLIT) cluster_sync_all();
@@ -1484,7 +1538,7 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_fwd_kernel(const __grid_consta
     }
     alive = __syncthreads_and(alive);
     if (!SPLIT && !alive) break;
-    if (tid < CH) raw_chain<false, SPLIT>(agg, carry, split, it, idle, alive);
+    if (tid < CH) raw_chain<false, SPLIT>(agg, carry, split, serial, serial_rounds, it, idle, alive);
     __syncthreads();
     if (idle) break;
     {
@@ -1535,6 +1589,8 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_bwd_kernel(const __grid_consta
   const int nchunks = (p.T + TC - 1) / TC;
   SplitChain<CH> split;
   if constexpr (SPLIT) split.init(reinterpret_cast<SplitSmem<CH>*>(smem + SM::OFF_SPLIT));
+  [[maybe_unused]] RawSerial* serial = reinterpret_cast<RawSerial*>(smem + SM::OFF_SERIAL);      // SPLIT only
+  [[maybe_unused]] int serial_rounds = 0;
   const int rank = SPLIT ? static_cast<int>(split.rank) : 0, nranks = SPLIT ? static_cast<int>(split.size) : 1;
   const int rounds = SPLIT ? (nchunks + nranks - 1) / nranks : nchunks;
   const int mine = SPLIT ? (nchunks - rank + nranks - 1) / nranks : nchunks;   // chunks this CTA loads and stores
@@ -1552,7 +1608,11 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_bwd_kernel(const __grid_consta
   if (USE_TMA) {
     if (tid == 0) {
       for (int s = 0; s < NSTAGE; ++s) mbar_init(&bars[s], 1);
-      if constexpr (SPLIT) { mbar_init(&split.sm->bar[0], 1); mbar_init(&split.sm->bar[1], 1); }
+      if constexpr (SPLIT) {
+        mbar_init(&split.sm->bar[0], 1);
+        mbar_init(&split.sm->bar[1], 1);
+        for (int r = 0; r < MAX_SPLIT; ++r) mbar_init(&serial->bar[r], 1);
+      }
       mbar_fence_init();
     }
     if constexpr (SPLIT) cluster_sync_all();
@@ -1613,7 +1673,7 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_bwd_kernel(const __grid_consta
     }
     alive = __syncthreads_and(alive);
     if (!SPLIT && !alive) break;
-    if (tid < CH) raw_chain<true, SPLIT>(agg, carry, split, q, idle, alive);
+    if (tid < CH) raw_chain<true, SPLIT>(agg, carry, split, serial, serial_rounds, q, idle, alive);
     __syncthreads();
     if (idle) break;
     {

@@ -96,3 +96,78 @@ def test_split_raw_scan(steps, width):
     for g, r in zip(dev, ref):
         assert orc.rel_l2(g.grad, r.grad) <= 1e-5
     assert _lib.device_status() == 0
+
+
+def _raw_both_ways(a, b, h0, dy):
+    from griffin_b200 import _lib, ops
+    dev = [t.to(DEV).requires_grad_(True) for t in (a, b, h0)]
+    got = ops.linear_scan(*dev)
+    (got * dy.to(DEV)).sum().backward()
+    assert _lib.device_status() == 0
+    return [t.detach().cpu() for t in (got, *(d.grad for d in dev))]
+
+
+def _raw_reference(a, b, h0, dy):
+    ref = [t.double().requires_grad_(True) for t in (a, b, h0)]
+    want = orc.linear_scan(*ref)
+    (want * dy.double()).sum().backward()
+    return [want.detach()] + [r.grad for r in ref]
+
+
+@pytest.mark.parametrize("steps", [200, 513, 64 * 17 - 1])
+def test_raw_scan_of_growing_decays_before_the_drive_starts(steps):
+    """A product of decays over a chunk may overflow where no state does: zeros times decays of five are zeros, in time order
+    for the states and against it for their gradients.  Every third channel decays throughout."""
+    gen = torch.Generator().manual_seed(steps)
+    B, D = 2, 72
+    a = torch.full((B, steps, D), 5.0)
+    a[..., ::3] = torch.rand(B, steps, D // 3, generator=gen) * 0.3 + 0.7
+    a[:, steps - 12:] = 0.9
+    b, dy, h0 = torch.randn(B, steps, D, generator=gen), torch.randn(B, steps, D, generator=gen), torch.zeros(B, D)
+    grows = torch.ones(D, dtype=torch.bool)
+    grows[::3] = False
+    b[:, :steps - 10, grows] = 0.0
+    dy[:, 10:, grows] = 0.0
+    for k, (got, want) in enumerate(zip(_raw_both_ways(a, b, h0, dy), _raw_reference(a, b, h0, dy))):
+        assert torch.isfinite(got).all(), k
+        assert orc.rel_l2(got, want) <= 1e-5, k
+        assert orc.rel_l2(got[..., grows], want[..., grows]) <= 1e-5, k
+
+
+@pytest.mark.parametrize("steps", [65, 512, 1100])
+def test_raw_scan_at_an_unstable_fixed_point(steps):
+    """h = 4 h - 3 from one, and its gradient's mirror image: exact in fp32 at every step, and lost (or NaN) once a chunk's
+    product meets its sum."""
+    B, D = 1, 36
+    a, b, h0 = torch.full((B, steps, D), 4.0), torch.full((B, steps, D), -3.0), torch.ones(B, D)
+    dy = torch.full((B, steps, D), -3.0)
+    dy[:, -1] = 1.0
+    h, da, db, dh0 = _raw_both_ways(a, b, h0, dy)
+    for t, value in ((h, 1.0), (db, 1.0), (da, 1.0), (dh0, 4.0)):
+        assert torch.equal(t, torch.full_like(t, value))
+
+
+@pytest.mark.parametrize("steps", [300, 1100])
+def test_raw_scan_of_decays_on_both_sides_of_one(steps):
+    """Uniform in (-2, 2): lanes that grow and lanes that shrink, contractive on the whole.  Every state is a sum of at most
+    a few dozen terms that count, each of as many roundings: 1e-5 norm-wise."""
+    gen = torch.Generator().manual_seed(steps)
+    a = torch.rand(2, steps, 72, generator=gen) * 4 - 2
+    b, dy = torch.randn(2, steps, 72, generator=gen), torch.randn(2, steps, 72, generator=gen)
+    h0 = torch.randn(2, 72, generator=gen)
+    for got, want in zip(_raw_both_ways(a, b, h0, dy), _raw_reference(a, b, h0, dy)):
+        assert orc.rel_l2(got, want) <= 1e-5
+
+
+def test_raw_scan_of_an_infinite_state():
+    """An infinite state times a decay is infinite, however small the product of the decays; a NaN stays one."""
+    steps, D = 640, 40
+    a, b = torch.full((1, steps, D), 0.1), torch.ones(1, steps, D)
+    b[0, 70, 3] = float("inf")
+    b[0, 5, 7] = float("nan")
+    from griffin_b200 import ops
+    h = ops.linear_scan(a.to(DEV), b.to(DEV), torch.zeros(1, D, device=DEV)).cpu()
+    assert torch.isinf(h[0, 70:, 3]).all() and torch.isfinite(h[0, :70, 3]).all()
+    assert torch.isnan(h[0, 5:, 7]).all() and torch.isfinite(h[0, :5, 7]).all()
+    rest = [c for c in range(D) if c not in (3, 7)]
+    assert torch.isfinite(h[0, :, rest]).all()
