@@ -1038,8 +1038,16 @@ int rglru_layer_bwd(const void* dout, const float* dh_last, const void* x, const
 
 int rglru_token_plan(const int64_t* seg_pos, const int64_t* prev_pos, const uint8_t* active, const uint8_t* reset,
                      int positions, uint8_t* flags, int64_t* last_pos, int B, int T, void* stream) {
+  return rglru_token_plan_ws(seg_pos, prev_pos, active, reset, positions, flags, last_pos, nullptr, 0, B, T, stream);
+}
+
+size_t rglru_token_plan_workspace_bytes(int B, int T) { return B > 0 && T > 0 ? token_plan_parts(B, T) : 0; }
+
+int rglru_token_plan_ws(const int64_t* seg_pos, const int64_t* prev_pos, const uint8_t* active, const uint8_t* reset,
+                        int positions, uint8_t* flags, int64_t* last_pos, void* ws, size_t ws_bytes, int B, int T, void* stream) {
   if (!flags) return RGLRU_ERR_NULL_POINTER;
   if (B <= 0 || T <= 0 || T > (1 << 30)) return RGLRU_ERR_BAD_SHAPE;
+  if (ws && ws_bytes < rglru_token_plan_workspace_bytes(B, T)) return RGLRU_ERR_WORKSPACE;
   if (!aligned(seg_pos, 8) || !aligned(prev_pos, 8) || !aligned(last_pos, 8)) return RGLRU_ERR_MISALIGNED;
   int* status = nullptr;
   const int rc = device_setup(&status);
@@ -1048,6 +1056,8 @@ int rglru_token_plan(const int64_t* seg_pos, const int64_t* prev_pos, const uint
   a.seg = reinterpret_cast<const long long*>(seg_pos); a.prev = reinterpret_cast<const long long*>(prev_pos);
   a.active = active; a.reset = reset; a.flags = flags; a.last = reinterpret_cast<long long*>(last_pos);
   a.positions = positions != 0; a.B = B; a.T = T;
+  a.nparts = ws && active && positions ? token_plan_parts(B, T) : 0;
+  a.parts = a.nparts > 0 ? static_cast<uint8_t*>(ws) : nullptr;
   const cudaError_t e = launch_token_plan(a, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
 }

@@ -16,24 +16,37 @@ constexpr int PLAN_TOKENS = 4;      // per thread and tile
 
 // Whether any byte of the mask is zero; the CTA stops looking at the first one it finds.
 __device__ __forceinline__ bool any_zero_byte(const uint8_t* m, long long n) {
-  const bool wide = (reinterpret_cast<uintptr_t>(m) & 15u) == 0;
-  const long long nw = wide ? n / 16 : 0;
+  const long long lead = min(static_cast<long long>((16 - (reinterpret_cast<uintptr_t>(m) & 15u)) & 15u), n);   // up to a 16-byte boundary
+  const uint4* mw = reinterpret_cast<const uint4*>(m + lead);
+  const long long nw = (n - lead) / 16;
   constexpr int FLIGHT = 4;
   for (long long w0 = 0; w0 < nw; w0 += PLAN_THREADS * FLIGHT) {
     uint4 v[FLIGHT];
 #pragma unroll
     for (int j = 0; j < FLIGHT; ++j) {
       const long long w = w0 + j * PLAN_THREADS + threadIdx.x;
-      v[j] = w < nw ? reinterpret_cast<const uint4*>(m)[w] : make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u);
+      v[j] = w < nw ? mw[w] : make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u);
     }
     uint32_t least = 0x01010101u;
 #pragma unroll
     for (int j = 0; j < FLIGHT; ++j) least = __vminu4(least, __vminu4(__vminu4(v[j].x, v[j].y), __vminu4(v[j].z, v[j].w)));
     if (__syncthreads_or(least != 0x01010101u)) return true;
   }
-  int zero = 0;
-  for (long long i = nw * 16 + threadIdx.x; i < n; i += PLAN_THREADS) zero |= m[i] == 0;
+  int zero = threadIdx.x < lead && m[threadIdx.x] == 0;
+  for (long long i = lead + nw * 16 + threadIdx.x; i < n; i += PLAN_THREADS) zero |= m[i] == 0;
   return __syncthreads_or(zero) != 0;
+}
+
+// One pass over the mask of the whole batch: block i notes whether its stretch of PLAN_STRETCH bytes, and every
+// gridDim.x-th one after it, has a zero.
+constexpr long long PLAN_STRETCH = 32768;
+constexpr long long PLAN_BLOCKS = 4 * 148;
+constexpr long long PLAN_LOOK = 65536;
+__global__ void __launch_bounds__(PLAN_THREADS) token_padding_kernel(const uint8_t* mask, long long n, uint8_t* part) {
+  bool zero = false;
+  for (long long i = blockIdx.x * PLAN_STRETCH; i < n && !zero; i += gridDim.x * PLAN_STRETCH)
+    zero = any_zero_byte(mask + i, min(PLAN_STRETCH, n - i));
+  if (threadIdx.x == 0) part[blockIdx.x] = zero;
 }
 
 __global__ void __launch_bounds__(PLAN_THREADS) token_plan_kernel(const TokenPlanArgs p) {
@@ -46,7 +59,16 @@ __global__ void __launch_bounds__(PLAN_THREADS) token_plan_kernel(const TokenPla
   uint8_t* flags = p.flags + static_cast<size_t>(b) * p.T;
   const long long prev = p.prev ? p.prev[b] : -1;
   // Padding anywhere in the batch: the first token of a document then wipes the history it would leave behind.
-  const bool padded = p.positions && p.active && (any_zero_byte(active, p.T) || any_zero_byte(p.active, static_cast<long long>(p.B) * p.T));
+  bool padded = false;
+  if (p.positions && p.active) {
+    if (p.parts) {
+      int zero = 0;
+      for (int i = tid; i < p.nparts; i += PLAN_THREADS) zero |= p.parts[i];
+      padded = __syncthreads_or(zero) != 0;
+    } else {
+      padded = any_zero_byte(active, p.T) || (p.B > 1 && any_zero_byte(p.active, static_cast<long long>(p.B) * p.T));
+    }
+  }
   if (tid == 0) s_last = -1;
   const bool counted = p.positions && p.active && !p.seg;      // positions are the running count of real tokens
   int carry = 0;
@@ -105,7 +127,16 @@ __global__ void __launch_bounds__(PLAN_THREADS) token_plan_kernel(const TokenPla
   if (last_t == s_last && (last_t >= 0 || tid == 0)) p.last[b] = last_pos;
 }
 
+// A mask of up to 64 KB is looked through by every row's CTA, which costs less than the launch of token_padding_kernel;
+// beyond, that is the batch's rows times the mask (an all-true 1024 x 2048 mask: 254 us, 13 in two launches; 256 x 2048: 25 and 7; 64 x 2048: 6.5 and 5.9).
+int token_plan_parts(int B, int T) {
+  const long long n = static_cast<long long>(B) * T;
+  if (B == 1 || n <= PLAN_LOOK) return 0;
+  const long long want = (n + PLAN_STRETCH - 1) / PLAN_STRETCH;
+  return static_cast<int>(want < PLAN_BLOCKS ? want : PLAN_BLOCKS);
+}
 cudaError_t launch_token_plan(const TokenPlanArgs& a, cudaStream_t s) {
+  if (a.parts) token_padding_kernel<<<a.nparts, PLAN_THREADS, 0, s>>>(a.active, static_cast<long long>(a.B) * a.T, a.parts);
   token_plan_kernel<<<a.B, PLAN_THREADS, 0, s>>>(a);
   return cudaGetLastError();
 }

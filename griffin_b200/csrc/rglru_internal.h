@@ -171,6 +171,8 @@ struct TokenPlanArgs {
   long long* last;
   bool positions;      // flags of a block call from positions, not of a bare layer from its reset mask
   int B, T;
+  uint8_t* parts;      // one byte for each of nparts parts of the mask (see token_plan_parts), or nullptr
+  int nparts;
 };
 // out = y * gelu(g), or with dout given out = dy and dg.
 struct GeluMulArgs {
@@ -260,6 +262,7 @@ int conv_tma_box_rows();
 int conv_tma_box_cols();
 cudaError_t launch_decode_conv(bool bf16, const ConvArgs& a, cudaStream_t s);
 cudaError_t launch_decode_step(bool bf16, const DecodeArgs& a, cudaStream_t s);
+int token_plan_parts(int B, int T);    // parts a pass over the mask has; 0: every row's CTA looks through it
 cudaError_t launch_token_plan(const TokenPlanArgs& a, cudaStream_t s);
 cudaError_t launch_gelu_mul(bool bf16, const GeluMulArgs& a, bool vector_ok, cudaStream_t s);
 cudaError_t launch_gate_pack(bool f32_weights, bool bf16, const GatePackArgs& a, cudaStream_t s);

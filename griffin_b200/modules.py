@@ -98,8 +98,7 @@ def token_flags(batch: int, steps: int, device, *, reset: Optional[Tensor] = Non
     if segment_pos is None and not ops._library_ops_active() and all(
             m is None or (m.is_cuda and m.dtype == torch.bool and m.shape == (batch, steps) and m.device == torch.device(device))
             for m in (reset, active)) and batch > 0 and steps > 0:
-        return ops.token_plan(batch, steps, device, reset=None if reset is None else reset.contiguous(),
-                              active=None if active is None else active.contiguous(), positions=False)[0]
+        return ops.token_plan(batch, steps, device, reset=reset, active=active, positions=False)[0]
     flags = torch.zeros(batch, steps, device=device, dtype=torch.uint8)
     if segment_pos is not None:
         cut = (3 - segment_pos.clamp(min=0, max=3)).to(torch.uint8)
@@ -512,10 +511,10 @@ class RecurrentBlock(nn.Module):
             split = active_mask is not None and steps > 1 and _needs_partition(active_mask, caller_mask)
             if (not split and x.is_cuda and not ops._library_ops_active() and batch > 0
                     and (previous is None or previous.shape == (batch,))):
-                as_long = lambda t: None if t is None else t.to(device=device, dtype=torch.long).contiguous()
+                as_long = lambda t: None if t is None else t.to(device=device, dtype=torch.long)
                 # (with positions of its own a call needs the cached ones only for rows that are all padding)
                 flags, last = ops.token_plan(batch, steps, device, segment_pos=as_long(segment_pos), previous=as_long(previous),
-                                             active=None if active_mask is None else active_mask.contiguous())
+                                             active=active_mask)
                 return flags, None, last, None
             pos = _positions(x, segment_pos, previous, active_mask)
             moves = None

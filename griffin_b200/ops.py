@@ -1229,15 +1229,26 @@ def token_plan(batch: int, steps: int, device, *, segment_pos: Optional[Tensor] 
     flags = torch.empty(batch, steps, device=device, dtype=torch.uint8)
     _require_cuda(flags)
     _same_device(flags, segment_pos, previous, active, reset)
-    _expect("segment_pos", segment_pos, (batch, steps), torch.long)
-    _expect("previous", previous, (batch,), torch.long)
-    _expect("active", active, (batch, steps), torch.bool)
-    _expect("reset", reset, (batch, steps), torch.bool)
-    segment_pos, previous, active, reset = (t if t is None else t.contiguous() for t in (segment_pos, previous, active, reset))
+    per_token = (batch, steps)
+    if segment_pos is not None:
+        _expect("segment_pos", segment_pos, per_token, torch.long)
+        segment_pos = segment_pos.contiguous()
+    if previous is not None:
+        _expect("previous", previous, (batch,), torch.long)
+        previous = previous.contiguous()
+    if active is not None:
+        _expect("active", active, per_token, torch.bool)
+        active = active.contiguous()
+    if reset is not None:
+        _expect("reset", reset, per_token, torch.bool)
+        reset = reset.contiguous()
     last = torch.empty(batch, device=device, dtype=torch.long) if positions else None
+    lib = _lib.load()
+    nbytes = lib.rglru_token_plan_workspace_bytes(batch, steps) if positions and active is not None else 0
+    ws = torch.empty(nbytes, device=device, dtype=torch.uint8) if nbytes else None
     with _on(flags, "rglru_token_plan"):
-        rc = _lib.load().rglru_token_plan(_ptr(segment_pos), _ptr(previous), _ptr(active), _ptr(reset), int(positions),
-                                          _ptr(flags), _ptr(last), batch, steps, _stream(flags))
+        rc = lib.rglru_token_plan_ws(_ptr(segment_pos), _ptr(previous), _ptr(active), _ptr(reset), int(positions), _ptr(flags),
+                                     _ptr(last), _ptr(ws), nbytes, batch, steps, _stream(flags))
     _lib.check(rc, "rglru_token_plan")
     return flags, last
 

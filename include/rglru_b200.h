@@ -342,6 +342,11 @@ int rglru_decode_step(const void* x, const void* u_r, const void* u_i, const flo
  *   flags : [B,T] out     last_pos : [B] out or NULL: position of the row's last active token, prev_pos if it has none */
 int rglru_token_plan(const int64_t* seg_pos, const int64_t* prev_pos, const uint8_t* active, const uint8_t* reset,
                      int positions, uint8_t* flags, int64_t* last_pos, int B, int T, void* stream);
+/* The same for masks of any size: `ws` (rglru_token_plan_workspace_bytes(B, T) bytes, none for small masks or without
+ * `active`) lets one pass find out whether there is any padding, where rglru_token_plan has every row look for it. */
+size_t rglru_token_plan_workspace_bytes(int B, int T);
+int rglru_token_plan_ws(const int64_t* seg_pos, const int64_t* prev_pos, const uint8_t* active, const uint8_t* reset,
+                        int positions, uint8_t* flags, int64_t* last_pos, void* ws, size_t ws_bytes, int B, int T, void* stream);
 
 /* out = y * gelu_tanh(branch) of n elements, and its gradient (griffin/griffin.py:464, 520). */
 int rglru_gelu_mul_fwd(const void* y, const void* branch, void* out, long long n, int io_dtype, void* stream);

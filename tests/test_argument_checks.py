@@ -83,7 +83,8 @@ def test_token_plan_makes_strided_masks_dense(ops, monkeypatch):
     ptr = ops._ptr
     monkeypatch.setattr(ops, "_ptr", lambda t: seen.append(t) or ptr(t))
     monkeypatch.setattr(ops, "_stream", lambda t: 0)
-    monkeypatch.setattr(ops._lib, "load", lambda: type("L", (), {"rglru_token_plan": staticmethod(lambda *a: 0)}))
+    monkeypatch.setattr(ops._lib, "load", lambda: type("L", (), {
+        "rglru_token_plan_ws": staticmethod(lambda *a: 0), "rglru_token_plan_workspace_bytes": staticmethod(lambda *a: 0)}))
     args = _plan_args()
     args["active"] = torch.ones(5, 3, dtype=torch.bool).T
     args["segment_pos"] = torch.zeros(5, 3, dtype=torch.long).T

@@ -75,3 +75,23 @@ def test_gelu_mul_far_out(value):
     y, g = torch.full((8,), 2.0, device=DEV), torch.full((8,), value, device=DEV)
     want = y * torch.nn.functional.gelu(g, approximate="tanh")
     torch.testing.assert_close(ops.gelu_mul(y, g), want, equal_nan=True)
+
+
+@pytest.mark.parametrize("batch,steps", [(1, 70000), (2, 32769), (9, 8192), (1024, 2048), (70000, 1)])
+@pytest.mark.parametrize("hole", [None, 0, 0.5, 1])
+def test_token_plan_of_large_masks(batch, steps, hole):
+    """Padding is looked for in parts: none, or one token of it at the first, a middle and the last place."""
+    from griffin_b200 import modules, ops
+    x = torch.empty(batch, steps, 1, device=DEV)
+    storage = torch.ones(batch * steps + 3, dtype=torch.bool, device=DEV)
+    for shift in (0, 3):                                  # a mask that does not start on a 16-byte boundary either
+        active = storage[shift:shift + batch * steps].view(batch, steps)
+        active.fill_(True)
+        if hole is not None:
+            active.view(-1)[int(hole * (batch * steps - 1))] = False
+        flags, last = ops.token_plan(batch, steps, DEV, active=active)
+        pos = modules._positions(x, None, None, active)
+        with ops.library_ops():
+            want = modules.token_flags(batch, steps, DEV, reset=pos == 0, active=active, segment_pos=pos, padded=~active.all())
+        assert torch.equal(flags, want)
+        assert torch.equal(last, modules._last_real_position(pos, active, None))
