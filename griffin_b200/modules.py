@@ -458,8 +458,8 @@ class RecurrentBlock(nn.Module):
                 lru.input_gate.weight, lru.input_gate.bias)
         either = (conv.weight, lru.Lambda) if conv.bias is None else (conv.weight, conv.bias, lru.Lambda)
         device = x.device
-        if not (all(t.dtype == x.dtype and t.device == device and t.is_contiguous() for t in same)
-                and all(t.dtype in (x.dtype, torch.float32) and t.device == device and t.is_contiguous() for t in either)):
+        if not (all([t.dtype == x.dtype and t.device == device for t in same])
+                and all([t.dtype in (x.dtype, torch.float32) and t.device == device for t in either])):
             return False
         return (cache.rnn_state.shape == (batch, width) and cache.conv_state.shape == (batch, 3, width)
                 and cache.segment_position.shape == (batch,) and (segment_pos is None or segment_pos.shape == (batch, 1)))
@@ -473,9 +473,9 @@ class RecurrentBlock(nn.Module):
             x_in, branch, conv.weight.squeeze(1), conv.bias, cache.conv_state.to(device=device, dtype=x.dtype),
             lru.recurrence_gate.weight, lru.recurrence_gate.bias, lru.input_gate.weight, lru.input_gate.bias, lru.Lambda,
             cache.rnn_state.to(device=device, dtype=torch.float32),
-            cache.segment_position.to(device=device, dtype=torch.long).contiguous(),
-            None if segment_pos is None else segment_pos.to(device=device, dtype=torch.long)[:, 0].contiguous(),
-            None if active_mask is None else active_mask[:, 0].contiguous(), lru.c)
+            cache.segment_position.to(device=device, dtype=torch.long),
+            None if segment_pos is None else segment_pos.to(device=device, dtype=torch.long)[:, 0],
+            None if active_mask is None else active_mask[:, 0], lru.c)
         out = _project(self.linear_out, y[:, None, :])
         if active_mask is not None:
             out = torch.where(active_mask[..., None], out, 0.0)

@@ -1338,7 +1338,6 @@ def decode_block(x_in: Tensor, branch: Optional[Tensor], conv_w: Tensor, conv_b:
     product with its GeLU.  ``x_in`` / ``branch`` [B, D]; conv weights, biases and Lambda in the activation dtype or
     (conv and Lambda) fp32; ``position`` / ``segment_pos`` [B] int64; ``active`` [B] bool.  The states are not modified."""
     _require_cuda(x_in)
-    _same_device(x_in, branch, conv_w, conv_b, conv_state, w_r, b_r, w_i, b_i, lam, h, position, segment_pos, active)
     dt = _io_dtype(x_in, "decode block")
     if x_in.dim() != 2 or w_r.dim() != 3:
         raise ValueError("x_in must be [batch, width] and the gate weights [heads, width/heads, width/heads]")
@@ -1346,26 +1345,35 @@ def decode_block(x_in: Tensor, branch: Optional[Tensor], conv_w: Tensor, conv_b:
     io, (G, bw) = x_in.dtype, w_r.shape[:2]
     if G * bw != D:
         raise ValueError(f"gate weights of {G} heads of {bw} channels do not make up a width of {D}")
-    _expect("branch", branch, (B, D), io)
-    _expect("conv_w", conv_w, (D, 4), io, torch.float32)
-    _expect("conv_b", conv_b, (D,), io, torch.float32)
-    _expect("conv_state", conv_state, (B, 3, D), io)
-    _expect("w_r", w_r, (G, bw, bw), io)
-    _expect("b_r", b_r, (G, bw), io)
-    _expect("w_i", w_i, (G, bw, bw), io)
-    _expect("b_i", b_i, (G, bw), io)
-    _expect("Lambda", lam, (D,), io, torch.float32)
-    _expect("h", h, (B, D), torch.float32)
-    _expect("position", position, (B,), torch.long)
-    _expect("segment_pos", segment_pos, (B,), torch.long)
-    _expect("active", active, (B,), torch.bool)
-    conv_b, b_r, b_i, lam, position, segment_pos, active = (
-        t if t is None else t.contiguous() for t in (conv_b, b_r, b_i, lam, position, segment_pos, active))
+    f32, bdd, per_row = torch.float32, (B, D), (B,)
+    either = (io, f32)
+    # (one expression each: this is on the path of every token)
+    d = x_in.get_device()
+    if not (d == w_r.get_device() == b_r.get_device() == w_i.get_device() == b_i.get_device() == conv_w.get_device()
+            == conv_state.get_device() == lam.get_device() == h.get_device() == position.get_device()
+            and (branch is None or branch.get_device() == d) and (conv_b is None or conv_b.get_device() == d)
+            and (segment_pos is None or segment_pos.get_device() == d) and (active is None or active.get_device() == d)):
+        raise RuntimeError("CUDA RG-LRU kernels require all tensors on one device")
+    if not (w_r.dtype == w_i.dtype == b_r.dtype == b_i.dtype == conv_state.dtype == io and h.dtype == f32
+            and conv_w.dtype in either and lam.dtype in either and position.dtype == torch.long
+            and w_r.shape == w_i.shape == (G, bw, bw) and b_r.shape == b_i.shape == (G, bw) and h.shape == bdd
+            and conv_state.shape == (B, 3, D) and conv_w.shape == (D, 4) and lam.shape == (D,) and position.shape == per_row
+            and (branch is None or (branch.dtype == io and branch.shape == bdd))
+            and (conv_b is None or (conv_b.dtype in either and conv_b.shape == (D,)))
+            and (segment_pos is None or (segment_pos.dtype == torch.long and segment_pos.shape == per_row))
+            and (active is None or (active.dtype == torch.bool and active.shape == per_row))):
+        raise ValueError(f"decode_block takes, at batch {B}, width {D}, {G} heads and activations of {io}: branch [B, D], conv_w "
+                         "[D, 4], conv_b [D], conv_state [B, 3, D], w_r and w_i [heads, D/heads, D/heads], b_r and b_i [heads, "
+                         "D/heads] and Lambda [D] of that dtype (conv_w, conv_b and Lambda: or float32), h [B, D] float32, "
+                         "position and segment_pos [B] int64, active [B] bool")
+    conv_b, segment_pos, active = (t if t is None or t.is_contiguous() else t.contiguous() for t in (conv_b, segment_pos, active))
+    b_r, b_i, lam, position = b_r.contiguous(), b_i.contiguous(), lam.contiguous(), position.contiguous()
     lib = _lib.load()
-    f32 = ((1 if conv_w.dtype == torch.float32 else 0) | (2 if conv_b is not None and conv_b.dtype == torch.float32 else 0)
-           | (4 if lam.dtype == torch.float32 else 0))
-    x_in, branch, conv_state, h = (_aligned_dense(t) for t in (x_in, branch, conv_state, h))
-    w_r, w_i, conv_w = _aligned_dense(w_r), _aligned_dense(w_i), _aligned_dense(conv_w)
+    f32_params = ((1 if conv_w.dtype == f32 else 0) | (2 if conv_b is not None and conv_b.dtype == f32 else 0)
+                  | (4 if lam.dtype == f32 else 0))
+    x_in, branch, conv_state, h, w_r, w_i, conv_w = [
+        t if t is None or (t.is_contiguous() and not t.data_ptr() & 15) else _aligned_dense(t)
+        for t in (x_in, branch, conv_state, h, w_r, w_i, conv_w)]
     y, h_new, conv_new = torch.empty_like(x_in), torch.empty_like(h), torch.empty_like(conv_state)
     pos_new = torch.empty_like(position)
     nbytes = B * D * x_in.element_size() + B
@@ -1374,6 +1382,6 @@ def decode_block(x_in: Tensor, branch: Optional[Tensor], conv_w: Tensor, conv_b:
         rc = lib.rglru_decode_block(_ptr(x_in), _ptr(branch), _ptr(conv_w), _ptr(conv_b), _ptr(conv_state), _ptr(conv_new),
                                     _ptr(w_r), _ptr(b_r), _ptr(w_i), _ptr(b_i), _ptr(lam), _ptr(h), _ptr(h_new),
                                     _ptr(position), _ptr(segment_pos), _ptr(active), _ptr(pos_new), _ptr(y), _ptr(ws),
-                                    nbytes, B, D, w_r.shape[1], float(c), dt, f32, _stream(x_in))
+                                    nbytes, B, D, bw, float(c), dt, f32_params, _stream(x_in))
     _lib.check(rc, "rglru_decode_block")
     return y, h_new, conv_new, pos_new
