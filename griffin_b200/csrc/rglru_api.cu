@@ -695,6 +695,14 @@ int rglru_gated_bwd(const void* dout, const float* dh_last, const void* x, const
                             dlambda, dh0, d_gate_bias, B, T, D, gate_width, c, io_dtype, stream, true);
 }
 
+int rglru_time_split(int op, int backward, int io_dtype, int B, int T, int D) {
+  if (io_dtype != RGLRU_F32 && io_dtype != RGLRU_BF16) return 0;
+  if (check_dims(B, T, D) != RGLRU_OK || op < RGLRU_SPLIT_SCAN || op > RGLRU_SPLIT_RAW) return 0;
+  const bool fwd = backward == 0, bf16 = io_dtype == RGLRU_BF16;
+  if (op == RGLRU_SPLIT_RAW) return raw_split(fwd, B, T, D);
+  return op == RGLRU_SPLIT_SCAN ? scan_split(fwd, bf16, B, T, D) : grouped_split(fwd, bf16, op == RGLRU_SPLIT_MERGED, B, T, D);
+}
+
 int rglru_linear_scan_fwd(const float* decay, const float* drive, const float* h0, float* out, int B, int T, int D,
                           void* stream) {
   if (!decay || !drive || !out) return RGLRU_ERR_NULL_POINTER;

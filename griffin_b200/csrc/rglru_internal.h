@@ -291,6 +291,7 @@ int grouped_box_cols();
 int scan_fwd_variant(int B, int T, int D, bool bf16);
 int scan_bwd_variant(int B, int T, int D, bool bf16);
 int scan_split(bool fwd, bool bf16, int B, int T, int D);
+int raw_split(bool fwd, int B, int T, int D);
 int grouped_split(bool fwd, bool bf16, bool merge, int B, int T, int D);
 int scan_fwd_box_rows(int variant);
 int scan_fwd_box_cols(int variant);

@@ -2215,7 +2215,11 @@ static int resident_clusters(int size) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int count = 0;
-    if (e != cudaSuccess || cudaOccupancyMaxActiveClusters(&count, kern, &cfg) != cudaSuccess) count = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&count, kern, &cfg);
+    if (e != cudaSuccess) {
+      cudaGetLastError();      // no split this time, and nothing remembered: the next call asks again
+      return 0;
+    }
     n = count + 1;
     slot.store(n, std::memory_order_relaxed);
   }
@@ -2462,17 +2466,22 @@ static cudaError_t launch_raw(const Maps& maps, const RawScanArgs& a, int split,
   if (e != cudaSuccess) return e;
   return launch_pdl(kern, dim3((a.D + CH - 1) / CH, a.B), K::THREADS, K::BYTES, s, maps, a, split);
 }
+using RawSplitFwd = RawFwdKern<RAW_STAGES, true, true>;
+using RawSplitBwd = RawBwdKern<RAW_STAGES, true, true>;
+int raw_split(bool fwd, int B, int T, int D) {
+  const long long tiles = static_cast<long long>(B) * ((D + CH - 1) / CH);
+  const int nchunks = (T + RAW_TC - 1) / RAW_TC;
+  return fwd ? pick_split<RawSplitFwd>(tiles, nchunks) : pick_split<RawSplitBwd>(tiles, nchunks);
+}
 cudaError_t launch_raw_fwd(bool use_tma, const RawFwdMaps& maps, const RawScanArgs& a, cudaStream_t s) {
   if (!use_tma) return launch_raw<RawFwdKern<1, false, false>>(maps, a, 1, s);
-  using Split = RawFwdKern<RAW_STAGES, true, true>;
-  const int split = pick_split<Split>(static_cast<long long>(a.B) * ((a.D + CH - 1) / CH), (a.T + RAW_TC - 1) / RAW_TC);
-  return split > 1 ? launch_raw<Split>(maps, a, split, s) : launch_raw<RawFwdKern<RAW_STAGES, true, false>>(maps, a, 1, s);
+  const int split = raw_split(true, a.B, a.T, a.D);
+  return split > 1 ? launch_raw<RawSplitFwd>(maps, a, split, s) : launch_raw<RawFwdKern<RAW_STAGES, true, false>>(maps, a, 1, s);
 }
 cudaError_t launch_raw_bwd(bool use_tma, const RawBwdMaps& maps, const RawScanArgs& a, cudaStream_t s) {
   if (!use_tma) return launch_raw<RawBwdKern<1, false, false>>(maps, a, 1, s);
-  using Split = RawBwdKern<RAW_STAGES, true, true>;
-  const int split = pick_split<Split>(static_cast<long long>(a.B) * ((a.D + CH - 1) / CH), (a.T + RAW_TC - 1) / RAW_TC);
-  return split > 1 ? launch_raw<Split>(maps, a, split, s) : launch_raw<RawBwdKern<RAW_STAGES, true, false>>(maps, a, 1, s);
+  const int split = raw_split(false, a.B, a.T, a.D);
+  return split > 1 ? launch_raw<RawSplitBwd>(maps, a, split, s) : launch_raw<RawBwdKern<RAW_STAGES, true, false>>(maps, a, 1, s);
 }
 
 int conv_tma_box_rows() { return 64 + 3; }

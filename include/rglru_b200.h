@@ -233,6 +233,15 @@ int rglru_layer_bwd(const void* dout, const float* dh_last, const void* x, const
                     int D, int head_width, int gate_width, float c, int weight_dtype, int bias_dtype, int lambda_dtype,
                     int io_dtype, void* stream);
 
+/* How many thread blocks share one (batch row, channel tile) along time in a call of this shape on 16-byte aligned tensors
+ * of whole 16-byte rows: 1 for none, 0 for bad arguments.  op: RGLRU_SPLIT_SCAN for rglru_fwd / rglru_bwd, _GATED for
+ * rglru_grouped_* and rglru_gated_* without a branch, _MERGED for those with one, _RAW for rglru_linear_scan_*. */
+#define RGLRU_SPLIT_SCAN 0
+#define RGLRU_SPLIT_GATED 1
+#define RGLRU_SPLIT_MERGED 2
+#define RGLRU_SPLIT_RAW 3
+int rglru_time_split(int op, int backward, int io_dtype, int B, int T, int D);
+
 /* Raw affine scan h_t = a_t h_{t-1} + b_t on fp32 tensors: the operator
  * fused_rglru_scan(decay, current_input, initial_state) of griffin/triton_scan.py:274-276
  * (forward kernel :31-60).  decay, drive, out: [B,T,D] fp32; h0: [B,D] fp32 or NULL. */

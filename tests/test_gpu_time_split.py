@@ -171,3 +171,84 @@ def test_raw_scan_of_an_infinite_state():
     assert torch.isnan(h[0, 5:, 7]).all() and torch.isfinite(h[0, :5, 7]).all()
     rest = [c for c in range(D) if c not in (3, 7)]
     assert torch.isfinite(h[0, :, rest]).all()
+
+
+SCAN, GATED, MERGED, RAW = range(4)
+
+
+def _split(op, backward, dtype, batch, steps, width):
+    from griffin_b200 import _lib, ops
+    return _lib.load().rglru_time_split(op, int(backward), ops._DTYPES[dtype], batch, steps, width)
+
+
+def test_the_shapes_above_do_split():
+    for backward in (False, True):
+        for dtype in (torch.float32, torch.bfloat16):
+            assert _split(SCAN, backward, dtype, 2, 64, 200) == 1                        # a single chunk
+            assert all(_split(SCAN, backward, dtype, 2, t, 200) >= 2 for t in (512, 513, 64 * 17 - 1, 64 * 21))
+            assert _split(SCAN, True, dtype, 2, 65, 200) == 2
+            for op in (GATED, MERGED):
+                assert _split(op, backward, dtype, 1, 65, 128) == 2 and _split(op, backward, dtype, 1, 64 * 9 + 3, 128) >= 3
+        assert all(_split(RAW, backward, torch.float32, 2, t, w) >= 2 for t in LENGTHS[1:] for w in (32, 72, 100))
+        assert _split(RAW, backward, torch.float32, 148, 4096, 1024) == 1                # a grid that fills the machine
+    assert _split(SCAN, False, torch.float32, 0, 64, 64) == 0 and _split(4, False, torch.float32, 1, 64, 64) == 0
+
+
+def _check_against_64_bits(op, dtype, batch, steps, width, monkeypatch):
+    from griffin_b200 import _lib, ops
+    # (the oracle's helper tensors are born on the CPU)
+    backward = orc.rglru_backward_linear
+
+    def on_device(*args, **kwargs):
+        with torch.device(DEV):
+            return backward(*args, **kwargs)
+    monkeypatch.setattr(orc, "rglru_backward_linear", on_device)
+    gen = torch.Generator(device=DEV).manual_seed(steps)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV)
+    h0 = rnd(batch, width)
+    if op == RAW:
+        given = [torch.rand(batch, steps, width, generator=gen, device=DEV) * 0.3 + 0.7, rnd(batch, steps, width), h0]
+    elif op == SCAN:
+        given = [rnd(batch, steps, width).to(dtype) for _ in range(3)] + [orc.init_lambda(width, 8.0, torch.Generator()).to(DEV), h0]
+    else:
+        weight = lambda: (rnd(1, width, width) / width ** 0.5).to(dtype).float()
+        given = [rnd(batch, steps, width).to(dtype), weight(), rnd(1, width) * 0.3, weight(), rnd(1, width) * 0.3,
+                 orc.init_lambda(width, 8.0, torch.Generator()).to(DEV), h0]
+        if op == MERGED:
+            given.append(rnd(batch, steps, width).to(dtype))
+    leaves = [t.clone().requires_grad_(True) for t in given]
+    ref = [t.double().requires_grad_(True) for t in given]
+    with torch.device(DEV):
+        if op == RAW:
+            got, want = [ops.linear_scan(*leaves)], [orc.linear_scan(*ref)]
+        elif op == SCAN:
+            got, want = ops.rglru(*leaves), orc._CoreLinearBackward.apply(*ref, None, None, 8.0)
+        else:
+            got = ops.rglru_grouped(*leaves[:7], branch=leaves[7] if op == MERGED else None)
+            names = ("recurrence_gate.weight", "recurrence_gate.bias", "input_gate.weight", "input_gate.bias", "Lambda")
+            want = list(orc.rglru_layer_linear_backward(ref[0], dict(zip(names, ref[1:6])), ref[6]))
+            if op == MERGED:
+                want[0] = want[0] * torch.nn.functional.gelu(ref[7], approximate="tanh")
+    up = [rnd(*t.shape).to(t.dtype) for t in got]
+    torch.autograd.backward(list(got), up)
+    torch.autograd.backward(list(want), [u.double() for u in up])
+    bound = 1e-5 if dtype == torch.float32 else 2e-2          # as in the tests above
+    for k, (a, b) in enumerate(zip([*got, *(t.grad for t in leaves)], [*want, *(t.grad for t in ref)])):
+        assert orc.rel_l2(a, b) <= bound, k
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("size", [3, 4, 5, 6, 7])
+@pytest.mark.parametrize("backward", [False, True])
+@pytest.mark.parametrize("op,dtype", [(SCAN, torch.float32), (SCAN, torch.bfloat16), (GATED, torch.bfloat16),
+                                      (MERGED, torch.float32), (RAW, torch.float32)])
+def test_clusters_of_every_size(op, dtype, backward, size, monkeypatch):
+    """The sizes between pairs and eights, which the number of tiles picks, with one block busy in the last round and with
+    one block idle in it."""
+    width = 32 if op == RAW else 64
+    for last in (1, size - 1):
+        steps = 64 * (2 * size + last) - 3
+        batch = next((b for b in range(1, 149) if _split(op, backward, dtype, b, steps, width) == size), None)
+        if batch is None:
+            pytest.skip(f"no number of tiles has clusters of {size} here")
+        _check_against_64_bits(op, dtype, batch, steps, width, monkeypatch)
