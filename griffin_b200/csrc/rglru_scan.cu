@@ -2432,8 +2432,15 @@ int scan_split(bool fwd, bool bf16, int B, int T, int D) {
   const int split = split_of<false, false>(fwd, bf16, B, T, D);
   return fwd && split < 3 ? 1 : split;      // see scan_fwd_variant
 }
+// In the layer the gate tensor has just been written and much of it is still in L2.  There the bf16 forward without the branch
+// product is faster unsplit than in pairs (D = 1024, forward of the layer unsplit / pairs: 96 tiles T = 2048 53 / 57 us,
+// T = 1200 34 / 38, 128 tiles T = 2048 57 / 60, T = 512 23 / 25, T = 16384 406 / 414, 16 tiles T = 128 10 / 12; three and more
+// win: 80 tiles 51 / 45, 64 tiles 48 / 36).
+// With the product (96 tiles 151 / 146, 128 tiles 182 / 174 in the block), and for fp32 (60 tiles 88 / 84), pairs win too.
 int grouped_split(bool fwd, bool bf16, bool merge, int B, int T, int D) {
-  return merge ? split_of<true, true>(fwd, bf16, B, T, D) : split_of<false, true>(fwd, bf16, B, T, D);
+  if (merge) return split_of<true, true>(fwd, bf16, B, T, D);
+  const int split = split_of<false, true>(fwd, bf16, B, T, D);
+  return fwd && bf16 && split < 3 ? 1 : split;
 }
 
 int raw_box_rows() { return RAW_TC; }
