@@ -18,6 +18,7 @@ from __future__ import annotations
 import contextlib
 import functools
 import os
+import threading
 from typing import Optional
 
 import torch
@@ -833,13 +834,50 @@ _grouped_fwd.register_autograd(_grouped_backward, setup_context=_grouped_setup)
 _GroupedNode = _eager_node("GroupedRGLRU", _grouped_fwd_impl, _grouped_setup, _grouped_backward, _grouped_bwd_parts)
 
 
-def _layer_in_library(x: Tensor, head_width: int) -> bool:
+def _layer_in_library(x: Tensor, head_width: int, differentiated: bool) -> bool:
     """Whether the layer's projections too are the library's kernels, each direction being one library call, or batched GEMMs
-    between its calls.  One call a direction saves some 105 us of host time in a training step; the batched GEMMs are
-    faster from a few hundred CTAs' worth of work on, by a time that grows with elements x head width.  The line is where
-    that reaches about half of what the host saves (see rglru_gates.cu for both sides' times)."""
-    work = x.numel() * head_width
-    return x.numel() <= 1 << 24 and work <= (1 << 30 if x.dtype == torch.bfloat16 else 1 << 29)
+    between its calls.
+
+    Called eagerly, one call a direction saves some 100 us of host time in a training step and 25 without gradients, and the
+    host is what such calls wait for; from some size on the GEMMs are faster by more.  Wall time of a training step, own
+    kernels / GEMMs, us: bf16 16384 tokens, 16 heads of 64 (2^24 elements, 2^30 elements x head width) 222 / 319; 512 tokens,
+    16 of 352 (2^29.9) 214 / 313; 65536 tokens, 32 of 8 (2^24, 2^27) 463 / 459; 131072 tokens, 16 of 16 (2^25) 532 / 556;
+    fp32 4096 tokens, 32 of 64 (2^23, 2^29) 298 / 300; 4096, 16 of 128 (2^23, 2^30) 459 / 440.  Without gradients: bf16 16384
+    tokens, 16 of 64 67 / 61; 4096, 16 of 128 (2^23, 2^30) 62 / 61; 4096, 32 of 64 (2^23, 2^29) 50 / 62; fp32 65536 tokens, 16 of
+    16 (2^24, 2^28) 114 / 152; 1024, 32 of 128 (2^22, 2^29) 89 / 85.
+
+    A captured call pays no host time when it is replayed, so there the faster on the device is taken (replay of the same
+    steps: bf16 202 / 158, 139 / 76; fp32 heads of 32 212 / 222, of 64 286 / 282, of 256 430 / 341).  bf16 heads of up to 32
+    channels over very many tokens keep the own kernels, whose weight gradient is split over the tokens (65536 tokens, 4 of 16
+    122 / 188; 16384, 16 of 8 85 / 106)."""
+    elements, width = x.numel(), x.shape[2]
+    work, half = elements * head_width, x.dtype == torch.bfloat16
+    if width // head_width > 65535:            # (heads are an axis of the kernels' grids)
+        return False
+    inside = elements <= (1 << 23 if half and not differentiated else 1 << 24) and work <= (1 << 30 if half else 1 << 29)
+    if not inside or not torch.cuda.is_current_stream_capturing():
+        return inside
+    return _own_projections_faster(elements // width, width, head_width, half, differentiated)
+
+
+def _own_projections_faster(rows: int, width: int, head_width: int, half: bool, differentiated: bool) -> bool:
+    """Which of the two takes less device time, for layers below the line of :func:`_layer_in_library`."""
+    if half:
+        return differentiated and head_width <= 32 and rows >= 128 * width
+    return head_width < 64
+
+
+_BLAS = threading.local()
+
+
+def _keep_gemms_capturable(device: torch.device, own_when_captured: bool) -> None:
+    """A stream capture cannot create a thread's cuBLAS handle.  A layer whose captured calls take GEMMs where its eager calls
+    do not makes sure of the handle while it is warmed up, on each thread (and device) that it runs on."""
+    if not own_when_captured and not torch.cuda.is_current_stream_capturing():
+        ready = _BLAS.__dict__.setdefault("devices", set())
+        if device.index not in ready:
+            torch.cuda.current_blas_handle()
+            ready.add(device.index)
 
 
 def _layer_fwd(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor, h0: Optional[Tensor],
@@ -856,6 +894,7 @@ def _layer_fwd(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, la
     nbytes = lib.rglru_layer_workspace_bytes(B, T, D, bw, dt, int(save))
     ws = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
     with _on(x, "rglru_layer_fwd"):
+        _keep_gemms_capturable(x.device, _own_projections_faster(B * T, D, bw, dt == _lib.BF16, save))
         rc = lib.rglru_layer_fwd(_ptr(x), _ptr(w_r), _ptr(b_r), _ptr(w_i), _ptr(b_i), _ptr(lam), _ptr(branch), _ptr(h0),
                                  _ptr(tok), _ptr(out), _ptr(h_last), _ptr(u), _ptr(ws), nbytes, int(save), B, T, D, bw,
                                  _gate_group(bw, x.element_size()), c, _DTYPES[w_r.dtype], _DTYPES[b_r.dtype],
@@ -896,6 +935,7 @@ class _LayerNode(torch.autograd.Function):
         nbytes = lib.rglru_layer_scratch_bytes(B, T, D, bw, dt)
         scratch = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
         with _on(x, "rglru_layer_bwd"):
+            _keep_gemms_capturable(x.device, _own_projections_faster(B * T, D, bw, dt == _lib.BF16, True))
             rc = lib.rglru_layer_bwd(_ptr(dout), _ptr(dh_last), _ptr(x), _ptr(u), _ptr(branch), _ptr(h0), _ptr(tok), _ptr(ws),
                                      ws.numel(), _ptr(dx), _ptr(du), _ptr(dbranch), _ptr(dw_r), _ptr(db_r), _ptr(dw_i),
                                      _ptr(db_i), _ptr(dlam), _ptr(dh0), _ptr(scratch), nbytes, B, T, D, bw,
@@ -931,7 +971,7 @@ def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, l
     traced = _library_ops_active()
     if traced or lam.dtype not in _DTYPES:
         lam = lam.to(torch.float32)
-    if not traced and _layer_in_library(x, bw):
+    if not traced and _layer_in_library(x, bw, save):
         args = (x.contiguous(), w_r, b_r, w_i, b_i, lam, None if h0 is None else h0.to(torch.float32).contiguous(),
                 None if tok is None else tok.contiguous(), float(c), None if branch is None else branch.to(x.dtype).contiguous())
         if save or torch.autograd.forward_ad._current_level >= 0:

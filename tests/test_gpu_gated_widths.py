@@ -146,3 +146,85 @@ def test_hooks_for_all_modules_see_the_gates():
     finally:
         handle.remove()
     assert seen.count(BlockDiagonalLinear) == 2
+
+
+def _step(layer, x, dy):
+    layer.zero_grad(set_to_none=True)
+    x.grad = None
+    y, h = layer(x, return_state=True)
+    y.backward(dy)
+    return [y.detach(), h.detach(), x.grad] + [p.grad for p in layer.parameters()]
+
+
+# (tokens, heads, head width, whether a captured call keeps the library's own projections)
+CAPTURED = [(torch.bfloat16, 512, 4, 64, False), (torch.bfloat16, 16384, 4, 16, True), (torch.float32, 512, 4, 32, True),
+            (torch.float32, 512, 4, 64, False)]
+
+
+@pytest.mark.parametrize("dtype,tokens,heads,bw,own", CAPTURED)
+def test_captured_training_step(dtype, tokens, heads, bw, own, monkeypatch):
+    """A captured step takes the projections that are faster on the device; its replay gives what the eager step gives."""
+    from griffin_b200 import RG_LRU, ops
+    torch.manual_seed(0)
+    layer = RG_LRU(heads * bw, gate_blocks=heads).to(DEV).to(dtype)
+    x = torch.randn(2, tokens // 2, heads * bw, device=DEV, dtype=dtype, requires_grad=True)
+    dy = torch.randn_like(x)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for _ in range(3):
+            want = [t.clone() for t in _step(layer, x, dy)]
+    torch.cuda.current_stream().wait_stream(side)
+    taken = []
+    one_call = ops._LayerNode.apply
+    monkeypatch.setattr(ops._LayerNode, "apply", staticmethod(lambda *a: taken.append(1) or one_call(*a)))
+    layer.zero_grad(set_to_none=True)
+    x.grad = None
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = _step(layer, x, dy)
+    assert bool(taken) == own
+    for _ in range(2):
+        for t in got:
+            t.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        for a, b in zip(got, want):
+            assert _rel(a, b) <= (1e-5 if dtype == torch.float32 else 2e-2)
+    assert ops._lib.device_status() == 0
+
+
+def test_a_process_that_only_ran_the_layer_can_capture_it():
+    """The eager layer uses no cuBLAS, its capture does: the warm-up leaves the threads of both directions with a handle."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import sys, torch
+sys.path[:0] = sys.argv[1:]
+from griffin_b200 import RG_LRU
+from test_gpu_gated_widths import _step
+layer = RG_LRU(256, gate_blocks=4).cuda().bfloat16()
+x = torch.randn(2, 256, 256, device='cuda', dtype=torch.bfloat16, requires_grad=True)
+dy = torch.randn_like(x)
+side = torch.cuda.Stream()
+side.wait_stream(torch.cuda.current_stream())
+with torch.cuda.stream(side):
+    for _ in range(3):
+        _step(layer, x, dy)
+    with torch.no_grad():
+        layer(x)
+torch.cuda.current_stream().wait_stream(side)
+layer.zero_grad(set_to_none=True); x.grad = None
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    _step(layer, x, dy)
+    with torch.no_grad():
+        layer(x)
+graph.replay(); torch.cuda.synchronize()
+del graph
+print("captured")
+"""
+    here = os.path.dirname(os.path.abspath(__file__))
+    done = subprocess.run([sys.executable, "-c", code, os.path.dirname(here), here], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0 and "captured" in done.stdout, done.stderr[-2000:]
