@@ -728,13 +728,20 @@ def _heads_first(t: Tensor, rows: int, G: int) -> Tensor:
     return t.as_strided((G, rows, C // G), (C // G, C, 1))
 
 
+def _tf32_allowed() -> bool:
+    """Whether the caller lets fp32 matrix products run in TF32."""
+    return torch.backends.cuda.matmul.fp32_precision == "tf32"
+
+
 def _gate_weight_grad(du: Tensor, x: Tensor, G: int, bw: int) -> Tensor:
     """d stacked weights [splits, G, 2 bw, bw] from the gate tensor's gradient: one batched GEMM; for fp32 with fewer 64 x 64
     output tiles than SMs, where that GEMM walks all tokens with the few CTAs so small an output gives (8 heads of 128,
     16384 tokens: 384 against 254 us; 16 of 176, 8192 tokens, the other way round: 321 against 529), ``rglru_gate_dw``,
-    whose partial sums over stretches of the tokens are left for the caller to add."""
-    rows, D = du.shape[0] * du.shape[1], G * bw
-    if du.dtype != torch.float32 or G * -(-2 * bw // 64) * -(-bw // 64) >= 148:
+    whose partial sums over stretches of the tokens are left for the caller to add.  Where the caller allows TF32 the GEMM
+    takes it, which ``rglru_gate_dw`` does not, and is faster from eight tiles on (a training step's replay with either,
+    16384 tokens: 16 heads of 64 283 against 362 us, 4 of 128 170 against 257; 65536 tokens, 4 of 32: 298 against 217)."""
+    rows, D, tiles = du.shape[0] * du.shape[1], G * bw, G * -(-2 * bw // 64) * -(-bw // 64)
+    if du.dtype != torch.float32 or tiles >= (8 if _tf32_allowed() else 148):
         return torch.bmm(_heads_first(du, rows, G).transpose(1, 2), _heads_first(x, rows, G))[None]
     lib = _lib.load()
     splits = lib.rglru_gate_dw_splits(rows, D, bw, _lib.F32)
@@ -849,12 +856,18 @@ def _layer_in_library(x: Tensor, head_width: int, differentiated: bool) -> bool:
     A captured call pays no host time when it is replayed, so there the faster on the device is taken (replay of the same
     steps: bf16 202 / 158, 139 / 76; fp32 heads of 32 212 / 222, of 64 286 / 282, of 256 430 / 341).  bf16 heads of up to 32
     channels over very many tokens keep the own kernels, whose weight gradient is split over the tokens (65536 tokens, 4 of 16
-    122 / 188; 16384, 16 of 8 85 / 106)."""
+    122 / 188; 16384, 16 of 8 85 / 106).
+
+    The own fp32 kernels are full fp32 whatever the caller allows.  With TF32 allowed the GEMMs are faster by more: replays
+    16384 tokens, 16 of 64 537 / 283, 4096 tokens, 16 of 24 73 / 68, of 16 60 / 60, 65536 tokens, 16 of 16 450 / 514; eagerly
+    4096, 32 of 48 (2^28.2) 240 / 317, 16384, 16 of 48 (2^29.2) 430 / 315, without gradients 4096, 16 of 48 (2^27.2) 69 / 67,
+    1024, 32 of 128 (2^29) 90 / 68."""
     elements, width = x.numel(), x.shape[2]
     work, half = elements * head_width, x.dtype == torch.bfloat16
     if width // head_width > 65535:            # (heads are an axis of the kernels' grids)
         return False
-    inside = elements <= (1 << 23 if half and not differentiated else 1 << 24) and work <= (1 << 30 if half else 1 << 29)
+    most = 1 << 30 if half else (1 << 29 if differentiated or not _tf32_allowed() else 1 << 27)
+    inside = elements <= (1 << 23 if half and not differentiated else 1 << 24) and work <= most
     if not inside or not torch.cuda.is_current_stream_capturing():
         return inside
     return _own_projections_faster(elements // width, width, head_width, half, differentiated)
@@ -862,8 +875,8 @@ def _layer_in_library(x: Tensor, head_width: int, differentiated: bool) -> bool:
 
 def _own_projections_faster(rows: int, width: int, head_width: int, half: bool, differentiated: bool) -> bool:
     """Which of the two takes less device time, for layers below the line of :func:`_layer_in_library`."""
-    if half:
-        return differentiated and head_width <= 32 and rows >= 128 * width
+    if half or _tf32_allowed():
+        return differentiated and head_width <= (32 if half else 16) and rows >= 128 * width
     return head_width < 64
 
 

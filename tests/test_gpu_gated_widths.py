@@ -228,3 +228,22 @@ print("captured")
     here = os.path.dirname(os.path.abspath(__file__))
     done = subprocess.run([sys.executable, "-c", code, os.path.dirname(here), here], capture_output=True, text=True, timeout=300)
     assert done.returncode == 0 and "captured" in done.stdout, done.stderr[-2000:]
+
+
+@pytest.mark.parametrize("heads,bw,gemm", [(16, 64, True), (1, 64, False)])
+def test_weight_gradient_takes_tf32_where_it_is_allowed(heads, bw, gemm):
+    from griffin_b200 import ops
+    torch.manual_seed(0)
+    du, x = torch.randn(2, 512, 2 * heads * bw, device=DEV), torch.randn(2, 512, heads * bw, device=DEV)
+    want = torch.einsum("ngo,ngi->goi", du.double().view(1024, heads, -1), x.double().view(1024, heads, -1))
+    full = ops._gate_weight_grad(du, x, heads, bw)
+    before = torch.get_float32_matmul_precision()
+    try:
+        torch.set_float32_matmul_precision("high")
+        got = ops._gate_weight_grad(du, x, heads, bw)
+    finally:
+        torch.set_float32_matmul_precision(before)
+    assert _rel(full.double().sum(0), want) <= 1e-6
+    # TF32 keeps eleven bits of the factors: 2^-11 each
+    assert _rel(got.double().sum(0), want) <= (2.0 ** -10 if gemm else 1e-6)
+    assert full.shape[0] > 1 and (got.shape[0] == 1) == gemm
