@@ -1260,8 +1260,9 @@ __global__ void __launch_bounds__(LANES*(CH / CV) + ((USE_TMA && !SELF_ISSUE) ? 
   bar_compute(NCOMP);
   if (!s_last) { drain(); return; }
   // Rows are added in index order whatever the load order; loads go out eight rows at a time so that the
-  // fold costs a few round trips to L2, not one per row.
-  if ((p.D & 3) == 0) {
+  // fold costs a few round trips to L2, not one per row.  (Lambda and the caller's buffers need not lie on 16-byte boundaries.)
+  const uintptr_t ends = reinterpret_cast<uintptr_t>(p.lambda) | reinterpret_cast<uintptr_t>(p.dlambda) | reinterpret_cast<uintptr_t>(p.dlam_part);
+  if ((p.D & 3) == 0 && (ends & 15u) == 0) {
     for (int d = tid * 4; d < p.D; d += NCOMP * 4) {
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
       for (int r0 = 0; r0 < p.B; r0 += 8) {
