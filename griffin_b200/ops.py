@@ -760,7 +760,7 @@ def _grouped_bwd_parts(dout: Tensor, dh_last: Optional[Tensor], x: Tensor, u: Te
     weights and biases the forward built.  The caller takes the two stacked gradients apart into the gates' own."""
     lib = _lib.load()
     with _no_autocast():
-        x = _aligned16(x)
+        x, u, bias, ws = (_aligned16(t) for t in (x, u, bias, ws))      # (saved-tensor hooks may have moved them)
         B, T, D = x.shape
         G, bw2, bw = wcat.shape
         dt = _io_dtype(x, "grouped backward")
@@ -866,8 +866,10 @@ def _layer_in_library(x: Tensor, head_width: int, differentiated: bool) -> bool:
     work, half = elements * head_width, x.dtype == torch.bfloat16
     if width // head_width > 65535:            # (heads are an axis of the kernels' grids)
         return False
-    most = 1 << 30 if half else (1 << 29 if differentiated or not _tf32_allowed() else 1 << 27)
-    inside = elements <= (1 << 23 if half and not differentiated else 1 << 24) and work <= most
+    if half:
+        inside = work <= 1 << 30 and elements <= (1 << 24 if differentiated else 1 << 23)
+    else:
+        inside = work <= 1 << 29 and elements <= 1 << 24 and (differentiated or work <= 1 << 27 or not _tf32_allowed())
     if not inside or not torch.cuda.is_current_stream_capturing():
         return inside
     return _own_projections_faster(elements // width, width, head_width, half, differentiated)
@@ -883,14 +885,16 @@ def _own_projections_faster(rows: int, width: int, head_width: int, half: bool, 
 _BLAS = threading.local()
 
 
-def _keep_gemms_capturable(device: torch.device, own_when_captured: bool) -> None:
-    """A stream capture cannot create a thread's cuBLAS handle.  A layer whose captured calls take GEMMs where its eager calls
-    do not makes sure of the handle while it is warmed up, on each thread (and device) that it runs on."""
-    if not own_when_captured and not torch.cuda.is_current_stream_capturing():
-        ready = _BLAS.__dict__.setdefault("devices", set())
-        if device.index not in ready:
-            torch.cuda.current_blas_handle()
-            ready.add(device.index)
+def _keep_gemms_capturable(device: torch.device) -> None:
+    """A stream capture cannot create a thread's cuBLAS handle, and the layer's captured calls may take GEMMs where its eager
+    calls do not: warmed up eagerly, it makes sure of the handle on each thread (and device) that it runs on."""
+    try:
+        ready = _BLAS.devices
+    except AttributeError:
+        ready = _BLAS.devices = set()
+    if device.index not in ready and not torch.cuda.is_current_stream_capturing():
+        torch.cuda.current_blas_handle()
+        ready.add(device.index)
 
 
 def _layer_fwd(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor, h0: Optional[Tensor],
@@ -907,7 +911,7 @@ def _layer_fwd(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, la
     nbytes = lib.rglru_layer_workspace_bytes(B, T, D, bw, dt, int(save))
     ws = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
     with _on(x, "rglru_layer_fwd"):
-        _keep_gemms_capturable(x.device, _own_projections_faster(B * T, D, bw, dt == _lib.BF16, save))
+        _keep_gemms_capturable(x.device)
         rc = lib.rglru_layer_fwd(_ptr(x), _ptr(w_r), _ptr(b_r), _ptr(w_i), _ptr(b_i), _ptr(lam), _ptr(branch), _ptr(h0),
                                  _ptr(tok), _ptr(out), _ptr(h_last), _ptr(u), _ptr(ws), nbytes, int(save), B, T, D, bw,
                                  _gate_group(bw, x.element_size()), c, _DTYPES[w_r.dtype], _DTYPES[b_r.dtype],
@@ -934,7 +938,7 @@ class _LayerNode(torch.autograd.Function):
     @torch.autograd.function.once_differentiable
     def backward(ctx, dout, dh_last):
         x, u, ws, branch, h0, tok = ctx.saved_tensors
-        x, branch = _aligned16(x), _aligned16(branch)
+        x, u, ws, branch = (_aligned16(t) for t in (x, u, ws, branch))      # (saved-tensor hooks may have moved them)
         lib = _lib.load()
         dt = _DTYPES[x.dtype]
         B, T, D = x.shape
@@ -948,7 +952,7 @@ class _LayerNode(torch.autograd.Function):
         nbytes = lib.rglru_layer_scratch_bytes(B, T, D, bw, dt)
         scratch = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
         with _on(x, "rglru_layer_bwd"):
-            _keep_gemms_capturable(x.device, _own_projections_faster(B * T, D, bw, dt == _lib.BF16, True))
+            _keep_gemms_capturable(x.device)
             rc = lib.rglru_layer_bwd(_ptr(dout), _ptr(dh_last), _ptr(x), _ptr(u), _ptr(branch), _ptr(h0), _ptr(tok), _ptr(ws),
                                      ws.numel(), _ptr(dx), _ptr(du), _ptr(dbranch), _ptr(dw_r), _ptr(db_r), _ptr(dw_i),
                                      _ptr(db_i), _ptr(dlam), _ptr(dh0), _ptr(scratch), nbytes, B, T, D, bw,
@@ -975,10 +979,15 @@ def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, l
         raise ValueError("branch must have the shape of x")
     if not gated_supported(x, bw):
         raise ValueError("the gate layout needs CUDA tensors and gate heads of whole 16-byte groups of channels")
-    _same_device(x, w_r, b_r, w_i, b_i, lam, h0, tok, branch)
-    if h0 is not None and h0.shape != (x.shape[0], x.shape[2]):
-        raise ValueError(f"h0 must be [batch, width], got {list(h0.shape)}")
-    _expect("tok", tok, (x.shape[0], x.shape[1]), torch.uint8)
+    device = x.device
+    if not (w_r.device == device and b_r.device == device and w_i.device == device and b_i.device == device
+            and lam.device == device):
+        _same_device(x, w_r, b_r, w_i, b_i, lam)
+    if h0 is not None or tok is not None or branch is not None:
+        _same_device(x, h0, tok, branch)
+        if h0 is not None and h0.shape != (x.shape[0], x.shape[2]):
+            raise ValueError(f"h0 must be [batch, width], got {list(h0.shape)}")
+        _expect("tok", tok, x.shape[:2], torch.uint8)
     save = torch.is_grad_enabled() and any(
         t is not None and t.requires_grad for t in (x, w_r, b_r, w_i, b_i, lam, h0, branch))
     traced = _library_ops_active()

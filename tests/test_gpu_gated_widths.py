@@ -247,3 +247,27 @@ def test_weight_gradient_takes_tf32_where_it_is_allowed(heads, bw, gemm):
     # TF32 keeps eleven bits of the factors: 2^-11 each
     assert _rel(got.double().sum(0), want) <= (2.0 ** -10 if gemm else 1e-6)
     assert full.shape[0] > 1 and (got.shape[0] == 1) == gemm
+
+
+@pytest.mark.parametrize("own_projections", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_saved_tensors_that_come_back_off_their_boundary(dtype, own_projections, monkeypatch):
+    """Saved-tensor hooks may bring what a backward needs back anywhere: here four bytes past a 16-byte boundary."""
+    from griffin_b200 import RG_LRU, ops
+    monkeypatch.setattr(ops, "_layer_in_library", lambda *a: own_projections)
+    torch.manual_seed(0)
+    layer = RG_LRU(128, gate_blocks=2).to(DEV).to(dtype)
+    x = torch.randn(2, 70, 128, device=DEV, dtype=dtype, requires_grad=True)
+    dy = torch.randn_like(x)
+    want = [t.clone() for t in _step(layer, x, dy)]
+
+    def back(t):
+        shift = 4 // t.element_size() if t.element_size() <= 4 else 0
+        buffer = torch.empty(t.numel() + shift, device=t.device, dtype=t.dtype)
+        return buffer[shift:].view(t.shape).copy_(t)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach().clone(), back):
+        got = _step(layer, x, dy)
+    # the own kernels give the same bits; a GEMM may choose by alignment: sums in another order, rounded once to the type
+    bound = 0.0 if own_projections else (1e-6 if dtype == torch.float32 else 2.0 ** -8)
+    for a, b in zip(got, want):
+        assert _rel(a, b) <= bound
