@@ -55,12 +55,17 @@ def _largest_block_count(width: int, requested: int) -> int:
     return count
 
 
+# (the registries themselves: a hook that is registered later is in them)
+_GLOBAL_HOOKS = (torch.nn.modules.module._global_forward_hooks, torch.nn.modules.module._global_forward_pre_hooks,
+                 torch.nn.modules.module._global_backward_hooks, torch.nn.modules.module._global_backward_pre_hooks)
+
+
 def _is_stock(layer: nn.Module, kind: type) -> bool:
     """Whether a submodule is the one this package put there: not replaced, not parametrised, without hooks of its own or
     for all modules (``torch.nn.modules.module.register_module_forward_hook`` and its like)."""
     return type(layer) is kind and "forward" not in layer.__dict__ and not (
         layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks
-        or torch.nn.modules.module._has_any_global_hook())
+        or _GLOBAL_HOOKS[0] or _GLOBAL_HOOKS[1] or _GLOBAL_HOOKS[2] or _GLOBAL_HOOKS[3])
 
 
 class BlockDiagonalLinear(nn.Module):
@@ -180,11 +185,10 @@ class RG_LRU(nn.Module):
             target = torch.empty_like(self.Lambda).uniform_(0.9, 0.999)
             self.Lambda.copy_(torch.logit(target.pow(1.0 / self.c)))
 
-    def _gates_in_node(self, xt: Tensor) -> bool:
+    def _gates_in_node(self, xt: Tensor, r: nn.Module, i: nn.Module) -> bool:
         """Whether both gate projections run inside the scan's autograd node (``ops.rglru_gated``).  Heads of a multiple of 64
         channels always do; of other widths, wherever the projections called as modules would compute the same thing:
         this package's own layers, in the dtype of ``xt`` or cast to it by autocast."""
-        r, i = self.recurrence_gate, self.input_gate
         if not self.group_gates:
             return False
         if ops.grouped_gates_supported(xt, r.block_width):
@@ -192,6 +196,8 @@ class RG_LRU(nn.Module):
         if not (ops.gated_supported(xt, r.block_width) and _is_stock(r, BlockDiagonalLinear) and _is_stock(i, BlockDiagonalLinear)):
             return False
         params = (r.weight, r.bias, i.weight, i.bias)
+        if i.weight.shape != r.weight.shape:       # (a gate of this package's with other heads in the place of one of them)
+            return False
         if torch.is_autocast_enabled("cuda"):
             alike = xt.dtype == torch.get_autocast_dtype("cuda") and all(t.dtype in (torch.float32, xt.dtype) for t in params)
         else:
@@ -224,13 +230,12 @@ class RG_LRU(nn.Module):
             raise TypeError(f"scan_mode='cuda' supports float32 and bfloat16 activations, got {xt.dtype}")
 
         flags = _flags if _flags is not None else token_flags(batch, steps, xt.device, reset=reset_mask, active=active_mask)
-        if self._gates_in_node(xt):
-            yt, h_last = ops.rglru_gated(xt, self.recurrence_gate.weight, self.recurrence_gate.bias,
-                                         self.input_gate.weight, self.input_gate.bias, self.Lambda, ht_minus_1, flags,
-                                         self.c, _branch)
+        r, i = self.recurrence_gate, self.input_gate
+        if self._gates_in_node(xt, r, i):
+            yt, h_last = ops.rglru_gated(xt, r.weight, r.bias, i.weight, i.bias, self.Lambda, ht_minus_1, flags, self.c, _branch)
             return (yt, h_last) if return_state else yt
-        u_r = self.recurrence_gate(xt).to(xt.dtype)
-        u_i = self.input_gate(xt).to(xt.dtype)
+        u_r = r(xt).to(xt.dtype)
+        u_i = i(xt).to(xt.dtype)
         if _branch is not None:   # the caller's GeLU branch, multiplied in by the kernels
             yt, h_last = ops.rglru_merged(xt, u_r, u_i, _branch, self.Lambda, ht_minus_1, flags, self.c)
         else:
@@ -438,44 +443,49 @@ class RecurrentBlock(nn.Module):
         for bias in (self.linear_x.bias, self.linear_y.bias, self.linear_out.bias, self.temporal_conv.bias):
             nn.init.zeros_(bias)
 
-    def _decodes_fused(self, x: Tensor, cache: RecurrentBlockCache, segment_pos: Optional[Tensor]) -> bool:
-        """Whether ``ops.decode_block`` does this cached token: this package's own layers in the dtype of ``x`` (the conv
-        and Lambda may be fp32), a cache of the right shapes, no autograd, no autocast, no tracing.  Whatever it does not
-        do -- and whatever has to be refused -- goes operator by operator."""
+    def _fused_token_parts(self, x: Tensor, cache: RecurrentBlockCache, segment_pos: Optional[Tensor]) -> Optional[tuple]:
+        """The parameters ``ops.decode_block`` does this cached token with, or None where it does not: it takes this package's
+        own layers in the dtype of ``x`` (the conv and Lambda may be fp32) and a cache of the right shapes, without autograd,
+        autocast or tracing.  Whatever it does not do -- and whatever has to be refused -- goes operator by operator."""
         if torch.is_grad_enabled() or not x.is_cuda or ops._library_ops_active() or torch.is_autocast_enabled("cuda"):
-            return False
-        lru, conv = self.rg_lru, self.temporal_conv
+            return None
+        lru, conv, lx, ly = self.rg_lru, self.temporal_conv, self.linear_x, self.linear_y
         # (replaced layers need not have any of the attributes read below)
-        if not (type(lru) is RG_LRU and _is_stock(self.linear_x, nn.Linear) and _is_stock(self.linear_y, nn.Linear)
-                and _is_stock(lru.recurrence_gate, BlockDiagonalLinear) and _is_stock(lru.input_gate, BlockDiagonalLinear)
-                and ops.decode_block_supported(x, lru.recurrence_gate.block_width)):
-            return False
-        batch, width = x.shape[0], self.rnn_width
-        for gate in (lru.recurrence_gate, lru.input_gate):
-            if gate.bias is None or gate.weight.shape != (gate.num_blocks, gate.block_width, gate.block_width):
-                return False
-        same = (self.linear_x.weight, self.linear_y.weight, lru.recurrence_gate.weight, lru.recurrence_gate.bias,
-                lru.input_gate.weight, lru.input_gate.bias)
-        either = (conv.weight, lru.Lambda) if conv.bias is None else (conv.weight, conv.bias, lru.Lambda)
-        device = x.device
-        if not (all([t.dtype == x.dtype and t.device == device for t in same])
-                and all([t.dtype in (x.dtype, torch.float32) and t.device == device for t in either])):
-            return False
-        return (cache.rnn_state.shape == (batch, width) and cache.conv_state.shape == (batch, 3, width)
-                and cache.segment_position.shape == (batch,) and (segment_pos is None or segment_pos.shape == (batch, 1)))
+        if type(lru) is not RG_LRU or not (_is_stock(lx, nn.Linear) and _is_stock(ly, nn.Linear)):
+            return None
+        r, i = lru.recurrence_gate, lru.input_gate
+        if not (_is_stock(r, BlockDiagonalLinear) and _is_stock(i, BlockDiagonalLinear)
+                and ops.decode_block_supported(x, r.block_width)):
+            return None
+        batch, width, dtype, device = x.shape[0], self.rnn_width, x.dtype, x.device
+        w_r, b_r, w_i, b_i, lam, conv_w, conv_b = r.weight, r.bias, i.weight, i.bias, lru.Lambda, conv.weight, conv.bias
+        if (b_r is None or b_i is None or w_r.shape != (r.num_blocks, r.block_width, r.block_width)
+                or w_i.shape != w_r.shape):
+            return None
+        w_x, w_y = lx.weight, ly.weight
+        for t in (w_x, w_y, w_r, b_r, w_i, b_i):
+            if t.dtype != dtype or t.device != device:
+                return None
+        for t in (conv_w, conv_b, lam):
+            if t is not None and (t.dtype != dtype and t.dtype != torch.float32 or t.device != device):
+                return None
+        if not (cache.rnn_state.shape == (batch, width) and cache.conv_state.shape == (batch, 3, width)
+                and cache.segment_position.shape == (batch,) and (segment_pos is None or segment_pos.shape == (batch, 1))):
+            return None
+        return (w_x, lx.bias, w_y, ly.bias), conv_w, conv_b, (w_r, b_r, w_i, b_i, lam), lru.c
 
-    def _decode_fused(self, x: Tensor, cache: RecurrentBlockCache, segment_pos: Optional[Tensor],
-                      active_mask: Optional[Tensor], return_cache: bool):
-        lru, conv, device = self.rg_lru, self.temporal_conv, x.device
-        branch = _project(self.linear_y, x)[:, 0]
-        x_in = _project(self.linear_x, x)[:, 0]
+    def _fused_token(self, parts: tuple, x: Tensor, cache: RecurrentBlockCache, segment_pos: Optional[Tensor],
+                     active_mask: Optional[Tensor], return_cache: bool):
+        (w_x, b_x, w_y, b_y), conv_w, conv_b, gates, c = parts
+        device = x.device
+        branch = ops.linear(x, w_y, b_y)[:, 0]
+        x_in = ops.linear(x, w_x, b_x)[:, 0]
         y, new_rnn, new_conv, position = ops.decode_block(
-            x_in, branch, conv.weight.squeeze(1), conv.bias, cache.conv_state.to(device=device, dtype=x.dtype),
-            lru.recurrence_gate.weight, lru.recurrence_gate.bias, lru.input_gate.weight, lru.input_gate.bias, lru.Lambda,
+            x_in, branch, conv_w.squeeze(1), conv_b, cache.conv_state.to(device=device, dtype=x.dtype), *gates,
             cache.rnn_state.to(device=device, dtype=torch.float32),
             cache.segment_position.to(device=device, dtype=torch.long),
             None if segment_pos is None else segment_pos.to(device=device, dtype=torch.long)[:, 0],
-            None if active_mask is None else active_mask[:, 0], lru.c)
+            None if active_mask is None else active_mask[:, 0], c)
         out = _project(self.linear_out, y[:, None, :])
         if active_mask is not None:
             out = torch.where(active_mask[..., None], out, 0.0)
@@ -491,8 +501,10 @@ class RecurrentBlock(nn.Module):
             if active_mask.shape != (batch, steps):
                 raise ValueError("active_mask must match the input [batch, sequence] dimensions")
             active_mask = active_mask.to(device=x.device, dtype=torch.bool)
-        if steps == 1 and cache is not None and self._decodes_fused(x, cache, segment_pos):
-            return self._decode_fused(x, cache, segment_pos, active_mask, return_cache)
+        if steps == 1 and cache is not None:
+            parts = self._fused_token_parts(x, cache, segment_pos)
+            if parts is not None:
+                return self._fused_token(parts, x, cache, segment_pos, active_mask, return_cache)
         previous = None if cache is None else cache.segment_position
         plain = segment_pos is None and cache is None and active_mask is None
         if plain and steps == 0:

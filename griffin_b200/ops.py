@@ -912,8 +912,9 @@ def _layer_fwd(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, la
     ws = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
     with _on(x, "rglru_layer_fwd"):
         _keep_gemms_capturable(x.device)
-        rc = lib.rglru_layer_fwd(_ptr(x), _ptr(w_r), _ptr(b_r), _ptr(w_i), _ptr(b_i), _ptr(lam), _ptr(branch), _ptr(h0),
-                                 _ptr(tok), _ptr(out), _ptr(h_last), _ptr(u), _ptr(ws), nbytes, int(save), B, T, D, bw,
+        rc = lib.rglru_layer_fwd(x.data_ptr(), w_r.data_ptr(), b_r.data_ptr(), w_i.data_ptr(), b_i.data_ptr(), lam.data_ptr(),
+                                 _ptr(branch), _ptr(h0), _ptr(tok), out.data_ptr(), h_last.data_ptr(), u.data_ptr(),
+                                 ws.data_ptr(), nbytes, int(save), B, T, D, bw,
                                  _gate_group(bw, x.element_size()), c, _DTYPES[w_r.dtype], _DTYPES[b_r.dtype],
                                  _DTYPES[lam.dtype], dt, _stream(x))
     _lib.check(rc, "rglru_layer_fwd")
@@ -953,9 +954,10 @@ class _LayerNode(torch.autograd.Function):
         scratch = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
         with _on(x, "rglru_layer_bwd"):
             _keep_gemms_capturable(x.device)
-            rc = lib.rglru_layer_bwd(_ptr(dout), _ptr(dh_last), _ptr(x), _ptr(u), _ptr(branch), _ptr(h0), _ptr(tok), _ptr(ws),
-                                     ws.numel(), _ptr(dx), _ptr(du), _ptr(dbranch), _ptr(dw_r), _ptr(db_r), _ptr(dw_i),
-                                     _ptr(db_i), _ptr(dlam), _ptr(dh0), _ptr(scratch), nbytes, B, T, D, bw,
+            rc = lib.rglru_layer_bwd(dout.data_ptr(), _ptr(dh_last), x.data_ptr(), u.data_ptr(), _ptr(branch), _ptr(h0), _ptr(tok),
+                                     ws.data_ptr(), ws.numel(), dx.data_ptr(), du.data_ptr(), _ptr(dbranch), dw_r.data_ptr(),
+                                     db_r.data_ptr(), dw_i.data_ptr(), db_i.data_ptr(), dlam.data_ptr(), _ptr(dh0),
+                                     scratch.data_ptr(), nbytes, B, T, D, bw,
                                      _gate_group(bw, x.element_size()), ctx.c, _DTYPES[dw_r.dtype], _DTYPES[db_r.dtype],
                                      _DTYPES[dlam.dtype], dt, _stream(x))
         _lib.check(rc, "rglru_layer_bwd")
@@ -970,10 +972,11 @@ def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, l
     computed inside the node by one grouped GEMM; with ``branch`` the first result is y * gelu_tanh(branch)."""
     if x.dim() != 3:
         raise ValueError("x must be [batch, sequence, width]")
+    B, T, D = x.shape
     G, bw, bw_in = w_r.shape
-    if bw != bw_in or w_i.shape != w_r.shape or G * bw != x.shape[2] or b_r.shape != (G, bw) or b_i.shape != (G, bw):
+    if bw != bw_in or w_i.shape != w_r.shape or G * bw != D or b_r.shape != (G, bw) or b_i.shape != (G, bw):
         raise ValueError("gate weights must be [heads, width/heads, width/heads] and biases [heads, width/heads]")
-    if lam.shape != (x.shape[2],):
+    if lam.shape != (D,):
         raise ValueError("Lambda must have shape [width]")
     if branch is not None and branch.shape != x.shape:
         raise ValueError("branch must have the shape of x")
@@ -985,11 +988,12 @@ def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, l
         _same_device(x, w_r, b_r, w_i, b_i, lam)
     if h0 is not None or tok is not None or branch is not None:
         _same_device(x, h0, tok, branch)
-        if h0 is not None and h0.shape != (x.shape[0], x.shape[2]):
+        if h0 is not None and h0.shape != (B, D):
             raise ValueError(f"h0 must be [batch, width], got {list(h0.shape)}")
-        _expect("tok", tok, x.shape[:2], torch.uint8)
-    save = torch.is_grad_enabled() and any(
-        t is not None and t.requires_grad for t in (x, w_r, b_r, w_i, b_i, lam, h0, branch))
+        _expect("tok", tok, (B, T), torch.uint8)
+    save = torch.is_grad_enabled() and (
+        x.requires_grad or w_r.requires_grad or b_r.requires_grad or w_i.requires_grad or b_i.requires_grad or lam.requires_grad
+        or (h0 is not None and h0.requires_grad) or (branch is not None and branch.requires_grad))
     traced = _library_ops_active()
     if traced or lam.dtype not in _DTYPES:
         lam = lam.to(torch.float32)

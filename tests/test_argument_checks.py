@@ -123,11 +123,11 @@ def test_a_cached_token_through_a_replaced_gate_is_not_taken_by_the_fused_form()
         block = RecurrentBlock(32, 64, gate_blocks=2)
         setattr(block.rg_lru, replace, torch.nn.Identity())
         with torch.no_grad():
-            assert block._decodes_fused(OnGpu(), None, None) is False
+            assert block._fused_token_parts(OnGpu(), None, None) is None
     block = RecurrentBlock(32, 64, gate_blocks=2)
     block.rg_lru = torch.nn.Identity()
     with torch.no_grad():
-        assert block._decodes_fused(OnGpu(), None, None) is False
+        assert block._fused_token_parts(OnGpu(), None, None) is None
 
 
 @pytest.mark.parametrize("register", ["register_module_forward_hook", "register_module_forward_pre_hook",

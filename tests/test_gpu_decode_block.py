@@ -118,3 +118,18 @@ def test_a_replaced_gate_goes_by_operators():
             want, ref = block(x, cache, return_cache=True)
     torch.testing.assert_close(out, want, rtol=1e-5, atol=1e-5)
     torch.testing.assert_close(new.rnn_state, ref.rnn_state, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("cached", [False, True])
+def test_gates_of_different_heads_run_as_modules(cached):
+    """A gate of this package's own class with other heads than its partner's: neither fused form can read it."""
+    from griffin_b200 import BlockDiagonalLinear
+    block, x, cache, _, _ = _setup(3, 2, 24, torch.float32, False, False)
+    gate = BlockDiagonalLinear(48, num_blocks=3).to(DEV)
+    block.rg_lru.input_gate = gate
+    with torch.no_grad():
+        out, new = block(x, cache if cached else None, return_cache=True)
+        block = _by_operators(block)
+        want, ref = block(x, cache if cached else None, return_cache=True)
+    torch.testing.assert_close(out, want, rtol=1e-5, atol=1e-6)
+    torch.testing.assert_close(new.rnn_state, ref.rnn_state, rtol=1e-5, atol=1e-6)
