@@ -561,7 +561,8 @@ class RecurrentBlock(nn.Module):
         if conv_state is not None and conv_state.shape != (batch, self.conv_kernel_size - 1, self.rnn_width):
             raise ValueError("Recurrent convolution cache has an incompatible shape")
 
-        conv_w = self.temporal_conv.weight.squeeze(1)      # (a view whose gradient is a view)
+        conv = self.temporal_conv
+        conv_w, conv_b = conv.weight.squeeze(1), conv.bias      # (a view whose gradient is a view)
         merged = self.fold_merge                           # whether the kernels form the branch product
         rnn_state = None if cache is None else cache.rnn_state
         if steps == 1 and cache is not None and not torch.is_grad_enabled() and x_in.is_cuda:
@@ -572,9 +573,8 @@ class RecurrentBlock(nn.Module):
             lru = self.rg_lru
             tok = flags[:, 0].contiguous()
             new_conv = conv_state.to(x_in.dtype).clone()
-            bias = self.temporal_conv.bias
             x_conv = ops.decode_conv(x_in[:, 0].contiguous(), conv_w.float().contiguous(),
-                                     None if bias is None else bias.float().contiguous(), new_conv, tok)
+                                     None if conv_b is None else conv_b.float().contiguous(), new_conv, tok)
             u_r = lru.recurrence_gate(x_conv).to(x_conv.dtype)
             u_i = lru.input_gate(x_conv).to(x_conv.dtype)
             new_rnn = rnn_state.to(device=x_in.device, dtype=torch.float32).clone()
@@ -587,11 +587,11 @@ class RecurrentBlock(nn.Module):
                 raise ValueError(f"ht_minus_1 must have shape ({batch}, {self.rnn_width}), got {tuple(rnn_state.shape)}")
             lru = self.rg_lru
             y, new_rnn, new_conv = ops.recurrent_core(
-                x_in, conv_w, self.temporal_conv.bias, conv_state, lru.recurrence_gate.weight, lru.recurrence_gate.bias,
+                x_in, conv_w, conv_b, conv_state, lru.recurrence_gate.weight, lru.recurrence_gate.bias,
                 lru.input_gate.weight, lru.input_gate.bias, lru.Lambda, rnn_state, flags, lru.c,
                 y_branch if self.fold_merge else None)
         else:
-            x_conv, new_conv = ops.causal_conv(x_in, conv_w, self.temporal_conv.bias, conv_state, flags,
+            x_conv, new_conv = ops.causal_conv(x_in, conv_w, conv_b, conv_state, flags,
                                                want_state=return_cache)
             y, new_rnn = self.rg_lru(x_conv, rnn_state, return_state=True, _flags=flags,
                                      _branch=y_branch if self.fold_merge else None)

@@ -986,11 +986,15 @@ def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, l
     if not (w_r.device == device and b_r.device == device and w_i.device == device and b_i.device == device
             and lam.device == device):
         _same_device(x, w_r, b_r, w_i, b_i, lam)
-    if h0 is not None or tok is not None or branch is not None:
-        _same_device(x, h0, tok, branch)
-        if h0 is not None and h0.shape != (B, D):
-            raise ValueError(f"h0 must be [batch, width], got {list(h0.shape)}")
+    if tok is not None and (tok.device != device or tok.dtype != torch.uint8 or tok.shape != (B, T)):
+        _same_device(x, tok)
         _expect("tok", tok, (B, T), torch.uint8)
+    if h0 is not None:
+        _same_device(x, h0)
+        if h0.shape != (B, D):
+            raise ValueError(f"h0 must be [batch, width], got {list(h0.shape)}")
+    if branch is not None:
+        _same_device(x, branch)
     save = torch.is_grad_enabled() and (
         x.requires_grad or w_r.requires_grad or b_r.requires_grad or w_i.requires_grad or b_i.requires_grad or lam.requires_grad
         or (h0 is not None and h0.requires_grad) or (branch is not None and branch.requires_grad))
