@@ -176,14 +176,21 @@ struct SplitChain {
     mbar_wait_or_flag(&sm->bar[it & 1], (it >> 1) & 1, dead, status, DEV_TIMEOUT_SPLIT);
     return fold(it, ch, carry, prod);
   }
-  __device__ __forceinline__ float receive(int it, int ch, float& carry, float& prod, bool& alive) {
+  // (`contractive`: no rank's product is above one, or NaN)
+  __device__ __forceinline__ float receive(int it, int ch, float& carry, bool& contractive, bool& alive) {
     if (alive) alive = mbar_wait_bounded(&sm->bar[it & 1], (it >> 1) & 1);
-    return fold(it, ch, carry, prod);
+    float unused = 1.0f;
+    return fold(it, ch, carry, unused, &contractive);
   }
-  __device__ __forceinline__ float fold(int it, int ch, float& carry, float& prod) {
+  __device__ __forceinline__ float fold(int it, int ch, float& carry, float& prod, bool* contractive = nullptr) {
     float2 v[MAX_SPLIT];
 #pragma unroll
     for (int r = 0; r < MAX_SPLIT; ++r) v[r] = r < static_cast<int>(size) ? sm->pair[it & 1][r][ch] : make_float2(1.0f, 0.0f);
+    if (contractive) {
+      *contractive = true;
+#pragma unroll
+      for (int r = 0; r < MAX_SPLIT; ++r) *contractive = *contractive && fabsf(v[r].x) <= 1.0f;
+    }
     float e = carry, enter = carry;
 #pragma unroll
     for (int r = 0; r < MAX_SPLIT; ++r) {
@@ -1390,38 +1397,34 @@ __device__ __forceinline__ void raw_chain(float2* agg, float& carry, SplitChain<
   float2 ag[LANES];
 #pragma unroll
   for (int j = 0; j < LANES; ++j) ag[j] = idle ? make_float2(1.0f, 0.0f) : agg[j * CH + tid];
-  if constexpr (!SPLIT) {
-    float e = carry;
+  auto chain = [&](float e) {       // lane by lane from the state entering the chunk; returns the state behind it
 #pragma unroll
     for (int q = 0; q < LANES; ++q) {
       const int j = REV ? LANES - 1 - q : q;
-      agg[j * CH + tid].x = e;
+      if (!idle) agg[j * CH + tid].x = e;
       e = fmaf(ag[j].x, e, ag[j].y);
     }
-    carry = e;
+    return e;
+  };
+  if constexpr (!SPLIT) {
+    carry = chain(carry);
   } else {
-    float2 m = make_float2(1.0f, 0.0f);        // map from the state entering the chunk to that entering the lane
+    float2 m = make_float2(1.0f, 0.0f);        // the map of the whole chunk
     bool composable = true;
 #pragma unroll
     for (int q = 0; q < LANES; ++q) {
-      const int j = REV ? LANES - 1 - q : q;
-      const float2 a = ag[j];
+      const float2 a = ag[REV ? LANES - 1 - q : q];
       composable = composable && fabsf(a.x) <= 1.0f;
-      ag[j] = m;
       m = make_float2(m.x * a.x, fmaf(a.x, m.y, a.y));
     }
     if (!composable) m.x = __int_as_float(0x7f800000);      // tells every rank
     split.send(it, tid, m, 0, 1);
-    float unused = 1.0f;
     const float before = carry;
-    const float e = split.receive(it, tid, carry, unused, alive);
-    bool steady = fabsf(carry) <= FLT_MAX;     // (a state that is not finite stays so to the end of the round)
-    for (uint32_t r = 0; r < split.size; ++r) steady = steady && fabsf(split.sm->pair[it & 1][r][tid].x) <= 1.0f;
+    bool contractive;
+    const float e = split.receive(it, tid, carry, contractive, alive);
+    const bool steady = contractive && fabsf(carry) <= FLT_MAX;     // (a state that is not finite stays so to the end of the round)
     const unsigned wild = __ballot_sync(0xffffffffu, !steady);
-    if (steady && !idle) {
-#pragma unroll
-      for (int j = 0; j < LANES; ++j) agg[j * CH + tid].x = fmaf(ag[j].x, e, ag[j].y);
-    }
+    if (steady) chain(e);
     if (wild) {
       if (tid == 0)
         for (uint32_t r = 0; r < split.size; ++r) mbar_expect_tx(&serial->bar[r], 4 * __popc(wild));
@@ -1429,14 +1432,7 @@ __device__ __forceinline__ void raw_chain(float2* agg, float& carry, SplitChain<
       float state = before;
       for (uint32_t r = 0; r < split.size; ++r) {
         if (r == split.rank && !steady) {
-          if (!idle) {
-            for (int q = 0; q < LANES; ++q) {
-              float2* lane = agg + (REV ? LANES - 1 - q : q) * CH + tid;
-              const float2 a = *lane;
-              lane->x = state;
-              state = fmaf(a.x, state, a.y);
-            }
-          }
+          state = chain(state);
           for (uint32_t to = 0; to < split.size; ++to)
             st_async_f32(cluster_map(&serial->exact[r][tid], to), state, cluster_map(&serial->bar[r], to));
         }
