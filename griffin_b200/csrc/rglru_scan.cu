@@ -151,7 +151,7 @@ struct ChainSmem {
 // round parity suffice: nobody can send round it + 2 before it has received everybody's round it + 1, which they
 // send after they are done reading round it.
 // What it buys: with fewer tiles than SMs a sequence is bound by one CTA walking it chunk by chunk.  B = 1, T = 16384,
-// D = 1024 bf16 (16 tiles, six CTAs each): forward 135 -> 67 us, backward 340 -> 80 us; B = 2, T = 2048: 25 -> 13 and
+// D = 1024 bf16 (16 tiles; eight CTAs each forward, six backward): forward 135 -> 67 us, backward 340 -> 80 us; B = 2, T = 2048: 25 -> 13 and
 // 47 -> 21 us; fp32 B = 1, T = 16384: 310 -> 76 and 407 -> 93 us.
 constexpr int MAX_SPLIT = 8;   // the portable cluster size
 template <int CH>
@@ -1388,9 +1388,10 @@ __device__ __forceinline__ void raw_entering(const float2* agg, int at, float2 (
   e[1] = make_float2(b.x, b.z);
 }
 // Level two of a chunk for one channel (thread): chain the lane aggregates onto the carry (lanes in increasing time order,
-// or decreasing with REV) and leave every lane's entering state in place.  `idle`: this CTA has no chunk in the round.
+// or decreasing with REV), leave every lane's entering state in place and return the state behind the chunk.  `idle`: this
+// CTA has no chunk in the round.
 template <bool REV, bool SPLIT>
-__device__ __forceinline__ void raw_chain(float2* agg, float& carry, SplitChain<CH>& split, RawSerial* serial, int& serial_rounds,
+__device__ __forceinline__ float raw_chain(float2* agg, float& carry, SplitChain<CH>& split, RawSerial* serial, int& serial_rounds,
                                           int it, bool idle, bool& alive) {
   constexpr int LANES = RAW_LANES;
   const int tid = threadIdx.x;
@@ -1407,7 +1408,7 @@ __device__ __forceinline__ void raw_chain(float2* agg, float& carry, SplitChain<
     return e;
   };
   if constexpr (!SPLIT) {
-    carry = chain(carry);
+    return carry = chain(carry);
   } else {
     float2 m = make_float2(1.0f, 0.0f);        // the map of the whole chunk
     bool composable = true;
@@ -1424,7 +1425,8 @@ __device__ __forceinline__ void raw_chain(float2* agg, float& carry, SplitChain<
     const float e = split.receive(it, tid, carry, contractive, alive);
     const bool steady = contractive && fabsf(carry) <= FLT_MAX;     // (a state that is not finite stays so to the end of the round)
     const unsigned wild = __ballot_sync(0xffffffffu, !steady);
-    if (steady) chain(e);
+    float behind = e;                          // state behind this CTA's chunk
+    if (steady) behind = chain(e);
     if (wild) {
       if (tid == 0)
         for (uint32_t r = 0; r < split.size; ++r) mbar_expect_tx(&serial->bar[r], 4 * __popc(wild));
@@ -1432,7 +1434,7 @@ __device__ __forceinline__ void raw_chain(float2* agg, float& carry, SplitChain<
       float state = before;
       for (uint32_t r = 0; r < split.size; ++r) {
         if (r == split.rank && !steady) {
-          state = chain(state);
+          behind = state = chain(state);
           for (uint32_t to = 0; to < split.size; ++to)
             st_async_f32(cluster_map(&serial->exact[r][tid], to), state, cluster_map(&serial->bar[r], to));
         }
@@ -1443,6 +1445,7 @@ __device__ __forceinline__ void raw_chain(float2* agg, float& carry, SplitChain<
       if (!steady) carry = state;
       ++serial_rounds;
     }
+    return behind;
   }
 }
 
@@ -1670,7 +1673,11 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_bwd_kernel(const __grid_consta
     }
     alive = __syncthreads_and(alive);
     if (!SPLIT && !alive) break;
-    if (tid < CH) raw_chain<true, SPLIT>(agg, carry, split, serial, serial_rounds, q, idle, alive);
+    if (tid < CH) {
+      const float behind = raw_chain<true, SPLIT>(agg, carry, split, serial, serial_rounds, q, idle, alive);
+      // (the first steps' own chunk has it to the bit, the folded carry to a rounding or two)
+      if (alive && k == 0 && dch < p.D && p.dh0) p.dh0[static_cast<size_t>(b) * p.D + dch] = behind;
+    }
     __syncthreads();
     if (idle) break;
     {
@@ -1713,7 +1720,6 @@ __global__ void __launch_bounds__(RAW_NT) rawscan_bwd_kernel(const __grid_consta
   if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }     // no CTA leaves while another may still send to it
   if (USE_TMA && tid == 0) tma_wait_all<0>();
   if (USE_TMA && !alive && tid < CH) atomicExch(p.status, DEV_TIMEOUT_LOAD);
-  if (alive && rank == 0 && tid < CH && dch < p.D && p.dh0) p.dh0[static_cast<size_t>(b) * p.D + dch] = carry;
 }
 
 // ======================================================================
