@@ -5,7 +5,7 @@
 // width: column (d / unit) * 2 unit + d % unit of the [B, T, 2 D] gate tensor is channel d's recurrence gate, `unit`
 // columns further its input gate, whatever head d is in.  A 64-channel scan tile may therefore straddle heads, and heads of any
 // width go through one GEMM without a re-layout.  bf16, B = 8, T = 8192, D = 5632, 16 heads of 352 channels, forward and
-// backward of the layer: 9.0 ms with the projections as modules (4.7 of it re-layouts), 3.4 ms this way.  Narrow groups
+// backward of the layer: 9.0 ms with the projections as modules (4.7 of it re-layouts), 3.7 ms this way (3.3 of kernels).  Narrow groups
 // cost the scan little: B = 8, T = 4096, D = 5632 bf16 forward / backward 306 / 530 us in groups of 8, 263 / 562 of 16,
 // 271 / 564 of 32, 256 / 537 of 64.
 //

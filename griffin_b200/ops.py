@@ -1,9 +1,11 @@
 """Differentiable torch operators over the C ABI.
 
-Every differentiable operator here -- the plain, merged, grouped and conv-folded scans, the raw
-affine scan and the conv -- is a ``torch.library`` custom op (namespace ``griffin_b200``) with an
-explicit backward op and a fake (shape-only) implementation, so autograd, DDP and ``torch.compile``
-see ordinary ops.  Tensors are passed to the library as raw device pointers on the current
+The plain, merged, grouped and conv-folded scans, the raw affine scan and the conv are ``torch.library``
+custom ops (namespace ``griffin_b200``) with an explicit backward op and a fake (shape-only) implementation,
+so autograd, DDP and ``torch.compile`` see ordinary ops; eager calls take an ``autograd.Function`` over the
+same implementation.  The layer in one call a direction, the pair of linear layers and the branch product
+(``_LayerNode``, ``_LinearPair``, ``_GeluMul``) are eager forms only: traced calls take the operators they
+stand for.  Tensors are passed to the library as raw device pointers on the current
 CUDA stream; nothing here computes on the CPU.
 
 * ``rglru``        -- gate epilogue + scan (griffin/griffin.py:237-286 of the reference)
@@ -969,7 +971,8 @@ def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, l
                 h0: Optional[Tensor] = None, tok: Optional[Tensor] = None, c: float = 8.0,
                 branch: Optional[Tensor] = None) -> tuple[Tensor, Tensor]:
     """y, h_last = RG-LRU(x) with both block-diagonal gate projections (weights [G, out, in], biases [G, out])
-    computed inside the node by one grouped GEMM; with ``branch`` the first result is y * gelu_tanh(branch)."""
+    computed inside the node, by the library's own projections or by batched GEMMs (:func:`_layer_in_library`); with
+    ``branch`` the first result is y * gelu_tanh(branch)."""
     if x.dim() != 3:
         raise ValueError("x must be [batch, sequence, width]")
     B, T, D = x.shape
