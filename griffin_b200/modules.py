@@ -458,6 +458,8 @@ class RecurrentBlock(nn.Module):
                 and ops.decode_block_supported(x, r.block_width)):
             return None
         batch, width, dtype, device = x.shape[0], self.rnn_width, x.dtype, x.device
+        if width > 1 << 24:                        # (what the library's first kernel has grid for)
+            return None
         w_r, b_r, w_i, b_i, lam, conv_w, conv_b = r.weight, r.bias, i.weight, i.bias, lru.Lambda, conv.weight, conv.bias
         if (b_r is None or b_i is None or w_r.shape != (r.num_blocks, r.block_width, r.block_width)
                 or w_i.shape != w_r.shape):

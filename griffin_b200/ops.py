@@ -855,7 +855,7 @@ def _layer_in_library(x: Tensor, head_width: int, differentiated: bool) -> bool:
     tokens, 16 of 64 67 / 61; 4096, 16 of 128 (2^23, 2^30) 62 / 61; 4096, 32 of 64 (2^23, 2^29) 50 / 62; fp32 65536 tokens, 16 of
     16 (2^24, 2^28) 114 / 152; 1024, 32 of 128 (2^22, 2^29) 89 / 85.
 
-    A captured call pays no host time when it is replayed, so there the faster on the device is taken (replay of the same
+    A captured call pays no host time when it is replayed, so there, warmed up, the faster on the device is taken (replay of the same
     steps: bf16 202 / 158, 139 / 76; fp32 heads of 32 212 / 222, of 64 286 / 282, of 256 430 / 341).  bf16 heads of up to 32
     channels over very many tokens keep the own kernels, whose weight gradient is split over the tokens (65536 tokens, 4 of 16
     122 / 188; 16384, 16 of 8 85 / 106).
@@ -874,7 +874,8 @@ def _layer_in_library(x: Tensor, head_width: int, differentiated: bool) -> bool:
         inside = work <= 1 << 29 and elements <= 1 << 24 and (differentiated or work <= 1 << 27 or not _tf32_allowed())
     if not inside or not torch.cuda.is_current_stream_capturing():
         return inside
-    return _own_projections_faster(elements // width, width, head_width, half, differentiated)
+    return (_own_projections_faster(elements // width, width, head_width, half, differentiated)
+            or not _gemms_capturable(x.device, differentiated))
 
 
 def _own_projections_faster(rows: int, width: int, head_width: int, half: bool, differentiated: bool) -> bool:
@@ -884,19 +885,28 @@ def _own_projections_faster(rows: int, width: int, head_width: int, half: bool, 
     return head_width < 64
 
 
-_BLAS = threading.local()
+_BLAS = threading.local()          # .devices: device indices for which the thread is known to have a cuBLAS handle
+_BACKWARD_BLAS: set = set()        # device indices whose backward passes are
 
 
-def _keep_gemms_capturable(device: torch.device) -> None:
+def _keep_gemms_capturable(device: torch.device, backward: bool) -> None:
     """A stream capture cannot create a thread's cuBLAS handle, and the layer's captured calls may take GEMMs where its eager
     calls do not: warmed up eagerly, it makes sure of the handle on each thread (and device) that it runs on."""
     try:
         ready = _BLAS.devices
     except AttributeError:
         ready = _BLAS.devices = set()
-    if device.index not in ready and not torch.cuda.is_current_stream_capturing():
+    index = device.index
+    if index not in ready and not torch.cuda.is_current_stream_capturing():
         torch.cuda.current_blas_handle()
-        ready.add(device.index)
+        ready.add(index)
+        if backward:
+            _BACKWARD_BLAS.add(index)
+
+
+def _gemms_capturable(device: torch.device, differentiated: bool) -> bool:
+    """Whether the layer has been warmed up so far on this thread, and on the one that runs backward passes."""
+    return device.index in getattr(_BLAS, "devices", ()) and (not differentiated or device.index in _BACKWARD_BLAS)
 
 
 def _layer_fwd(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor, h0: Optional[Tensor],
@@ -913,7 +923,7 @@ def _layer_fwd(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, la
     nbytes = lib.rglru_layer_workspace_bytes(B, T, D, bw, dt, int(save))
     ws = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
     with _on(x, "rglru_layer_fwd"):
-        _keep_gemms_capturable(x.device)
+        _keep_gemms_capturable(x.device, False)
         rc = lib.rglru_layer_fwd(x.data_ptr(), w_r.data_ptr(), b_r.data_ptr(), w_i.data_ptr(), b_i.data_ptr(), lam.data_ptr(),
                                  _ptr(branch), _ptr(h0), _ptr(tok), out.data_ptr(), h_last.data_ptr(), u.data_ptr(),
                                  ws.data_ptr(), nbytes, int(save), B, T, D, bw,
@@ -955,7 +965,7 @@ class _LayerNode(torch.autograd.Function):
         nbytes = lib.rglru_layer_scratch_bytes(B, T, D, bw, dt)
         scratch = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
         with _on(x, "rglru_layer_bwd"):
-            _keep_gemms_capturable(x.device)
+            _keep_gemms_capturable(x.device, True)
             rc = lib.rglru_layer_bwd(dout.data_ptr(), _ptr(dh_last), x.data_ptr(), u.data_ptr(), _ptr(branch), _ptr(h0), _ptr(tok),
                                      ws.data_ptr(), ws.numel(), dx.data_ptr(), du.data_ptr(), _ptr(dbranch), dw_r.data_ptr(),
                                      db_r.data_ptr(), dw_i.data_ptr(), db_i.data_ptr(), dlam.data_ptr(), _ptr(dh0),

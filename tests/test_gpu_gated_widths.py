@@ -194,15 +194,17 @@ def test_captured_training_step(dtype, tokens, heads, bw, own, monkeypatch):
     assert ops._lib.device_status() == 0
 
 
-def test_a_process_that_only_ran_the_layer_can_capture_it():
-    """The eager layer uses no cuBLAS, its capture does: the warm-up leaves the threads of both directions with a handle."""
+@pytest.mark.parametrize("warm_up", ["both", "forward", "none"])
+def test_a_process_that_only_ran_the_layer_can_capture_it(warm_up):
+    """The eager layer uses no cuBLAS, its capture does: the warm-up leaves the threads of both directions with a handle, and
+    what has not been warmed up stays with the kernels that need none."""
     import os
     import subprocess
     import sys
     code = """
 import sys, torch
-sys.path[:0] = sys.argv[1:]
-from griffin_b200 import RG_LRU
+sys.path[:0] = sys.argv[2:]
+from griffin_b200 import RG_LRU, ops
 from test_gpu_gated_widths import _step
 layer = RG_LRU(256, gate_blocks=4).cuda().bfloat16()
 x = torch.randn(2, 256, 256, device='cuda', dtype=torch.bfloat16, requires_grad=True)
@@ -211,22 +213,30 @@ side = torch.cuda.Stream()
 side.wait_stream(torch.cuda.current_stream())
 with torch.cuda.stream(side):
     for _ in range(3):
-        _step(layer, x, dy)
-    with torch.no_grad():
-        layer(x)
+        if sys.argv[1] == 'both':
+            _step(layer, x, dy)
+        if sys.argv[1] != 'none':
+            with torch.no_grad():
+                layer(x)
 torch.cuda.current_stream().wait_stream(side)
 layer.zero_grad(set_to_none=True); x.grad = None
+taken = []
+one_call = ops._LayerNode.apply
+ops._LayerNode.apply = staticmethod(lambda *a: taken.append(1) or one_call(*a))
 graph = torch.cuda.CUDAGraph()
 with torch.cuda.graph(graph):
-    _step(layer, x, dy)
+    got = _step(layer, x, dy)
     with torch.no_grad():
         layer(x)
+assert bool(taken) == (sys.argv[1] != 'both'), taken
 graph.replay(); torch.cuda.synchronize()
+assert all(torch.isfinite(t).all() for t in got)
 del graph
 print("captured")
 """
     here = os.path.dirname(os.path.abspath(__file__))
-    done = subprocess.run([sys.executable, "-c", code, os.path.dirname(here), here], capture_output=True, text=True, timeout=300)
+    done = subprocess.run([sys.executable, "-c", code, warm_up, os.path.dirname(here), here], capture_output=True, text=True,
+                          timeout=300)
     assert done.returncode == 0 and "captured" in done.stdout, done.stderr[-2000:]
 
 

@@ -10,6 +10,7 @@ import torch
 def ops(monkeypatch):
     from griffin_b200 import ops
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(ops, "_gemms_capturable", lambda *a: True)
     return ops
 
 
@@ -52,3 +53,10 @@ def test_projections_where_tf32_is_allowed(ops, precision, monkeypatch):
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
     assert not ops._layer_in_library(x, 32, True) and not ops._layer_in_library(x, 32, False)
     assert ops._layer_in_library(_x(65536, 256, torch.float32), 16, True)
+
+
+def test_what_was_not_warmed_up_is_captured_without_gemms(ops, monkeypatch):
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    monkeypatch.setattr(ops, "_gemms_capturable", lambda *a: False)
+    assert ops._layer_in_library(_x(16384, 1024, torch.bfloat16), 64, True)
+    assert not ops._layer_in_library(_x(16385, 1024, torch.bfloat16), 64, True)
