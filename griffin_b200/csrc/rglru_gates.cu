@@ -99,19 +99,20 @@ __global__ void __launch_bounds__(32 * GATE_WARPS) gate_unpack_kernel(const Gate
 // ---------------------------------------------------------------- fp32 weight gradient
 // dw[g][o][i] = sum over tokens n of du[n, 2 bw g + o] x[n, bw g + i].  The output is small (2 bw x bw per head) and the
 // contraction long, so a CTA takes a 64 x TI tile of one head and one stretch of the tokens, 32 of them per stage, and
-// leaves a partial sum for gate_unpack_kernel.  A thread owns 4 x 4 outputs; both operands lie with the contracted axis
-// outermost, so it reads two float4 per token.
+// leaves a partial sum for gate_unpack_kernel.  Both operands lie with the contracted axis outermost; a thread owns 8 x 4
+// outputs as pairs along o, which the eight values it reads come in, and so issues 16 packed FMAs per three 16-byte loads.
 // A library's batched GEMM walks all tokens with the few CTAs the output has: at 7685 tokens and 16 heads of 48 channels
-// two calls took 359 us, this kernel takes 51.
+// two calls took 359 us, this kernel takes 47 (55 with 4 x 4 outputs and single FMAs).
 constexpr int DW_TO = 64, DW_TK = 32;
 
 template <int TI>
-__global__ void __launch_bounds__(16 * (TI / 4)) gate_dw_kernel(const GateDwArgs p) {
+__global__ void __launch_bounds__(8 * (TI / 4)) gate_dw_kernel(const GateDwArgs p) {
   const float* du_all = static_cast<const float*>(p.du);
   const float* x_all = static_cast<const float*>(p.x);
-  constexpr int NT = 16 * (TI / 4);
+  constexpr int NT = 8 * (TI / 4);
   __shared__ __align__(16) float sa[2][DW_TK][DW_TO];
   __shared__ __align__(16) float sb[2][DW_TK][TI];
+  // (a thread's eight rows of o lie in two groups of four 32 apart, so that the threads of a warp read adjacent pieces)
   const int tid = threadIdx.x, to = (tid / (TI / 4)) * 4, ti = (tid % (TI / 4)) * 4;
   const int tiles_i = (p.bw + TI - 1) / TI;
   const int o0 = (blockIdx.x / tiles_i) * DW_TO, i0 = (blockIdx.x % tiles_i) * TI, head = blockIdx.y;
@@ -120,11 +121,13 @@ __global__ void __launch_bounds__(16 * (TI / 4)) gate_dw_kernel(const GateDwArgs
   const float* x = x_all + static_cast<size_t>(head) * p.bw;
 
   auto load = [&](int st, long long n) {
+#pragma unroll
     for (int i = tid; i < DW_TK * DW_TO / 4; i += NT) {
       const int k = i / (DW_TO / 4), c = (i % (DW_TO / 4)) * 4;
       const bool ok = n + k < n1 && o0 + c < 2 * p.bw;
       cp_async16(smem_u32(&sa[st][k][c]), ok ? du + (n + k) * 2 * p.D + o0 + c : du_all, ok);
     }
+#pragma unroll
     for (int i = tid; i < DW_TK * TI / 4; i += NT) {
       const int k = i / (TI / 4), c = (i % (TI / 4)) * 4;
       const bool ok = n + k < n1 && i0 + c < p.bw;
@@ -132,11 +135,11 @@ __global__ void __launch_bounds__(16 * (TI / 4)) gate_dw_kernel(const GateDwArgs
     }
     cp_async_commit();
   };
-  float acc[4][4];
+  float2 acc[4][4];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.0f;
+    for (int b = 0; b < 4; ++b) acc[a][b] = f2(0.0f);
   load(0, n0);
   int st = 0;
   for (long long n = n0; n < n1; n += DW_TK, st ^= 1) {
@@ -145,22 +148,27 @@ __global__ void __launch_bounds__(16 * (TI / 4)) gate_dw_kernel(const GateDwArgs
     if (n + DW_TK < n1) load(st ^ 1, n + DW_TK);
 #pragma unroll 8
     for (int k = 0; k < DW_TK; ++k) {
-      const float4 a4 = *reinterpret_cast<const float4*>(&sa[st][k][to]);
+      const float4 l4 = *reinterpret_cast<const float4*>(&sa[st][k][to]);
+      const float4 h4 = *reinterpret_cast<const float4*>(&sa[st][k][to + 32]);
       const float4 b4 = *reinterpret_cast<const float4*>(&sb[st][k][ti]);
-      const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+      const float2 a[4] = {make_float2(l4.x, l4.y), make_float2(l4.z, l4.w), make_float2(h4.x, h4.y), make_float2(h4.z, h4.w)};
+      const float b[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+      for (int v = 0; v < 4; ++v)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
+        for (int u = 0; u < 4; ++u) acc[u][v] = fma2(a[u], f2(b[v]), acc[u][v]);
     }
   }
   if (i0 + ti >= p.bw) return;             // bw is a multiple of 4
   float* out = p.part + (static_cast<size_t>(blockIdx.z) * 2 * p.D + static_cast<size_t>(head) * 2 * p.bw) * p.bw;
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
-    if (o0 + to + u < 2 * p.bw)
-      *reinterpret_cast<float4*>(out + static_cast<size_t>(o0 + to + u) * p.bw + i0 + ti) =
-          make_float4(acc[u][0], acc[u][1], acc[u][2], acc[u][3]);
+  for (int u = 0; u < 8; ++u) {
+    const int o = o0 + to + (u >> 2) * 32 + (u & 3);
+    const float2(&r)[4] = acc[u >> 1];
+    if (o < 2 * p.bw)
+      *reinterpret_cast<float4*>(out + static_cast<size_t>(o) * p.bw + i0 + ti) =
+          (u & 1) ? make_float4(r[0].y, r[1].y, r[2].y, r[3].y) : make_float4(r[0].x, r[1].x, r[2].x, r[3].x);
+  }
 }
 
 // ---------------------------------------------------------------- fp32 projections
@@ -517,9 +525,9 @@ cudaError_t launch_gate_dw(bool bf16, const GateDwArgs& args, int splits, cudaSt
   const int ti = dw_tile(a.bw);
   const dim3 grid(static_cast<unsigned>(((2 * a.bw + DW_TO - 1) / DW_TO) * ((a.bw + ti - 1) / ti)),
                   static_cast<unsigned>(a.D / a.bw), static_cast<unsigned>(splits));
-  if (ti == 64) gate_dw_kernel<64><<<grid, 256, 0, s>>>(a);
-  else if (ti == 48) gate_dw_kernel<48><<<grid, 192, 0, s>>>(a);
-  else gate_dw_kernel<32><<<grid, 128, 0, s>>>(a);
+  if (ti == 64) gate_dw_kernel<64><<<grid, 128, 0, s>>>(a);
+  else if (ti == 48) gate_dw_kernel<48><<<grid, 96, 0, s>>>(a);
+  else gate_dw_kernel<32><<<grid, 64, 0, s>>>(a);
   return cudaGetLastError();
 }
 
