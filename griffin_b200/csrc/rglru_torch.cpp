@@ -1,0 +1,619 @@
+// The eager operators as native autograd nodes over the C ABI: what griffin_b200/ops.py does in Python for a call, without the
+// interpreter.  A step forward and backward, Python forms / these, us: scan B8 T2048 D1024 bf16 134 / 81 (78 of them kernels), raw
+// scan B3 T1999 D1000 102 / 65 (42), fp32 layer B2 T256 D256 220 / 134 (49), block under autocast B8 T2048 1019 / 680 (635);
+// one cached token of a small block 109 / 89 (19), a padded prompt of 6 x 1200 tokens 221 / 150 (131).
+//
+// Every entry point takes the plain case only -- dense CUDA tensors on one device, in the kernels' types and shapes, outside
+// tracing, dispatch modes, functorch and dual numbers -- and returns None for anything else, before it has launched or
+// allocated anything: the Python operators then do the call, or refuse it, as they always did.  Nothing is kept between calls.
+
+#include <ATen/ATen.h>
+#include <ATen/autocast_mode.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <pybind11/stl.h>
+#include <torch/csrc/autograd/forward_grad.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <atomic>
+#include <mutex>
+#include <optional>
+#include <string>
+#include <tuple>
+#include <vector>
+
+#include "../../include/rglru_b200.h"
+
+namespace {
+
+using at::Tensor;
+using Opt = std::optional<Tensor>;
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+// ---------------------------------------------------------------- what a plain call is
+int kernel_dtype(at::ScalarType t) { return t == at::kFloat ? RGLRU_F32 : (t == at::kBFloat16 ? RGLRU_BF16 : -1); }
+int kernel_dtype(const Tensor& t) { return kernel_dtype(t.scalar_type()); }
+
+// Nothing between this call and the CUDA backend that wants to see it (dispatch modes, functorch levels, dual numbers).
+bool unobserved() {
+  return !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
+         !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) &&
+         !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::Functionalize) &&
+         torch::autograd::ForwardADLevel::try_get_by_idx(0) == nullptr;
+}
+// An ordinary dense tensor on `device`.
+bool dense(const Tensor& t, const at::Device& device) {
+  return t.device() == device && t.layout() == at::kStrided && t.is_contiguous() && !t.is_neg() &&
+         !t.key_set().has(c10::DispatchKey::Python) && t.has_storage();
+}
+bool dense(const Opt& t, const at::Device& device) { return !t || dense(*t, device); }
+bool aligned16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15) == 0; }
+bool aligned16(const Opt& t) { return !t || aligned16(*t); }
+bool shape_is(const Tensor& t, at::IntArrayRef s) { return t.sizes() == s; }
+const void* ptr(const Opt& t) { return t ? t->const_data_ptr() : nullptr; }
+const void* ptr(const Tensor& t) { return t.defined() ? t.const_data_ptr() : nullptr; }
+template <typename T, typename X>
+const T* ptr_as(const X& t) { return static_cast<const T*>(ptr(t)); }
+bool wants_grad(const Tensor& t) { return t.defined() && t.requires_grad(); }
+bool wants_grad(const Opt& t) { return t && t->requires_grad(); }
+Tensor or_undefined(const Opt& t) { return t ? *t : Tensor(); }
+bool in_int(int64_t n) { return n > 0 && n <= 0x7fffffff; }
+bool dims_ok(const Tensor& x) {
+  return x.dim() == 3 && in_int(x.size(0)) && x.size(0) <= 65535 && in_int(x.size(1)) && in_int(x.size(2));
+}
+bool mask_ok(const Opt& m, int64_t B, int64_t T, const at::Device& d) {
+  return !m || (dense(*m, d) && m->scalar_type() == at::kBool && shape_is(*m, {B, T}));
+}
+
+void* stream_of(const at::Device& d) { return c10::cuda::getCurrentCUDAStream(d.index()).stream(); }
+Tensor empty(at::IntArrayRef s, const Tensor& like, at::ScalarType t) { return at::empty(s, like.options().dtype(t).requires_grad(false)); }
+Tensor empty_as(const Tensor& like) { return empty(like.sizes(), like, like.scalar_type()); }
+Tensor bytes(size_t n, const Tensor& like) { return empty({static_cast<int64_t>(n)}, like, at::kByte); }
+
+// The exception classes of griffin_b200._lib.check.
+void check(int rc, const char* what) {
+  if (rc == RGLRU_OK) return;
+  std::string text = std::string(what) + ": " + rglru_status_string(rc);
+  if (rc == RGLRU_ERR_BAD_SHAPE || rc == RGLRU_ERR_NULL_POINTER || rc == RGLRU_ERR_MISALIGNED || rc == RGLRU_ERR_WORKSPACE ||
+      rc == RGLRU_ERR_TOO_LARGE)
+    TORCH_CHECK_VALUE(false, text);
+  if (rc == RGLRU_ERR_BAD_DTYPE) TORCH_CHECK_TYPE(false, text);
+  if (rc == RGLRU_ERR_LAUNCH) text += std::string(" (") + rglru_last_cuda_error() + ")";
+  TORCH_CHECK(false, "CUDA RG-LRU ", text);
+}
+
+// ---------------------------------------------------------------- nodes
+// A node whose backward cannot itself be differentiated: under create_graph its results carry an error node, as those of a
+// Python Function marked once_differentiable do.
+struct KernelNode : Node {
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    const bool recorded = at::GradMode::is_enabled();
+    variable_list out;
+    {
+      at::AutoGradMode off(false);
+      out = backward(grads);
+    }
+    if (!recorded) return out;
+    bool any = false;
+    for (const Tensor& g : grads) any = any || wants_grad(g);
+    if (!any) return out;
+    for (Tensor& t : out) {
+      if (!t.defined()) continue;
+      auto error = std::make_shared<torch::autograd::DelayedError>(
+          "trying to differentiate twice a function that was marked with @once_differentiable", 1);
+      Tensor leaf = t.detach();
+      leaf.set_requires_grad(true);
+      t = (*error)({leaf})[0];
+    }
+    return out;
+  }
+  virtual variable_list backward(const variable_list& grads) = 0;
+  bool wants(size_t i) const { return task_should_compute_output(i); }
+};
+template <typename N, typename... Inputs>
+std::shared_ptr<N> make_node(const Inputs&... inputs) {
+  std::shared_ptr<N> node(new N(), torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(inputs...));
+  return node;
+}
+SavedVariable keep(const Tensor& t) { return SavedVariable(t, false); }
+SavedVariable keep(const Opt& t) { return SavedVariable(or_undefined(t), false); }
+Tensor saved(SavedVariable& v) { return v.unpack(); }
+// (what saved-tensor hooks bring back may lie anywhere)
+Tensor saved16(SavedVariable& v) {
+  Tensor t = v.unpack();
+  return !t.defined() || (t.is_contiguous() && aligned16(t)) ? t : t.clone(at::MemoryFormat::Contiguous);
+}
+Tensor dense_grad(const Tensor& g, const Tensor& like, at::ScalarType t) {
+  return g.defined() ? g.to(t).contiguous() : at::zeros(like.sizes(), like.options().dtype(t));
+}
+
+// ---------------------------------------------------------------- the scan on given pre-activations
+struct ScanNode final : KernelNode {
+  SavedVariable x, u_r, u_i, lam, h0, tok, ws;
+  float c = 0;
+  std::string name() const override { return "RglruScanBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (SavedVariable* v : {&x, &u_r, &u_i, &lam, &h0, &tok, &ws}) v->reset_data();
+  }
+  variable_list backward(const variable_list& g) override {
+    const Tensor x_ = saved(x), ur = saved(u_r), ui = saved(u_i), l = saved(lam), h = saved(h0), tk = saved(tok), w = saved(ws);
+    const c10::cuda::CUDAGuard on(x_.device());
+    const Tensor dy = dense_grad(g[0], x_, x_.scalar_type());
+    const Tensor dh = g[1].defined() ? g[1].to(at::kFloat).contiguous() : Tensor();
+    const int64_t B = x_.size(0), T = x_.size(1), D = x_.size(2);
+    Tensor dx = empty_as(x_), dur = empty_as(x_), dui = empty_as(x_), dlam = empty({D}, x_, at::kFloat), dh0;
+    if (h.defined() && wants(4)) dh0 = empty({B, D}, x_, at::kFloat);
+    check(rglru_bwd(ptr(dy), ptr_as<float>(dh), ptr(x_), ptr(ur), ptr(ui), ptr_as<float>(l), ptr_as<float>(h), ptr_as<uint8_t>(tk),
+                    w.data_ptr(), w.numel(), dx.data_ptr(), dur.data_ptr(), dui.data_ptr(), dlam.data_ptr<float>(),
+                    dh0.defined() ? dh0.data_ptr<float>() : nullptr, B, T, D, c, kernel_dtype(x_), stream_of(x_.device())),
+          "rglru_bwd");
+    return {dx, dur, dui, dlam, dh0};
+  }
+};
+
+std::optional<std::tuple<Tensor, Tensor>> scan(const Tensor& x, const Tensor& u_r, const Tensor& u_i, const Tensor& lam, const Opt& h0,
+                                               const Opt& tok, double c) {
+  const at::Device d = x.device();
+  if (!x.is_cuda() || !dims_ok(x) || kernel_dtype(x) < 0 || !unobserved() || !dense(x, d) || !dense(u_r, d) || !dense(u_i, d) ||
+      !dense(lam, d) || !dense(h0, d) || !dense(tok, d) || u_r.sizes() != x.sizes() || u_i.sizes() != x.sizes() ||
+      u_r.scalar_type() != x.scalar_type() || u_i.scalar_type() != x.scalar_type() || lam.scalar_type() != at::kFloat)
+    return std::nullopt;
+  const int64_t B = x.size(0), T = x.size(1), D = x.size(2);
+  if (!shape_is(lam, {D}) || (h0 && (h0->scalar_type() != at::kFloat || !shape_is(*h0, {B, D}))) ||
+      (tok && (tok->scalar_type() != at::kByte || !shape_is(*tok, {B, T}))))
+    return std::nullopt;
+  const bool save = at::GradMode::is_enabled() && (wants_grad(x) || wants_grad(u_r) || wants_grad(u_i) || wants_grad(lam) || wants_grad(h0));
+  Tensor y, h_last, ws;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    const c10::cuda::CUDAGuard on(d);
+    y = empty_as(x);
+    h_last = empty({B, D}, x, at::kFloat);
+    const size_t n = save ? rglru_workspace_bytes(B, T, D, kernel_dtype(x)) : 0;
+    if (save) ws = bytes(n, x);
+    check(rglru_fwd(ptr(x), ptr(u_r), ptr(u_i), ptr_as<float>(lam), ptr_as<float>(h0), ptr_as<uint8_t>(tok), y.data_ptr(),
+                    h_last.data_ptr<float>(), save ? ws.data_ptr() : nullptr, n, B, T, D, c, kernel_dtype(x), stream_of(d)),
+          "rglru_fwd");
+  }
+  if (save) {
+    auto node = make_node<ScanNode>(x, u_r, u_i, lam, or_undefined(h0));
+    node->x = keep(x); node->u_r = keep(u_r); node->u_i = keep(u_i); node->lam = keep(lam); node->h0 = keep(h0); node->tok = keep(tok);
+    node->ws = keep(ws);
+    node->c = c;
+    torch::autograd::set_history(y, node);
+    torch::autograd::set_history(h_last, node);
+  }
+  return std::make_tuple(y, h_last);
+}
+
+// ---------------------------------------------------------------- raw affine scan
+struct AffineNode final : KernelNode {
+  SavedVariable decay, h0, out;
+  std::string name() const override { return "LinearScanBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (SavedVariable* v : {&decay, &h0, &out}) v->reset_data();
+  }
+  variable_list backward(const variable_list& g) override {
+    const Tensor a = saved(decay), h = saved(h0), o = out.unpack(shared_from_this());
+    const c10::cuda::CUDAGuard on(a.device());
+    const Tensor dout = dense_grad(g[0], a, at::kFloat);
+    Tensor da = empty_as(a), dd = empty_as(a), dh = empty_as(h);
+    check(rglru_linear_scan_bwd(dout.const_data_ptr<float>(), a.const_data_ptr<float>(), h.const_data_ptr<float>(), o.const_data_ptr<float>(),
+                                da.data_ptr<float>(), dd.data_ptr<float>(), dh.data_ptr<float>(), a.size(0), a.size(1), a.size(2),
+                                stream_of(a.device())),
+          "rglru_linear_scan_bwd");
+    return {da, dd, dh};
+  }
+};
+
+std::optional<Tensor> affine(const Tensor& decay, const Tensor& drive, const Tensor& h0) {
+  const at::Device d = decay.device();
+  if (!decay.is_cuda() || !dims_ok(decay) || !unobserved() || !dense(decay, d) || !dense(drive, d) || !dense(h0, d) ||
+      decay.scalar_type() != at::kFloat || drive.scalar_type() != at::kFloat || h0.scalar_type() != at::kFloat ||
+      drive.sizes() != decay.sizes() || !shape_is(h0, {decay.size(0), decay.size(2)}))
+    return std::nullopt;
+  Tensor out;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    const c10::cuda::CUDAGuard on(d);
+    out = empty_as(drive);
+    check(rglru_linear_scan_fwd(decay.const_data_ptr<float>(), drive.const_data_ptr<float>(), h0.const_data_ptr<float>(),
+                                out.data_ptr<float>(), decay.size(0), decay.size(1), decay.size(2), stream_of(d)),
+          "rglru_linear_scan_fwd");
+  }
+  if (at::GradMode::is_enabled() && (wants_grad(decay) || wants_grad(drive) || wants_grad(h0))) {
+    auto node = make_node<AffineNode>(decay, drive, h0);
+    torch::autograd::set_history(out, node);
+    node->decay = keep(decay); node->h0 = keep(h0); node->out = SavedVariable(out, true);
+  }
+  return out;
+}
+
+// ---------------------------------------------------------------- the layer, each direction as one library call
+// Which threads and devices have a cuBLAS handle (see _keep_gemms_capturable in ops.py).
+thread_local uint64_t t_blas = 0;
+std::atomic<uint64_t> g_backward_blas{0};
+void keep_gemms_capturable(const at::Device& d, bool backward) {
+  const uint64_t bit = 1ull << (d.index() & 63);
+  if (t_blas & bit) return;
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return;
+  at::cuda::getCurrentCUDABlasHandle();
+  t_blas |= bit;
+  if (backward) g_backward_blas |= bit;
+}
+bool gemms_capturable(int64_t index, bool differentiated) {
+  const uint64_t bit = 1ull << (index & 63);
+  return (t_blas & bit) && (!differentiated || (g_backward_blas.load() & bit));
+}
+
+struct Gates {
+  Tensor w_r, b_r, w_i, b_i, lam;
+  double c;
+  int64_t heads() const { return w_r.size(0); }
+  int64_t width() const { return w_r.size(1); }
+  bool want_grad() const { return wants_grad(w_r) || wants_grad(b_r) || wants_grad(w_i) || wants_grad(b_i) || wants_grad(lam); }
+};
+int64_t gate_group(int64_t bw) { return std::min<int64_t>(bw & -bw, 64); }
+
+// Whether the layer is a plain call.  Whether it is made in one piece at all is the caller's decision (ops._layer_in_library); a call
+// that is being captured is not taken from here.
+bool layer_plain(at::ScalarType dtype, int64_t D, const at::Device& d, const Gates& g) {
+  const Tensor& w = g.w_r;
+  if (w.dim() != 3 || w.size(1) != w.size(2) || w.size(0) < 1 || w.size(1) < 1 || g.w_i.sizes() != w.sizes() ||
+      !shape_is(g.b_r, {w.size(0), w.size(1)}) || g.b_i.sizes() != g.b_r.sizes() || w.size(0) * w.size(1) != D)
+    return false;
+  if (!shape_is(g.lam, {D}) || kernel_dtype(w) < 0 || g.w_i.scalar_type() != w.scalar_type() || kernel_dtype(g.b_r) < 0 ||
+      g.b_i.scalar_type() != g.b_r.scalar_type() || kernel_dtype(g.lam) < 0 || !dense(w, d) || !dense(g.w_i, d) || !dense(g.b_r, d) ||
+      !dense(g.b_i, d) || !dense(g.lam, d) || !aligned16(w) || !aligned16(g.w_i))
+    return false;
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return false;
+  return gate_group(g.width()) * (dtype == at::kBFloat16 ? 2 : 4) >= 16 && g.heads() <= 65535;
+}
+
+// What the layer keeps for its backward beside the tensors.
+struct LayerShape {
+  int64_t heads = 0, bw = 0;
+  at::ScalarType wt = at::kFloat, bt = at::kFloat, lt = at::kFloat;
+  float c = 0;
+};
+LayerShape layer_shape(const Gates& g) {
+  return {g.heads(), g.width(), g.w_r.scalar_type(), g.b_r.scalar_type(), g.lam.scalar_type(), static_cast<float>(g.c)};
+}
+struct LayerOut {
+  Tensor out, h_last, u, ws;
+};
+LayerOut layer_forward(const Tensor& x, const Gates& g, const Opt& h0, const Opt& tok, const Opt& branch, bool save) {
+  const at::Device d = x.device();
+  const int64_t B = x.size(0), T = x.size(1), D = x.size(2), bw = g.width();
+  const int io = kernel_dtype(x), wd = kernel_dtype(g.w_r), bd = kernel_dtype(g.b_r), ld = kernel_dtype(g.lam);
+  LayerOut r;
+  r.out = empty_as(x);
+  r.h_last = empty({B, D}, x, at::kFloat);
+  keep_gemms_capturable(d, false);
+  r.u = empty({B, T, 2 * D}, x, x.scalar_type());
+  const size_t n = rglru_layer_workspace_bytes(B, T, D, bw, io, save);
+  r.ws = bytes(n, x);
+  check(rglru_layer_fwd(ptr(x), ptr(g.w_r), ptr(g.b_r), ptr(g.w_i), ptr(g.b_i), ptr(g.lam), ptr(branch), ptr_as<float>(h0),
+                        ptr_as<uint8_t>(tok), r.out.data_ptr(), r.h_last.data_ptr<float>(), r.u.data_ptr(), r.ws.data_ptr(), n, save, B,
+                        T, D, bw, gate_group(bw), g.c, wd, bd, ld, io, stream_of(d)),
+        "rglru_layer_fwd");
+  return r;
+}
+struct LayerGrads {
+  Tensor dx, dw_r, db_r, dw_i, db_i, dlam, dh0, dbranch;
+};
+LayerGrads layer_backward(const LayerShape& s, const Tensor& dout, const Tensor& dh, const Tensor& x, const Tensor& u, const Tensor& ws,
+                          const Tensor& branch, const Tensor& h0, const Tensor& tok, bool want_dh0) {
+  const at::Device d = x.device();
+  const int64_t B = x.size(0), T = x.size(1), D = x.size(2);
+  LayerGrads g;
+  g.dx = empty_as(x);
+  if (branch.defined()) g.dbranch = empty_as(x);
+  if (want_dh0) g.dh0 = empty({B, D}, x, at::kFloat);
+  g.dw_r = empty({s.heads, s.bw, s.bw}, x, s.wt); g.db_r = empty({s.heads, s.bw}, x, s.bt);
+  g.dw_i = empty({s.heads, s.bw, s.bw}, x, s.wt); g.db_i = empty({s.heads, s.bw}, x, s.bt);
+  g.dlam = empty({D}, x, s.lt);
+  const int io = kernel_dtype(x), wd = kernel_dtype(s.wt), bd = kernel_dtype(s.bt), ld = kernel_dtype(s.lt);
+  float* dh0 = want_dh0 ? g.dh0.data_ptr<float>() : nullptr;
+  void* dbranch = branch.defined() ? g.dbranch.data_ptr() : nullptr;
+  keep_gemms_capturable(d, true);
+  const size_t n = rglru_layer_scratch_bytes(B, T, D, s.bw, io);
+  Tensor scratch = bytes(n, x), du = empty_as(u);
+  check(rglru_layer_bwd(ptr(dout), ptr_as<float>(dh), ptr(x), ptr(u), ptr(branch), ptr_as<float>(h0), ptr_as<uint8_t>(tok), ws.data_ptr(),
+                        ws.numel(), g.dx.data_ptr(), du.data_ptr(), dbranch, g.dw_r.data_ptr(), g.db_r.data_ptr(), g.dw_i.data_ptr(),
+                        g.db_i.data_ptr(), g.dlam.data_ptr(), dh0, scratch.data_ptr(), n, B, T, D, s.bw, gate_group(s.bw), s.c, wd, bd,
+                        ld, io, stream_of(d)),
+        "rglru_layer_bwd");
+  return g;
+}
+
+struct LayerNode final : KernelNode {
+  SavedVariable x, u, ws, branch, h0, tok;
+  LayerShape shape;
+  std::string name() const override { return "LayerBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (SavedVariable* v : {&x, &u, &ws, &branch, &h0, &tok}) v->reset_data();
+  }
+  variable_list backward(const variable_list& g) override {
+    const Tensor x_ = saved16(x), u_ = saved16(u), w = saved16(ws), br = saved16(branch), h = saved(h0), tk = saved(tok);
+    const c10::cuda::CUDAGuard on(x_.device());
+    Tensor dout = dense_grad(g[0], x_, x_.scalar_type());
+    if (!aligned16(dout)) dout = dout.clone();
+    const Tensor dh = g[1].defined() ? g[1].to(at::kFloat).contiguous() : Tensor();
+    const LayerGrads r = layer_backward(shape, dout, dh, x_, u_, w, br, h, tk, h.defined() && wants(6));
+    return {r.dx, r.dw_r, r.db_r, r.dw_i, r.db_i, r.dlam, r.dh0, r.dbranch};
+  }
+};
+
+// ops.rglru_gated, where it takes one call a direction: (y, h_last).
+std::optional<std::tuple<Tensor, Tensor>> layer(const Tensor& x, const Tensor& w_r, const Tensor& b_r, const Tensor& w_i, const Tensor& b_i,
+                                                const Tensor& lam, const Opt& h0, const Opt& tok, const Opt& branch, double c) {
+  const at::Device d = x.device();
+  if (!x.is_cuda() || !dims_ok(x) || kernel_dtype(x) < 0 || !unobserved() || !dense(x, d) || !aligned16(x)) return std::nullopt;
+  const int64_t B = x.size(0), T = x.size(1), D = x.size(2);
+  if (!dense(h0, d) || (h0 && (h0->scalar_type() != at::kFloat || !shape_is(*h0, {B, D}))) || !dense(tok, d) ||
+      (tok && (tok->scalar_type() != at::kByte || !shape_is(*tok, {B, T}))) || !dense(branch, d) || !aligned16(branch) ||
+      (branch && (branch->sizes() != x.sizes() || branch->scalar_type() != x.scalar_type())))
+    return std::nullopt;
+  const Gates g{w_r, b_r, w_i, b_i, lam, c};
+  if (!layer_plain(x.scalar_type(), D, d, g)) return std::nullopt;
+  const bool save = at::GradMode::is_enabled() && (wants_grad(x) || g.want_grad() || wants_grad(h0) || wants_grad(branch));
+  LayerOut r;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    const c10::cuda::CUDAGuard on(d);
+    r = layer_forward(x, g, h0, tok, branch, save);
+  }
+  if (save) {
+    auto node = make_node<LayerNode>(x, w_r, b_r, w_i, b_i, lam, or_undefined(h0), or_undefined(branch));
+    node->x = keep(x); node->u = keep(r.u); node->ws = keep(r.ws); node->branch = keep(branch); node->h0 = keep(h0); node->tok = keep(tok);
+    node->shape = layer_shape(g);
+    torch::autograd::set_history(r.out, node);
+    torch::autograd::set_history(r.h_last, node);
+  }
+  return std::make_tuple(r.out, r.h_last);
+}
+
+// ---------------------------------------------------------------- the block
+Tensor column_sums(const Tensor& m, at::ScalarType t) {
+  const int64_t rows = m.size(0), cols = m.size(1);
+  Tensor out = empty({cols}, m, t);
+  const size_t n = rglru_column_sums_workspace_bytes(rows, cols);
+  Tensor ws = bytes(n, m);
+  check(rglru_column_sums_as(ptr(m), out.data_ptr(), ws.data_ptr(), n, rows, cols, kernel_dtype(m), kernel_dtype(out), stream_of(m.device())),
+        "rglru_column_sums");
+  return out;
+}
+Tensor mm_as(const Tensor& a, const Tensor& b, at::ScalarType t) { return a.scalar_type() == t ? at::mm(a, b) : at::mm(a, b, t); }
+Tensor rows_of(const Tensor& t) { return t.view({-1, t.size(-1)}); }
+
+// RecurrentBlock.forward after its masks as one node: linear_x and linear_y, conv, layer, branch product, linear_out.  Bias gradients
+// come from rglru_column_sums, weight gradients leave their GEMMs in the weights' types, and the two shares of the input gradient
+// meet in the second GEMM's accumulator (as in ops._LinearPair).
+enum BlockParam { WX, BX, WY, BY, CW, CB, WR, BR, WI, BI, LAM, WO, BO, BLOCK_PARAMS };
+struct BlockNode final : KernelNode {
+  SavedVariable x, wx, wy, wo, x_in, branch, cw, x_conv, u, ws, y, mixed, flags, active, conv_state, h0;
+  LayerShape layer;
+  at::ScalarType xt = at::kFloat, pt[BLOCK_PARAMS];
+  bool merge = false;
+  std::string name() const override { return "RecurrentBlockBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (SavedVariable* v : {&x, &wx, &wy, &wo, &x_in, &branch, &cw, &x_conv, &u, &ws, &y, &mixed, &flags, &active, &conv_state, &h0})
+      v->reset_data();
+  }
+  variable_list backward(const variable_list& g) override {
+    const Tensor x_ = saved16(x), x_in_ = saved16(x_in), branch_ = saved16(branch), x_conv_ = saved16(x_conv), mixed_ = saved16(mixed),
+                 wx_ = saved(wx), wy_ = saved(wy), wo_ = saved(wo), flags_ = saved(flags), active_ = saved(active), cw_ = saved(cw),
+                 h = saved(h0), conv_state_ = saved16(conv_state), u_ = saved16(u), ws_ = saved16(ws), y_ = saved16(y);
+    const at::Device d = x_.device();
+    const c10::cuda::CUDAGuard on(d);
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(at::autocast_dispatch_keyset);
+    const at::ScalarType io = x_in_.scalar_type();
+    const int64_t B = x_.size(0), T = x_.size(1), D = x_in_.size(2);
+    auto p = [](int k) { return 1 + k; };                // a parameter's place among the inputs
+    variable_list out(1 + BLOCK_PARAMS + 1);
+
+    Tensor dout = g[0].defined() ? g[0].to(io) : at::zeros({B, T, wo_.size(0)}, x_in_.options());
+    if (active_.defined()) dout = at::where(active_.unsqueeze(-1), dout, 0.0);
+    dout = rows_of(dout.contiguous());
+    if (wants(p(WO))) out[p(WO)] = mm_as(dout.t(), rows_of(mixed_), pt[WO]);
+    if (wants(p(BO))) out[p(BO)] = column_sums(dout, pt[BO]);
+    Tensor dy = at::mm(dout, wo_).view({B, T, D}), dbranch;
+    if (!merge) {
+      const Tensor dm = dy;
+      dy = empty_as(y_);
+      dbranch = empty_as(branch_);
+      check(rglru_gelu_mul_bwd(ptr(dm), ptr(y_), ptr(branch_), dy.data_ptr(), dbranch.data_ptr(), y_.numel(), kernel_dtype(y_), stream_of(d)),
+            "rglru_gelu_mul_bwd");
+    }
+    const Tensor dh = g[1].defined() ? g[1].to(at::kFloat).contiguous() : Tensor();
+    const LayerGrads r = layer_backward(layer, dy, dh, x_conv_, u_, ws_, merge ? branch_ : Tensor(), h, flags_, h.defined() && wants(1 + BLOCK_PARAMS));
+    if (merge) dbranch = r.dbranch;
+    out[p(WR)] = r.dw_r; out[p(BR)] = r.db_r; out[p(WI)] = r.dw_i; out[p(BI)] = r.db_i; out[p(LAM)] = r.dlam;
+    out[1 + BLOCK_PARAMS] = r.dh0;
+
+    Tensor dx_in = empty_as(x_in_), dcw = empty_as(cw_), dcb = empty({D}, x_in_, at::kFloat);
+    const size_t n = rglru_conv_bwd_workspace_bytes(B, T, D);
+    Tensor scratch = bytes(n, x_in_);
+    check(rglru_conv_bwd(ptr(r.dx), ptr(x_in_), cw_.const_data_ptr<float>(), ptr(conv_state_), ptr_as<uint8_t>(flags_), dx_in.data_ptr(),
+                         dcw.data_ptr<float>(), dcb.data_ptr<float>(), nullptr, scratch.data_ptr(), n, B, T, D, kernel_dtype(x_in_),
+                         stream_of(d)),
+          "rglru_conv_bwd");
+    out[p(CW)] = dcw.to(pt[CW]); out[p(CB)] = dcb.to(pt[CB]);
+
+    const Tensor d1 = rows_of(dx_in), d2 = rows_of(dbranch), rows = rows_of(x_);
+    if (wants(0)) {
+      Tensor dx = mm_as(d1, wx_, xt);
+      if (d2.scalar_type() == xt) dx.addmm_(d2, wy_);
+      else at::addmm_outf(dx, d2, wy_, xt, 1, 1, dx);
+      out[0] = dx.view(x_.sizes());
+    }
+    if (wants(p(WX))) out[p(WX)] = mm_as(d1.t(), rows, pt[WX]);
+    if (wants(p(BX))) out[p(BX)] = column_sums(d1, pt[BX]);
+    if (wants(p(WY))) out[p(WY)] = mm_as(d2.t(), rows, pt[WY]);
+    if (wants(p(BY))) out[p(BY)] = column_sums(d2, pt[BY]);
+    return out;
+  }
+};
+
+// For stock layers whose gated layer is one library call a direction: (out, final state, next conv state or None).  `flags` are the
+// call's flag bytes, `active` its padding mask for the output.
+std::optional<std::tuple<Tensor, Tensor, Opt>> block(const Tensor& x, const std::vector<Opt>& params, const Tensor& flags, const Opt& active,
+                                                     const Opt& conv_state, const Opt& rnn_state, double c, bool merge, bool want_state) {
+  const at::Device d = x.device();
+  if (!x.is_cuda() || !dims_ok(x) || !unobserved() || !dense(x, d) || params.size() != BLOCK_PARAMS) return std::nullopt;
+  Tensor p[BLOCK_PARAMS];
+  bool grad = wants_grad(x) || wants_grad(rnn_state);
+  for (int k = 0; k < BLOCK_PARAMS; ++k) {
+    if (!params[k] || !dense(params[k], d)) return std::nullopt;
+    p[k] = *params[k];
+    grad = grad || wants_grad(p[k]);
+  }
+  grad = grad && at::GradMode::is_enabled();
+  const Gates g{p[WR], p[BR], p[WI], p[BI], p[LAM], c};
+  const bool autocast = at::autocast::is_autocast_enabled(at::kCUDA);
+  const at::ScalarType dtype = autocast ? at::autocast::get_autocast_dtype(at::kCUDA) : x.scalar_type();
+  if (kernel_dtype(dtype) < 0) return std::nullopt;
+  auto alike = [&](const Tensor& t) { return t.scalar_type() == dtype || (autocast && t.scalar_type() == at::kFloat); };
+  if (!alike(x)) return std::nullopt;
+  for (int k : {WX, BX, WY, BY, WO, BO, WR, BR, WI, BI})
+    if (!alike(p[k])) return std::nullopt;
+  const int64_t B = x.size(0), T = x.size(1), I = x.size(2), D = p[BX].numel();
+  if (!shape_is(p[WX], {D, I}) || !shape_is(p[WY], {D, I}) || !shape_is(p[BX], {D}) || !shape_is(p[BY], {D}) || p[WO].dim() != 2 ||
+      p[WO].size(1) != D || !shape_is(p[BO], {p[WO].size(0)}) || !shape_is(p[CW], {D, 1, 4}) || !shape_is(p[CB], {D}) ||
+      kernel_dtype(p[CW]) < 0 || kernel_dtype(p[CB]) < 0 || !dense(flags, d) || flags.scalar_type() != at::kByte || !shape_is(flags, {B, T}) ||
+      !mask_ok(active, B, T, d) || !in_int(D) || p[WO].size(0) < 1)
+    return std::nullopt;
+  if (conv_state && (!dense(*conv_state, d) || conv_state->scalar_type() != dtype || !shape_is(*conv_state, {B, 3, D}) ||
+                     (at::GradMode::is_enabled() && wants_grad(conv_state))))
+    return std::nullopt;
+  if (rnn_state && (!dense(*rnn_state, d) || rnn_state->scalar_type() != at::kFloat || !shape_is(*rnn_state, {B, D}))) return std::nullopt;
+  if (!layer_plain(dtype, D, d, g)) return std::nullopt;
+
+  Tensor xc, wxc, wyc, woc, x_in, branch, cw, x_conv, next, mixed, out;
+  LayerOut r;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(at::autocast_dispatch_keyset);
+    const c10::cuda::CUDAGuard on(d);
+    xc = x.to(dtype); wxc = p[WX].to(dtype); wyc = p[WY].to(dtype); woc = p[WO].to(dtype);
+    x_in = at::linear(xc, wxc, p[BX].to(dtype));
+    branch = at::linear(xc, wyc, p[BY].to(dtype));
+    x_conv = empty_as(x_in);
+    if (want_state) next = empty({B, 3, D}, x_in, dtype);
+    cw = p[CW].to(at::kFloat);
+    const Tensor cb = p[CB].to(at::kFloat);
+    check(rglru_conv_fwd(ptr(x_in), cw.const_data_ptr<float>(), cb.const_data_ptr<float>(), ptr(conv_state), ptr_as<uint8_t>(flags),
+                         x_conv.data_ptr(), want_state ? next.data_ptr() : nullptr, B, T, D, kernel_dtype(x_in), stream_of(d)),
+          "rglru_conv_fwd");
+    r = layer_forward(x_conv, g, rnn_state, flags, merge ? Opt(branch) : Opt(), grad);
+    mixed = r.out;
+    if (!merge) {
+      mixed = empty_as(r.out);
+      check(rglru_gelu_mul_fwd(ptr(r.out), ptr(branch), mixed.data_ptr(), mixed.numel(), kernel_dtype(mixed), stream_of(d)),
+            "rglru_gelu_mul_fwd");
+    }
+    out = at::linear(mixed, woc, p[BO].to(dtype));
+    if (active) out = at::where(active->unsqueeze(-1), out, 0.0);
+  }
+  if (grad) {
+    auto node = make_node<BlockNode>(x, p[WX], p[BX], p[WY], p[BY], p[CW], p[CB], p[WR], p[BR], p[WI], p[BI], p[LAM], p[WO], p[BO],
+                                     or_undefined(rnn_state));
+    node->x = keep(xc); node->wx = keep(wxc); node->wy = keep(wyc); node->wo = keep(woc); node->x_in = keep(x_in);
+    node->branch = keep(branch); node->cw = keep(cw); node->x_conv = keep(x_conv); node->u = keep(r.u); node->ws = keep(r.ws);
+    node->y = keep(merge ? Tensor() : r.out); node->mixed = keep(mixed); node->flags = keep(flags); node->active = keep(active);
+    node->conv_state = keep(conv_state); node->h0 = keep(rnn_state);
+    node->layer = layer_shape(g);
+    node->xt = x.scalar_type();
+    for (int k = 0; k < BLOCK_PARAMS; ++k) node->pt[k] = p[k].scalar_type();
+    node->merge = merge;
+    torch::autograd::set_history(out, node);
+    torch::autograd::set_history(r.h_last, node);
+  }
+  return std::make_tuple(out, r.h_last, want_state ? Opt(next) : Opt());
+}
+
+// ops.token_plan with positions: (flag bytes, position of every row's last real token).
+std::optional<std::tuple<Tensor, Tensor>> plan(int64_t B, int64_t T, const Tensor& like, const Opt& seg, const Opt& prev, const Opt& active) {
+  const at::Device d = like.device();
+  auto longs = [&](const Opt& t, at::IntArrayRef s) { return !t || (dense(*t, d) && t->scalar_type() == at::kLong && shape_is(*t, s)); };
+  if (!like.is_cuda() || !unobserved() || !in_int(B) || !in_int(T) || !longs(seg, {B, T}) || !longs(prev, {B}) || !mask_ok(active, B, T, d))
+    return std::nullopt;
+  at::AutoDispatchBelowADInplaceOrView below;
+  const c10::cuda::CUDAGuard on(d);
+  Tensor flags = empty({B, T}, like, at::kByte), last = empty({B}, like, at::kLong), ws;
+  const size_t n = active ? rglru_token_plan_workspace_bytes(B, T) : 0;
+  if (n) ws = bytes(n, like);
+  check(rglru_token_plan_ws(ptr_as<int64_t>(seg), ptr_as<int64_t>(prev), ptr_as<uint8_t>(active), nullptr, 1, flags.data_ptr<uint8_t>(),
+                            last.data_ptr<int64_t>(), n ? ws.data_ptr() : nullptr, n, B, T, stream_of(d)),
+        "rglru_token_plan");
+  return std::make_tuple(flags, last);
+}
+
+// ops.decode_block: (y, next state, next conv state, next position).
+std::optional<std::tuple<Tensor, Tensor, Tensor, Tensor>> decode(const Tensor& x, const Opt& branch, const Tensor& cw, const Opt& cb,
+                                                                 const Tensor& conv_state, const Tensor& wr, const Tensor& br,
+                                                                 const Tensor& wi, const Tensor& bi, const Tensor& lam, const Tensor& h,
+                                                                 const Tensor& position, const Opt& seg, const Opt& active, double c) {
+  const at::Device d = x.device();
+  if (!x.is_cuda() || x.dim() != 2 || wr.dim() != 3 || kernel_dtype(x) < 0 || !unobserved()) return std::nullopt;
+  const at::ScalarType io = x.scalar_type();
+  for (const Tensor* t : {&x, &conv_state, &wr, &wi, &cw, &h})
+    if (!dense(*t, d) || !aligned16(*t)) return std::nullopt;
+  for (const Tensor* t : {&br, &bi, &lam, &position})
+    if (!dense(*t, d)) return std::nullopt;
+  for (const Tensor* t : {&conv_state, &wr, &br, &wi, &bi})
+    if (t->scalar_type() != io) return std::nullopt;
+  auto either = [&](const Tensor& t) { return t.scalar_type() == io || t.scalar_type() == at::kFloat; };
+  const int64_t B = x.size(0), D = x.size(1), G = wr.size(0), bw = wr.size(1);
+  if (B < 1 || B > RGLRU_DECODE_BLOCK_MAX_BATCH || D < 1 || D > RGLRU_DECODE_BLOCK_MAX_WIDTH || G * bw != D ||
+      bw * x.element_size() % 16 != 0 || h.scalar_type() != at::kFloat || position.scalar_type() != at::kLong || !either(cw) || !either(lam) ||
+      !shape_is(wr, {G, bw, bw}) || !shape_is(wi, {G, bw, bw}) || !shape_is(br, {G, bw}) || !shape_is(bi, {G, bw}) || !shape_is(h, {B, D}) ||
+      !shape_is(conv_state, {B, 3, D}) || !shape_is(cw, {D, 4}) || !shape_is(lam, {D}) || !shape_is(position, {B}) ||
+      (branch && (!dense(branch, d) || !aligned16(branch) || branch->scalar_type() != io || !shape_is(*branch, {B, D}))) ||
+      (cb && (!dense(cb, d) || !either(*cb) || !shape_is(*cb, {D}))) ||
+      (seg && (!dense(seg, d) || seg->scalar_type() != at::kLong || !shape_is(*seg, {B}))) ||
+      (active && (!dense(active, d) || active->scalar_type() != at::kBool || !shape_is(*active, {B}))))
+    return std::nullopt;
+  at::AutoDispatchBelowADInplaceOrView below;
+  const c10::cuda::CUDAGuard on(d);
+  Tensor y = empty_as(x), h_new = empty_as(h), conv_new = empty_as(conv_state), pos_new = empty_as(position);
+  const size_t n = rglru_decode_block_workspace_bytes(B, D, kernel_dtype(x));
+  Tensor ws = bytes(n, x);
+  const int f32 = (cw.scalar_type() == at::kFloat ? RGLRU_F32_CONV_W : 0) | (cb && cb->scalar_type() == at::kFloat ? RGLRU_F32_CONV_B : 0) |
+                  (lam.scalar_type() == at::kFloat ? RGLRU_F32_LAMBDA : 0);
+  check(rglru_decode_block(ptr(x), ptr(branch), ptr(cw), ptr(cb), ptr(conv_state), conv_new.data_ptr(), ptr(wr), ptr(br), ptr(wi), ptr(bi),
+                           ptr(lam), h.const_data_ptr<float>(), h_new.data_ptr<float>(), position.const_data_ptr<int64_t>(),
+                           ptr_as<int64_t>(seg), ptr_as<uint8_t>(active), pos_new.data_ptr<int64_t>(), y.data_ptr(), ws.data_ptr(), n, B, D,
+                           bw, c, kernel_dtype(x), f32, stream_of(d)),
+        "rglru_decode_block");
+  return std::make_tuple(y, h_new, conv_new, pos_new);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_native, m) {
+  m.doc() = "Native forms of the eager operators; every function returns None for a call it does not take.";
+  m.def("scan", &scan);
+  m.def("affine", &affine);
+  m.def("layer", &layer);
+  m.def("plan", &plan);
+  m.def("block", &block);
+  m.def("decode", &decode);
+  m.def("gemms_capturable", &gemms_capturable);
+}

@@ -204,6 +204,15 @@ class RG_LRU(nn.Module):
             alike = all(t.dtype == xt.dtype for t in params)
         return alike and all(t.device == xt.device for t in params)
 
+    def _stock_gates(self) -> Optional[tuple]:
+        """(w_r, b_r, w_i, b_i, Lambda) where both gates are this package's own layers as it put them there, or None."""
+        r, i = self._modules.get("recurrence_gate"), self._modules.get("input_gate")
+        if not (_is_stock(r, BlockDiagonalLinear) and _is_stock(i, BlockDiagonalLinear)):
+            return None
+        r, i = r._parameters, i._parameters
+        parts = r.get("weight"), r.get("bias"), i.get("weight"), i.get("bias"), self._parameters.get("Lambda")
+        return None if any(p is None for p in parts) else parts
+
     def forward(self, xt: Tensor, ht_minus_1: Optional[Tensor] = None, *, reset_mask: Optional[Tensor] = None,
                 active_mask: Optional[Tensor] = None, return_state: bool = False, _flags: Optional[Tensor] = None,
                 _branch: Optional[Tensor] = None):
@@ -476,6 +485,26 @@ class RecurrentBlock(nn.Module):
             return None
         return (w_x, lx.bias, w_y, ly.bias), conv_w, conv_b, (w_r, b_r, w_i, b_i, lam), lru.c
 
+    def _stock_parts(self) -> Optional[list]:
+        """The parameters of the native block call, in its order, where every layer is as this package put it there, or None."""
+        m = self._modules
+        lx, ly, lo, conv, lru = (m.get(k) for k in ("linear_x", "linear_y", "linear_out", "temporal_conv", "rg_lru"))
+        if not (_is_stock(lx, nn.Linear) and _is_stock(ly, nn.Linear) and _is_stock(lo, nn.Linear) and type(conv) is nn.Conv1d
+                and _is_stock(lru, RG_LRU) and lru.group_gates and lru.rnn_width == self.rnn_width):
+            return None
+        gates = lru._stock_gates()
+        if gates is None:
+            return None
+        lx, ly, lo, conv = lx._parameters, ly._parameters, lo._parameters, conv._parameters
+        return [lx.get("weight"), lx.get("bias"), ly.get("weight"), ly.get("bias"), conv.get("weight"), conv.get("bias"), *gates,
+                lo.get("weight"), lo.get("bias")]
+
+    def _layer_in_library(self, x: Tensor, parts: list) -> bool:
+        """:func:`ops._layer_in_library` of the layer inside a native block call on ``x``."""
+        dtype = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
+        save = torch.is_grad_enabled() and (x.requires_grad or any(p is not None and p.requires_grad for p in parts))
+        return ops._sizes_in_library(x.shape[0] * x.shape[1] * self.rnn_width, self.rnn_width, dtype, x.device, parts[6].shape[-1], save)
+
     def _fused_token(self, parts: tuple, x: Tensor, cache: RecurrentBlockCache, segment_pos: Optional[Tensor],
                      active_mask: Optional[Tensor], return_cache: bool):
         (w_x, b_x, w_y, b_y), conv_w, conv_b, gates, c = parts
@@ -550,6 +579,19 @@ class RecurrentBlock(nn.Module):
             if return_cache and last is not None:
                 last = last.clone()         # the plan is shared between blocks, a cache belongs to one
 
+        native = None
+        if x.is_cuda and moves is None and not self.fold_conv and (steps > 1 or cache is None or torch.is_grad_enabled()):
+            native = self._stock_parts() if ops._native_call() else None
+        if native is not None and self._layer_in_library(x, native):
+            done = ops._native().block(x, native, flags, active_mask, None if cache is None else cache.conv_state,
+                                       None if cache is None else cache.rnn_state, float(self._modules["rg_lru"].c), self.fold_merge,
+                                       return_cache)
+            if done is not None:
+                if not return_cache:
+                    return done[0]
+                if last is None:
+                    last = _last_real_position(pos, active_mask, previous)
+                return done[0], RecurrentBlockCache(done[1], done[2], last)
         lx, ly = self.linear_x, self.linear_y
         if _is_stock(lx, nn.Linear) and _is_stock(ly, nn.Linear):
             x_in, y_branch = ops.linear_pair(x, lx.weight, lx.bias, ly.weight, ly.bias)

@@ -94,6 +94,29 @@ def _stream(t: Tensor) -> int:
     return torch.cuda.current_stream(t.device).cuda_stream
 
 
+_NATIVE = None
+
+
+def _native():
+    """The extension module with the native forms of the eager operators (csrc/rglru_torch.cpp)."""
+    global _NATIVE
+    if _NATIVE is None:
+        try:
+            from . import _native as module
+        except ImportError as error:
+            raise RuntimeError("griffin_b200/_native.so has not been built for this PyTorch; run `python -m griffin_b200.build`. "
+                               "Eager calls on CUDA tensors need it.") from error
+        _NATIVE = module
+    return _NATIVE
+
+
+def _native_call() -> bool:
+    """Whether an eager call on CUDA tensors is offered to its native form first: outside tracing, forward-mode differentiation
+    and NVTX ranges.  The native form looks the tensors over and declines (None) whatever is not a plain call of ordinary dense
+    tensors in the kernels' types and shapes; that goes through the Python form, checks and error messages included."""
+    return not (_FORCE_LIBRARY_OPS or _NVTX or torch.compiler.is_compiling() or torch.autograd.forward_ad._current_level >= 0)
+
+
 # Every differentiable operator exists in two forms over the same implementation functions: a ``torch.library``
 # custom op (with fake implementation and registered backward), which is what ``torch.compile`` and other
 # tracers see, and a plain ``torch.autograd.Function``, which is what eager calls use because it costs a
@@ -243,6 +266,10 @@ _RglruNode = _eager_node("RglruScan", _rglru_fwd_impl, _rglru_setup, _rglru_back
 def rglru(x: Tensor, u_r: Tensor, u_i: Tensor, lam: Tensor, h0: Optional[Tensor] = None,
           tok: Optional[Tensor] = None, c: float = 8.0) -> tuple[Tensor, Tensor]:
     """y, h_last = RG-LRU(x | gate pre-activations u_r, u_i).  ``lam`` and ``h0`` are fp32."""
+    if x.is_cuda and _native_call():
+        done = _native().scan(x, u_r, u_i, lam, h0, tok, float(c))
+        if done is not None:
+            return done
     if x.dim() != 3 or u_r.shape != x.shape or u_i.shape != x.shape:
         raise ValueError("x, u_r and u_i must share shape [batch, sequence, width]")
     if u_r.dtype != x.dtype or u_i.dtype != x.dtype:
@@ -320,6 +347,10 @@ def linear_scan(decay: Tensor, current_input: Tensor, initial_state: Tensor) -> 
     ``fused_rglru_scan`` (griffin/triton_scan.py:211-224, 274-276)."""
     if not decay.is_cuda or not current_input.is_cuda or not initial_state.is_cuda:
         raise RuntimeError("CUDA linear scan requires CUDA tensors")
+    if decay.is_cuda and _native_call():
+        done = _native().affine(decay, current_input, initial_state)
+        if done is not None:
+            return done
     if decay.shape != current_input.shape or decay.dim() != 3:
         raise ValueError("decay and current_input must share shape [batch, sequence, width]")
     if initial_state.shape != (decay.size(0), decay.size(2)):
@@ -864,8 +895,12 @@ def _layer_in_library(x: Tensor, head_width: int, differentiated: bool) -> bool:
     16384 tokens, 16 of 64 537 / 283, 4096 tokens, 16 of 24 73 / 68, of 16 60 / 60, 65536 tokens, 16 of 16 450 / 514; eagerly
     4096, 32 of 48 (2^28.2) 240 / 317, 16384, 16 of 48 (2^29.2) 430 / 315, without gradients 4096, 16 of 48 (2^27.2) 69 / 67,
     1024, 32 of 128 (2^29) 90 / 68."""
-    elements, width = x.numel(), x.shape[2]
-    work, half = elements * head_width, x.dtype == torch.bfloat16
+    return _sizes_in_library(x.numel(), x.shape[2], x.dtype, x.device, head_width, differentiated)
+
+
+def _sizes_in_library(elements: int, width: int, dtype: torch.dtype, device: torch.device, head_width: int, differentiated: bool) -> bool:
+    """:func:`_layer_in_library` from the sizes."""
+    work, half = elements * head_width, dtype == torch.bfloat16
     if width // head_width > 65535:            # (heads are an axis of the kernels' grids)
         return False
     if half:
@@ -875,7 +910,7 @@ def _layer_in_library(x: Tensor, head_width: int, differentiated: bool) -> bool:
     if not inside or not torch.cuda.is_current_stream_capturing():
         return inside
     return (_own_projections_faster(elements // width, width, head_width, half, differentiated)
-            or not _gemms_capturable(x.device, differentiated))
+            or not _gemms_capturable(device, differentiated))
 
 
 def _own_projections_faster(rows: int, width: int, head_width: int, half: bool, differentiated: bool) -> bool:
@@ -906,6 +941,8 @@ def _keep_gemms_capturable(device: torch.device, backward: bool) -> None:
 
 def _gemms_capturable(device: torch.device, differentiated: bool) -> bool:
     """Whether the layer has been warmed up so far on this thread, and on the one that runs backward passes."""
+    if _native().gemms_capturable(device.index, differentiated):
+        return True
     return device.index in getattr(_BLAS, "devices", ()) and (not differentiated or device.index in _BACKWARD_BLAS)
 
 
@@ -985,6 +1022,13 @@ def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, l
     ``branch`` the first result is y * gelu_tanh(branch)."""
     if x.dim() != 3:
         raise ValueError("x must be [batch, sequence, width]")
+    save = torch.is_grad_enabled() and (
+        x.requires_grad or w_r.requires_grad or b_r.requires_grad or w_i.requires_grad or b_i.requires_grad or lam.requires_grad
+        or (h0 is not None and h0.requires_grad) or (branch is not None and branch.requires_grad))
+    if x.is_cuda and w_r.dim() == 3 and w_r.shape[1] > 0 and _native_call() and _layer_in_library(x, w_r.shape[1], save):
+        done = _native().layer(x, w_r, b_r, w_i, b_i, lam, h0, tok, branch, float(c))
+        if done is not None:
+            return done
     B, T, D = x.shape
     G, bw, bw_in = w_r.shape
     if bw != bw_in or w_i.shape != w_r.shape or G * bw != D or b_r.shape != (G, bw) or b_i.shape != (G, bw):
@@ -1008,9 +1052,6 @@ def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, l
             raise ValueError(f"h0 must be [batch, width], got {list(h0.shape)}")
     if branch is not None:
         _same_device(x, branch)
-    save = torch.is_grad_enabled() and (
-        x.requires_grad or w_r.requires_grad or b_r.requires_grad or w_i.requires_grad or b_i.requires_grad or lam.requires_grad
-        or (h0 is not None and h0.requires_grad) or (branch is not None and branch.requires_grad))
     traced = _library_ops_active()
     if traced or lam.dtype not in _DTYPES:
         lam = lam.to(torch.float32)
@@ -1309,6 +1350,11 @@ def token_plan(batch: int, steps: int, device, *, segment_pos: Optional[Tensor] 
     """(flag bytes [B, T], position of every row's last real token [B]) of a block call's masks, or with
     ``positions=False`` (flag bytes, None) of a bare layer's reset and padding masks, in one launch (``rglru_token_plan``).
     CUDA tensors on ``device``: int64 positions [B, T] and [B], bool masks [B, T]."""
+    given = segment_pos if segment_pos is not None else previous if previous is not None else active
+    if positions and given is not None and given.is_cuda and given.device == torch.device(device) and _native_call():
+        done = _native().plan(batch, steps, given, segment_pos, previous, active)
+        if done is not None:
+            return done
     flags = torch.empty(batch, steps, device=device, dtype=torch.uint8)
     _require_cuda(flags)
     _same_device(flags, segment_pos, previous, active, reset)
@@ -1420,6 +1466,11 @@ def decode_block(x_in: Tensor, branch: Optional[Tensor], conv_w: Tensor, conv_b:
     output projection (``rglru_decode_block``): conv, both gate projections, the update and, with ``branch`` given, the
     product with its GeLU.  ``x_in`` / ``branch`` [B, D]; conv weights, biases and Lambda in the activation dtype or
     (conv and Lambda) fp32; ``position`` / ``segment_pos`` [B] int64; ``active`` [B] bool.  The states are not modified."""
+    if x_in.is_cuda and _native_call():
+        done = _native().decode(x_in, branch, conv_w, conv_b, conv_state, w_r, b_r, w_i, b_i, lam, h, position, segment_pos, active,
+                                float(c))
+        if done is not None:
+            return done
     _require_cuda(x_in)
     dt = _io_dtype(x_in, "decode block")
     if x_in.dim() != 2 or w_r.dim() != 3:

@@ -1,0 +1,204 @@
+"""The native operator forms (csrc/rglru_torch.cpp) against the Python ones: the same kernels on the same tensors, so the same bits
+wherever both make the same library calls; and what the native forms leave to the Python ones."""
+
+from __future__ import annotations
+
+import contextlib
+import threading
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture
+def python_form(monkeypatch):
+    """A switch: calls made inside ``with`` go through the Python forms."""
+    from griffin_b200 import ops
+
+    @contextlib.contextmanager
+    def only_python():
+        with monkeypatch.context() as m:
+            m.setattr(ops, "_native_call", lambda: False)
+            yield
+    return only_python
+
+
+def _n(*shape, dtype=torch.float32, scale=1.0):
+    return (torch.randn(*shape, device=DEV) * scale).to(dtype)
+
+
+def _step(call, leaves, grads):
+    for t in leaves:
+        t.grad = None
+    outs = call(*leaves)
+    outs = outs if isinstance(outs, tuple) else (outs,)
+    torch.autograd.backward(list(outs), list(grads))
+    return [o.detach() for o in outs] + [t.grad for t in leaves]
+
+
+def _operators(dtype, steps):
+    from griffin_b200 import ops, token_flags
+    torch.manual_seed(0)
+    batch, heads, bw = 2, 2, 64
+    width = heads * bw
+    active = torch.arange(steps, device=DEV)[None] < torch.tensor([[steps], [max(1, steps // 2)]], device=DEV)
+    flags = token_flags(batch, steps, torch.device(DEV), active=active)
+    seq, state = (batch, steps, width), (batch, width)
+    leaf = lambda *s, dt=dtype, scale=1.0: _n(*s, dtype=dt, scale=scale).requires_grad_(True)
+    lam = lambda: torch.logit(torch.rand(width, device=DEV) * 0.09 + 0.9).requires_grad_(True)
+    gates = [leaf(heads, bw, bw, scale=bw ** -0.5), leaf(heads, bw, scale=0.3), leaf(heads, bw, bw, scale=bw ** -0.5), leaf(heads, bw, scale=0.3)]
+    yield (lambda x, r, i, l, h: ops.rglru(x, r, i, l, h, flags), [leaf(*seq), leaf(*seq), leaf(*seq), lam(), leaf(*state, dt=torch.float32)],
+           [_n(*seq, dtype=dtype), _n(*state)])
+    yield (lambda x, *p: ops.rglru_gated(x, *p[:5], p[5], flags, 8.0, p[6]),
+           [leaf(*seq), *gates, lam(), leaf(*state, dt=torch.float32), leaf(*seq)], [_n(*seq, dtype=dtype), _n(*state)])
+    if dtype == torch.float32:
+        yield (ops.linear_scan, [(torch.rand(*seq, device=DEV) * 0.3 + 0.7).requires_grad_(True), leaf(*seq), leaf(*state)], [_n(*seq)])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("steps", [1, 65, 200])
+def test_operators_give_the_same_bits(dtype, steps, python_form):
+    for call, leaves, grads in _operators(dtype, steps):
+        got = [t.clone() for t in _step(call, leaves, grads)]
+        with python_form():
+            want = _step(call, leaves, grads)
+        for a, b in zip(got, want):
+            assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(a, b)
+
+
+def _block(dtype, autocast, merge, heads=2, bw=64):
+    from griffin_b200 import RecurrentBlock
+    torch.manual_seed(1)
+    block = RecurrentBlock(96, heads * bw, gate_blocks=heads, fold_merge=merge).to(DEV)
+    with torch.no_grad():
+        for p in block.parameters():
+            if p.dim() <= 2 and p.numel() <= heads * bw:
+                p.add_(torch.randn_like(p) * 0.1)
+    return block.to(torch.float32 if autocast else dtype)
+
+
+@pytest.mark.parametrize("dtype,autocast", [(torch.float32, False), (torch.bfloat16, False), (torch.bfloat16, True)])
+@pytest.mark.parametrize("merge", [False, True])
+@pytest.mark.parametrize("mask", ["none", "positions", "right", "cache"])
+@pytest.mark.parametrize("steps,bw", [(70, 64), (5, 24)])
+def test_block_agrees_with_its_operators(dtype, autocast, merge, mask, steps, bw, python_form):
+    block = _block(dtype, autocast, merge, bw=bw)
+    batch = 3
+    x = _n(batch, steps, 96, dtype=torch.float32 if autocast else dtype).requires_grad_(True)
+    dy = _n(batch, steps, 96, dtype=dtype)
+    pos = torch.arange(steps, device=DEV).expand(batch, steps) % 7 if mask == "positions" else None
+    active = torch.arange(steps, device=DEV)[None] < torch.tensor([[steps], [2], [1]], device=DEV) if mask == "right" else None
+    with torch.no_grad(), torch.autocast("cuda", torch.bfloat16, enabled=autocast):
+        cache = block(x.detach(), return_cache=True)[1] if mask == "cache" else None
+
+    def run():
+        block.zero_grad(set_to_none=True)
+        x.grad = None
+        with torch.autocast("cuda", torch.bfloat16, enabled=autocast):
+            y, new = block(x, cache, pos, active_mask=active, return_cache=True)
+        y.backward(dy)
+        with torch.no_grad(), torch.autocast("cuda", torch.bfloat16, enabled=autocast):
+            z, new2 = block(x, cache, pos, active_mask=active, return_cache=True)
+        return [y.detach(), new.rnn_state.detach(), new.conv_state, new.segment_position, x.grad, z, new2.rnn_state, new2.conv_state,
+                new2.segment_position] + [p.grad.clone() for p in block.parameters()]
+    got = run()
+    with python_form():
+        want = run()
+    # the same kernels; under autocast linear_out's weight gradient is no longer rounded to bf16 on its way to fp32, and GEMMs of
+    # other layouts may add in another order: one rounding of the type
+    bound = 1e-5 if dtype == torch.float32 else 2.0 ** -7
+    for a, b in zip(got, want):
+        assert a.dtype == b.dtype and a.shape == b.shape
+        if a.is_floating_point():
+            assert (a.double() - b.double()).norm() <= bound * b.double().norm().clamp_min(1e-30)
+        else:
+            assert torch.equal(a, b)
+
+
+def test_backward_twice_needs_the_graph_kept_and_is_not_differentiable():
+    for call, leaves, grads in _operators(torch.float32, 65):
+        outs = call(*leaves)
+        outs = outs if isinstance(outs, tuple) else (outs,)
+        first = torch.autograd.grad(outs, leaves, grads, retain_graph=True)
+        again = torch.autograd.grad(outs, leaves, grads)
+        assert all(torch.equal(a, b) for a, b in zip(first, again))
+        with pytest.raises(RuntimeError, match="second time"):
+            torch.autograd.grad(outs, leaves, grads)
+        outs = call(*leaves)
+        outs = outs if isinstance(outs, tuple) else (outs,)
+        wanted = [g.clone().requires_grad_(True) for g in grads]
+        (dx, *_) = torch.autograd.grad(outs, leaves, wanted, create_graph=True)
+        with pytest.raises(RuntimeError, match="once_differentiable"):
+            dx.sum().backward()
+
+
+def test_saved_tensor_hooks_and_partial_gradients():
+    for call, leaves, grads in _operators(torch.bfloat16, 65):
+        want = [t.clone() for t in _step(call, leaves, grads)]
+        packed = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(1) or t.detach().cpu(), lambda t: t.to(DEV)):
+            got = _step(call, leaves, grads)
+        assert packed and all(torch.equal(a, b) for a, b in zip(got, want))
+        for t in leaves[1:]:
+            t.requires_grad_(False)
+        leaves[0].grad = None
+        torch.autograd.backward(list(call(*leaves)), list(grads))
+        assert torch.equal(leaves[0].grad, want[2])
+
+
+def test_what_is_not_plain_goes_by_the_python_forms():
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from griffin_b200 import ops
+    seen = []
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return func(*args, **(kwargs or {}))
+    a, b, h = torch.rand(2, 70, 64, device=DEV), _n(2, 70, 64), _n(2, 64)
+    want = ops.linear_scan(a, b, h)
+    with Watch():
+        assert torch.equal(ops.linear_scan(a, b, h), want)
+    assert seen
+    # strided views, other types, shapes and devices
+    wide = torch.rand(2, 70, 128, device=DEV)
+    assert torch.equal(ops.linear_scan(wide[..., ::2], b, h), ops.linear_scan(wide[..., ::2].contiguous(), b, h))
+    native = ops._native()
+    assert native.affine(wide[..., ::2], b, h) is None and native.affine(a.double(), b, h) is None
+    assert native.affine(a, b, h[:1]) is None and native.affine(a.cpu(), b, h) is None
+    assert native.scan(a, a, a, h[0], None, None, 8.0) is not None and native.scan(a, a, a.bfloat16(), h[0], None, None, 8.0) is None
+    with pytest.raises(TypeError):
+        ops.linear_scan(a.bfloat16(), b, h)
+    with pytest.raises(ValueError):
+        ops.linear_scan(a, b, h[:1])
+    with torch.autograd.forward_ad.dual_level(), pytest.raises((RuntimeError, NotImplementedError)):
+        ops.linear_scan(torch.autograd.forward_ad.make_dual(a, b), b, h)
+
+
+def test_threads_and_streams_of_their_own():
+    from griffin_b200 import ops
+    cases = []
+    for k in range(3):
+        torch.manual_seed(k)
+        a, b, h, g = torch.rand(2, 300, 96, device=DEV), _n(2, 300, 96), _n(2, 96), _n(2, 300, 96)
+        cases.append([t.requires_grad_(True) for t in (a, b, h)] + [g])
+    wants = [[t.clone() for t in _step(ops.linear_scan, c[:3], [c[3]])] for c in cases]
+    torch.cuda.synchronize()
+    failed = []
+
+    def work(c, want):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(10):
+                got = _step(ops.linear_scan, c[:3], [c[3]])
+                torch.cuda.current_stream().synchronize()
+                if not all(torch.equal(x, y) for x, y in zip(got, want)):
+                    failed.append(1)
+    threads = [threading.Thread(target=work, args=cw) for cw in zip(cases, wants)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
