@@ -617,9 +617,10 @@ def _timed(fn, steps, warmup, d: Dist):
     return d.max_over_ranks(e0.elapsed_time(e1) / steps)
 
 
-# Library kernels per forward+backward of one recurrent block on the TMA-staged conv path: conv forward, scan forward,
-# scan backward, conv backward and its partial-row fold, and two column-sum kernels for each of the three bias gradients.
-BLOCK_LAUNCHES = 11
+# Library kernels per forward+backward of one recurrent block on the TMA-staged conv path: conv forward, layer forward,
+# layer backward and its fold, conv backward and its partial-row fold, and two column-sum kernels for each of the three bias
+# gradients.
+BLOCK_LAUNCHES = 12
 
 
 def run_block(args, d: Dist) -> dict:

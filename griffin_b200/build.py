@@ -21,8 +21,8 @@ SRC_DIR = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(SRC_DIR, "_build")
 LIB_PATH = os.path.join(PKG_DIR, "librglru_b200.so")
 NATIVE_PATH = os.path.join(PKG_DIR, "_native.so")
-SOURCES = ["rglru_scan.cu", "rglru_conv.cu", "rglru_decode.cu", "rglru_gates.cu", "rglru_block.cu", "rglru_api.cu", "rglru_noalloc.cu"]
-HEADERS = ["rglru_device.cuh", "rglru_vec.cuh", "rglru_mma.cuh", "rglru_internal.h", os.path.join("..", "..", "include", "rglru_b200.h")]
+SOURCES = ["rglru_scan.cu", "rglru_conv.cu", "rglru_decode.cu", "rglru_gates.cu", "rglru_block.cu", "rglru_fused.cu", "rglru_api.cu", "rglru_noalloc.cu"]
+HEADERS = ["rglru_device.cuh", "rglru_scan.cuh", "rglru_tc.cuh", "rglru_vec.cuh", "rglru_mma.cuh", "rglru_internal.h", os.path.join("..", "..", "include", "rglru_b200.h")]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",

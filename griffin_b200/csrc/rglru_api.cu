@@ -66,7 +66,8 @@ static EncodeTiledFn encode_fn() {
 
 // 3-D map over a dense [B, T, D] tensor with a [1, rows, cols] box; out-of-range parts
 // of a box read as zero and are dropped on store.
-static bool encode_map(CUtensorMap* map, const void* base, bool bf16, int B, int T, int D, int rows, int cols) {
+static bool encode_map(CUtensorMap* map, const void* base, bool bf16, int B, int T, int D, int rows, int cols,
+                       CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
   const size_t es = bf16 ? 2 : 4;
@@ -76,7 +77,7 @@ static bool encode_map(CUtensorMap* map, const void* base, bool bf16, int B, int
   const cuuint32_t estr[3] = {1u, 1u, 1u};
   const CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                         const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
@@ -125,8 +126,9 @@ static bool encode_map_gates(CUtensorMap* map, const void* base, bool bf16, int 
 // the same handful of buffers step after step (the caching allocator hands the same blocks back), so encoded
 // maps are kept in a small per-thread table: a hit costs a compare and a 128-byte copy instead of a driver call
 // per map (seven to nine of them per backward call).
-// `form` is 0 for the plain 3-D map, MAP_PAIRED, or the group width of an interleaved gate tensor.
-constexpr int MAP_PAIRED = -1;
+// `form` is 0 for the plain 3-D map, MAP_PAIRED, MAP_SWIZZLED (the plain map with the copy engine's 128-byte swizzle), or the
+// group width of an interleaved gate tensor.
+constexpr int MAP_PAIRED = -1, MAP_SWIZZLED = -2;
 struct MapKey {
   const void* base;
   int B, T, D, rows, cols, bf16, form;
@@ -157,6 +159,7 @@ static bool make_map(CUtensorMap* map, const void* base, bool bf16, int B, int T
   }
   auto encode = [&]() {
     if (form == 0) return encode_map(map, base, bf16, B, T, D, rows, cols);
+    if (form == MAP_SWIZZLED) return encode_map(map, base, bf16, B, T, D, rows, cols, CU_TENSOR_MAP_SWIZZLE_128B);
     if (form == MAP_PAIRED) return encode_map_paired(map, base, bf16, B, T, D, rows, cols);
     return encode_map_gates(map, base, bf16, B, T, D, rows, cols, form);
   };
@@ -1042,6 +1045,110 @@ int rglru_layer_bwd(const void* dout, const float* dh_last, const void* x, const
                          weight_dtype, bias_dtype, lambda_dtype, stream);
   if (rc != RGLRU_OK) return rc;
   return rglru_gate_project(du, w, dx, 1, rows, D, head_width, io_dtype, stream);
+}
+
+// The fused layer's workspace holds the chunk-entry states, the weights in the kernels' operand form, Lambda and the biases;
+// its scratch the partial sums of the parameter gradients.
+static int check_fused(int B, int T, int D, int head_width, int io_dtype) {
+  if (io_dtype != RGLRU_BF16) return RGLRU_ERR_BAD_DTYPE;
+  const int rc = check_dims(B, T, D);
+  if (rc != RGLRU_OK) return rc;
+  return fused_head_width(head_width) && D % head_width == 0 && tma_shape_ok(T, D, 2) ? RGLRU_OK : RGLRU_ERR_BAD_SHAPE;
+}
+int rglru_fused_layer_ok(int B, int T, int D, int head_width, int io_dtype) {
+  return check_fused(B, T, D, head_width, io_dtype) == RGLRU_OK ? 1 : 0;
+}
+static size_t fused_states_bytes(int B, int T, int D) {
+  return up256(static_cast<size_t>(B) * ((static_cast<size_t>(T) + SAVE_EVERY - 1) / SAVE_EVERY) * D * sizeof(float));
+}
+static size_t fused_pack_bytes(int D) { return (static_cast<size_t>(D) + 63) / 64 * (128 * 64 * 2); }
+size_t rglru_fused_layer_workspace_bytes(int B, int T, int D) {
+  if (check_dims(B, T, D) != RGLRU_OK) return 0;
+  return fused_states_bytes(B, T, D) + fused_pack_bytes(D) + static_cast<size_t>(3) * D * sizeof(float);
+}
+static size_t fused_dw_bytes(int B, int D, int split) {
+  return static_cast<size_t>(B) * split * ((static_cast<size_t>(D) + 63) / 64) * 128 * 64 * sizeof(float);
+}
+size_t rglru_fused_layer_scratch_bytes(int B, int T, int D, int merged) {
+  if (check_dims(B, T, D) != RGLRU_OK) return 0;
+  return fused_dw_bytes(B, D, fused_split(false, merged != 0, B, T, D)) + static_cast<size_t>(B) * 3 * D * sizeof(float);
+}
+
+int rglru_fused_layer_fwd(const void* x, const void* w_r, const void* b_r, const void* w_i, const void* b_i, const void* lambda,
+                          const void* branch, const float* h0, const uint8_t* tok, void* out, float* h_last, void* ws,
+                          size_t ws_bytes, int B, int T, int D, int head_width, float c, int weight_dtype, int bias_dtype,
+                          int lambda_dtype, int io_dtype, void* stream) {
+  int rc = check_fused(B, T, D, head_width, io_dtype);
+  if (rc != RGLRU_OK) return rc;
+  if (!io_dtype_ok(weight_dtype) || !io_dtype_ok(bias_dtype) || !io_dtype_ok(lambda_dtype)) return RGLRU_ERR_BAD_DTYPE;
+  if (!x || !w_r || !b_r || !w_i || !b_i || !lambda || !out) return RGLRU_ERR_NULL_POINTER;
+  const size_t bs = bias_dtype == RGLRU_BF16 ? 2 : 4, ls = lambda_dtype == RGLRU_BF16 ? 2 : 4;
+  if (!aligned(x, 16) || !aligned(w_r, 16) || !aligned(w_i, 16) || !aligned(branch, 16) || !aligned(out, 16) || !aligned(b_r, bs) ||
+      !aligned(b_i, bs) || !aligned(lambda, ls) || !aligned(h0, 4) || !aligned(h_last, 4) || !aligned(ws, 16))
+    return RGLRU_ERR_MISALIGNED;
+  if (ws && ws_bytes < rglru_fused_layer_workspace_bytes(B, T, D)) return RGLRU_ERR_WORKSPACE;
+  int* status = nullptr;
+  rc = device_setup(&status);
+  if (rc != RGLRU_OK) return rc;
+  FusedFwdArgs a = {};
+  a.w_r = w_r; a.w_i = w_i; a.b_r = b_r; a.b_i = b_i; a.lambda = lambda; a.h0 = h0; a.tok = tok; a.h_last = h_last;
+  if (ws) {
+    a.states = static_cast<float*>(ws);
+    a.pack = static_cast<uint8_t*>(ws) + fused_states_bytes(B, T, D);
+    a.params = reinterpret_cast<float*>(static_cast<uint8_t*>(a.pack) + fused_pack_bytes(D));
+  }
+  a.split = fused_split(true, branch != nullptr, B, T, D);
+  a.B = B; a.T = T; a.D = D; a.bw = head_width; a.c = c; a.status = status;
+  a.f32_w = weight_dtype == RGLRU_F32; a.f32_bias = bias_dtype == RGLRU_F32; a.f32_lambda = lambda_dtype == RGLRU_F32;
+  FusedMaps maps = {};
+  bool ok = make_map(&maps.x, x, true, B, T, D, 64, 64, MAP_SWIZZLED) && make_map(&maps.out, out, true, B, T, D, 64, 64, MAP_SWIZZLED);
+  if (ok && branch) ok = make_map(&maps.g, branch, true, B, T, D, 64, 64, MAP_SWIZZLED);
+  if (!ok) return RGLRU_ERR_UNSUPPORTED;
+  const cudaError_t e = launch_fused_fwd(branch != nullptr, maps, a, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
+}
+
+int rglru_fused_layer_bwd(const void* dout, const float* dh_last, const void* x, const void* branch, const float* h0,
+                          const uint8_t* tok, const void* ws, size_t ws_bytes, void* dx, void* dbranch, void* dw_r, void* db_r,
+                          void* dw_i, void* db_i, void* dlambda, float* dh0, void* scratch, size_t scratch_bytes, int B, int T,
+                          int D, int head_width, float c, int weight_dtype, int bias_dtype, int lambda_dtype, int io_dtype,
+                          void* stream) {
+  int rc = check_fused(B, T, D, head_width, io_dtype);
+  if (rc != RGLRU_OK) return rc;
+  if (!io_dtype_ok(weight_dtype) || !io_dtype_ok(bias_dtype) || !io_dtype_ok(lambda_dtype)) return RGLRU_ERR_BAD_DTYPE;
+  if (!dout || !x || !ws || !dx || (branch && !dbranch) || !dw_r || !db_r || !dw_i || !db_i || !dlambda) return RGLRU_ERR_NULL_POINTER;
+  const size_t bs = bias_dtype == RGLRU_BF16 ? 2 : 4, ls = lambda_dtype == RGLRU_BF16 ? 2 : 4;
+  if (!aligned(dout, 16) || !aligned(x, 16) || !aligned(branch, 16) || !aligned(dx, 16) || !aligned(dbranch, 16) || !aligned(dw_r, 16) ||
+      !aligned(dw_i, 16) || !aligned(scratch, 16) || !aligned(db_r, bs) || !aligned(db_i, bs) || !aligned(dlambda, ls) ||
+      !aligned(h0, 4) || !aligned(dh_last, 4) || !aligned(dh0, 4) || !aligned(ws, 16))
+    return RGLRU_ERR_MISALIGNED;
+  if (ws_bytes < rglru_fused_layer_workspace_bytes(B, T, D)) return RGLRU_ERR_WORKSPACE;
+  int* status = nullptr;
+  rc = device_setup(&status);
+  if (rc != RGLRU_OK) return rc;
+  FusedBwdArgs a = {};
+  a.split = fused_split(false, branch != nullptr, B, T, D);
+  const size_t sum_bytes = static_cast<size_t>(B) * 3 * D * sizeof(float);
+  if (scratch_bytes < fused_dw_bytes(B, D, a.split) + sum_bytes) a.split = 1;     // (sized when the device could not be asked)
+  const size_t dw_bytes = fused_dw_bytes(B, D, a.split);
+  if (!scratch || scratch_bytes < dw_bytes + sum_bytes) return RGLRU_ERR_WORKSPACE;
+  a.h0 = h0; a.dh_last = dh_last; a.tok = tok;
+  a.states = static_cast<const float*>(ws);
+  a.pack = static_cast<const uint8_t*>(ws) + fused_states_bytes(B, T, D);
+  a.params = reinterpret_cast<const float*>(static_cast<const uint8_t*>(a.pack) + fused_pack_bytes(D));
+  a.dw_part = static_cast<float*>(scratch);
+  a.sum_part = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + dw_bytes);
+  a.dh0 = dh0; a.dw_r = dw_r; a.dw_i = dw_i; a.db_r = db_r; a.db_i = db_i; a.dlambda = dlambda;
+  a.B = B; a.T = T; a.D = D; a.bw = head_width; a.c = c; a.status = status;
+  a.f32_w = weight_dtype == RGLRU_F32; a.f32_bias = bias_dtype == RGLRU_F32; a.f32_lambda = lambda_dtype == RGLRU_F32;
+  FusedMaps maps = {};
+  bool ok = make_map(&maps.dy, dout, true, B, T, D, 64, 64, MAP_SWIZZLED) && make_map(&maps.x, x, true, B, T, D, 64, 64, MAP_SWIZZLED) &&
+            make_map(&maps.out, dx, true, B, T, D, 64, 64, MAP_SWIZZLED);
+  if (ok && branch)
+    ok = make_map(&maps.g, branch, true, B, T, D, 64, 64, MAP_SWIZZLED) && make_map(&maps.dg, dbranch, true, B, T, D, 64, 64, MAP_SWIZZLED);
+  if (!ok) return RGLRU_ERR_UNSUPPORTED;
+  const cudaError_t e = launch_fused_bwd(branch != nullptr, maps, a, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
 }
 
 int rglru_token_plan(const int64_t* seg_pos, const int64_t* prev_pos, const uint8_t* active, const uint8_t* reset,

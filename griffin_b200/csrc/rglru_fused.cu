@@ -1,0 +1,843 @@
+// The bf16 layer with its gate projections inside the scan kernels, for gate heads of 16, 32 or 64 channels: a channel tile
+// of the scan (64 channels) then holds whole heads, so everything the projections contract is in the CTA that scans.
+//
+// Per 64-step chunk, beside the scan (rglru_scan.cu has its decomposition, and what its template switches mean):
+//   forward   u[64 x 128] = x W^T by tcgen05.mma, rounded to bf16 into the shared tiles the scan reads its gates from;
+//   backward  the same again (nothing of u is kept), then from the chunk's du tiles
+//             dx[64 x 64] += du W, and dW[128 x 64] += du^T x, accumulated in tensor memory over the CTA's whole sequence.
+// Neither u nor du ever leaves the SM: a forward reads x and writes y, a backward reads dy and x and writes dx, where the
+// kernels of rglru_gates.cu and rglru_scan.cu move 3 and 6 more elements per element (u out and in twice, du out and in).
+// Two warps take the accumulators out of tensor memory (and issue the multiplications): in the forward ahead of the eight
+// scan warps by up to two chunks, in the backward u two chunks ahead and dx behind.  One more warp issues the bulk copies.
+// The scan warps take registers over from those (setmaxnreg): held at the launch's share they spill 100 to 300 bytes.
+// B8 T2048 D1024, 16 heads of 64, us: 52 forward, 73 backward and 4 for the fold of the weight gradient, where gate kernels
+// around the scan took 202 in all; T16384 at B1 (clusters of eight) 108 + 211 warm and 240 in a loop, where 282; B16 with the
+// branch product 88 + 183 + 9, where batched GEMMs around the scan took some 350.  Bound by the serial chain of a chunk: u out of
+// tensor memory, scan, du into it, with one CTA's eight scan warps on an SM.
+// All tiles are staged with the copy engine's 128-byte swizzle, which is the operand layout of the tensor cores and leaves
+// the scan's accesses as free of bank conflicts as dense rows.
+//
+// An operand tile of 64 time rows is given to the tensor cores as 128 rows (the unit's full height; the second half is
+// whatever follows in shared memory, and lands in accumulator rows nobody reads).  Heads of 16 and 32 channels are contracted
+// head by head, so that nothing but a head's own channels enters its sums.
+//
+// Reference: griffin/griffin.py:129-154, 190-286.
+
+#include "rglru_scan.cuh"
+#include "rglru_tc.cuh"
+
+namespace rglru {
+
+namespace {
+
+template <int N>
+__device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+using BF = __nv_bfloat16;
+constexpr int FT = 64 * 128;                 // bytes of a tile: 64 rows of 64 channels
+constexpr int FCH = 64, FLANES = 16, FTS = 4, FNCV = FCH / CV, FCOMP = FLANES * FNCV;
+constexpr int FTHREADS = FCOMP + 128;        // scan warps; a warpgroup of two tensor-memory warps, the copy warp, and one idle
+// Registers a thread of the scan warps and of the others: their sum over the block stays below what it is launched with.
+constexpr int FWD_SCAN = 88, FWD_AUX = 56, BWD_SCAN = 200, BWD_AUX = 96;
+constexpr int W_BYTES = 2 * FT;              // both gates' weights of the tile, rows r 0 .. 63, i 0 .. 63
+constexpr int BAR_TC = 4;                    // named barriers: the two tensor-memory warps; those and the scan warps (2)
+
+__device__ __forceinline__ float param(const void* p, int i, bool f32) {
+  return f32 ? static_cast<const float*>(p)[i] : __bfloat162float(static_cast<const BF*>(p)[i]);
+}
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// The weights of a tile's heads as one [128 x 64] operand (gate g, channel c in row 64 g + c; its head's channels in the columns
+// they have in the tile, zeros elsewhere), by the scan warps.  `pack`: where the operand is kept for the backward, or nullptr.
+__device__ __forceinline__ void load_weights(uint8_t* sw, uint4* pack, const void* w_r, const void* w_i, bool f32, int d0, int D, int bw, int tid) {
+  for (int idx = tid; idx < 1024; idx += FCOMP) {
+    const int row = idx >> 3, piece = idx & 7, c = row & 63, k = piece * 8;
+    const void* w = row < 64 ? w_r : w_i;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (d0 + c < D && k / bw == c / bw) {
+      const size_t at = static_cast<size_t>(d0 + c) * bw + k % bw;
+      if (f32) {
+        const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(w) + at);
+        const float4 b = *reinterpret_cast<const float4*>(static_cast<const float*>(w) + at + 4);
+        v = make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+      } else {
+        v = *reinterpret_cast<const uint4*>(static_cast<const BF*>(w) + at);
+      }
+    }
+    *reinterpret_cast<uint4*>(sw + row * 128 + ((piece ^ (row & 7)) << 4)) = v;
+    if (pack) pack[idx] = v;
+  }
+}
+__device__ __forceinline__ void load_packed_weights(uint8_t* sw, const uint4* pack, int tid) {
+#pragma unroll
+  for (int i = 0; i < 1024 / FCOMP; ++i) {
+    const int idx = tid + i * FCOMP, row = idx >> 3, piece = idx & 7;
+    *reinterpret_cast<uint4*>(sw + row * 128 + ((piece ^ (row & 7)) << 4)) = pack[idx];
+  }
+}
+
+struct ThreadParams {
+  float2 K[2];
+  GateBias gb;
+};
+// `keep`: [3 D] fp32 for the backward (Lambda, then the two biases), or nullptr.
+__device__ __forceinline__ ThreadParams load_params(const void* lambda, const void* b_r, const void* b_i, bool f32_lambda, bool f32_bias,
+                                                    int d, int D, float c, float* keep) {
+  float k[4], r[4], i[4];
+  const float sc = gate_bias_scale<true>();
+#pragma unroll
+  for (int ch = 0; ch < 4; ++ch) {
+    const bool ok = d + ch < D;
+    const float lam = ok ? param(lambda, d + ch, f32_lambda) : 0.0f;
+    r[ch] = ok ? param(b_r, d + ch, f32_bias) : 0.0f;
+    i[ch] = ok ? param(b_i, d + ch, f32_bias) : 0.0f;
+    if (keep && ok) { keep[d + ch] = lam; keep[D + d + ch] = r[ch]; keep[2 * D + d + ch] = i[ch]; }
+    k[ch] = ok ? decay_rate(lam, c) : 0.0f;
+    r[ch] *= sc;
+    i[ch] *= sc;
+  }
+  ThreadParams t;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    t.K[h] = make_float2(k[2 * h], k[2 * h + 1]);
+    t.gb.r[h] = make_float2(r[2 * h], r[2 * h + 1]);
+    t.gb.i[h] = make_float2(i[2 * h], i[2 * h + 1]);
+  }
+  return t;
+}
+
+// u = x W^T of one chunk into 128 accumulator columns (64 g + c), by one thread.
+__device__ __forceinline__ void mma_gates(uint32_t acc, uint32_t x, uint32_t w, int bw) {
+  if (bw == 64) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      tc_mma(acc, tc_desc(x + 32 * k), tc_desc(w + 32 * k), tc_idesc(128, 128, false, false), k > 0);
+    return;
+  }
+  const uint32_t idesc = bw == 32 ? tc_idesc(128, 32, false, false) : tc_idesc(128, 16, false, false);
+  for (int c = 0; c < 64; c += bw)
+    for (int g = 0; g < 2; ++g)
+      for (int k = c; k < c + bw; k += 16)
+        tc_mma(acc + 64 * g + c, tc_desc(x + 2 * k), tc_desc(w + (64 * g + c) * 128 + 2 * k), idesc, k > c);
+}
+// The gates' share of dx of one chunk, du W, into 64 accumulator columns.
+__device__ __forceinline__ void mma_dx(uint32_t acc, uint32_t du, uint32_t w, int bw) {
+  const uint32_t idesc = bw == 64 ? tc_idesc(128, 64, false, true) : (bw == 32 ? tc_idesc(128, 32, false, true) : tc_idesc(128, 16, false, true));
+  for (int c = 0; c < 64; c += bw)
+    for (int g = 0; g < 2; ++g)
+      for (int k = c; k < c + bw; k += 16)
+        tc_mma(acc + c, tc_desc(du + g * FT + 2 * k), tc_desc(w + (64 * g + k) * 128 + 2 * c), idesc, g > 0 || k > c);
+}
+// dW += du^T x over one chunk, 128 accumulator rows (64 g + c) of 64 columns.
+__device__ __forceinline__ void mma_dw(uint32_t acc, uint32_t du, uint32_t x, bool first) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    tc_mma(acc, tc_desc(du + 2048 * k, FT), tc_desc(x + 2048 * k), tc_idesc(128, 64, true, true), !first || k > 0);
+}
+// A thread's row of u from tensor memory into the two gate tiles.
+__device__ __forceinline__ void store_gates(uint8_t* u, uint32_t acc, int row) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float v[32];
+    tc_load32(acc + 32 * q, v);
+    uint8_t* dst = u + (q >> 1) * FT + row * 128;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      *reinterpret_cast<uint4*>(dst + ((((q & 1) * 4 + j) ^ (row & 7)) << 4)) =
+          make_uint4(pack_bf16(v[8 * j], v[8 * j + 1]), pack_bf16(v[8 * j + 2], v[8 * j + 3]), pack_bf16(v[8 * j + 4], v[8 * j + 5]),
+                     pack_bf16(v[8 * j + 6], v[8 * j + 7]));
+  }
+}
+
+// ---------------------------------------------------------------- forward
+template <bool MERGE, bool SPLIT>
+struct FusedFwdSmem {
+  static constexpr int NSTAGE = MERGE ? 3 : 4;
+  static constexpr int OFF_G = FT;
+  static constexpr int STAGE = MERGE ? 2 * FT : FT;
+  static constexpr int OFF_U = NSTAGE * STAGE;               // two slots of both gates' tiles
+  static constexpr int OFF_W = OFF_U + 4 * FT;
+  static constexpr int OFF_AGG = OFF_W + W_BYTES;
+  static constexpr int OFF_EIN = OFF_AGG + ChainSmem<FLANES, FCH>::AGG;
+  static constexpr int OFF_BAR = OFF_EIN + ChainSmem<FLANES, FCH>::EIN;   // full, ready [NSTAGE], gates [2], tensor cores, flag, address
+  static constexpr int OFF_SPLIT = OFF_BAR + (2 * NSTAGE + 3) * 8 + 16;
+  static constexpr int BYTES = OFF_SPLIT + (SPLIT ? static_cast<int>(sizeof(SplitSmem<FCH>)) : 0) + 1024;   // (to align the tiles)
+};
+
+template <bool MERGE, bool SPLIT>
+__global__ void __launch_bounds__(FTHREADS, 2) fused_fwd_kernel(const __grid_constant__ FusedMaps maps, const FusedFwdArgs p) {
+  using SM = FusedFwdSmem<MERGE, SPLIT>;
+  constexpr int NSTAGE = SM::NSTAGE, TS = FTS, LANES = FLANES, CH = FCH;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+  float2* agg = reinterpret_cast<float2*>(smem + SM::OFF_AGG);
+  float* ein = reinterpret_cast<float*>(smem + SM::OFF_EIN);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + SM::OFF_BAR);
+  uint64_t* ready = full + NSTAGE;
+  uint64_t* gates = ready + NSTAGE;
+  uint64_t* done = gates + 2;
+  volatile int* dead = reinterpret_cast<volatile int*>(done + 1);
+  uint32_t* tmem_at = reinterpret_cast<uint32_t*>(done + 1) + 1;
+
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int b = blockIdx.y, d0 = blockIdx.x * CH;
+  const int nchunks = (p.T + 63) / 64;
+  SplitChain<CH> split{};
+  if constexpr (SPLIT) split.init(reinterpret_cast<SplitSmem<CH>*>(smem + SM::OFF_SPLIT));
+  const int rank = SPLIT ? static_cast<int>(split.rank) : 0, nranks = SPLIT ? static_cast<int>(split.size) : 1;
+  const int rounds = SPLIT ? (nchunks + nranks - 1) / nranks : nchunks;
+  const int mine = SPLIT ? (nchunks - rank + nranks - 1) / nranks : nchunks;   // chunks this CTA takes, at least one
+
+  auto issue = [&](int it) {
+    const int sidx = it % NSTAGE, k = it * nranks + rank;
+    mbar_expect_tx(&full[sidx], SM::STAGE);
+    tma_load_3d(smem + sidx * SM::STAGE, &maps.x, d0, k * 64, b, &full[sidx]);
+    if (MERGE) tma_load_3d(smem + sidx * SM::STAGE + SM::OFF_G, &maps.g, d0, k * 64, b, &full[sidx]);
+  };
+  if (tid == FCOMP + 64) {
+    *dead = 0;
+    for (int s = 0; s < NSTAGE; ++s) { mbar_init(&full[s], 1); mbar_init(&ready[s], FCOMP / 32); }
+    mbar_init(&gates[0], 2); mbar_init(&gates[1], 2); mbar_init(done, 1);
+    if constexpr (SPLIT) { mbar_init(&split.sm->bar[0], 1); mbar_init(&split.sm->bar[1], 1); }
+    mbar_fence_init();
+    prefetch_map(&maps.x); prefetch_map(&maps.out);
+    if (MERGE) prefetch_map(&maps.g);
+    tma_prefetch_3d(&maps.x, d0, rank * 64, b);
+    if (MERGE) tma_prefetch_3d(&maps.g, d0, rank * 64, b);
+  }
+  if (warp == 8) tc_alloc<128>(tmem_at);
+  tc_fence_before();
+  if constexpr (SPLIT) cluster_sync_all();   // the barriers of every CTA are there before anybody sends
+  else __syncthreads();
+  tc_fence_after();
+  // Only now may the next kernel of the stream come in: were it to take tensor memory while it waits for this one, a CTA of
+  // this one could be left without.
+  pdl_launch_dependents();
+  pdl_wait();
+
+  if (warp >= 8) {
+  regs_down<FWD_AUX>();
+  if (warp == 10) {            // ---- copies: loads run NSTAGE - 1 chunks ahead (see rglru_fwd_body)
+    if (tid == FCOMP + 64) {
+      issue(0);
+      mbar_wait_or_flag(&full[0], 0, dead, p.status, DEV_TIMEOUT_LOAD);
+      for (int it = 1; it < NSTAGE && it < mine; ++it) issue(it);
+      for (int it = 0; it < mine; ++it) {
+        const int sidx = it % NSTAGE, k = it * nranks + rank;
+        mbar_wait_or_flag(&ready[sidx], (it / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
+        tma_store_3d(&maps.out, smem + sidx * SM::STAGE, d0, k * 64, b);
+        tma_commit();
+        if (it + NSTAGE < mine) {
+          tma_wait_read<0>();
+          issue(it + NSTAGE);
+        }
+      }
+      tma_wait_all<0>();
+    }
+    if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }
+    return;
+  }
+  if (warp < 10) {             // ---- gates
+    const uint32_t acc = *tmem_at, mine_acc = acc + (static_cast<uint32_t>(warp - 8) << 21);   // this warp's 32 rows
+    const int row = tid - FCOMP;
+    bar_all(FCOMP + 64);       // the weights are there
+    for (int it = 0; it < mine; ++it) {
+      const int s = it % NSTAGE, slot = it & 1;
+      if (it >= 2) mbar_wait_or_flag(&ready[(it - 2) % NSTAGE], ((it - 2) / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
+      mbar_wait_or_flag(&full[s], (it / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+      __syncwarp();
+      if (row == 0) {
+        tc_fence_after();
+        mma_gates(acc, smem_u32(smem + s * SM::STAGE), smem_u32(smem + SM::OFF_W), p.bw);
+        tc_commit(done);
+      }
+      __syncwarp();
+      mbar_wait_or_flag(done, it & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+      __syncwarp();
+      tc_fence_after();
+      store_gates(smem + SM::OFF_U + slot * 2 * FT, mine_acc, row);
+      tc_fence_before();
+      __syncwarp();
+      if ((tid & 31) == 0) mbar_arrive(&gates[slot]);
+      __syncwarp();
+      asm volatile("bar.sync %0, 64;" ::"n"(BAR_TC) : "memory");       // both are done with the accumulators
+    }
+    __syncwarp();
+    tc_fence_after();
+    if (warp == 8) tc_free<128>(acc);
+    if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }
+    return;
+  }
+
+  if constexpr (SPLIT) cluster_sync_all();      // the idle warp
+  return;
+  }
+  regs_up<FWD_SCAN>();
+  // ---- scan
+  const int lane_t = tid / FNCV, vec = tid % FNCV;
+  const bool keeps = p.pack && b == 0 && rank == 0;
+  load_weights(smem + SM::OFF_W, keeps ? static_cast<uint4*>(p.pack) + blockIdx.x * 1024 : nullptr, p.w_r, p.w_i, p.f32_w, d0, p.D, p.bw, tid);
+  fence_async_smem();
+  bar_all(FCOMP + 64);
+  const ThreadParams tp = load_params(p.lambda, p.b_r, p.b_i, p.f32_lambda, p.f32_bias, d0 + vec * CV, p.D, p.c,
+                                      keeps && lane_t == 0 ? p.params : nullptr);
+  const float2(&K)[2] = tp.K;
+  const bool poly = bar_compute_and(FCOMP, fmaxf(fmaxf(K[0].x, K[0].y), fmaxf(K[1].x, K[1].y)) <= -POLY_RANGE);
+  const int nsave = (p.T + SAVE_EVERY - 1) / SAVE_EVERY;
+  const bool chain_thread = tid < CH;
+  const int dch = d0 + tid;
+  float carry = 0.0f;
+  if (chain_thread && dch < p.D && p.h0) carry = p.h0[static_cast<size_t>(b) * p.D + dch];
+  ConvTaps ct;
+  const int off0 = lane_t * TS * 128 + (((vec >> 1) ^ ((lane_t & 1) << 2)) << 4) + (vec & 1) * 8;
+
+  for (int it = 0; it < rounds; ++it) {
+    const int k = it * nranks + rank;
+    const bool idle = SPLIT && it >= mine;     // last round: no chunk left for this CTA, it only takes part in the exchange
+    if constexpr (SPLIT) { if (tid == 0) split.arm(it); }
+    uint8_t* tiles = smem + (it % NSTAGE) * SM::STAGE;
+    const int t0 = k * 64;
+    uint32_t fl[1];
+    const bool masked = p.tok != nullptr || t0 + 64 > p.T;
+    if (masked) load_flags<TS>(p.tok, b, p.T, t0 + lane_t * TS, fl);
+
+    float2 P[TS][2], S[TS][2];
+    if (!idle) {
+      mbar_wait_or_flag(&full[it % NSTAGE], (it / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+      mbar_wait_or_flag(&gates[it & 1], (it >> 1) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+      const uint8_t* tr = smem + SM::OFF_U + (it & 1) * 2 * FT;
+      const uint8_t* ti = tr + FT;
+      if (masked && any_flag(fl)) {
+        if (poly) fwd_local<BF, TS, CH, true, true, false, true, 128, true>(tiles, tr, ti, off0, K, fl, ct, nullptr, tp.gb, P, S);
+        else fwd_local<BF, TS, CH, true, false, false, true, 128, true>(tiles, tr, ti, off0, K, fl, ct, nullptr, tp.gb, P, S);
+      } else {
+        if (poly) fwd_local<BF, TS, CH, false, true, false, true, 128, true>(tiles, tr, ti, off0, K, fl, ct, nullptr, tp.gb, P, S);
+        else fwd_local<BF, TS, CH, false, false, false, true, 128, true>(tiles, tr, ti, off0, K, fl, ct, nullptr, tp.gb, P, S);
+      }
+      float4* dst = reinterpret_cast<float4*>(agg + lane_t * CH + vec * CV);
+      dst[0] = make_float4(P[TS - 1][0].x, S[TS - 1][0].x, P[TS - 1][0].y, S[TS - 1][0].y);
+      dst[1] = make_float4(P[TS - 1][1].x, S[TS - 1][1].x, P[TS - 1][1].y, S[TS - 1][1].y);
+    }
+    bar_compute(FCOMP);
+
+    if (chain_thread) {
+      float2 ag[LANES];
+#pragma unroll
+      for (int j = 0; j < LANES; ++j) ag[j] = idle ? make_float2(1.0f, 0.0f) : agg[j * CH + tid];
+      if constexpr (!SPLIT) {
+        if (p.states && dch < p.D) p.states[(static_cast<size_t>(b) * nsave + k) * p.D + dch] = carry;
+        float e = carry;
+#pragma unroll
+        for (int j = 0; j < LANES; ++j) {
+          ein[j * CH + tid] = e;
+          e = fmaf(ag[j].x, e, ag[j].y);
+        }
+        carry = e;
+      } else {
+        float pp[LANES], sp[LANES], pa = 1.0f, sa = 0.0f, unused = 1.0f;
+#pragma unroll
+        for (int j = 0; j < LANES; ++j) {
+          pp[j] = pa;
+          sp[j] = sa;
+          sa = fmaf(ag[j].x, sa, ag[j].y);
+          pa *= ag[j].x;
+        }
+        split.send(it, tid, make_float2(pa, sa), 0, 1);
+        const float enter = split.receive(it, tid, carry, unused, dead, p.status);
+        if (!idle) {
+          if (p.states && dch < p.D) p.states[(static_cast<size_t>(b) * nsave + k) * p.D + dch] = enter;
+#pragma unroll
+          for (int j = 0; j < LANES; ++j) ein[j * CH + tid] = fmaf(pp[j], enter, sp[j]);
+        }
+      }
+    }
+    bar_compute(FCOMP);
+    if (idle) break;
+
+    const float4 e4 = *reinterpret_cast<const float4*>(ein + lane_t * CH + vec * CV);
+    const float2 e[2] = {make_float2(e4.x, e4.y), make_float2(e4.z, e4.w)};
+#pragma unroll
+    for (int st = 0; st < TS; ++st) {
+      const int off = step_at<128, true>(off0, st);
+      float2 yv[2];
+#pragma unroll
+      for (int cp = 0; cp < 2; ++cp) yv[cp] = fma2(P[st][cp], e[cp], S[st][cp]);
+      if constexpr (SPLIT) {     // the final state is the last step's output to the bit, not the folded carry
+        if (p.h_last && t0 + lane_t * TS + st == p.T - 1) {
+          float* hl = p.h_last + static_cast<size_t>(b) * p.D + d0 + vec * CV;
+          const float v[4] = {yv[0].x, yv[0].y, yv[1].x, yv[1].y};
+#pragma unroll
+          for (int ch = 0; ch < 4; ++ch)
+            if (d0 + vec * CV + ch < p.D) hl[ch] = v[ch];
+        }
+      }
+      if (MERGE) {
+        float2 gv[2];
+        Pack<BF>::unpack2(Pack<BF>::load(tiles + SM::OFF_G + off), gv);
+#pragma unroll
+        for (int cp = 0; cp < 2; ++cp) yv[cp] = mul2(yv[cp], mul2(gv[cp], gelu_sigmoid2<true>(gv[cp])));
+      }
+      Pack<BF>::store2(tiles + off, yv);     // over x in place
+    }
+    fence_async_smem();
+    __syncwarp();
+    if ((tid & 31) == 0) mbar_arrive(&ready[it % NSTAGE]);
+  }
+  if constexpr (SPLIT) {
+    __syncwarp();
+    cluster_sync_all();        // no CTA leaves while another may still send to it
+  } else {
+    if (chain_thread && dch < p.D && p.h_last) p.h_last[static_cast<size_t>(b) * p.D + dch] = carry;
+  }
+}
+
+// ---------------------------------------------------------------- backward
+template <bool MERGE, bool SPLIT>
+struct FusedBwdSmem {
+  static constexpr int NSTAGE = MERGE ? 4 : 5;
+  static constexpr int OFF_X = FT, OFF_G = 2 * FT;          // behind the dy tile, which dx takes over
+  static constexpr int STAGE = MERGE ? 3 * FT : 2 * FT;
+  static constexpr int OFF_U = NSTAGE * STAGE;
+  static constexpr int OFF_W = OFF_U + 4 * FT;
+  static constexpr int PLANE = FLANES * FCH * 4;            // (see BwdSmem)
+  static constexpr int OFF_AGGP = OFF_W + W_BYTES;
+  static constexpr int OFF_AGGS = OFF_AGGP + PLANE;
+  static constexpr int OFF_AGGC = OFF_AGGS + PLANE;
+  static constexpr int OFF_EINF = OFF_AGGC + PLANE;
+  static constexpr int OFF_EINR = OFF_EINF + PLANE;
+  static constexpr int OFF_BAR = OFF_EINR + PLANE;          // full, ready, out [NSTAGE], gates [2], tensor cores [2], flag, address
+  static constexpr int OFF_SPLIT = OFF_BAR + (3 * NSTAGE + 4) * 8 + 16;
+  static constexpr int BYTES = OFF_SPLIT + (SPLIT ? static_cast<int>(sizeof(SplitSmem<FCH>)) : 0) + 1024;
+};
+// Accumulator columns: u, dx, dW.
+constexpr int ACC_DX = 128, ACC_DW = 192, ACC_COLS = 256;
+
+template <bool MERGE, bool SPLIT>
+__global__ void __launch_bounds__(FTHREADS, 1) fused_bwd_kernel(const __grid_constant__ FusedMaps maps, const FusedBwdArgs p) {
+  using SM = FusedBwdSmem<MERGE, SPLIT>;
+  constexpr int NSTAGE = SM::NSTAGE, TS = FTS, LANES = FLANES, CH = FCH;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+  float* aggP = reinterpret_cast<float*>(smem + SM::OFF_AGGP);
+  float* aggS = reinterpret_cast<float*>(smem + SM::OFF_AGGS);
+  float* aggC = reinterpret_cast<float*>(smem + SM::OFF_AGGC);
+  float* einF = reinterpret_cast<float*>(smem + SM::OFF_EINF);
+  float* einR = reinterpret_cast<float*>(smem + SM::OFF_EINR);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + SM::OFF_BAR);
+  uint64_t* ready = full + NSTAGE;
+  uint64_t* outs = ready + NSTAGE;
+  uint64_t* gates = outs + NSTAGE;
+  uint64_t* done = gates + 2;                 // [0] u, [1] dx and dW of a chunk
+  volatile int* dead = reinterpret_cast<volatile int*>(done + 2);
+  uint32_t* tmem_at = reinterpret_cast<uint32_t*>(done + 2) + 1;
+
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int b = blockIdx.y, d0 = blockIdx.x * CH;
+  const int nchunks = (p.T + 63) / 64;
+  SplitChain<CH> split{};
+  if constexpr (SPLIT) split.init(reinterpret_cast<SplitSmem<CH>*>(smem + SM::OFF_SPLIT));
+  const int rank = SPLIT ? static_cast<int>(split.rank) : 0, nranks = SPLIT ? static_cast<int>(split.size) : 1;
+  const int rounds = SPLIT ? (nchunks + nranks - 1) / nranks : nchunks;
+  const int mine = SPLIT ? (nchunks - rank + nranks - 1) / nranks : nchunks;
+
+  auto issue = [&](int q) {    // this CTA's q-th chunk in processing order, which runs from the end of the sequence
+    const int k = nchunks - 1 - (q * nranks + rank), sidx = q % NSTAGE;
+    uint8_t* st = smem + sidx * SM::STAGE;
+    mbar_expect_tx(&full[sidx], SM::STAGE);
+    tma_load_3d(st + SM::OFF_X, &maps.x, d0, k * 64, b, &full[sidx]);
+    tma_load_3d(st, &maps.dy, d0, k * 64, b, &full[sidx]);
+    if (MERGE) tma_load_3d(st + SM::OFF_G, &maps.g, d0, k * 64, b, &full[sidx]);
+  };
+  if (tid == FCOMP + 64) {
+    *dead = 0;
+    for (int s = 0; s < NSTAGE; ++s) { mbar_init(&full[s], 1); mbar_init(&ready[s], FCOMP / 32); mbar_init(&outs[s], 2); }
+    mbar_init(&gates[0], 2); mbar_init(&gates[1], 2); mbar_init(&done[0], 1); mbar_init(&done[1], 1);
+    if constexpr (SPLIT) { mbar_init(&split.sm->bar[0], 1); mbar_init(&split.sm->bar[1], 1); }
+    mbar_fence_init();
+    prefetch_map(&maps.x); prefetch_map(&maps.dy); prefetch_map(&maps.out);
+    if (MERGE) { prefetch_map(&maps.g); prefetch_map(&maps.dg); }
+    const int kl = nchunks - 1 - rank;
+    tma_prefetch_3d(&maps.x, d0, kl * 64, b);
+    tma_prefetch_3d(&maps.dy, d0, kl * 64, b);
+    if (MERGE) tma_prefetch_3d(&maps.g, d0, kl * 64, b);
+  }
+  if (warp == 0) tc_alloc<ACC_COLS>(tmem_at);
+  tc_fence_before();
+  if constexpr (SPLIT) cluster_sync_all();
+  else __syncthreads();
+  tc_fence_after();
+  pdl_launch_dependents();     // (see the forward)
+  pdl_wait();
+  const uint32_t acc = *tmem_at;
+
+  if (warp >= 8) {
+  regs_down<BWD_AUX>();
+  if (warp == 10) {            // ---- copies
+    if (tid == FCOMP + 64) {
+      issue(0);
+      mbar_wait_or_flag(&full[0], 0, dead, p.status, DEV_TIMEOUT_LOAD);
+      for (int q = 1; q < NSTAGE && q < mine; ++q) issue(q);
+      for (int q = 0; q < mine; ++q) {
+        const int sidx = q % NSTAGE, k = nchunks - 1 - (q * nranks + rank);
+        uint8_t* st = smem + sidx * SM::STAGE;
+        mbar_wait_or_flag(&outs[sidx], (q / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
+        tma_store_3d(&maps.out, st, d0, k * 64, b);
+        if (MERGE) tma_store_3d(&maps.dg, st + SM::OFF_G, d0, k * 64, b);
+        tma_commit();
+        if (q + NSTAGE < mine) {
+          tma_wait_read<0>();
+          issue(q + NSTAGE);
+        }
+      }
+      tma_wait_all<0>();
+    }
+    if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }
+    return;
+  }
+  if (warp < 10) {             // ---- gates ahead of the scan, input and weight gradients behind it
+    const uint32_t rows = static_cast<uint32_t>(warp - 8) << 21;      // this warp's 32 accumulator rows
+    const int row = tid - FCOMP;
+    const uint32_t sw = smem_u32(smem + SM::OFF_W);
+    bar_all(FCOMP + 64);       // the weights are there
+    auto make_gates = [&](int q) {
+      const int s = q % NSTAGE, slot = q & 1;
+      mbar_wait_or_flag(&full[s], (q / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+      __syncwarp();
+      if (row == 0) {
+        tc_fence_after();
+        mma_gates(acc, smem_u32(smem + s * SM::STAGE + SM::OFF_X), sw, p.bw);
+        tc_commit(&done[0]);
+      }
+      __syncwarp();
+      mbar_wait_or_flag(&done[0], q & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+      __syncwarp();
+      tc_fence_after();
+      store_gates(smem + SM::OFF_U + slot * 2 * FT, acc + rows, row);
+      tc_fence_before();
+      __syncwarp();
+      if ((tid & 31) == 0) mbar_arrive(&gates[slot]);
+      __syncwarp();
+      asm volatile("bar.sync %0, 64;" ::"n"(BAR_TC) : "memory");       // both are done with the accumulators
+    };
+    make_gates(0);
+    if (mine > 1) make_gates(1);
+    for (int q = 0; q < mine; ++q) {
+      const int s = q % NSTAGE;
+      uint8_t* st = smem + s * SM::STAGE;
+      mbar_wait_or_flag(&ready[s], (q / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
+      __syncwarp();
+      if (row == 0) {
+        const uint32_t du = smem_u32(smem + SM::OFF_U + (q & 1) * 2 * FT);
+        tc_fence_after();
+        mma_dx(acc + ACC_DX, du, sw, p.bw);
+        mma_dw(acc + ACC_DW, du, smem_u32(st + SM::OFF_X), q == 0);
+        tc_commit(&done[1]);
+      }
+      __syncwarp();
+      mbar_wait_or_flag(&done[1], q & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+      __syncwarp();
+      tc_fence_after();
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float v[32];
+        tc_load32(acc + ACC_DX + rows + 32 * h, v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint4* at = reinterpret_cast<uint4*>(st + row * 128 + (((h * 4 + j) ^ (row & 7)) << 4));
+          const uint4 d = *at;
+          const uint32_t in[4] = {d.x, d.y, d.z, d.w};
+          uint32_t o[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            o[e] = pack_bf16(v[8 * j + 2 * e] + __uint_as_float(in[e] << 16), v[8 * j + 2 * e + 1] + __uint_as_float(in[e] & 0xffff0000u));
+          *at = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+      }
+      tc_fence_before();
+      fence_async_smem();
+      __syncwarp();
+      if ((tid & 31) == 0) mbar_arrive(&outs[s]);
+      __syncwarp();
+      asm volatile("bar.sync %0, 64;" ::"n"(BAR_TC) : "memory");
+      if (q + 2 < mine) make_gates(q + 2);
+    }
+    tc_fence_before();
+    bar_all(FCOMP + 64);       // dW is whole
+    if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }
+    return;
+  }
+
+  if constexpr (SPLIT) cluster_sync_all();
+  return;
+  }
+  regs_up<BWD_SCAN>();
+  // ---- scan
+  const int lane_t = tid / FNCV, vec = tid % FNCV;
+  load_packed_weights(smem + SM::OFF_W, static_cast<const uint4*>(p.pack) + blockIdx.x * 1024, tid);
+  fence_async_smem();
+  bar_all(FCOMP + 64);
+  const ThreadParams tp = load_params(p.params, p.params + p.D, p.params + 2 * p.D, true, true, d0 + vec * CV, p.D, p.c, nullptr);
+  const float2(&K)[2] = tp.K;
+  const bool poly = bar_compute_and(FCOMP, fmaxf(fmaxf(K[0].x, K[0].y), fmaxf(K[1].x, K[1].y)) <= -POLY_RANGE);
+  const int nsave = (p.T + SAVE_EVERY - 1) / SAVE_EVERY;
+  const int cch = tid & (CH - 1), dch = d0 + cch;
+  const bool fwd_chain = tid < CH, rev_chain = tid >= CH && tid < 2 * CH;
+  float carry_rev = 0.0f;
+  if (rev_chain && dch < p.D && p.dh_last) carry_rev = p.dh_last[static_cast<size_t>(b) * p.D + dch];
+  float2 dlam[2] = {f2(0.0f), f2(0.0f)}, dsr[2] = {f2(0.0f), f2(0.0f)}, dsi[2] = {f2(0.0f), f2(0.0f)};
+  ConvTaps ct;
+  const int off0 = lane_t * TS * 128 + (((vec >> 1) ^ ((lane_t & 1) << 2)) << 4) + (vec & 1) * 8;
+
+  for (int q = 0; q < rounds; ++q) {
+    const int k = nchunks - 1 - (q * nranks + rank);
+    const bool idle = SPLIT && q >= mine;
+    if constexpr (SPLIT) { if (tid == 0) split.arm(q); }
+    const int stage = q % NSTAGE;
+    uint8_t* tiles = smem + stage * SM::STAGE;
+    uint8_t* tr = smem + SM::OFF_U + (q & 1) * 2 * FT;
+    const int t0 = k * 64;
+    uint32_t fl[1];
+    const bool masked = p.tok != nullptr || t0 + 64 > p.T;
+    if (masked && !idle) load_flags<TS>(p.tok, b, p.T, t0 + lane_t * TS, fl);
+
+    // State entering this chunk (saved by the forward kernel; chunk 0 starts from h0).
+    float enter = 0.0f;
+    if (fwd_chain && dch < p.D && !idle) {
+      if (k == 0) enter = p.h0 ? p.h0[static_cast<size_t>(b) * p.D + dch] : 0.0f;
+      else enter = p.states[(static_cast<size_t>(b) * nsave + k) * p.D + dch];
+    }
+    BwdRegs<BF, TS> R;
+    bool flagged = false;
+    if (!idle) {
+      mbar_wait_or_flag(&full[stage], (q / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+      mbar_wait_or_flag(&gates[q & 1], (q >> 1) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+      float2 prod[2], sfwd[2], crev[2];
+      flagged = masked && any_flag(fl);
+      uint8_t* tg = tiles + SM::OFF_G;
+      const uint8_t* tx = tiles + SM::OFF_X;
+      const uint8_t* ti = tr + FT;
+      if (flagged) {
+        if (poly) bwd_local<BF, TS, CH, true, true, false, MERGE, true, true>(tiles, tg, tx, tr, ti, off0, K, fl, ct, nullptr, tp.gb, R, prod, sfwd, crev);
+        else bwd_local<BF, TS, CH, true, false, false, MERGE, true, true>(tiles, tg, tx, tr, ti, off0, K, fl, ct, nullptr, tp.gb, R, prod, sfwd, crev);
+      } else {
+        if (poly) bwd_local<BF, TS, CH, false, true, false, MERGE, true, true>(tiles, tg, tx, tr, ti, off0, K, fl, ct, nullptr, tp.gb, R, prod, sfwd, crev);
+        else bwd_local<BF, TS, CH, false, false, false, MERGE, true, true>(tiles, tg, tx, tr, ti, off0, K, fl, ct, nullptr, tp.gb, R, prod, sfwd, crev);
+      }
+      const int ao = lane_t * CH + vec * CV;
+      *reinterpret_cast<float4*>(aggP + ao) = make_float4(prod[0].x, prod[0].y, prod[1].x, prod[1].y);
+      *reinterpret_cast<float4*>(aggS + ao) = make_float4(sfwd[0].x, sfwd[0].y, sfwd[1].x, sfwd[1].y);
+      *reinterpret_cast<float4*>(aggC + ao) = make_float4(crev[0].x, crev[0].y, crev[1].x, crev[1].y);
+    }
+    bar_compute(FCOMP);
+
+    if ((fwd_chain && !idle) || rev_chain) {
+      const float* plane = fwd_chain ? aggS : aggC;
+      float* ein = fwd_chain ? einF : einR;
+      float ap[LANES], as[LANES];
+#pragma unroll
+      for (int j = 0; j < LANES; ++j) { ap[j] = aggP[j * CH + cch]; as[j] = plane[j * CH + cch]; }
+      if (fwd_chain) {
+        float e = enter;
+#pragma unroll
+        for (int j = 0; j < LANES; ++j) {
+          ein[j * CH + cch] = e;
+          e = fmaf(ap[j], e, as[j]);
+        }
+      } else if constexpr (!SPLIT) {
+        float e = carry_rev;
+#pragma unroll
+        for (int j = LANES - 1; j >= 0; --j) {
+          ein[j * CH + cch] = e;
+          e = fmaf(ap[j], e, as[j]);
+        }
+        carry_rev = e;
+      } else {
+        float pa = 1.0f, sa = 0.0f, unused = 1.0f;      // (see rglru_bwd_kernel)
+        if (!idle) {
+#pragma unroll
+          for (int j = LANES - 1; j >= 0; --j) {
+            const float pj = ap[j], sj = as[j];
+            ap[j] = pa;
+            as[j] = sa;
+            sa = fmaf(pj, sa, sj);
+            pa *= pj;
+          }
+        }
+        split.send(q, cch, make_float2(pa, sa), 0, 1);
+        const float e = split.receive(q, cch, carry_rev, unused, dead, p.status);
+        if (!idle) {
+#pragma unroll
+          for (int j = 0; j < LANES; ++j) ein[j * CH + cch] = fmaf(ap[j], e, as[j]);
+        }
+      }
+    }
+    bar_compute(FCOMP);
+    if (idle) break;
+
+    {
+      const float4 f4 = *reinterpret_cast<const float4*>(einF + lane_t * CH + vec * CV);
+      const float4 r4 = *reinterpret_cast<const float4*>(einR + lane_t * CH + vec * CV);
+      const float2 hin[2] = {make_float2(f4.x, f4.y), make_float2(f4.z, f4.w)};
+      const float2 cin[2] = {make_float2(r4.x, r4.y), make_float2(r4.z, r4.w)};
+      const int off_u = static_cast<int>(tr - tiles);
+      if (flagged) bwd_apply<BF, TS, CH, true, false, MERGE, true, true>(tiles, 0, off_u, off_u + FT, SM::OFF_G, off0, K, hin, cin, R, dlam, dsr, dsi);
+      else bwd_apply<BF, TS, CH, false, false, MERGE, true, true>(tiles, 0, off_u, off_u + FT, SM::OFF_G, off0, K, hin, cin, R, dlam, dsr, dsi);
+    }
+    fence_async_smem();
+    __syncwarp();
+    if ((tid & 31) == 0) mbar_arrive(&ready[stage]);
+  }
+
+  if (rev_chain && rank == 0 && dch < p.D && p.dh0) p.dh0[static_cast<size_t>(b) * p.D + dch] = carry_rev;
+
+  // Sums over time, the time-lanes folded in a fixed order.
+  bar_compute(FCOMP);
+  *reinterpret_cast<float4*>(einF + lane_t * CH + vec * CV) = make_float4(dlam[0].x, dlam[0].y, dlam[1].x, dlam[1].y);
+  *reinterpret_cast<float4*>(einR + lane_t * CH + vec * CV) = make_float4(dsr[0].x, dsr[0].y, dsr[1].x, dsr[1].y);
+  *reinterpret_cast<float4*>(aggP + lane_t * CH + vec * CV) = make_float4(dsi[0].x, dsi[0].y, dsi[1].x, dsi[1].y);
+  bar_compute(FCOMP);
+  float* sums = p.sum_part + static_cast<size_t>(b) * 3 * p.D;
+  if (tid < 3 * CH && dch < p.D) {
+    const int which = tid / CH;
+    const float* plane = which == 0 ? einF : (which == 1 ? einR : aggP);
+    float a = 0.0f;
+#pragma unroll
+    for (int j = 0; j < LANES; ++j) a += plane[j * CH + cch];
+    if constexpr (SPLIT) st_cluster_f32(cluster_map(&split.sm->sums[rank][tid], 0), a);
+    else sums[which * p.D + dch] = a;
+  }
+  bar_all(FCOMP + 64);         // dW is whole: four warps read its 128 rows
+  __syncwarp();
+  tc_fence_after();
+  if (warp < 4) {
+    float* out = p.dw_part + ((static_cast<size_t>(b) * nranks + rank) * gridDim.x + blockIdx.x) * (128 * 64) + tid * 64;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float v[32];
+      tc_load32(acc + ACC_DW + 32 * h + (static_cast<uint32_t>(warp) << 21), v);
+#pragma unroll
+      for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(out + 32 * h + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    }
+  }
+  tc_fence_before();
+  __syncwarp();
+  bar_compute(FCOMP);
+  __syncwarp();
+  tc_fence_after();
+  if (warp == 0) tc_free<ACC_COLS>(acc);
+  if constexpr (SPLIT) {       // rank 0 folds the sums of the cluster in rank order
+    __syncwarp();
+    cluster_sync_all();
+    if (rank == 0 && tid < 3 * CH && dch < p.D) {
+      float a = 0.0f;
+      for (int r = 0; r < nranks; ++r) a += split.sm->sums[r][tid];
+      sums[(tid / CH) * p.D + dch] = a;
+    }
+  }
+}
+
+// Gradients of the five parameters from the partial sums, added in index order, in the parameters' own types.  The first
+// `wblocks` blocks take four weights a thread, the others one bias or Lambda.
+template <typename P>
+__global__ void __launch_bounds__(256) fused_fold_kernel(const FusedBwdArgs p, int wblocks, int splits) {
+  if (static_cast<int>(blockIdx.x) < wblocks) {
+    const long long e = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) * 4, n = static_cast<long long>(p.D) * p.bw;
+    if (e >= 2 * n) return;
+    const int gate = e >= n;
+    const long long at = gate ? e - n : e;
+    const int d = static_cast<int>(at / p.bw), k = static_cast<int>(at % p.bw), c = d & 63;
+    const int ntiles = (p.D + 63) / 64;
+    const float* src = p.dw_part + static_cast<size_t>(d >> 6) * (128 * 64) + (64 * gate + c) * 64 + c / p.bw * p.bw + k;
+    const size_t stride = static_cast<size_t>(ntiles) * (128 * 64);
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s0 = 0; s0 < splits; s0 += 8) {
+      float4 v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        v[j] = s0 + j < splits ? *reinterpret_cast<const float4*>(src + (s0 + j) * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) { a.x += v[j].x; a.y += v[j].y; a.z += v[j].z; a.w += v[j].w; }
+    }
+    const float o[4] = {a.x, a.y, a.z, a.w};
+    Pack<P>::store(static_cast<P*>(gate ? p.dw_i : p.dw_r) + at, o);
+    return;
+  }
+  const int i = (static_cast<int>(blockIdx.x) - wblocks) * 256 + threadIdx.x;
+  if (i >= 3 * p.D) return;
+  float a = 0.0f;
+  for (int r0 = 0; r0 < p.B; r0 += 8) {
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = r0 + j < p.B ? p.sum_part[static_cast<size_t>(r0 + j) * 3 * p.D + i] : 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a += v[j];
+  }
+  const int which = i / p.D, d = i % p.D;
+  if (which == 0) a *= (1.0f / (1.0f + expf(p.params[d]))) * p.c;
+  void* dst = which == 0 ? p.dlambda : (which == 1 ? p.db_r : p.db_i);
+  if (which == 0 ? p.f32_lambda : p.f32_bias) static_cast<float*>(dst)[d] = a;
+  else static_cast<BF*>(dst)[d] = __float2bfloat16_rn(a);
+}
+
+template <bool MERGE, bool SPLIT>
+struct FusedFwdKern {
+  static constexpr int THREADS = FTHREADS, BYTES = FusedFwdSmem<MERGE, SPLIT>::BYTES;
+  static_assert(BYTES <= 232448, "shared memory of one CTA");
+  using Fn = void (*)(FusedMaps, FusedFwdArgs);
+  static Fn get(cudaError_t& e) {
+    Fn kern = fused_fwd_kernel<MERGE, SPLIT>;
+    e = set_smem<FusedFwdKern>(kern, BYTES);
+    return kern;
+  }
+};
+template <bool MERGE, bool SPLIT>
+struct FusedBwdKern {
+  static constexpr int THREADS = FTHREADS, BYTES = FusedBwdSmem<MERGE, SPLIT>::BYTES;
+  static_assert(BYTES <= 232448, "shared memory of one CTA");
+  using Fn = void (*)(FusedMaps, FusedBwdArgs);
+  static Fn get(cudaError_t& e) {
+    Fn kern = fused_bwd_kernel<MERGE, SPLIT>;
+    e = set_smem<FusedBwdKern>(kern, BYTES);
+    return kern;
+  }
+};
+template <typename K, typename Args>
+cudaError_t launch_fused(const FusedMaps& maps, const Args& a, cudaStream_t s) {
+  cudaError_t e;
+  auto kern = K::get(e);
+  if (e != cudaSuccess) return e;
+  return launch_pdl(kern, dim3((a.D + 63) / 64, a.B), K::THREADS, K::BYTES, s, maps, a, a.split);
+}
+
+}  // namespace
+
+bool fused_head_width(int head_width) { return head_width == 16 || head_width == 32 || head_width == 64; }
+
+int fused_split(bool fwd, bool merge, int B, int T, int D) {
+  const long long tiles = static_cast<long long>(B) * ((D + 63) / 64);
+  const int nchunks = (T + 63) / 64;
+  if (fwd) return merge ? pick_split<FusedFwdKern<true, true>>(tiles, nchunks) : pick_split<FusedFwdKern<false, true>>(tiles, nchunks);
+  return merge ? pick_split<FusedBwdKern<true, true>>(tiles, nchunks) : pick_split<FusedBwdKern<false, true>>(tiles, nchunks);
+}
+cudaError_t launch_fused_fwd(bool merge, const FusedMaps& maps, const FusedFwdArgs& a, cudaStream_t s) {
+  if (a.split > 1) return merge ? launch_fused<FusedFwdKern<true, true>>(maps, a, s) : launch_fused<FusedFwdKern<false, true>>(maps, a, s);
+  return merge ? launch_fused<FusedFwdKern<true, false>>(maps, a, s) : launch_fused<FusedFwdKern<false, false>>(maps, a, s);
+}
+cudaError_t launch_fused_bwd(bool merge, const FusedMaps& maps, const FusedBwdArgs& a, cudaStream_t s) {
+  cudaError_t e;
+  if (a.split > 1) e = merge ? launch_fused<FusedBwdKern<true, true>>(maps, a, s) : launch_fused<FusedBwdKern<false, true>>(maps, a, s);
+  else e = merge ? launch_fused<FusedBwdKern<true, false>>(maps, a, s) : launch_fused<FusedBwdKern<false, false>>(maps, a, s);
+  if (e != cudaSuccess) return e;
+  const int wblocks = static_cast<int>((2ll * a.D * a.bw / 4 + 255) / 256), vblocks = (3 * a.D + 255) / 256;
+  const int splits = a.B * (a.split > 1 ? a.split : 1);
+  if (a.f32_w) fused_fold_kernel<float><<<wblocks + vblocks, 256, 0, s>>>(a, wblocks, splits);
+  else fused_fold_kernel<BF><<<wblocks + vblocks, 256, 0, s>>>(a, wblocks, splits);
+  return cudaGetLastError();
+}
+
+}  // namespace rglru

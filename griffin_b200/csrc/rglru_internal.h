@@ -223,6 +223,48 @@ struct GateDwArgs {
   int D, bw;
 };
 
+// The layer with its gate projections inside the scan kernels (see rglru_fused.cu).
+struct FusedFwdArgs {
+  const void* w_r;       // [G, bw, bw], 16-byte aligned
+  const void* w_i;
+  const void* b_r;       // [D]
+  const void* b_i;
+  const void* lambda;    // [D]
+  const float* h0;
+  const uint8_t* tok;
+  float* h_last;
+  float* states;         // [B, ceil(T/SAVE_EVERY), D] or nullptr; with it, what the backward needs of the parameters:
+  void* pack;            // [ceil(D / 64), 128, 64] bf16, each channel tile's weights as the kernels' operand
+  float* params;         // [3 D]: Lambda and the two biases
+  int split, B, T, D, bw;
+  bool f32_w, f32_bias, f32_lambda;
+  float c;
+  int* status;
+};
+struct FusedBwdArgs {
+  const float* h0;
+  const float* dh_last;
+  const uint8_t* tok;
+  const float* states;
+  const void* pack;
+  const float* params;
+  float* dw_part;        // [B * split, ceil(D / 64), 128, 64]: rows r 0 .. 63, i 0 .. 63 of a channel tile
+  float* sum_part;       // [B, 3, D]: sums over time of dl * r, du_r, du_i
+  float* dh0;
+  void* dw_r;
+  void* dw_i;
+  void* db_r;
+  void* db_i;
+  void* dlambda;
+  int split, B, T, D, bw;
+  bool f32_w, f32_bias, f32_lambda;
+  float c;
+  int* status;
+};
+struct FusedMaps {
+  CUtensorMap x, out, g, dy, dg;     // forward: x, out, g; backward: dy, x, g, out (dx), dg
+};
+
 // One cached token of the recurrent block (see rglru_decode_block in the public header).
 struct DecodeBlockArgs {
   const void* x_in;
@@ -288,6 +330,10 @@ cudaError_t launch_merge_bwd(bool bf16, bool use_tma, bool conv, const BwdMaps& 
 cudaError_t launch_grouped_fwd(bool bf16, bool merge, const FwdMaps& maps, const ScanFwdArgs& args, cudaStream_t s);
 cudaError_t launch_grouped_bwd(bool bf16, bool merge, const BwdMaps& maps, const ScanBwdArgs& args, cudaStream_t s);
 int grouped_box_cols();
+bool fused_head_width(int head_width);
+int fused_split(bool fwd, bool merge, int B, int T, int D);
+cudaError_t launch_fused_fwd(bool merge, const FusedMaps& maps, const FusedFwdArgs& args, cudaStream_t s);
+cudaError_t launch_fused_bwd(bool merge, const FusedMaps& maps, const FusedBwdArgs& args, cudaStream_t s);
 int scan_fwd_variant(int B, int T, int D, bool bf16);
 int scan_bwd_variant(int B, int T, int D, bool bf16);
 int scan_split(bool fwd, bool bf16, int B, int T, int D);

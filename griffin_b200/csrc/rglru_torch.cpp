@@ -268,34 +268,39 @@ struct Gates {
 };
 int64_t gate_group(int64_t bw) { return std::min<int64_t>(bw & -bw, 64); }
 
-// Whether the layer is a plain call.  Whether it is made in one piece at all is the caller's decision (ops._layer_in_library); a call
-// that is being captured is not taken from here.
-bool layer_plain(at::ScalarType dtype, int64_t D, const at::Device& d, const Gates& g) {
+enum class Layer { none, fused, library };
+
+// How the layer is called in the plain case: with the projections inside the scan kernels, or as the library's own kernels in
+// front of them.  Whether it is called in one piece at all is the caller's decision (ops._layer_in_library, ops._layer_fused); a
+// call that is being captured is not taken from here.
+Layer layer_route(int64_t B, int64_t T, at::ScalarType dtype, int64_t D, const at::Device& d, const Gates& g) {
   const Tensor& w = g.w_r;
   if (w.dim() != 3 || w.size(1) != w.size(2) || w.size(0) < 1 || w.size(1) < 1 || g.w_i.sizes() != w.sizes() ||
       !shape_is(g.b_r, {w.size(0), w.size(1)}) || g.b_i.sizes() != g.b_r.sizes() || w.size(0) * w.size(1) != D)
-    return false;
+    return Layer::none;
   if (!shape_is(g.lam, {D}) || kernel_dtype(w) < 0 || g.w_i.scalar_type() != w.scalar_type() || kernel_dtype(g.b_r) < 0 ||
       g.b_i.scalar_type() != g.b_r.scalar_type() || kernel_dtype(g.lam) < 0 || !dense(w, d) || !dense(g.w_i, d) || !dense(g.b_r, d) ||
       !dense(g.b_i, d) || !dense(g.lam, d) || !aligned16(w) || !aligned16(g.w_i))
-    return false;
-  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return false;
-  return gate_group(g.width()) * (dtype == at::kBFloat16 ? 2 : 4) >= 16 && g.heads() <= 65535;
+    return Layer::none;
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return Layer::none;
+  if (dtype == at::kBFloat16 && rglru_fused_layer_ok(B, T, D, g.width(), RGLRU_BF16)) return Layer::fused;
+  return gate_group(g.width()) * (dtype == at::kBFloat16 ? 2 : 4) < 16 || g.heads() > 65535 ? Layer::none : Layer::library;
 }
 
 // What the layer keeps for its backward beside the tensors.
 struct LayerShape {
+  bool fused = false;
   int64_t heads = 0, bw = 0;
   at::ScalarType wt = at::kFloat, bt = at::kFloat, lt = at::kFloat;
   float c = 0;
 };
-LayerShape layer_shape(const Gates& g) {
-  return {g.heads(), g.width(), g.w_r.scalar_type(), g.b_r.scalar_type(), g.lam.scalar_type(), static_cast<float>(g.c)};
+LayerShape layer_shape(Layer route, const Gates& g) {
+  return {route == Layer::fused, g.heads(), g.width(), g.w_r.scalar_type(), g.b_r.scalar_type(), g.lam.scalar_type(), static_cast<float>(g.c)};
 }
 struct LayerOut {
   Tensor out, h_last, u, ws;
 };
-LayerOut layer_forward(const Tensor& x, const Gates& g, const Opt& h0, const Opt& tok, const Opt& branch, bool save) {
+LayerOut layer_forward(Layer route, const Tensor& x, const Gates& g, const Opt& h0, const Opt& tok, const Opt& branch, bool save) {
   const at::Device d = x.device();
   const int64_t B = x.size(0), T = x.size(1), D = x.size(2), bw = g.width();
   const int io = kernel_dtype(x), wd = kernel_dtype(g.w_r), bd = kernel_dtype(g.b_r), ld = kernel_dtype(g.lam);
@@ -303,6 +308,15 @@ LayerOut layer_forward(const Tensor& x, const Gates& g, const Opt& h0, const Opt
   r.out = empty_as(x);
   r.h_last = empty({B, D}, x, at::kFloat);
   keep_gemms_capturable(d, false);
+  if (route == Layer::fused) {
+    const size_t n = save ? rglru_fused_layer_workspace_bytes(B, T, D) : 0;
+    if (save) r.ws = bytes(n, x);
+    check(rglru_fused_layer_fwd(ptr(x), ptr(g.w_r), ptr(g.b_r), ptr(g.w_i), ptr(g.b_i), ptr(g.lam), ptr(branch), ptr_as<float>(h0),
+                                ptr_as<uint8_t>(tok), r.out.data_ptr(), r.h_last.data_ptr<float>(), save ? r.ws.data_ptr() : nullptr, n, B,
+                                T, D, bw, g.c, wd, bd, ld, io, stream_of(d)),
+          "rglru_fused_layer_fwd");
+    return r;
+  }
   r.u = empty({B, T, 2 * D}, x, x.scalar_type());
   const size_t n = rglru_layer_workspace_bytes(B, T, D, bw, io, save);
   r.ws = bytes(n, x);
@@ -330,6 +344,16 @@ LayerGrads layer_backward(const LayerShape& s, const Tensor& dout, const Tensor&
   float* dh0 = want_dh0 ? g.dh0.data_ptr<float>() : nullptr;
   void* dbranch = branch.defined() ? g.dbranch.data_ptr() : nullptr;
   keep_gemms_capturable(d, true);
+  if (s.fused) {
+    const size_t n = rglru_fused_layer_scratch_bytes(B, T, D, branch.defined());
+    Tensor scratch = bytes(n, x);
+    check(rglru_fused_layer_bwd(ptr(dout), ptr_as<float>(dh), ptr(x), ptr(branch), ptr_as<float>(h0), ptr_as<uint8_t>(tok), ptr(ws),
+                                ws.numel(), g.dx.data_ptr(), dbranch, g.dw_r.data_ptr(), g.db_r.data_ptr(), g.dw_i.data_ptr(),
+                                g.db_i.data_ptr(), g.dlam.data_ptr(), dh0, scratch.data_ptr(), n, B, T, D, s.bw, s.c, wd, bd, ld, io,
+                                stream_of(d)),
+          "rglru_fused_layer_bwd");
+    return g;
+  }
   const size_t n = rglru_layer_scratch_bytes(B, T, D, s.bw, io);
   Tensor scratch = bytes(n, x), du = empty_as(u);
   check(rglru_layer_bwd(ptr(dout), ptr_as<float>(dh), ptr(x), ptr(u), ptr(branch), ptr_as<float>(h0), ptr_as<uint8_t>(tok), ws.data_ptr(),
@@ -370,18 +394,19 @@ std::optional<std::tuple<Tensor, Tensor>> layer(const Tensor& x, const Tensor& w
       (branch && (branch->sizes() != x.sizes() || branch->scalar_type() != x.scalar_type())))
     return std::nullopt;
   const Gates g{w_r, b_r, w_i, b_i, lam, c};
-  if (!layer_plain(x.scalar_type(), D, d, g)) return std::nullopt;
+  const Layer route = layer_route(B, T, x.scalar_type(), D, d, g);
+  if (route == Layer::none) return std::nullopt;
   const bool save = at::GradMode::is_enabled() && (wants_grad(x) || g.want_grad() || wants_grad(h0) || wants_grad(branch));
   LayerOut r;
   {
     at::AutoDispatchBelowADInplaceOrView below;
     const c10::cuda::CUDAGuard on(d);
-    r = layer_forward(x, g, h0, tok, branch, save);
+    r = layer_forward(route, x, g, h0, tok, branch, save);
   }
   if (save) {
     auto node = make_node<LayerNode>(x, w_r, b_r, w_i, b_i, lam, or_undefined(h0), or_undefined(branch));
     node->x = keep(x); node->u = keep(r.u); node->ws = keep(r.ws); node->branch = keep(branch); node->h0 = keep(h0); node->tok = keep(tok);
-    node->shape = layer_shape(g);
+    node->shape = layer_shape(route, g);
     torch::autograd::set_history(r.out, node);
     torch::autograd::set_history(r.h_last, node);
   }
@@ -471,10 +496,11 @@ struct BlockNode final : KernelNode {
   }
 };
 
-// For stock layers whose gated layer is one library call a direction: (out, final state, next conv state or None).  `flags` are the
-// call's flag bytes, `active` its padding mask for the output.
+// For stock layers: (out, final state, next conv state or None).  `flags` are the call's flag bytes, `active` its padding mask for
+// the output, `in_library` what ops._layer_in_library says of its layer.
 std::optional<std::tuple<Tensor, Tensor, Opt>> block(const Tensor& x, const std::vector<Opt>& params, const Tensor& flags, const Opt& active,
-                                                     const Opt& conv_state, const Opt& rnn_state, double c, bool merge, bool want_state) {
+                                                     const Opt& conv_state, const Opt& rnn_state, double c, bool merge, bool want_state,
+                                                     bool in_library) {
   const at::Device d = x.device();
   if (!x.is_cuda() || !dims_ok(x) || !unobserved() || !dense(x, d) || params.size() != BLOCK_PARAMS) return std::nullopt;
   Tensor p[BLOCK_PARAMS];
@@ -503,7 +529,8 @@ std::optional<std::tuple<Tensor, Tensor, Opt>> block(const Tensor& x, const std:
                      (at::GradMode::is_enabled() && wants_grad(conv_state))))
     return std::nullopt;
   if (rnn_state && (!dense(*rnn_state, d) || rnn_state->scalar_type() != at::kFloat || !shape_is(*rnn_state, {B, D}))) return std::nullopt;
-  if (!layer_plain(dtype, D, d, g)) return std::nullopt;
+  const Layer route = layer_route(B, T, dtype, D, d, g);
+  if (route == Layer::none || (route == Layer::library && !in_library)) return std::nullopt;
 
   Tensor xc, wxc, wyc, woc, x_in, branch, cw, x_conv, next, mixed, out;
   LayerOut r;
@@ -521,7 +548,7 @@ std::optional<std::tuple<Tensor, Tensor, Opt>> block(const Tensor& x, const std:
     check(rglru_conv_fwd(ptr(x_in), cw.const_data_ptr<float>(), cb.const_data_ptr<float>(), ptr(conv_state), ptr_as<uint8_t>(flags),
                          x_conv.data_ptr(), want_state ? next.data_ptr() : nullptr, B, T, D, kernel_dtype(x_in), stream_of(d)),
           "rglru_conv_fwd");
-    r = layer_forward(x_conv, g, rnn_state, flags, merge ? Opt(branch) : Opt(), grad);
+    r = layer_forward(route, x_conv, g, rnn_state, flags, merge ? Opt(branch) : Opt(), grad);
     mixed = r.out;
     if (!merge) {
       mixed = empty_as(r.out);
@@ -538,7 +565,7 @@ std::optional<std::tuple<Tensor, Tensor, Opt>> block(const Tensor& x, const std:
     node->branch = keep(branch); node->cw = keep(cw); node->x_conv = keep(x_conv); node->u = keep(r.u); node->ws = keep(r.ws);
     node->y = keep(merge ? Tensor() : r.out); node->mixed = keep(mixed); node->flags = keep(flags); node->active = keep(active);
     node->conv_state = keep(conv_state); node->h0 = keep(rnn_state);
-    node->layer = layer_shape(g);
+    node->layer = layer_shape(route, g);
     node->xt = x.scalar_type();
     for (int k = 0; k < BLOCK_PARAMS; ++k) node->pt[k] = p[k].scalar_type();
     node->merge = merge;

@@ -582,10 +582,10 @@ class RecurrentBlock(nn.Module):
         native = None
         if x.is_cuda and moves is None and not self.fold_conv and (steps > 1 or cache is None or torch.is_grad_enabled()):
             native = self._stock_parts() if ops._native_call() else None
-        if native is not None and self._layer_in_library(x, native):
+        if native is not None:
             done = ops._native().block(x, native, flags, active_mask, None if cache is None else cache.conv_state,
                                        None if cache is None else cache.rnn_state, float(self._modules["rg_lru"].c), self.fold_merge,
-                                       return_cache)
+                                       return_cache, self._layer_in_library(x, native))
             if done is not None:
                 if not return_cache:
                     return done[0]

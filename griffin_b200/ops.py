@@ -970,48 +970,95 @@ def _layer_fwd(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, la
     return out, h_last, u, ws
 
 
-class _LayerNode(torch.autograd.Function):
-    """The layer with both directions as one library call each."""
+_FUSED_HEADS = (16, 32, 64)
 
-    @staticmethod
-    def forward(ctx, x, w_r, b_r, w_i, b_i, lam, h0, tok, c, branch):
-        ctx.set_materialize_grads(False)
-        x, branch = _aligned16(x), _aligned16(branch)
+
+def _layer_fused(x: Tensor, head_width: int) -> bool:
+    """Whether the layer's projections run inside the scan kernels (``rglru_fused_layer_fwd``), at any size: bf16, whole gate heads
+    in a 64-channel tile of the scan."""
+    return x.dtype == torch.bfloat16 and head_width in _FUSED_HEADS and x.shape[2] % 8 == 0 and x.shape[0] <= 65535
+
+
+def _fused_fwd(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor, h0: Optional[Tensor],
+               tok: Optional[Tensor], c: float, branch: Optional[Tensor], save: bool) -> tuple[Tensor, Tensor, Optional[Tensor]]:
+    """(out, h_last, workspace) of the whole layer in one kernel; ``x`` and ``branch`` dense and aligned."""
+    lib = _lib.load()
+    B, T, D = x.shape
+    w_r, b_r, w_i, b_i, lam = _kernel_params(w_r, b_r, w_i, b_i, lam)
+    out = torch.empty_like(x)
+    h_last = torch.empty(B, D, device=x.device, dtype=torch.float32)
+    nbytes = lib.rglru_fused_layer_workspace_bytes(B, T, D) if save else 0
+    ws = torch.empty(nbytes, device=x.device, dtype=torch.uint8) if save else None
+    with _on(x, "rglru_fused_layer_fwd"):
+        _keep_gemms_capturable(x.device, False)
+        rc = lib.rglru_fused_layer_fwd(x.data_ptr(), w_r.data_ptr(), b_r.data_ptr(), w_i.data_ptr(), b_i.data_ptr(), lam.data_ptr(),
+                                       _ptr(branch), _ptr(h0), _ptr(tok), out.data_ptr(), h_last.data_ptr(), _ptr(ws), nbytes,
+                                       B, T, D, w_r.shape[1], c, _DTYPES[w_r.dtype], _DTYPES[b_r.dtype], _DTYPES[lam.dtype],
+                                       _lib.BF16, _stream(x))
+    _lib.check(rc, "rglru_fused_layer_fwd")
+    return out, h_last, ws
+
+
+def _layer_forward(ctx, x, w_r, b_r, w_i, b_i, lam, h0, tok, c, branch):
+    ctx.set_materialize_grads(False)
+    x, branch = _aligned16(x), _aligned16(branch)
+    if _layer_fused(x, w_r.shape[1]):
+        out, h_last, ws = _fused_fwd(x, w_r, b_r, w_i, b_i, lam, h0, tok, c, branch, True)
+        u = None
+    else:
         out, h_last, u, ws = _layer_fwd(x, w_r, b_r, w_i, b_i, lam, h0, tok, c, branch, True)
-        ctx.save_for_backward(x, u, ws, branch, h0, tok)
-        ctx.c, ctx.heads = c, w_r.shape[:2]
-        ctx.param_dtypes = (w_r.dtype, b_r.dtype, w_i.dtype, b_i.dtype, lam.dtype)
-        ctx.want_dh0 = h0 is not None and ctx.needs_input_grad[6]
-        return out, h_last
+    ctx.save_for_backward(x, u, ws, branch, h0, tok)
+    ctx.c, ctx.heads = c, w_r.shape[:2]
+    ctx.param_dtypes = (w_r.dtype, b_r.dtype, w_i.dtype, b_i.dtype, lam.dtype)
+    ctx.want_dh0 = h0 is not None and ctx.needs_input_grad[6]
+    return out, h_last
 
-    @staticmethod
-    @torch.autograd.function.once_differentiable
-    def backward(ctx, dout, dh_last):
-        x, u, ws, branch, h0, tok = ctx.saved_tensors
-        x, u, ws, branch = (_aligned16(t) for t in (x, u, ws, branch))      # (saved-tensor hooks may have moved them)
-        lib = _lib.load()
-        dt = _DTYPES[x.dtype]
-        B, T, D = x.shape
-        G, bw = ctx.heads
-        dout = torch.zeros_like(x) if dout is None else _aligned16(dout.to(x.dtype).contiguous())
-        dh_last = None if dh_last is None else dh_last.to(torch.float32).contiguous()
-        dx, du = torch.empty_like(x), torch.empty_like(u)
-        dbranch = None if branch is None else torch.empty_like(x)
-        dh0 = torch.empty(B, D, device=x.device, dtype=torch.float32) if ctx.want_dh0 else None
-        dw_r, db_r, dw_i, db_i, dlam = grads = _gate_grad_buffers(ctx.param_dtypes, G, bw, x.device)
-        nbytes = lib.rglru_layer_scratch_bytes(B, T, D, bw, dt)
-        scratch = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
-        with _on(x, "rglru_layer_bwd"):
-            _keep_gemms_capturable(x.device, True)
+
+@torch.autograd.function.once_differentiable
+def _layer_backward(ctx, dout, dh_last):
+    x, u, ws, branch, h0, tok = ctx.saved_tensors
+    x, u, ws, branch = (_aligned16(t) for t in (x, u, ws, branch))      # (saved-tensor hooks may have moved them)
+    lib = _lib.load()
+    dt = _DTYPES[x.dtype]
+    B, T, D = x.shape
+    G, bw = ctx.heads
+    dout = torch.zeros_like(x) if dout is None else _aligned16(dout.to(x.dtype).contiguous())
+    dh_last = None if dh_last is None else dh_last.to(torch.float32).contiguous()
+    dx = torch.empty_like(x)
+    dbranch = None if branch is None else torch.empty_like(x)
+    dh0 = torch.empty(B, D, device=x.device, dtype=torch.float32) if ctx.want_dh0 else None
+    dw_r, db_r, dw_i, db_i, dlam = grads = _gate_grad_buffers(ctx.param_dtypes, G, bw, x.device)
+    outs = (dw_r.data_ptr(), db_r.data_ptr(), dw_i.data_ptr(), db_i.data_ptr(), dlam.data_ptr(), _ptr(dh0))
+    types = (_DTYPES[dw_r.dtype], _DTYPES[db_r.dtype], _DTYPES[dlam.dtype], dt)
+    with _on(x, "rglru_layer_bwd"):
+        _keep_gemms_capturable(x.device, True)
+        if u is None:
+            nbytes = lib.rglru_fused_layer_scratch_bytes(B, T, D, branch is not None)
+            scratch = torch.empty(nbytes, device=x.device, dtype=torch.uint8)
+            rc = lib.rglru_fused_layer_bwd(dout.data_ptr(), _ptr(dh_last), x.data_ptr(), _ptr(branch), _ptr(h0), _ptr(tok),
+                                           ws.data_ptr(), ws.numel(), dx.data_ptr(), _ptr(dbranch), *outs, scratch.data_ptr(), nbytes,
+                                           B, T, D, bw, ctx.c, *types, _stream(x))
+        else:
+            nbytes = lib.rglru_layer_scratch_bytes(B, T, D, bw, dt)
+            scratch, du = torch.empty(nbytes, device=x.device, dtype=torch.uint8), torch.empty_like(u)
             rc = lib.rglru_layer_bwd(dout.data_ptr(), _ptr(dh_last), x.data_ptr(), u.data_ptr(), _ptr(branch), _ptr(h0), _ptr(tok),
-                                     ws.data_ptr(), ws.numel(), dx.data_ptr(), du.data_ptr(), _ptr(dbranch), dw_r.data_ptr(),
-                                     db_r.data_ptr(), dw_i.data_ptr(), db_i.data_ptr(), dlam.data_ptr(), _ptr(dh0),
-                                     scratch.data_ptr(), nbytes, B, T, D, bw,
-                                     _gate_group(bw, x.element_size()), ctx.c, _DTYPES[dw_r.dtype], _DTYPES[db_r.dtype],
-                                     _DTYPES[dlam.dtype], dt, _stream(x))
-        _lib.check(rc, "rglru_layer_bwd")
-        dw_r, db_r, dw_i, db_i, dlam = (g if g.dtype == t else g.to(t) for g, t in zip(grads, ctx.param_dtypes))
-        return dx, dw_r, db_r, dw_i, db_i, dlam, dh0, None, None, dbranch
+                                     ws.data_ptr(), ws.numel(), dx.data_ptr(), du.data_ptr(), _ptr(dbranch), *outs, scratch.data_ptr(),
+                                     nbytes, B, T, D, bw, _gate_group(bw, x.element_size()), ctx.c, *types, _stream(x))
+    _lib.check(rc, "rglru_layer_bwd" if u is not None else "rglru_fused_layer_bwd")
+    dw_r, db_r, dw_i, db_i, dlam = (g if g.dtype == t else g.to(t) for g, t in zip(grads, ctx.param_dtypes))
+    return dx, dw_r, db_r, dw_i, db_i, dlam, dh0, None, None, dbranch
+
+
+class _LayerNode(torch.autograd.Function):
+    """The layer with both directions as one library call each, below the line of :func:`_layer_in_library`."""
+
+    forward, backward = staticmethod(_layer_forward), staticmethod(_layer_backward)
+
+
+class _FusedNode(torch.autograd.Function):
+    """The same beyond that line, for the layers :func:`_layer_fused` names."""
+
+    forward, backward = staticmethod(_layer_forward), staticmethod(_layer_backward)
 
 
 def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, lam: Tensor,
@@ -1025,7 +1072,8 @@ def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, l
     save = torch.is_grad_enabled() and (
         x.requires_grad or w_r.requires_grad or b_r.requires_grad or w_i.requires_grad or b_i.requires_grad or lam.requires_grad
         or (h0 is not None and h0.requires_grad) or (branch is not None and branch.requires_grad))
-    if x.is_cuda and w_r.dim() == 3 and w_r.shape[1] > 0 and _native_call() and _layer_in_library(x, w_r.shape[1], save):
+    if x.is_cuda and w_r.dim() == 3 and w_r.shape[1] > 0 and _native_call() and (
+            _layer_fused(x, w_r.shape[1]) or _layer_in_library(x, w_r.shape[1], save)):
         done = _native().layer(x, w_r, b_r, w_i, b_i, lam, h0, tok, branch, float(c))
         if done is not None:
             return done
@@ -1055,12 +1103,13 @@ def rglru_gated(x: Tensor, w_r: Tensor, b_r: Tensor, w_i: Tensor, b_i: Tensor, l
     traced = _library_ops_active()
     if traced or lam.dtype not in _DTYPES:
         lam = lam.to(torch.float32)
-    if not traced and _layer_in_library(x, bw, save):
+    inside, fused = (not traced and _layer_in_library(x, bw, save)), (not traced and _layer_fused(x, bw))
+    if inside or fused:
         args = (x.contiguous(), w_r, b_r, w_i, b_i, lam, None if h0 is None else h0.to(torch.float32).contiguous(),
                 None if tok is None else tok.contiguous(), float(c), None if branch is None else branch.to(x.dtype).contiguous())
         if save or torch.autograd.forward_ad._current_level >= 0:
-            return _LayerNode.apply(*args)
-        return _layer_fwd(_aligned16(args[0]), *args[1:9], _aligned16(args[9]), False)[:2]
+            return (_LayerNode if inside else _FusedNode).apply(*args)
+        return (_fused_fwd if fused else _layer_fwd)(_aligned16(args[0]), *args[1:9], _aligned16(args[9]), False)[:2]
     out, h_last, _, _, _, _ = (_grouped_fwd if traced else functools.partial(_GroupedNode.run, save))(
         x.contiguous(), w_r, b_r, w_i, b_i, lam.contiguous(),
         None if h0 is None else h0.to(torch.float32).contiguous(), None if tok is None else tok.contiguous(), float(c),

@@ -233,6 +233,25 @@ int rglru_layer_bwd(const void* dout, const float* dh_last, const void* x, const
                     int D, int head_width, int gate_width, float c, int weight_dtype, int bias_dtype, int lambda_dtype,
                     int io_dtype, void* stream);
 
+/* The same for bf16 tensors and gate heads of 16, 32 or 64 channels with the projections inside the scan kernels: neither the
+ * gate tensor nor its gradient exists.  rglru_fused_layer_ok says whether a shape qualifies.
+ *   ws      : rglru_fused_layer_workspace_bytes bytes, 16-byte aligned, or NULL where no backward follows; besides the states
+ *             it keeps what the backward needs of the parameters
+ *   scratch : rglru_fused_layer_scratch_bytes bytes, 16-byte aligned (merged: whether branch is given)
+ *   weights and their gradients 16-byte aligned; everything else as in rglru_layer_fwd / rglru_layer_bwd */
+int rglru_fused_layer_ok(int B, int T, int D, int head_width, int io_dtype);
+size_t rglru_fused_layer_workspace_bytes(int B, int T, int D);
+size_t rglru_fused_layer_scratch_bytes(int B, int T, int D, int merged);
+int rglru_fused_layer_fwd(const void* x, const void* w_r, const void* b_r, const void* w_i, const void* b_i, const void* lambda,
+                          const void* branch, const float* h0, const uint8_t* tok, void* out, float* h_last, void* ws,
+                          size_t ws_bytes, int B, int T, int D, int head_width, float c, int weight_dtype, int bias_dtype,
+                          int lambda_dtype, int io_dtype, void* stream);
+int rglru_fused_layer_bwd(const void* dout, const float* dh_last, const void* x, const void* branch, const float* h0,
+                          const uint8_t* tok, const void* ws, size_t ws_bytes, void* dx, void* dbranch, void* dw_r, void* db_r,
+                          void* dw_i, void* db_i, void* dlambda, float* dh0, void* scratch, size_t scratch_bytes, int B, int T,
+                          int D, int head_width, float c, int weight_dtype, int bias_dtype, int lambda_dtype, int io_dtype,
+                          void* stream);
+
 /* How many thread blocks share one (batch row, channel tile) along time in a call of this shape on 16-byte aligned tensors
  * of whole 16-byte rows: 1 for none, 0 for bad arguments.  op: RGLRU_SPLIT_SCAN for rglru_fwd / rglru_bwd, _GATED for
  * rglru_grouped_* and rglru_gated_* without a branch, _MERGED for those with one, _RAW for rglru_linear_scan_*. */

@@ -1,0 +1,115 @@
+"""The bf16 layer with its gate projections inside the scan kernels (``rglru_fused_layer_fwd/bwd``) against the layer's arithmetic in
+64 bits: heads of 16, 32 and 64 channels, sequences around the 64-step chunk, a last channel tile that is cut off, padding, resets,
+carried state, the branch product, parameters of both types, one cluster and many rows."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from oracle import rglru_oracle as orc
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+# bf16 tensors: one rounding of the pre-activations and of every result, hardware tanh (2.5e-4); the bound of the layer's other tests
+BF16_REL = 2e-2
+
+
+def _case(batch, steps, heads, bw, masked, merge, weights, seed=0):
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    width = heads * bw
+    n = lambda *s: torch.randn(*s, device=DEV, generator=gen)
+    half = lambda t: t.to(torch.bfloat16)
+    case = dict(x=half(n(batch, steps, width)), w_r=half(n(heads, bw, bw) * bw ** -0.5).to(weights), b_r=half(0.3 * n(heads, bw)).to(weights),
+                w_i=half(n(heads, bw, bw) * bw ** -0.5).to(weights), b_i=half(0.3 * n(heads, bw)).to(weights),
+                lam=orc.init_lambda(width, 8.0, torch.Generator().manual_seed(seed)).to(DEV), h0=n(batch, width))
+    case["branch"] = half(n(batch, steps, width)) if merge else None
+    resets = torch.rand(batch, steps, device=DEV, generator=gen) < 0.05 if masked else None
+    active = (torch.arange(steps, device=DEV)[None] < torch.randint(1, steps + 1, (batch, 1), device=DEV, generator=gen)) if masked else None
+    return case, resets, active, half(n(batch, steps, width)), n(batch, width)
+
+
+def _run(case, flags, dy, dh):
+    from griffin_b200 import ops
+    c = {k: None if v is None else v.clone().requires_grad_(True) for k, v in case.items()}
+    y, h = ops.rglru_gated(c["x"], c["w_r"], c["b_r"], c["w_i"], c["b_i"], c["lam"], c["h0"], flags, 8.0, c["branch"])
+    torch.autograd.backward([y, h], [dy, dh])
+    return {"y": y.detach(), "h_last": h.detach(), **{k: v.grad for k, v in c.items() if v is not None}}
+
+
+def _reference(case, resets, active, dy, dh):
+    """In 64 bits, the projections by einsum and the scan one step after another."""
+    c = {k: None if v is None else v.double().requires_grad_(True) for k, v in case.items()}
+    batch, steps, width = c["x"].shape
+    heads, bw, _ = c["w_r"].shape
+    xh = c["x"].view(batch, steps, heads, bw)
+    gate = lambda w, b: torch.sigmoid((torch.einsum("btgi,goi->btgo", xh, w) + b).reshape(batch, steps, width))
+    r, i = gate(c["w_r"], c["b_r"]), gate(c["w_i"], c["b_i"])
+    log_a = 8.0 * r * torch.nn.functional.logsigmoid(c["lam"])
+    a, gamma = torch.exp(log_a), torch.sqrt(-torch.expm1(2 * log_a))
+    if resets is not None:
+        keep = (~resets)[..., None].double()
+        a, gamma = a * keep, gamma * keep + (1 - keep)
+    b = gamma * i * c["x"]
+    if active is not None:
+        live = active[..., None].double()
+        a, b = a * live + (1 - live), b * live
+    h, out = c["h0"], []
+    for t in range(steps):
+        h = a[:, t] * h + b[:, t]
+        out.append(h)
+    y = torch.stack(out, 1)
+    if c["branch"] is not None:
+        y = y * torch.nn.functional.gelu(c["branch"], approximate="tanh")
+    torch.autograd.backward([y, h], [dy.double(), dh.double()])
+    return {"y": y.detach(), "h_last": h.detach(), **{k: v.grad for k, v in c.items() if v is not None}}
+
+
+@pytest.mark.parametrize("weights", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("merge", [False, True])
+@pytest.mark.parametrize("batch,steps,heads,bw,masked", [
+    (2, 64, 1, 64, False), (1, 1, 1, 16, False), (2, 63, 3, 16, True), (3, 64, 4, 64, False), (1, 65, 5, 32, True), (2, 128, 2, 64, False),
+    (4, 200, 7, 32, False), (1, 700, 1, 64, True), (40, 130, 5, 64, True), (70, 65, 2, 16, False), (20, 300, 16, 64, True)])
+def test_against_64_bits(batch, steps, heads, bw, masked, merge, weights):
+    from griffin_b200 import _lib, token_flags
+    case, resets, active, dy, dh = _case(batch, steps, heads, bw, masked, merge, weights)
+    flags = token_flags(batch, steps, torch.device(DEV), reset=resets, active=active)
+    got, want = _run(case, flags, dy, dh), _reference(case, resets, active, dy, dh)
+    assert _lib.device_status() == 0
+    for key, ref in want.items():
+        kept = case[key].dtype if key in case else (torch.bfloat16 if key == "y" else torch.float32)
+        assert got[key].shape == ref.shape and got[key].dtype == kept
+        assert torch.isfinite(got[key]).all()
+        assert orc.rel_l2(got[key], ref) <= BF16_REL, (key, orc.rel_l2(got[key], ref))
+
+
+@pytest.mark.parametrize("bw", [16, 32])
+def test_a_head_keeps_its_infinities_to_itself(bw):
+    """Heads that share a channel tile do not enter each other's sums: what is not finite in one leaves the others alone."""
+    case, _, _, dy, dh = _case(2, 70, 8, bw, False, False, torch.bfloat16)
+    clean = _run(case, None, dy, dh)
+    spoilt = dict(case, x=case["x"].clone())
+    spoilt["x"][0, 3, bw] = float("inf")           # head 1
+    spoilt["x"][1, 5, bw + 1] = float("nan")
+    got = _run(spoilt, None, dy, dh)
+    others = [c for c in range(8 * bw) if not bw <= c < 2 * bw]
+    for key in ("y", "x"):
+        assert torch.equal(got[key][..., others], clean[key][..., others])
+    for key in ("w_r", "b_r", "w_i", "b_i"):
+        assert torch.equal(got[key][[0, *range(2, 8)]], clean[key][[0, *range(2, 8)]])
+    assert not torch.isfinite(got["y"][..., bw:2 * bw]).all()
+
+
+def test_parameters_may_change_between_the_passes():
+    """The forward keeps the weights it has used: an update before the backward does not reach it."""
+    from griffin_b200 import ops
+    case, _, _, dy, dh = _case(2, 100, 2, 64, False, False, torch.float32)
+    want = _run(case, None, dy, dh)
+    c = {k: None if v is None else v.clone().requires_grad_(True) for k, v in case.items()}
+    y, h = ops.rglru_gated(c["x"], c["w_r"], c["b_r"], c["w_i"], c["b_i"], c["lam"], c["h0"], None, 8.0, None)
+    with torch.no_grad():
+        for k in ("w_r", "b_r", "w_i", "b_i", "lam"):
+            c[k].add_(1.0)
+    torch.autograd.backward([y, h], [dy, dh])
+    for k in ("x", "w_r", "b_r", "w_i", "b_i", "lam", "h0"):
+        assert torch.equal(c[k].grad, want[k]), k
