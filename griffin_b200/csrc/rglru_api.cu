@@ -192,6 +192,7 @@ static bool tma_shape_ok(int T, int D, size_t es) {
 // once those pairs fill the 148 SMs, below that the kernels that also split the time axis are used.
 static bool conv_tma_pays(int B, int D) { return static_cast<long long>(B) * ((D + 63) / 64) >= 148; }
 
+static bool io_dtype_ok(int t) { return t == RGLRU_F32 || t == RGLRU_BF16; }
 static int check_dims(int B, int T, int D) {
   if (B <= 0 || T <= 0 || D <= 0) return RGLRU_ERR_BAD_SHAPE;
   if (B > 65535) return RGLRU_ERR_BAD_SHAPE;  // batch rows map to gridDim.y
@@ -756,26 +757,26 @@ int rglru_linear_scan_bwd(const float* d_out, const float* decay, const float* h
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
 }
 
-int rglru_conv_fwd(const void* x_in, const float* conv_w, const float* conv_b, const void* conv_state,
-                   const uint8_t* tok, void* x_conv, void* new_state, int B, int T, int D, int io_dtype,
+int rglru_conv_fwd_as(const void* x_in, const void* conv_w, const void* conv_b, const void* conv_state,
+                   const uint8_t* tok, void* x_conv, void* new_state, int B, int T, int D, int weight_dtype, int bias_dtype, int io_dtype,
                    void* stream) {
-  if (io_dtype != RGLRU_F32 && io_dtype != RGLRU_BF16) return RGLRU_ERR_BAD_DTYPE;
+  if (!io_dtype_ok(io_dtype) || !io_dtype_ok(weight_dtype) || !io_dtype_ok(bias_dtype)) return RGLRU_ERR_BAD_DTYPE;
   if (!x_in || !conv_w || !x_conv) return RGLRU_ERR_NULL_POINTER;
   int rc = check_dims(B, T, D);
   if (rc != RGLRU_OK) return rc;
   const bool bf16 = io_dtype == RGLRU_BF16;
   const size_t es = bf16 ? 2 : 4;
   if (!aligned(x_in, es) || !aligned(x_conv, es) || !aligned(conv_state, es) || !aligned(new_state, es) ||
-      !aligned(conv_w, 4) || !aligned(conv_b, 4))
+      !aligned(conv_w, weight_dtype == RGLRU_BF16 ? 2 : 4) || !aligned(conv_b, bias_dtype == RGLRU_BF16 ? 2 : 4))
     return RGLRU_ERR_MISALIGNED;
   int* status = nullptr;
   rc = device_setup(&status);
   if (rc != RGLRU_OK) return rc;
   ConvArgs a = {};
-  a.x_in = x_in; a.w = conv_w; a.bias = conv_b; a.state = conv_state; a.tok = tok; a.out = x_conv;
+  a.x_in = x_in; a.w = conv_w; a.bias = conv_b; a.half_w = weight_dtype == RGLRU_BF16; a.half_b = bias_dtype == RGLRU_BF16; a.state = conv_state; a.tok = tok; a.out = x_conv;
   a.new_state = new_state; a.B = B; a.T = T; a.D = D;
   a.vector_ok = (static_cast<size_t>(D) * es) % 16 == 0 && aligned(x_in, 16) && aligned(x_conv, 16) &&
-                aligned(conv_state, 16) && aligned(conv_w, 16);
+                aligned(conv_state, 16) && (a.half_w || aligned(conv_w, 16));
   ConvMaps maps;
   a.maps = nullptr;
   a.status = status;
@@ -787,22 +788,29 @@ int rglru_conv_fwd(const void* x_in, const float* conv_w, const float* conv_b, c
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
 }
 
+int rglru_conv_fwd(const void* x_in, const float* conv_w, const float* conv_b, const void* conv_state, const uint8_t* tok, void* x_conv,
+                   void* new_state, int B, int T, int D, int io_dtype, void* stream) {
+  return rglru_conv_fwd_as(x_in, conv_w, conv_b, conv_state, tok, x_conv, new_state, B, T, D, RGLRU_F32, RGLRU_F32, io_dtype, stream);
+}
+
 size_t rglru_conv_bwd_workspace_bytes(int B, int T, int D) {
   if (B <= 0 || T <= 0 || D <= 0) return 0;
   return static_cast<size_t>(conv_bwd_partial_rows(B, T)) * 5 * D * sizeof(float);
 }
 
-int rglru_conv_bwd(const void* d_conv, const void* x_in, const float* conv_w, const void* conv_state,
-                   const uint8_t* tok, void* dx_in, float* d_w, float* d_b, void* d_state, void* ws, size_t ws_bytes,
-                   int B, int T, int D, int io_dtype, void* stream) {
-  if (io_dtype != RGLRU_F32 && io_dtype != RGLRU_BF16) return RGLRU_ERR_BAD_DTYPE;
+int rglru_conv_bwd_as(const void* d_conv, const void* x_in, const void* conv_w, const void* conv_state,
+                   const uint8_t* tok, void* dx_in, void* d_w, void* d_b, void* d_state, void* ws, size_t ws_bytes,
+                   int B, int T, int D, int weight_dtype, int grad_weight_dtype, int grad_bias_dtype, int io_dtype, void* stream) {
+  if (!io_dtype_ok(io_dtype) || !io_dtype_ok(weight_dtype) || !io_dtype_ok(grad_weight_dtype) || !io_dtype_ok(grad_bias_dtype))
+    return RGLRU_ERR_BAD_DTYPE;
   if (!d_conv || !x_in || !conv_w || !dx_in || !d_w) return RGLRU_ERR_NULL_POINTER;
   int rc = check_dims(B, T, D);
   if (rc != RGLRU_OK) return rc;
   const bool bf16 = io_dtype == RGLRU_BF16;
   const size_t es = bf16 ? 2 : 4;
   if (!aligned(d_conv, es) || !aligned(x_in, es) || !aligned(dx_in, es) || !aligned(conv_state, es) ||
-      !aligned(d_state, es) || !aligned(conv_w, 4) || !aligned(d_w, 4) || !aligned(d_b, 4) || !aligned(ws, 4))
+      !aligned(d_state, es) || !aligned(conv_w, weight_dtype == RGLRU_BF16 ? 2 : 4) ||
+      !aligned(d_w, grad_weight_dtype == RGLRU_BF16 ? 2 : 4) || !aligned(d_b, grad_bias_dtype == RGLRU_BF16 ? 2 : 4) || !aligned(ws, 4))
     return RGLRU_ERR_MISALIGNED;
   if (!ws || ws_bytes < rglru_conv_bwd_workspace_bytes(B, T, D)) return RGLRU_ERR_WORKSPACE;
   int* status = nullptr;
@@ -810,10 +818,11 @@ int rglru_conv_bwd(const void* d_conv, const void* x_in, const float* conv_w, co
   if (rc != RGLRU_OK) return rc;
   ConvBwdArgs a = {};
   a.d_conv = d_conv; a.x_in = x_in; a.w = conv_w; a.state = conv_state; a.tok = tok; a.dx_in = dx_in;
-  a.d_w = d_w; a.d_b = d_b; a.d_state = d_state; a.part = static_cast<float*>(ws);
+  a.d_w = d_w; a.d_b = d_b; a.half_w = weight_dtype == RGLRU_BF16; a.half_dw = grad_weight_dtype == RGLRU_BF16;
+  a.half_db = grad_bias_dtype == RGLRU_BF16; a.d_state = d_state; a.part = static_cast<float*>(ws);
   a.B = B; a.T = T; a.D = D;
   a.vector_ok = (static_cast<size_t>(D) * es) % 16 == 0 && aligned(d_conv, 16) && aligned(x_in, 16) &&
-                aligned(dx_in, 16) && aligned(conv_state, 16) && aligned(d_state, 16) && aligned(conv_w, 16);
+                aligned(dx_in, 16) && aligned(conv_state, 16) && aligned(d_state, 16) && (a.half_w || aligned(conv_w, 16));
   ConvMaps maps;
   a.maps = nullptr;
   a.status = status;
@@ -824,6 +833,12 @@ int rglru_conv_bwd(const void* d_conv, const void* x_in, const float* conv_w, co
     a.maps = &maps;
   const cudaError_t e = launch_conv_bwd(bf16, a, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
+}
+
+int rglru_conv_bwd(const void* d_conv, const void* x_in, const float* conv_w, const void* conv_state, const uint8_t* tok, void* dx_in,
+                   float* d_w, float* d_b, void* d_state, void* ws, size_t ws_bytes, int B, int T, int D, int io_dtype, void* stream) {
+  return rglru_conv_bwd_as(d_conv, x_in, conv_w, conv_state, tok, dx_in, d_w, d_b, d_state, ws, ws_bytes, B, T, D, RGLRU_F32, RGLRU_F32,
+                           RGLRU_F32, io_dtype, stream);
 }
 
 size_t rglru_column_sums_workspace_bytes(long long rows, int cols) {
@@ -902,7 +917,6 @@ int rglru_decode_step(const void* x, const void* u_r, const void* u_i, const flo
 static bool gate_groups_ok(int D, int head_width, int gate_width) {
   return D > 0 && head_width > 0 && D % head_width == 0 && gate_width >= 4 && gate_width % 4 == 0 && head_width % gate_width == 0;
 }
-static bool io_dtype_ok(int t) { return t == RGLRU_F32 || t == RGLRU_BF16; }
 
 int rglru_gate_pack(const void* w_r, const void* b_r, const void* w_i, const void* b_i, const void* lambda, void* wcat,
                     float* params, int D, int head_width, int gate_width, int weight_dtype, int bias_dtype,

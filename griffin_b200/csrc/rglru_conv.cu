@@ -25,14 +25,15 @@ struct ConvUnroll { static constexpr int value = sizeof(IO) == 2 ? 8 : 4; };
 // kernels, with nothing to keep, use full 16-byte accesses (vec_width).
 constexpr int CONV_VEC = 4;
 
-// The four taps of VEC channels starting at d: wt[k][v] = w[d + v, k] (one 16-byte load per channel).
+// The four taps of VEC channels starting at d: wt[k][v] = w[d + v, k] (fp32: one 16-byte load per channel).
 template <int VEC>
-__device__ __forceinline__ void load_conv_weights(const float* __restrict__ w, int d, float (&wt)[CONV_TAPS][VEC]) {
+__device__ __forceinline__ void load_conv_weights(const void* __restrict__ taps, bool half, int d, float (&wt)[CONV_TAPS][VEC]) {
+  const float* w = static_cast<const float*>(taps);
 #pragma unroll
   for (int v = 0; v < VEC; ++v) {
-    if constexpr (VEC == 1) {
+    if (VEC == 1 || half) {
 #pragma unroll
-      for (int k = 0; k < CONV_TAPS; ++k) wt[k][v] = w[(d + v) * CONV_TAPS + k];
+      for (int k = 0; k < CONV_TAPS; ++k) wt[k][v] = param_as_float(taps, static_cast<size_t>(d + v) * CONV_TAPS + k, half);
     } else {
       const float4 q = *reinterpret_cast<const float4*>(w + static_cast<size_t>(d + v) * CONV_TAPS);
       wt[0][v] = q.x; wt[1][v] = q.y; wt[2][v] = q.z; wt[3][v] = q.w;
@@ -43,8 +44,8 @@ __device__ __forceinline__ void load_conv_weights(const float* __restrict__ w, i
 // ---------------------------------------------------------------- forward
 // Thread = (batch row, run of RUN time-steps, VEC channels).
 template <typename IO, int VEC, int RUN>
-__global__ void __launch_bounds__(256, 3) conv_fwd_kernel(const IO* __restrict__ xin, const float* __restrict__ w,
-                                                       const float* __restrict__ bias, const IO* __restrict__ state,
+__global__ void __launch_bounds__(256, 3) conv_fwd_kernel(const IO* __restrict__ xin, const void* __restrict__ w,
+                                                       const void* __restrict__ bias, bool half_w, bool half_b, const IO* __restrict__ state,
                                                        const uint8_t* __restrict__ tok, IO* __restrict__ out, int B,
                                                        int T, int D) {
   constexpr int UNROLL = ConvUnroll<IO>::value;
@@ -60,9 +61,9 @@ __global__ void __launch_bounds__(256, 3) conv_fwd_kernel(const IO* __restrict__
   const int t_end = min(T, t_begin + RUN);
 
   float wt[CONV_TAPS][VEC], bs[VEC];
-  load_conv_weights<VEC>(w, d, wt);
+  load_conv_weights<VEC>(w, half_w, d, wt);
 #pragma unroll
-  for (int v = 0; v < VEC; ++v) bs[v] = bias ? bias[d + v] : 0.0f;
+  for (int v = 0; v < VEC; ++v) bs[v] = bias ? param_as_float(bias, d + v, half_b) : 0.0f;
   // hist[l-1] holds the input l steps before the current one.
   float hist[CONV_TAPS - 1][VEC];
 #pragma unroll
@@ -188,7 +189,7 @@ __global__ void conv_state_kernel(const IO* __restrict__ xin, const IO* __restri
 // partial row [5, D] is written per (row, 8*RUN time-steps).
 template <typename IO, int VEC, int RUN>
 __global__ void __launch_bounds__(256, 2) conv_bwd_kernel(const IO* __restrict__ dconv, const IO* __restrict__ xin,
-                                                       const float* __restrict__ w, const IO* __restrict__ state,
+                                                       const void* __restrict__ w, bool half_w, const IO* __restrict__ state,
                                                        const uint8_t* __restrict__ tok, IO* __restrict__ dxin,
                                                        IO* __restrict__ dstate, float* __restrict__ part, int B, int T,
                                                        int D) {
@@ -214,7 +215,7 @@ __global__ void __launch_bounds__(256, 2) conv_bwd_kernel(const IO* __restrict__
 
   if (live && t_begin < T) {
     float wt[CONV_TAPS][VEC];
-    load_conv_weights<VEC>(w, d, wt);
+    load_conv_weights<VEC>(w, half_w, d, wt);
 
     auto load_in = [&](int t, float (&v)[VEC]) {
       if (t >= 0) Vec<IO, VEC>::load(xin + (static_cast<size_t>(b) * T + t) * D + d, v);
@@ -380,15 +381,18 @@ __global__ void __launch_bounds__(256, 2) conv_bwd_kernel(const IO* __restrict__
 }
 
 // d_w[d, k] = sum over partial rows; d_b[d] likewise.  Rows are added in index order.
-__global__ void conv_bwd_reduce_kernel(const float* __restrict__ part, float* __restrict__ dw, float* __restrict__ db,
-                                       int rows, int D) {
+__global__ void conv_bwd_reduce_kernel(const float* __restrict__ part, void* __restrict__ dw, void* __restrict__ db,
+                                       bool half_w, bool half_b, int rows, int D) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= 5 * D) return;
   const int k = idx / D, d = idx % D;
   float acc = 0.0f;
   for (int r = 0; r < rows; ++r) acc += part[(static_cast<size_t>(r) * 5 + k) * D + d];
-  if (k < 4) dw[d * CONV_TAPS + k] = acc;
-  else if (db) db[d] = acc;
+  void* dst = k < 4 ? dw : db;
+  const size_t at = k < 4 ? static_cast<size_t>(d) * CONV_TAPS + k : d;
+  if (!dst) return;
+  if (k < 4 ? half_w : half_b) static_cast<__nv_bfloat16*>(dst)[at] = __float2bfloat16_rn(acc);
+  else static_cast<float*>(dst)[at] = acc;
 }
 
 // ---------------------------------------------------------------- column sums
@@ -667,11 +671,11 @@ static cudaError_t conv_fwd_t(const ConvArgs& a, cudaStream_t s) {
   cudaError_t e;
   if (a.maps) {   // enough (row, channel-tile) pairs to fill the machine: the TMA-staged kernel
     ConvTmaArgs t = {};
-    t.w = a.w; t.bias = a.bias; t.state = a.state; t.tok = a.tok; t.B = a.B; t.T = a.T; t.D = a.D; t.status = a.status;
+    t.w = a.w; t.bias = a.bias; t.half_w = a.half_w; t.half_b = a.half_b; t.state = a.state; t.tok = a.tok; t.B = a.B; t.T = a.T; t.D = a.D; t.status = a.status;
     e = launch_conv_tma_fwd(sizeof(IO) == 2, *a.maps, t, s);
   } else {
-    if (vec_ok) conv_fwd_kernel<IO, V, CONV_RUN><<<blocks, 256, 0, s>>>(xin, a.w, a.bias, st, a.tok, out, a.B, a.T, a.D);
-    else conv_fwd_kernel<IO, 1, CONV_RUN><<<blocks, 256, 0, s>>>(xin, a.w, a.bias, st, a.tok, out, a.B, a.T, a.D);
+    if (vec_ok) conv_fwd_kernel<IO, V, CONV_RUN><<<blocks, 256, 0, s>>>(xin, a.w, a.bias, a.half_w, a.half_b, st, a.tok, out, a.B, a.T, a.D);
+    else conv_fwd_kernel<IO, 1, CONV_RUN><<<blocks, 256, 0, s>>>(xin, a.w, a.bias, a.half_w, a.half_b, st, a.tok, out, a.B, a.T, a.D);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess || !a.new_state) return e;
@@ -702,17 +706,17 @@ static cudaError_t conv_bwd_t(const ConvBwdArgs& a, cudaStream_t s) {
   int part_rows = a.B * tblocks;
   if (a.maps) {   // the TMA-staged kernel leaves one partial row per batch row
     ConvTmaArgs t = {};
-    t.w = a.w; t.state = a.state; t.tok = a.tok; t.d_state = a.d_state; t.part = a.part;
+    t.w = a.w; t.half_w = a.half_w; t.state = a.state; t.tok = a.tok; t.d_state = a.d_state; t.part = a.part;
     t.B = a.B; t.T = a.T; t.D = a.D; t.status = a.status;
     e = launch_conv_tma_bwd(sizeof(IO) == 2, *a.maps, t, s);
     part_rows = a.B;
   } else {
-    if (vec_ok) conv_bwd_kernel<IO, V, CONV_RUN><<<grid, 256, 0, s>>>(dc, xin, a.w, st, a.tok, dx, ds, a.part, a.B, a.T, a.D);
-    else conv_bwd_kernel<IO, 1, CONV_RUN><<<grid, 256, 0, s>>>(dc, xin, a.w, st, a.tok, dx, ds, a.part, a.B, a.T, a.D);
+    if (vec_ok) conv_bwd_kernel<IO, V, CONV_RUN><<<grid, 256, 0, s>>>(dc, xin, a.w, a.half_w, st, a.tok, dx, ds, a.part, a.B, a.T, a.D);
+    else conv_bwd_kernel<IO, 1, CONV_RUN><<<grid, 256, 0, s>>>(dc, xin, a.w, a.half_w, st, a.tok, dx, ds, a.part, a.B, a.T, a.D);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) return e;
-  conv_bwd_reduce_kernel<<<(5 * a.D + 255) / 256, 256, 0, s>>>(a.part, a.d_w, a.d_b, part_rows, a.D);
+  conv_bwd_reduce_kernel<<<(5 * a.D + 255) / 256, 256, 0, s>>>(a.part, a.d_w, a.d_b, a.half_dw, a.half_db, part_rows, a.D);
   return cudaGetLastError();
 }
 
@@ -729,8 +733,8 @@ static cudaError_t decode_conv_t(const ConvArgs& a, cudaStream_t s) {
   const IO* xin = static_cast<const IO*>(a.x_in);
   IO* st = static_cast<IO*>(a.new_state);
   IO* out = static_cast<IO*>(a.out);
-  if (a.vector_ok) decode_conv_kernel<IO, V><<<blocks, 256, 0, s>>>(xin, a.w, a.bias, st, a.tok, out, a.B, a.D);
-  else decode_conv_kernel<IO, 1><<<blocks, 256, 0, s>>>(xin, a.w, a.bias, st, a.tok, out, a.B, a.D);
+  if (a.vector_ok) decode_conv_kernel<IO, V><<<blocks, 256, 0, s>>>(xin, static_cast<const float*>(a.w), static_cast<const float*>(a.bias), st, a.tok, out, a.B, a.D);
+  else decode_conv_kernel<IO, 1><<<blocks, 256, 0, s>>>(xin, static_cast<const float*>(a.w), static_cast<const float*>(a.bias), st, a.tok, out, a.B, a.D);
   return cudaGetLastError();
 }
 

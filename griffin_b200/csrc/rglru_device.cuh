@@ -453,6 +453,11 @@ struct Pack<__nv_bfloat16> {
   static __device__ __forceinline__ __nv_bfloat16 from_float(float x) { return __float2bfloat16_rn(x); }
 };
 
+// A parameter that may be in either type.
+__device__ __forceinline__ float param_as_float(const void* p, size_t i, bool half) {
+  return half ? __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]) : static_cast<const float*>(p)[i];
+}
+
 // Token flag bits (mirrors include/rglru_b200.h).
 constexpr uint32_t TOK_CUT_MASK = 0x03u;
 constexpr uint32_t TOK_RESET = 0x04u;

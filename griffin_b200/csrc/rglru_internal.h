@@ -109,8 +109,9 @@ struct ConvMaps {
   CUtensorMap in0, in1, out0;
 };
 struct ConvTmaArgs {
-  const float* w;
-  const float* bias;
+  const void* w;
+  const void* bias;
+  bool half_w, half_b;   // taps / bias in bf16, else fp32
   const void* state;     // [B, 3, D] history before t = 0 or nullptr
   const uint8_t* tok;
   void* d_state;         // backward only: gradient of the history, or nullptr
@@ -119,10 +120,13 @@ struct ConvTmaArgs {
   int* status;
 };
 
+// Taps, bias and their gradients come in the parameters' own types: casting them around the kernels took two launches of 2 to
+// 4 us a direction, a sixth of a padded prompt of 6 x 1200 tokens.
 struct ConvArgs {
   const void* x_in;
-  const float* w;
-  const float* bias;
+  const void* w;
+  const void* bias;
+  bool half_w, half_b;   // taps / bias in bf16, else fp32
   const void* state;  // history before t = 0 (forward) or nullptr
   const uint8_t* tok;
   void* out;
@@ -135,12 +139,13 @@ struct ConvArgs {
 struct ConvBwdArgs {
   const void* d_conv;
   const void* x_in;
-  const float* w;
+  const void* w;
   const void* state;
   const uint8_t* tok;
   void* dx_in;
-  float* d_w;
-  float* d_b;
+  void* d_w;
+  void* d_b;
+  bool half_w, half_dw, half_db;   // taps / their gradient / the bias's gradient in bf16, else fp32
   void* d_state;
   float* part;
   int B, T, D;

@@ -1292,7 +1292,7 @@ __global__ void __launch_bounds__(288) conv_tma_fwd_kernel(const __grid_constant
   }
 
   ConvTaps ct;
-  load_taps(p.w, p.bias, d0 + vec * CV, p.D, ct);
+  load_taps(p.w, p.bias, d0 + vec * CV, p.D, ct, p.half_w, p.half_b);
   const int off0 = (lane_t * TS) * ROWB + vec * Pack<IO>::BYTES;
 
   for (int k = 0; k < nchunks; ++k) {
@@ -1475,7 +1475,7 @@ __global__ void __maxnreg__(96) conv_tma_bwd_kernel(const __grid_constant__ Conv
   }
 
   ConvTaps ct;
-  load_taps(p.w, nullptr, d0 + vec * CV, p.D, ct);
+  load_taps(p.w, nullptr, d0 + vec * CV, p.D, ct, p.half_w);
   float2 gw[5][2];
 #pragma unroll
   for (int q = 0; q < 5; ++q) { gw[q][0] = f2(0.0f); gw[q][1] = f2(0.0f); }

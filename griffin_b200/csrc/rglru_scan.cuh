@@ -219,14 +219,15 @@ struct ConvTaps {
   float2 bias[2];
 };
 
-__device__ __forceinline__ void load_taps(const float* conv_w, const float* conv_b, int d, int D, ConvTaps& ct) {
+__device__ __forceinline__ void load_taps(const void* conv_w, const void* conv_b, int d, int D, ConvTaps& ct, bool half_w = false,
+                                          bool half_b = false) {
   float w[4][4], bz[4];
 #pragma unroll
   for (int ch = 0; ch < 4; ++ch) {
     const bool ok = d + ch < D;
-    bz[ch] = (ok && conv_b) ? conv_b[d + ch] : 0.0f;
+    bz[ch] = (ok && conv_b) ? param_as_float(conv_b, d + ch, half_b) : 0.0f;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) w[k][ch] = ok ? conv_w[(d + ch) * 4 + k] : 0.0f;
+    for (int k = 0; k < 4; ++k) w[k][ch] = ok ? param_as_float(conv_w, static_cast<size_t>(d + ch) * 4 + k, half_w) : 0.0f;
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k) { ct.w[k][0] = make_float2(w[k][0], w[k][1]); ct.w[k][1] = make_float2(w[k][2], w[k][3]); }

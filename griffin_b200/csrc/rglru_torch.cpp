@@ -472,14 +472,14 @@ struct BlockNode final : KernelNode {
     out[p(WR)] = r.dw_r; out[p(BR)] = r.db_r; out[p(WI)] = r.dw_i; out[p(BI)] = r.db_i; out[p(LAM)] = r.dlam;
     out[1 + BLOCK_PARAMS] = r.dh0;
 
-    Tensor dx_in = empty_as(x_in_), dcw = empty_as(cw_), dcb = empty({D}, x_in_, at::kFloat);
+    Tensor dx_in = empty_as(x_in_), dcw = empty(cw_.sizes(), x_in_, pt[CW]), dcb = empty({D}, x_in_, pt[CB]);
     const size_t n = rglru_conv_bwd_workspace_bytes(B, T, D);
     Tensor scratch = bytes(n, x_in_);
-    check(rglru_conv_bwd(ptr(r.dx), ptr(x_in_), cw_.const_data_ptr<float>(), ptr(conv_state_), ptr_as<uint8_t>(flags_), dx_in.data_ptr(),
-                         dcw.data_ptr<float>(), dcb.data_ptr<float>(), nullptr, scratch.data_ptr(), n, B, T, D, kernel_dtype(x_in_),
-                         stream_of(d)),
+    check(rglru_conv_bwd_as(ptr(r.dx), ptr(x_in_), ptr(cw_), ptr(conv_state_), ptr_as<uint8_t>(flags_), dx_in.data_ptr(), dcw.data_ptr(),
+                            dcb.data_ptr(), nullptr, scratch.data_ptr(), n, B, T, D, kernel_dtype(cw_), kernel_dtype(pt[CW]),
+                            kernel_dtype(pt[CB]), kernel_dtype(x_in_), stream_of(d)),
           "rglru_conv_bwd");
-    out[p(CW)] = dcw.to(pt[CW]); out[p(CB)] = dcb.to(pt[CB]);
+    out[p(CW)] = dcw; out[p(CB)] = dcb;
 
     const Tensor d1 = rows_of(dx_in), d2 = rows_of(dbranch), rows = rows_of(x_);
     if (wants(0)) {
@@ -543,10 +543,11 @@ std::optional<std::tuple<Tensor, Tensor, Opt>> block(const Tensor& x, const std:
     branch = at::linear(xc, wyc, p[BY].to(dtype));
     x_conv = empty_as(x_in);
     if (want_state) next = empty({B, 3, D}, x_in, dtype);
-    cw = p[CW].to(at::kFloat);
-    const Tensor cb = p[CB].to(at::kFloat);
-    check(rglru_conv_fwd(ptr(x_in), cw.const_data_ptr<float>(), cb.const_data_ptr<float>(), ptr(conv_state), ptr_as<uint8_t>(flags),
-                         x_conv.data_ptr(), want_state ? next.data_ptr() : nullptr, B, T, D, kernel_dtype(x_in), stream_of(d)),
+    // The backward keeps bf16 taps as an fp32 copy: the parameter may change before it runs.
+    cw = grad ? p[CW].to(at::kFloat) : p[CW];
+    check(rglru_conv_fwd_as(ptr(x_in), ptr(cw), ptr(p[CB]), ptr(conv_state), ptr_as<uint8_t>(flags), x_conv.data_ptr(),
+                            want_state ? next.data_ptr() : nullptr, B, T, D, kernel_dtype(cw), kernel_dtype(p[CB]), kernel_dtype(x_in),
+                            stream_of(d)),
           "rglru_conv_fwd");
     r = layer_forward(route, x_conv, g, rnn_state, flags, merge ? Opt(branch) : Opt(), grad);
     mixed = r.out;

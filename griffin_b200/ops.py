@@ -375,8 +375,9 @@ def _conv_fwd_impl(x_in: Tensor, w: Tensor, b: Optional[Tensor], state: Optional
     out = torch.empty_like(x_in)
     new_state = torch.empty((B, 3, D) if want_state else (0,), device=x_in.device, dtype=x_in.dtype)
     with _on(x_in, "rglru_conv_fwd"):
-        rc = lib.rglru_conv_fwd(_ptr(x_in), _ptr(w), _ptr(b), _ptr(state), _ptr(tok), _ptr(out),
-                                _ptr(new_state) if want_state else None, B, T, D, dt, _stream(x_in))
+        rc = lib.rglru_conv_fwd_as(_ptr(x_in), _ptr(w), _ptr(b), _ptr(state), _ptr(tok), _ptr(out),
+                                   _ptr(new_state) if want_state else None, B, T, D, _io_dtype(w, "conv"),
+                                   _lib.F32 if b is None else _io_dtype(b, "conv"), dt, _stream(x_in))
     _lib.check(rc, "rglru_conv_fwd")
     return out, new_state
 
@@ -449,10 +450,11 @@ def causal_conv(x_in: Tensor, weight: Tensor, bias: Optional[Tensor], conv_state
         raise ValueError("conv input must be [batch, sequence, width]")
     if weight.shape != (x_in.shape[2], 4):
         raise ValueError("CUDA causal conv supports kernel width 4 with weight [width, 4]")
-    w = weight.to(torch.float32).contiguous()
-    b = None if bias is None else bias.to(torch.float32).contiguous()
     st = None if conv_state is None else conv_state.to(x_in.dtype).contiguous()
-    differentiated = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x_in, w, b, st))
+    differentiated = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x_in, weight, bias, st))
+    # The kernel reads taps and bias in either type; a differentiated call keeps its fp32 copy of them for the backward.
+    w, b = (t if t is None or (not differentiated and t.dtype in _DTYPES) else t.to(torch.float32) for t in (weight, bias))
+    w, b = w.contiguous(), None if b is None else b.contiguous()
     return (_conv_fwd if _library_ops_active() else functools.partial(_ConvNode.run, differentiated))(
         x_in.contiguous(), w, b, st, None if tok is None else tok.contiguous(), want_state)
 

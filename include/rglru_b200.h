@@ -288,6 +288,10 @@ int rglru_linear_scan_bwd(const float* d_out, const float* decay, const float* h
 int rglru_conv_fwd(const void* x_in, const float* conv_w, const float* conv_b, const void* conv_state,
                    const uint8_t* tok, void* x_conv, void* new_state, int B, int T, int D,
                    int io_dtype, void* stream);
+/* The same with taps and bias in types of their own (RGLRU_F32 or RGLRU_BF16 each). */
+int rglru_conv_fwd_as(const void* x_in, const void* conv_w, const void* conv_b, const void* conv_state, const uint8_t* tok,
+                      void* x_conv, void* new_state, int B, int T, int D, int weight_dtype, int bias_dtype, int io_dtype,
+                      void* stream);
 
 /* Backward of rglru_conv_fwd for the dense (no padding) case: the reference gets it from
  * autograd over griffin/griffin.py:478-486.
@@ -300,6 +304,10 @@ size_t rglru_conv_bwd_workspace_bytes(int B, int T, int D);
 int rglru_conv_bwd(const void* d_conv, const void* x_in, const float* conv_w, const void* conv_state,
                    const uint8_t* tok, void* dx_in, float* d_w, float* d_b, void* d_state, void* ws,
                    size_t ws_bytes, int B, int T, int D, int io_dtype, void* stream);
+/* The same with conv_w, d_w and d_b in types of their own. */
+int rglru_conv_bwd_as(const void* d_conv, const void* x_in, const void* conv_w, const void* conv_state, const uint8_t* tok,
+                      void* dx_in, void* d_w, void* d_b, void* d_state, void* ws, size_t ws_bytes, int B, int T, int D,
+                      int weight_dtype, int grad_weight_dtype, int grad_bias_dtype, int io_dtype, void* stream);
 
 /* Conv backward for callers that cannot allocate device memory.  (No counterpart in the reference:
  * it exists for hosts of this library that may not call cudaMalloc or any allocating routine at the

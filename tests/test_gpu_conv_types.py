@@ -1,0 +1,72 @@
+"""The conv's entries with taps, bias and their gradients in types of their own against the fp32 entries on converted tensors: the
+same arithmetic, so the same bits."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+BF, F32 = torch.bfloat16, torch.float32
+# Widths of one channel a thread, of whole vectors, and (enough tiles) of the copy engine's kernels; ragged and one-step sequences.
+SHAPES = [(1, 1, 64), (2, 5, 33), (2, 70, 128), (3, 300, 200), (8, 1030, 768)]
+
+
+def _code(dtype):
+    from griffin_b200 import _lib
+    return _lib.BF16 if dtype == BF else _lib.F32
+
+
+def _p(t):
+    return None if t is None else t.data_ptr()
+
+
+def _tensors(shape, io, with_state):
+    torch.manual_seed(sum(shape))
+    B, T, D = shape
+    x, dy = (torch.randn(shape, device=DEV).to(io) for _ in range(2))
+    state = torch.randn(B, 3, D, device=DEV).to(io) if with_state else None
+    tok = torch.randint(0, 32, (B, T), device=DEV).to(torch.uint8)
+    return x, dy, torch.randn(D, 4, device=DEV).to(BF), torch.randn(D, device=DEV).to(BF), state, tok if T > 1 else None
+
+
+@pytest.mark.parametrize("io", [BF, F32])
+@pytest.mark.parametrize("weight,bias", [(BF, BF), (BF, F32), (F32, BF)])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_types_of_their_own(shape, weight, bias, io):
+    from griffin_b200 import _lib
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    B, T, D = shape
+    x, dy, w, b, state, tok = _tensors(shape, io, True)
+    outs, grads = [], []
+    for wt, bt in ((F32, F32), (weight, bias)):
+        y, nxt = torch.empty_like(x), torch.empty_like(state)
+        args = (_p(x), _p(wc := w.to(wt)), _p(bc := b.to(bt)), _p(state), _p(tok), _p(y), _p(nxt), B, T, D)
+        as32 = wt == bt == F32
+        _lib.check(lib.rglru_conv_fwd(*args, _code(io), stream) if as32 else
+                   lib.rglru_conv_fwd_as(*args, _code(wt), _code(bt), _code(io), stream), "forward")
+        dx, dw, db = torch.empty_like(x), torch.empty(D, 4, device=DEV, dtype=wt), torch.empty(D, device=DEV, dtype=bt)
+        ds = torch.empty_like(state)
+        n = lib.rglru_conv_bwd_workspace_bytes(B, T, D)
+        ws = torch.empty(n, device=DEV, dtype=torch.uint8)
+        args = (_p(dy), _p(x), _p(wc), _p(state), _p(tok), _p(dx), _p(dw), _p(db), _p(ds), _p(ws), n, B, T, D)
+        _lib.check(lib.rglru_conv_bwd(*args, _code(io), stream) if as32 else
+                   lib.rglru_conv_bwd_as(*args, _code(wt), _code(wt), _code(bt), _code(io), stream), "backward")
+        outs.append((y, nxt, dx, ds))
+        grads.append((dw.to(wt), db.to(bt)))
+        del wc, bc
+    for a, c in zip(*outs):
+        assert torch.equal(a, c)
+    assert torch.equal(grads[0][0].to(weight), grads[1][0]) and torch.equal(grads[0][1].to(bias), grads[1][1])
+
+
+def test_refused_types_and_addresses():
+    from griffin_b200 import _lib
+    lib = _lib.load()
+    shape = (2, 5, 64)
+    x, _, w, b, state, tok = _tensors(shape, BF, True)
+    y = torch.empty_like(x)
+    call = lambda wp, wt, bt: lib.rglru_conv_fwd_as(_p(x), wp, _p(b), None, None, _p(y), None, *shape, wt, bt, _lib.BF16, None)
+    assert call(_p(w), 7, _lib.BF16) != 0 and call(_p(w), _lib.BF16, 7) != 0
+    assert call(_p(w) + 1, _lib.BF16, _lib.BF16) != 0 and call(_p(w) + 2, _lib.F32, _lib.BF16) != 0
