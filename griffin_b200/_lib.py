@@ -73,6 +73,7 @@ SIGNATURES = {
     "rglru_token_plan": (_i, [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _vp]),
     "rglru_token_plan_workspace_bytes": (_sz, [_i, _i]),
     "rglru_token_plan_ws": (_i, [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _sz, _i, _i, _vp]),
+    "rglru_zero_rows": (_i, [_vp, _vp, ctypes.c_longlong, _i, _vp]),
     "rglru_gelu_mul_fwd": (_i, [_vp, _vp, _vp, ctypes.c_longlong, _i, _vp]),
     "rglru_gelu_mul_bwd": (_i, [_vp, _vp, _vp, _vp, _vp, ctypes.c_longlong, _i, _vp]),
     "rglru_decode_conv": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]),

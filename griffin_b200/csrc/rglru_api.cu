@@ -1206,6 +1206,16 @@ static int gelu_mul(const GeluMulArgs& a, int io_dtype, void* stream) {
   const cudaError_t e = launch_gelu_mul(io_dtype == RGLRU_BF16, a, vector_ok, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
 }
+int rglru_zero_rows(void* x, const uint8_t* keep, long long rows, int row_bytes, void* stream) {
+  if (!x || !keep) return RGLRU_ERR_NULL_POINTER;
+  if (rows <= 0 || rows > (1ll << 33) || row_bytes <= 0 || row_bytes % 16 != 0) return RGLRU_ERR_BAD_SHAPE;
+  if (!aligned(x, 16)) return RGLRU_ERR_MISALIGNED;
+  int* status = nullptr;
+  const int rc = device_setup(&status);
+  if (rc != RGLRU_OK) return rc;
+  const cudaError_t e = launch_zero_rows(x, keep, rows, row_bytes / 16, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? RGLRU_OK : fail_cuda(e);
+}
 int rglru_gelu_mul_fwd(const void* y, const void* branch, void* out, long long n, int io_dtype, void* stream) {
   return gelu_mul(GeluMulArgs{y, branch, nullptr, out, nullptr, n}, io_dtype, stream);
 }

@@ -174,6 +174,19 @@ __global__ void __launch_bounds__(256) gelu_mul_kernel(const GeluMulArgs p) {
   if constexpr (BWD) V::store(static_cast<IO*>(p.dg) + i, reinterpret_cast<float (&)[VEC]>(c));
 }
 
+// ---------------------------------------------------------------- padding rows of the output
+// The block's output is zero at padding tokens (griffin/griffin.py:488-510).  In place, a warp per row, only the padding rows
+// are written and only the mask is read; a select over the whole tensor takes 13.5 us for 6 x 1200 rows of 768 bf16, this 3.0.
+__global__ void __launch_bounds__(256) zero_rows_kernel(uint4* __restrict__ x, const uint8_t* __restrict__ keep, long long rows, int pieces) {
+  const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (row >= rows || keep[row]) return;
+  for (int i = threadIdx.x & 31; i < pieces; i += 32) x[row * pieces + i] = make_uint4(0u, 0u, 0u, 0u);
+}
+cudaError_t launch_zero_rows(void* x, const uint8_t* keep, long long rows, int pieces, cudaStream_t s) {
+  zero_rows_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, s>>>(static_cast<uint4*>(x), keep, rows, pieces);
+  return cudaGetLastError();
+}
+
 template <typename IO, bool BWD>
 static cudaError_t gelu_mul_t(const GeluMulArgs& a, bool vector_ok, cudaStream_t s) {
   constexpr int V = vec_width<IO>();

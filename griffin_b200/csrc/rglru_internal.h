@@ -311,6 +311,7 @@ cudaError_t launch_decode_conv(bool bf16, const ConvArgs& a, cudaStream_t s);
 cudaError_t launch_decode_step(bool bf16, const DecodeArgs& a, cudaStream_t s);
 int token_plan_parts(int B, int T);    // parts a pass over the mask has; 0: every row's CTA looks through it
 cudaError_t launch_token_plan(const TokenPlanArgs& a, cudaStream_t s);
+cudaError_t launch_zero_rows(void* x, const uint8_t* keep, long long rows, int pieces, cudaStream_t s);   // pieces of 16 bytes a row
 cudaError_t launch_gelu_mul(bool bf16, const GeluMulArgs& a, bool vector_ok, cudaStream_t s);
 cudaError_t launch_gate_pack(bool f32_weights, bool bf16, const GatePackArgs& a, cudaStream_t s);
 cudaError_t launch_gate_unpack(bool bf16, bool f32_weights, const GateUnpackArgs& a, cudaStream_t s);

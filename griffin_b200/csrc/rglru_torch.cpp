@@ -557,7 +557,13 @@ std::optional<std::tuple<Tensor, Tensor, Opt>> block(const Tensor& x, const std:
             "rglru_gelu_mul_fwd");
     }
     out = at::linear(mixed, woc, p[BO].to(dtype));
-    if (active) out = at::where(active->unsqueeze(-1), out, 0.0);
+    if (active) {
+      const int64_t row = out.size(2) * out.element_size();
+      if (row % 16 == 0 && in_int(row) && out.is_contiguous() && aligned16(out))
+        check(rglru_zero_rows(out.data_ptr(), ptr_as<uint8_t>(active), B * T, row, stream_of(d)), "rglru_zero_rows");
+      else
+        out = at::where(active->unsqueeze(-1), out, 0.0);
+    }
   }
   if (grad) {
     auto node = make_node<BlockNode>(x, p[WX], p[BX], p[WY], p[BY], p[CW], p[CB], p[WR], p[BR], p[WI], p[BI], p[LAM], p[WO], p[BO],
