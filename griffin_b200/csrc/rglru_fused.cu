@@ -8,12 +8,14 @@
 // Neither u nor du ever leaves the SM: a forward reads x and writes y, a backward reads dy and x and writes dx, where the
 // kernels of rglru_gates.cu and rglru_scan.cu move 3 and 6 more elements per element (u out and in twice, du out and in).
 // Two warps take the accumulators out of tensor memory (and issue the multiplications): in the forward ahead of the eight
-// scan warps by up to two chunks, in the backward u two chunks ahead and dx behind.  One more warp issues the bulk copies.
+// scan warps by up to two chunks, in the backward u two chunks ahead (hence three slots of gate tiles) and dx behind.  One more
+// warp issues the bulk copies.
 // The scan warps take registers over from those (setmaxnreg): held at the launch's share they spill 100 to 300 bytes.
-// B8 T2048 D1024, 16 heads of 64, us: 52 forward, 73 backward and 4 for the fold of the weight gradient, where gate kernels
-// around the scan took 202 in all; T16384 at B1 (clusters of eight) 108 + 211 warm and 240 in a loop, where 282; B16 with the
-// branch product 88 + 183 + 9, where batched GEMMs around the scan took some 350.  Bound by the serial chain of a chunk: u out of
-// tensor memory, scan, du into it, with one CTA's eight scan warps on an SM.
+// B8 T2048 D1024, 16 heads of 64, us: 44 forward, 73 backward and 4 for the fold of the weight gradient, where gate kernels
+// around the scan took 202 in all; T16384 at B1 (clusters of eight) 216 a step, where 282; B16 with the branch product
+// 89 + 180 + 9, where batched GEMMs around the scan took some 350.  Bound by the serial chain of a chunk in the scan warps, eight
+// on an SM: multiplying a chunk ahead and a third slot of gate tiles, which took the tensor-memory warps out of that chain, gave
+// 2 us of 127.
 // All tiles are staged with the copy engine's 128-byte swizzle, which is the operand layout of the tensor cores and leaves
 // the scan's accesses as free of bank conflicts as dense rows.
 //
@@ -40,7 +42,7 @@ constexpr int FT = 64 * 128;                 // bytes of a tile: 64 rows of 64 c
 constexpr int FCH = 64, FLANES = 16, FTS = 4, FNCV = FCH / CV, FCOMP = FLANES * FNCV;
 constexpr int FTHREADS = FCOMP + 128;        // scan warps; a warpgroup of two tensor-memory warps, the copy warp, and one idle
 // Registers a thread of the scan warps and of the others: their sum over the block stays below what it is launched with.
-constexpr int FWD_SCAN = 88, FWD_AUX = 56, BWD_SCAN = 200, BWD_AUX = 96;
+constexpr int FWD_SCAN = 88, FWD_AUX = 56, FWD_SCAN_ALONE = 184, FWD_AUX_ALONE = 96, BWD_SCAN = 200, BWD_AUX = 96;
 constexpr int W_BYTES = 2 * FT;              // both gates' weights of the tile, rows r 0 .. 63, i 0 .. 63
 constexpr int BAR_TC = 4;                    // named barriers: the two tensor-memory warps; those and the scan warps (2)
 
@@ -169,8 +171,9 @@ struct FusedFwdSmem {
   static constexpr int BYTES = OFF_SPLIT + (SPLIT ? static_cast<int>(sizeof(SplitSmem<FCH>)) : 0) + 1024;   // (to align the tiles)
 };
 
-template <bool MERGE, bool SPLIT>
-__global__ void __launch_bounds__(FTHREADS, 2) fused_fwd_kernel(const __grid_constant__ FusedMaps maps, const FusedFwdArgs p) {
+// ALONE: at most one CTA per SM, which may then have twice the registers.
+template <bool MERGE, bool SPLIT, bool ALONE>
+__global__ void __launch_bounds__(FTHREADS, ALONE ? 1 : 2) fused_fwd_kernel(const __grid_constant__ FusedMaps maps, const FusedFwdArgs p) {
   using SM = FusedFwdSmem<MERGE, SPLIT>;
   constexpr int NSTAGE = SM::NSTAGE, TS = FTS, LANES = FLANES, CH = FCH;
   extern __shared__ uint8_t smem_raw[];
@@ -221,63 +224,65 @@ __global__ void __launch_bounds__(FTHREADS, 2) fused_fwd_kernel(const __grid_con
   pdl_wait();
 
   if (warp >= 8) {
-  regs_down<FWD_AUX>();
-  if (warp == 10) {            // ---- copies: loads run NSTAGE - 1 chunks ahead (see rglru_fwd_body)
-    if (tid == FCOMP + 64) {
-      issue(0);
-      mbar_wait_or_flag(&full[0], 0, dead, p.status, DEV_TIMEOUT_LOAD);
-      for (int it = 1; it < NSTAGE && it < mine; ++it) issue(it);
-      for (int it = 0; it < mine; ++it) {
-        const int sidx = it % NSTAGE, k = it * nranks + rank;
-        mbar_wait_or_flag(&ready[sidx], (it / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
-        tma_store_3d(&maps.out, smem + sidx * SM::STAGE, d0, k * 64, b);
-        tma_commit();
-        if (it + NSTAGE < mine) {
-          tma_wait_read<0>();
-          issue(it + NSTAGE);
+    regs_down<ALONE ? FWD_AUX_ALONE : FWD_AUX>();
+    if (warp == 10) {            // ---- copies: loads run NSTAGE - 1 chunks ahead (see rglru_fwd_body)
+      if (tid == FCOMP + 64) {
+        issue(0);
+        mbar_wait_or_flag(&full[0], 0, dead, p.status, DEV_TIMEOUT_LOAD);
+        for (int it = 1; it < NSTAGE && it < mine; ++it) issue(it);
+        for (int it = 0; it < mine; ++it) {
+          const int sidx = it % NSTAGE, k = it * nranks + rank;
+          mbar_wait_or_flag(&ready[sidx], (it / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
+          tma_store_3d(&maps.out, smem + sidx * SM::STAGE, d0, k * 64, b);
+          tma_commit();
+          if (it + NSTAGE < mine) {
+            tma_wait_read<0>();
+            issue(it + NSTAGE);
+          }
         }
+        tma_wait_all<0>();
       }
-      tma_wait_all<0>();
+      if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }
+      return;
     }
-    if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }
-    return;
-  }
-  if (warp < 10) {             // ---- gates
-    const uint32_t acc = *tmem_at, mine_acc = acc + (static_cast<uint32_t>(warp - 8) << 21);   // this warp's 32 rows
-    const int row = tid - FCOMP;
-    bar_all(FCOMP + 64);       // the weights are there
-    for (int it = 0; it < mine; ++it) {
-      const int s = it % NSTAGE, slot = it & 1;
-      if (it >= 2) mbar_wait_or_flag(&ready[(it - 2) % NSTAGE], ((it - 2) / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
-      mbar_wait_or_flag(&full[s], (it / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
-      __syncwarp();
-      if (row == 0) {
+    if (warp < 10) {             // ---- gates
+      const uint32_t acc = *tmem_at, mine_acc = acc + (static_cast<uint32_t>(warp - 8) << 21);   // this warp's 32 rows
+      const int row = tid - FCOMP;
+      bar_all(FCOMP + 64);       // the weights are there
+      auto multiply = [&](int it) {
+        const int s = it % NSTAGE;
+        mbar_wait_or_flag(&full[s], (it / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
         tc_fence_after();
         mma_gates(acc, smem_u32(smem + s * SM::STAGE), smem_u32(smem + SM::OFF_W), p.bw);
         tc_commit(done);
+      };
+      if (row == 0) multiply(0);
+      for (int it = 0; it < mine; ++it) {
+        const int slot = it & 1;
+        __syncwarp();
+        if (it >= 2) mbar_wait_or_flag(&ready[(it - 2) % NSTAGE], ((it - 2) / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
+        mbar_wait_or_flag(done, it & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+        __syncwarp();
+        tc_fence_after();
+        store_gates(smem + SM::OFF_U + slot * 2 * FT, mine_acc, row);
+        tc_fence_before();
+        __syncwarp();
+        if ((tid & 31) == 0) mbar_arrive(&gates[slot]);
+        __syncwarp();
+        asm volatile("bar.sync %0, 64;" ::"n"(BAR_TC) : "memory");       // both are done with the accumulators
+        if (row == 0 && it + 1 < mine) multiply(it + 1);
       }
       __syncwarp();
-      mbar_wait_or_flag(done, it & 1, dead, p.status, DEV_TIMEOUT_LOAD);
-      __syncwarp();
       tc_fence_after();
-      store_gates(smem + SM::OFF_U + slot * 2 * FT, mine_acc, row);
-      tc_fence_before();
-      __syncwarp();
-      if ((tid & 31) == 0) mbar_arrive(&gates[slot]);
-      __syncwarp();
-      asm volatile("bar.sync %0, 64;" ::"n"(BAR_TC) : "memory");       // both are done with the accumulators
+      if (warp == 8) tc_free<128>(acc);
+      if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }
+      return;
     }
-    __syncwarp();
-    tc_fence_after();
-    if (warp == 8) tc_free<128>(acc);
-    if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }
+
+    if constexpr (SPLIT) cluster_sync_all();      // the idle warp
     return;
   }
-
-  if constexpr (SPLIT) cluster_sync_all();      // the idle warp
-  return;
-  }
-  regs_up<FWD_SCAN>();
+  regs_up<ALONE ? FWD_SCAN_ALONE : FWD_SCAN>();
   // ---- scan
   const int lane_t = tid / FNCV, vec = tid % FNCV;
   const bool keeps = p.pack && b == 0 && rank == 0;
@@ -400,18 +405,19 @@ __global__ void __launch_bounds__(FTHREADS, 2) fused_fwd_kernel(const __grid_con
 template <bool MERGE, bool SPLIT>
 struct FusedBwdSmem {
   static constexpr int NSTAGE = MERGE ? 4 : 5;
+  static constexpr int NSLOT = 3;                           // of both gates' tiles
   static constexpr int OFF_X = FT, OFF_G = 2 * FT;          // behind the dy tile, which dx takes over
   static constexpr int STAGE = MERGE ? 3 * FT : 2 * FT;
   static constexpr int OFF_U = NSTAGE * STAGE;
-  static constexpr int OFF_W = OFF_U + 4 * FT;
+  static constexpr int OFF_W = OFF_U + NSLOT * 2 * FT;
   static constexpr int PLANE = FLANES * FCH * 4;            // (see BwdSmem)
   static constexpr int OFF_AGGP = OFF_W + W_BYTES;
   static constexpr int OFF_AGGS = OFF_AGGP + PLANE;
   static constexpr int OFF_AGGC = OFF_AGGS + PLANE;
   static constexpr int OFF_EINF = OFF_AGGC + PLANE;
   static constexpr int OFF_EINR = OFF_EINF + PLANE;
-  static constexpr int OFF_BAR = OFF_EINR + PLANE;          // full, ready, out [NSTAGE], gates [2], tensor cores [2], flag, address
-  static constexpr int OFF_SPLIT = OFF_BAR + (3 * NSTAGE + 4) * 8 + 16;
+  static constexpr int OFF_BAR = OFF_EINR + PLANE;          // full, ready, out [NSTAGE], gates [NSLOT], tensor cores [2], flag, address
+  static constexpr int OFF_SPLIT = OFF_BAR + (3 * NSTAGE + NSLOT + 2 + 1) / 2 * 16 + 16;
   static constexpr int BYTES = OFF_SPLIT + (SPLIT ? static_cast<int>(sizeof(SplitSmem<FCH>)) : 0) + 1024;
 };
 // Accumulator columns: u, dx, dW.
@@ -420,7 +426,7 @@ constexpr int ACC_DX = 128, ACC_DW = 192, ACC_COLS = 256;
 template <bool MERGE, bool SPLIT>
 __global__ void __launch_bounds__(FTHREADS, 1) fused_bwd_kernel(const __grid_constant__ FusedMaps maps, const FusedBwdArgs p) {
   using SM = FusedBwdSmem<MERGE, SPLIT>;
-  constexpr int NSTAGE = SM::NSTAGE, TS = FTS, LANES = FLANES, CH = FCH;
+  constexpr int NSTAGE = SM::NSTAGE, NSLOT = SM::NSLOT, TS = FTS, LANES = FLANES, CH = FCH;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
   float* aggP = reinterpret_cast<float*>(smem + SM::OFF_AGGP);
@@ -432,7 +438,7 @@ __global__ void __launch_bounds__(FTHREADS, 1) fused_bwd_kernel(const __grid_con
   uint64_t* ready = full + NSTAGE;
   uint64_t* outs = ready + NSTAGE;
   uint64_t* gates = outs + NSTAGE;
-  uint64_t* done = gates + 2;                 // [0] u, [1] dx and dW of a chunk
+  uint64_t* done = gates + NSLOT;                 // [0] u, [1] dx and dW of a chunk
   volatile int* dead = reinterpret_cast<volatile int*>(done + 2);
   uint32_t* tmem_at = reinterpret_cast<uint32_t*>(done + 2) + 1;
 
@@ -456,7 +462,8 @@ __global__ void __launch_bounds__(FTHREADS, 1) fused_bwd_kernel(const __grid_con
   if (tid == FCOMP + 64) {
     *dead = 0;
     for (int s = 0; s < NSTAGE; ++s) { mbar_init(&full[s], 1); mbar_init(&ready[s], FCOMP / 32); mbar_init(&outs[s], 2); }
-    mbar_init(&gates[0], 2); mbar_init(&gates[1], 2); mbar_init(&done[0], 1); mbar_init(&done[1], 1);
+    for (int s = 0; s < NSLOT; ++s) mbar_init(&gates[s], 2);
+    mbar_init(&done[0], 1); mbar_init(&done[1], 1);
     if constexpr (SPLIT) { mbar_init(&split.sm->bar[0], 1); mbar_init(&split.sm->bar[1], 1); }
     mbar_fence_init();
     prefetch_map(&maps.x); prefetch_map(&maps.dy); prefetch_map(&maps.out);
@@ -476,104 +483,104 @@ __global__ void __launch_bounds__(FTHREADS, 1) fused_bwd_kernel(const __grid_con
   const uint32_t acc = *tmem_at;
 
   if (warp >= 8) {
-  regs_down<BWD_AUX>();
-  if (warp == 10) {            // ---- copies
-    if (tid == FCOMP + 64) {
-      issue(0);
-      mbar_wait_or_flag(&full[0], 0, dead, p.status, DEV_TIMEOUT_LOAD);
-      for (int q = 1; q < NSTAGE && q < mine; ++q) issue(q);
+    regs_down<BWD_AUX>();
+    if (warp == 10) {            // ---- copies
+      if (tid == FCOMP + 64) {
+        issue(0);
+        mbar_wait_or_flag(&full[0], 0, dead, p.status, DEV_TIMEOUT_LOAD);
+        for (int q = 1; q < NSTAGE && q < mine; ++q) issue(q);
+        for (int q = 0; q < mine; ++q) {
+          const int sidx = q % NSTAGE, k = nchunks - 1 - (q * nranks + rank);
+          uint8_t* st = smem + sidx * SM::STAGE;
+          mbar_wait_or_flag(&outs[sidx], (q / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
+          tma_store_3d(&maps.out, st, d0, k * 64, b);
+          if (MERGE) tma_store_3d(&maps.dg, st + SM::OFF_G, d0, k * 64, b);
+          tma_commit();
+          if (q + NSTAGE < mine) {
+            tma_wait_read<0>();
+            issue(q + NSTAGE);
+          }
+        }
+        tma_wait_all<0>();
+      }
+      if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }
+      return;
+    }
+    if (warp < 10) {             // ---- gates ahead of the scan, input and weight gradients behind it
+      const uint32_t rows = static_cast<uint32_t>(warp - 8) << 21;      // this warp's 32 accumulator rows
+      const int row = tid - FCOMP;
+      const uint32_t sw = smem_u32(smem + SM::OFF_W);
+      bar_all(FCOMP + 64);       // the weights are there
+      auto make_gates = [&](int q) {
+        const int s = q % NSTAGE, slot = q % NSLOT;
+        mbar_wait_or_flag(&full[s], (q / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+        __syncwarp();
+        if (row == 0) {
+          tc_fence_after();
+          mma_gates(acc, smem_u32(smem + s * SM::STAGE + SM::OFF_X), sw, p.bw);
+          tc_commit(&done[0]);
+        }
+        __syncwarp();
+        mbar_wait_or_flag(&done[0], q & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+        __syncwarp();
+        tc_fence_after();
+        store_gates(smem + SM::OFF_U + slot * 2 * FT, acc + rows, row);
+        tc_fence_before();
+        __syncwarp();
+        if ((tid & 31) == 0) mbar_arrive(&gates[slot]);
+        __syncwarp();
+        asm volatile("bar.sync %0, 64;" ::"n"(BAR_TC) : "memory");       // both are done with the accumulators
+      };
+      make_gates(0);
+      if (mine > 1) make_gates(1);
       for (int q = 0; q < mine; ++q) {
-        const int sidx = q % NSTAGE, k = nchunks - 1 - (q * nranks + rank);
-        uint8_t* st = smem + sidx * SM::STAGE;
-        mbar_wait_or_flag(&outs[sidx], (q / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
-        tma_store_3d(&maps.out, st, d0, k * 64, b);
-        if (MERGE) tma_store_3d(&maps.dg, st + SM::OFF_G, d0, k * 64, b);
-        tma_commit();
-        if (q + NSTAGE < mine) {
-          tma_wait_read<0>();
-          issue(q + NSTAGE);
+        const int s = q % NSTAGE;
+        uint8_t* st = smem + s * SM::STAGE;
+        if (q + 2 < mine) make_gates(q + 2);     // (the slot's last reader, the multiplications of chunk q - 1, was waited for)
+        mbar_wait_or_flag(&ready[s], (q / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
+        __syncwarp();
+        if (row == 0) {
+          const uint32_t du = smem_u32(smem + SM::OFF_U + q % NSLOT * 2 * FT);
+          tc_fence_after();
+          mma_dx(acc + ACC_DX, du, sw, p.bw);
+          mma_dw(acc + ACC_DW, du, smem_u32(st + SM::OFF_X), q == 0);
+          tc_commit(&done[1]);
         }
-      }
-      tma_wait_all<0>();
-    }
-    if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }
-    return;
-  }
-  if (warp < 10) {             // ---- gates ahead of the scan, input and weight gradients behind it
-    const uint32_t rows = static_cast<uint32_t>(warp - 8) << 21;      // this warp's 32 accumulator rows
-    const int row = tid - FCOMP;
-    const uint32_t sw = smem_u32(smem + SM::OFF_W);
-    bar_all(FCOMP + 64);       // the weights are there
-    auto make_gates = [&](int q) {
-      const int s = q % NSTAGE, slot = q & 1;
-      mbar_wait_or_flag(&full[s], (q / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
-      __syncwarp();
-      if (row == 0) {
+        __syncwarp();
+        mbar_wait_or_flag(&done[1], q & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+        __syncwarp();
         tc_fence_after();
-        mma_gates(acc, smem_u32(smem + s * SM::STAGE + SM::OFF_X), sw, p.bw);
-        tc_commit(&done[0]);
-      }
-      __syncwarp();
-      mbar_wait_or_flag(&done[0], q & 1, dead, p.status, DEV_TIMEOUT_LOAD);
-      __syncwarp();
-      tc_fence_after();
-      store_gates(smem + SM::OFF_U + slot * 2 * FT, acc + rows, row);
-      tc_fence_before();
-      __syncwarp();
-      if ((tid & 31) == 0) mbar_arrive(&gates[slot]);
-      __syncwarp();
-      asm volatile("bar.sync %0, 64;" ::"n"(BAR_TC) : "memory");       // both are done with the accumulators
-    };
-    make_gates(0);
-    if (mine > 1) make_gates(1);
-    for (int q = 0; q < mine; ++q) {
-      const int s = q % NSTAGE;
-      uint8_t* st = smem + s * SM::STAGE;
-      mbar_wait_or_flag(&ready[s], (q / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_STORE);
-      __syncwarp();
-      if (row == 0) {
-        const uint32_t du = smem_u32(smem + SM::OFF_U + (q & 1) * 2 * FT);
-        tc_fence_after();
-        mma_dx(acc + ACC_DX, du, sw, p.bw);
-        mma_dw(acc + ACC_DW, du, smem_u32(st + SM::OFF_X), q == 0);
-        tc_commit(&done[1]);
-      }
-      __syncwarp();
-      mbar_wait_or_flag(&done[1], q & 1, dead, p.status, DEV_TIMEOUT_LOAD);
-      __syncwarp();
-      tc_fence_after();
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float v[32];
-        tc_load32(acc + ACC_DX + rows + 32 * h, v);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint4* at = reinterpret_cast<uint4*>(st + row * 128 + (((h * 4 + j) ^ (row & 7)) << 4));
-          const uint4 d = *at;
-          const uint32_t in[4] = {d.x, d.y, d.z, d.w};
-          uint32_t o[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            o[e] = pack_bf16(v[8 * j + 2 * e] + __uint_as_float(in[e] << 16), v[8 * j + 2 * e + 1] + __uint_as_float(in[e] & 0xffff0000u));
-          *at = make_uint4(o[0], o[1], o[2], o[3]);
+  #pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float v[32];
+          tc_load32(acc + ACC_DX + rows + 32 * h, v);
+  #pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            uint4* at = reinterpret_cast<uint4*>(st + row * 128 + (((h * 4 + j) ^ (row & 7)) << 4));
+            const uint4 d = *at;
+            const uint32_t in[4] = {d.x, d.y, d.z, d.w};
+            uint32_t o[4];
+  #pragma unroll
+            for (int e = 0; e < 4; ++e)
+              o[e] = pack_bf16(v[8 * j + 2 * e] + __uint_as_float(in[e] << 16), v[8 * j + 2 * e + 1] + __uint_as_float(in[e] & 0xffff0000u));
+            *at = make_uint4(o[0], o[1], o[2], o[3]);
+          }
         }
+        tc_fence_before();
+        fence_async_smem();
+        __syncwarp();
+        if ((tid & 31) == 0) mbar_arrive(&outs[s]);
+        __syncwarp();
+        asm volatile("bar.sync %0, 64;" ::"n"(BAR_TC) : "memory");
       }
       tc_fence_before();
-      fence_async_smem();
-      __syncwarp();
-      if ((tid & 31) == 0) mbar_arrive(&outs[s]);
-      __syncwarp();
-      asm volatile("bar.sync %0, 64;" ::"n"(BAR_TC) : "memory");
-      if (q + 2 < mine) make_gates(q + 2);
+      bar_all(FCOMP + 64);       // dW is whole
+      if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }
+      return;
     }
-    tc_fence_before();
-    bar_all(FCOMP + 64);       // dW is whole
-    if constexpr (SPLIT) { __syncwarp(); cluster_sync_all(); }
-    return;
-  }
 
-  if constexpr (SPLIT) cluster_sync_all();
-  return;
+    if constexpr (SPLIT) cluster_sync_all();
+    return;
   }
   regs_up<BWD_SCAN>();
   // ---- scan
@@ -599,7 +606,7 @@ __global__ void __launch_bounds__(FTHREADS, 1) fused_bwd_kernel(const __grid_con
     if constexpr (SPLIT) { if (tid == 0) split.arm(q); }
     const int stage = q % NSTAGE;
     uint8_t* tiles = smem + stage * SM::STAGE;
-    uint8_t* tr = smem + SM::OFF_U + (q & 1) * 2 * FT;
+    uint8_t* tr = smem + SM::OFF_U + q % NSLOT * 2 * FT;
     const int t0 = k * 64;
     uint32_t fl[1];
     const bool masked = p.tok != nullptr || t0 + 64 > p.T;
@@ -615,7 +622,7 @@ __global__ void __launch_bounds__(FTHREADS, 1) fused_bwd_kernel(const __grid_con
     bool flagged = false;
     if (!idle) {
       mbar_wait_or_flag(&full[stage], (q / NSTAGE) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
-      mbar_wait_or_flag(&gates[q & 1], (q >> 1) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
+      mbar_wait_or_flag(&gates[q % NSLOT], (q / NSLOT) & 1, dead, p.status, DEV_TIMEOUT_LOAD);
       float2 prod[2], sfwd[2], crev[2];
       flagged = masked && any_flag(fl);
       uint8_t* tg = tiles + SM::OFF_G;
@@ -784,13 +791,13 @@ __global__ void __launch_bounds__(256) fused_fold_kernel(const FusedBwdArgs p, i
   else static_cast<BF*>(dst)[d] = __float2bfloat16_rn(a);
 }
 
-template <bool MERGE, bool SPLIT>
+template <bool MERGE, bool SPLIT, bool ALONE>
 struct FusedFwdKern {
   static constexpr int THREADS = FTHREADS, BYTES = FusedFwdSmem<MERGE, SPLIT>::BYTES;
   static_assert(BYTES <= 232448, "shared memory of one CTA");
   using Fn = void (*)(FusedMaps, FusedFwdArgs);
   static Fn get(cudaError_t& e) {
-    Fn kern = fused_fwd_kernel<MERGE, SPLIT>;
+    Fn kern = fused_fwd_kernel<MERGE, SPLIT, ALONE>;
     e = set_smem<FusedFwdKern>(kern, BYTES);
     return kern;
   }
@@ -821,12 +828,20 @@ bool fused_head_width(int head_width) { return head_width == 16 || head_width ==
 int fused_split(bool fwd, bool merge, int B, int T, int D) {
   const long long tiles = static_cast<long long>(B) * ((D + 63) / 64);
   const int nchunks = (T + 63) / 64;
-  if (fwd) return merge ? pick_split<FusedFwdKern<true, true>>(tiles, nchunks) : pick_split<FusedFwdKern<false, true>>(tiles, nchunks);
+  if (fwd) return merge ? pick_split<FusedFwdKern<true, true, true>>(tiles, nchunks) : pick_split<FusedFwdKern<false, true, true>>(tiles, nchunks);
   return merge ? pick_split<FusedBwdKern<true, true>>(tiles, nchunks) : pick_split<FusedBwdKern<false, true>>(tiles, nchunks);
 }
+// A grid of at most one CTA per SM (a split one always is: all its clusters are resident at once) takes the kernels with twice
+// the registers: held at two per SM they spill about 100 bytes, 50 us forward against 44 at 128 CTAs (B8 T2048 D1024), 106
+// against 76 at sixteen clusters of eight (B1 T16384).  From there on two per SM hide each other's waits.
+template <bool MERGE>
+static cudaError_t launch_fused_fwd_t(const FusedMaps& maps, const FusedFwdArgs& a, cudaStream_t s) {
+  if (a.split > 1) return launch_fused<FusedFwdKern<MERGE, true, true>>(maps, a, s);
+  const bool alone = static_cast<long long>(a.B) * ((a.D + 63) / 64) <= 148;
+  return alone ? launch_fused<FusedFwdKern<MERGE, false, true>>(maps, a, s) : launch_fused<FusedFwdKern<MERGE, false, false>>(maps, a, s);
+}
 cudaError_t launch_fused_fwd(bool merge, const FusedMaps& maps, const FusedFwdArgs& a, cudaStream_t s) {
-  if (a.split > 1) return merge ? launch_fused<FusedFwdKern<true, true>>(maps, a, s) : launch_fused<FusedFwdKern<false, true>>(maps, a, s);
-  return merge ? launch_fused<FusedFwdKern<true, false>>(maps, a, s) : launch_fused<FusedFwdKern<false, false>>(maps, a, s);
+  return merge ? launch_fused_fwd_t<true>(maps, a, s) : launch_fused_fwd_t<false>(maps, a, s);
 }
 cudaError_t launch_fused_bwd(bool merge, const FusedMaps& maps, const FusedBwdArgs& a, cudaStream_t s) {
   cudaError_t e;

@@ -121,7 +121,7 @@ struct ConvTmaArgs {
 };
 
 // Taps, bias and their gradients come in the parameters' own types: casting them around the kernels took two launches of 2 to
-// 4 us a direction, a sixth of a padded prompt of 6 x 1200 tokens.
+// 4 us a direction, 8 of the 130 us of kernels of a padded prompt of 6 x 1200 tokens.
 struct ConvArgs {
   const void* x_in;
   const void* w;
